@@ -1303,7 +1303,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         auto t_sample = clk::now();
         const uint32_t nc = (uint32_t)cands.size();
         std::vector<PlanCand> pc(nc);
-        u64 total = 0;
+        u64 total = 0, most = 0;
         for (uint32_t c = 0; c < nc; c++) {
             const int dir = cands[c][5] - '0', order = cands[c][9] - '0';
             PlanCand &q = pc[c];
@@ -1325,7 +1325,9 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
             q.eb = layer_eb;
             q.neg_2_eb = neg_2_layer_eb;
             q.dir = dir;
-            total += q.cnt[0] * q.cnt[1] * q.cnt[2];
+            const u64 own = q.cnt[0] * q.cnt[1] * q.cnt[2];
+            most = std::max(most, own);
+            total += (own + kPlanAlign - 1) / kPlanAlign * kPlanAlign;
         }
         std::vector<u64> num(nc);
         for (uint32_t c = 0; c < nc; c++) num[c] = pc[c].cnt[0] * pc[c].cnt[1] * pc[c].cnt[2];
@@ -1345,7 +1347,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         int32_t *d_qb = ctx->plan_qb.as<int32_t>();
         {
             ProfScope ps_(ctx, "plan_sample", total * 8);
-            CK(launch_plan_sample(d_in, dims[1], dims[2], d_pc, nc, total, d_qb, ctx->plan_e.as<float>(), (int32_t *)(aux + aux_range),
+            CK(launch_plan_sample(d_in, dims[1], dims[2], d_pc, nc, most, d_qb, ctx->plan_e.as<float>(), (int32_t *)(aux + aux_range),
                                   st));
         }
         {

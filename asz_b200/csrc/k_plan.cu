@@ -4,51 +4,57 @@
 #include <cuda_runtime.h>
 
 #include "dev_common.cuh"
+#include "float_chain.cuh"
 #include "launch.h"
 
 namespace asz {
 namespace {
 
-__device__ __forceinline__ uint32_t cand_of(const PlanCand *__restrict__ c, uint32_t nc, uint64_t k) {
-    uint32_t lo = 0, hi = nc;  // last candidate with off <= k
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (c[mid].off <= k) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // dot_sample_compress (generate_config.tpp:227-254) as GCC emits it for the reference build: the
 // edge stencils below, the interior 1D4R in double with a float product in between, the residual
 // quantised in float (diff * neg_2_eb) and e = fmaf(-eb, (float)(2 * qb), diff) for the error sum.
-__global__ void plan_sample_kernel(const float *__restrict__ d, uint64_t n1, uint64_t n2, const PlanCand *__restrict__ cands,
-                                   uint32_t ncands, uint64_t total, int32_t *__restrict__ qb_out, float *__restrict__ e_out,
-                                   int32_t *__restrict__ qb_range) {
+//
+// A row of CTAs per candidate (grid y), so the loop nest's divisors are the CTA's own and the QB
+// extremes are reduced in the CTA before they reach the candidate's two words: one pair of atomics
+// a CTA. Every thread's own pair, on the same two words, was most of the kernel (100x500x500, the
+// search's 14 layers, nine candidates of 0.5 M samples in the first: 11.1 ms with it, 0.24 without).
+constexpr int kSampleThreads = 256;
+
+__global__ void __launch_bounds__(kSampleThreads)
+    plan_sample_kernel(const float *__restrict__ d, uint64_t n1, uint64_t n2, const PlanCand *__restrict__ cands,
+                       int32_t *__restrict__ qb_out, float *__restrict__ e_out, int32_t *__restrict__ qb_range) {
+    __shared__ int32_t rlo[kSampleThreads / 32], rhi[kSampleThreads / 32];
+    const PlanCand &c = cands[blockIdx.y];
+    const uint64_t n = c.cnt[0] * c.cnt[1] * c.cnt[2];
+    const int a0 = c.ax[0], a1 = c.ax[1], a2 = c.ax[2];  // loop nest: outer to inner
+    const uint64_t c2 = c.cnt[a2], c1 = c.cnt[a1];
+    const uint64_t lo0 = c.lo[a0], lo1 = c.lo[a1], lo2 = c.lo[a2], st0 = c.st[a0], st1 = c.st[a1], st2 = c.st[a2];
+    auto extent = [&](int a) { return a == 0 ? n1 * n2 : a == 1 ? n2 : (uint64_t)1; };
+    const uint64_t x0 = extent(a0), x1 = extent(a1), x2 = extent(a2);
+    const int dir = c.dir;
+    const double td = (double)c.t;
+    const float neg_2_eb = c.neg_2_eb, eb = c.eb;
+    int32_t *const qb = qb_out + c.off;
+    float *const eo = e_out + c.off;
+    const uint64_t hs = c.hs, right = c.right, dist = c.dist;
+    const bool narrow = n < (1ull << 32);
     int32_t lo = INT32_MAX, hi = INT32_MIN;
-    uint32_t ci_last = 0xffffffffu;
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < total; k += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t ci = cand_of(cands, ncands, k);
-        if (ci != ci_last) {
-            if (ci_last != 0xffffffffu && lo <= hi) {
-                atomicMin(&qb_range[2 * ci_last], lo);
-                atomicMax(&qb_range[2 * ci_last + 1], hi);
-            }
-            lo = INT32_MAX;
-            hi = INT32_MIN;
-            ci_last = ci;
+    for (uint64_t kl = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; kl < n; kl += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t k0, k1, k2;
+        if (narrow) {  // 32-bit divisions
+            const uint32_t r = (uint32_t)kl / (uint32_t)c2;
+            k2 = (uint32_t)kl - r * (uint32_t)c2;
+            k0 = r / (uint32_t)c1;
+            k1 = r - (uint32_t)k0 * (uint32_t)c1;
+        } else {
+            const uint64_t r = kl / c2;
+            k2 = kl - r * c2;
+            k0 = r / c1;
+            k1 = r - k0 * c1;
         }
-        const PlanCand c = cands[ci];
-        const uint64_t kl = k - c.off;
-        // Loop nest: axes ax[0] (outer) .. ax[2] (inner).
-        const uint64_t c2 = c.cnt[c.ax[2]], c1 = c.cnt[c.ax[1]];
-        const uint64_t k2 = kl % c2, r = kl / c2, k1 = r % c1, k0 = r / c1;
-        uint64_t ii[3];
-        ii[c.ax[0]] = c.lo[c.ax[0]] + k0 * c.st[c.ax[0]];
-        ii[c.ax[1]] = c.lo[c.ax[1]] + k1 * c.st[c.ax[1]];
-        ii[c.ax[2]] = c.lo[c.ax[2]] + k2 * c.st[c.ax[2]];
-        const uint64_t pos = (ii[0] * n1 + ii[1]) * n2 + ii[2];
-        const uint64_t i = ii[c.dir], hs = c.hs, right = c.right, dist = c.dist;
+        const uint64_t i0 = lo0 + k0 * st0, i1 = lo1 + k1 * st1, i2 = lo2 + k2 * st2;
+        const uint64_t pos = i0 * x0 + i1 * x1 + i2 * x2;
+        const uint64_t i = dir == a0 ? i0 : dir == a1 ? i1 : i2;
         const float xm1 = d[pos - dist];
         float pred;
         if (i <= hs) {
@@ -63,101 +69,81 @@ __global__ void plan_sample_kernel(const float *__restrict__ d, uint64_t n1, uin
                 pred = __fmul_rn(__fsub_rn(__fmaf_rn(xm1, 6.0f, __fmul_rn(d[pos + dist], 3.0f)), xm3), 0.125f);
             } else {
                 const float s1 = __fadd_rn(d[pos + dist], xm1), s3 = __fadd_rn(xm3, d[pos + 3 * dist]);
-                const double td = (double)c.t;
                 const float p1 = __double2float_rn(__dmul_rn((double)s3, __dsub_rn(0.25, td)));
                 pred = __double2float_rn(__fma_rn(__dadd_rn(0.25, td), (double)s1, (double)p1));
             }
         }
         const float diff = __fsub_rn(pred, d[pos]);
-        const int32_t q = (int32_t)lround_f(__fmul_rn(diff, c.neg_2_eb));
+        const int32_t q = (int32_t)lround_f(__fmul_rn(diff, neg_2_eb));
         const float q2 = __int2float_rn((int32_t)((uint32_t)q * 2u));
-        qb_out[k] = q;
-        e_out[k] = __fmaf_rn(-c.eb, q2, diff);
+        qb[kl] = q;
+        eo[kl] = __fmaf_rn(-eb, q2, diff);
         lo = min(lo, q);
         hi = max(hi, q);
     }
-    if (ci_last != 0xffffffffu && lo <= hi) {
-        atomicMin(&qb_range[2 * ci_last], lo);
-        atomicMax(&qb_range[2 * ci_last + 1], hi);
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        rlo[threadIdx.x >> 5] = lo;
+        rhi[threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kSampleThreads / 32; w++) {
+            lo = min(lo, rlo[w]);
+            hi = max(hi, rhi[w]);
+        }
+        if (lo <= hi) {
+            atomicMin(&qb_range[2 * blockIdx.y], lo);
+            atomicMax(&qb_range[2 * blockIdx.y + 1], hi);
+        }
     }
 }
 
-// mse = fmaf(e, e, mse) over each candidate's samples in loop order (one warp per candidate), the
-// reference's float sum (generate_config.tpp:227-254), bit for bit.
-//
-// Batches of kBatch terms, kPer consecutive ones per lane. While the running sum s stays in one
-// binade [2^E, 2^(E+1)), with ulp u = 2^(E-23) and s = m*u (m in [2^23, 2^24)), every step
-// s' = RN(s + x*x) equals (m + r)*u with r = x*x/u rounded to the nearest integer, unless the
-// fraction of x*x/u is exactly one half (round-half-even then depends on m). The terms are not
-// negative, so the partial sums grow: if the batch's total stays below 2^24 no step leaves the
-// binade, and the batch adds sum(r)*u in one step. x*x is exact in double and u a power of two,
-// so r and the tie test are exact. A batch with a tie, a crossing, or a sum below the normal range
-// is replayed term by term (the exact chain).
-constexpr uint32_t kPer = 8, kBatch = 32 * kPer;
+// mse = fmaf(e, e, mse) over each candidate's samples in loop order, the reference's float sum
+// (generate_config.tpp:227-254), bit for bit: a CTA per candidate over batches of 8192 terms
+// (float_chain.cuh). For the same 14 layers a warp per candidate with batches of 256 took 3.6 ms,
+// a CTA each takes 0.56: what is left is the scan and two barriers a batch, and one more pass for
+// each of the sum's binades.
+constexpr int kMsePer = 8;
 
-__global__ void plan_mse_kernel(const PlanCand *__restrict__ cands, uint32_t ncands, const float *__restrict__ e,
-                                float *__restrict__ mse_out) {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= ncands) return;
-    const PlanCand c = cands[warp];
+__global__ void __launch_bounds__(1024) plan_mse_kernel(const PlanCand *__restrict__ cands, const float *__restrict__ e,
+                                                        float *__restrict__ mse_out) {
+    __shared__ ChainShared sh;
+    const PlanCand &c = cands[blockIdx.x];
     const uint64_t n = c.cnt[0] * c.cnt[1] * c.cnt[2];
-    const float *p = e + c.off;
-    float mse = 0.0f;
-    for (uint64_t b = 0; b < n; b += kBatch) {
-        float v[kPer];
-#pragma unroll
-        for (uint32_t i = 0; i < kPer; i++) {
-            const uint64_t k = b + lane * kPer + i;
-            v[i] = k < n ? p[k] : 0.0f;
-        }
-        if (mse >= 0x1p-100f) {
-            int ex;
-            frexpf(mse, &ex);  // mse = f * 2^ex, f in [0.5, 1): binade 2^(ex-1), ulp 2^(ex-24)
-            const double inv_u = ldexp(1.0, 24 - ex);
-            const uint32_t m = (uint32_t)__double2uint_rz((double)mse * inv_u);
-            bool ok = true;
-            uint32_t sum = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < kPer; i++) {
-                const double t = __dmul_rn(__dmul_rn((double)v[i], (double)v[i]), inv_u);
-                const double r = rint(t);
-                ok = ok && r < 0x1p24 && fabs(t - r) != 0.5;
-                sum += ok ? (uint32_t)r : 0u;
+    const float *p = e + c.off;  // off is a multiple of kPlanAlign
+    const float mse = block_chain<kMsePer>(
+        sh, 0.0f, n,
+        [&](uint64_t k, float (&x)[kMsePer]) {
+            if (k + kMsePer <= n) {
+                const float4 u = *reinterpret_cast<const float4 *>(p + k), v = *reinterpret_cast<const float4 *>(p + k + 4);
+                x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
+                x[4] = v.x, x[5] = v.y, x[6] = v.z, x[7] = v.w;
+            } else {
+                for (int i = 0; i < kMsePer; i++) x[i] = k + i < n ? p[k + i] : 0.0f;
             }
-            ok = __all_sync(0xffffffffu, ok);
-            const uint32_t tot = __reduce_add_sync(0xffffffffu, sum);
-            if (ok && (uint64_t)m + tot < (1ull << 24)) {
-                mse = ldexpf((float)(m + tot), ex - 24);
-                continue;
-            }
-        }
-        const uint32_t cnt = n - b < kBatch ? (uint32_t)(n - b) : kBatch;
-        for (uint32_t j = 0; j < cnt; j++) {
-            const uint32_t i = j % kPer;
-            float vi = v[0];
-#pragma unroll
-            for (uint32_t q = 1; q < kPer; q++) vi = i == q ? v[q] : vi;
-            const float x = __shfl_sync(0xffffffffu, vi, j / kPer);
-            mse = __fmaf_rn(x, x, mse);
-        }
-    }
-    if (lane == 0) mse_out[warp] = mse;
+        },
+        [](float s, float x) { return __fmaf_rn(x, x, s); });
+    if (threadIdx.x == 0) mse_out[blockIdx.x] = mse;
 }
 
 }  // namespace
 
-cudaError_t launch_plan_sample(const float *d, uint64_t n1, uint64_t n2, const PlanCand *cands, uint32_t ncands, uint64_t total,
+cudaError_t launch_plan_sample(const float *d, uint64_t n1, uint64_t n2, const PlanCand *cands, uint32_t ncands, uint64_t most,
                                int32_t *qb, float *e, int32_t *qb_range, cudaStream_t st) {
-    if (total == 0) return cudaSuccess;
-    const uint64_t b = (total + 255) / 256;
-    plan_sample_kernel<<<(unsigned)(b < 148 * 16 ? b : 148 * 16), 256, 0, st>>>(d, n1, n2, cands, ncands, total, qb, e, qb_range);
+    if (most == 0 || ncands == 0) return cudaSuccess;
+    // CTAs a candidate: enough for its samples, and about 16 an SM over all candidates.
+    const uint64_t want = (most + kSampleThreads - 1) / kSampleThreads, share = (148 * 16 + ncands - 1) / ncands;
+    plan_sample_kernel<<<dim3((unsigned)(want < share ? want : share), ncands), kSampleThreads, 0, st>>>(d, n1, n2, cands, qb, e,
+                                                                                                        qb_range);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_plan_mse(const PlanCand *cands, uint32_t ncands, const float *e, float *mse, cudaStream_t st) {
     if (ncands == 0) return cudaSuccess;
-    plan_mse_kernel<<<(ncands * 32 + 127) / 128, 128, 0, st>>>(cands, ncands, e, mse);
+    plan_mse_kernel<<<ncands, 1024, 0, st>>>(cands, e, mse);
     count_launch();
     return cudaGetLastError();
 }
