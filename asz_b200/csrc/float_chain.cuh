@@ -23,10 +23,10 @@ namespace asz {
 struct ChainSum {
     float s;
     uint32_t m;
-    double inv_u;
     int ex;
-    bool normal;  // far enough above the smallest floats for the products below
-    __device__ __forceinline__ explicit ChainSum(float v) : s(v), m(0), inv_u(0.0), ex(0), normal(v >= 0x1p-100f && v < 0x1p120f) {
+    double inv_u;
+    bool normal;  // well inside the normal floats
+    __device__ __forceinline__ explicit ChainSum(float v) : s(v), m(0), ex(0), inv_u(0.0), normal(v >= 0x1p-100f && v < 0x1p120f) {
         if (normal) {
             ex = (int)(__float_as_uint(v) >> 23) - 126;  // v = f 2^ex, f in [1/2, 1): ulp 2^(ex - 24)
             m = (__float_as_uint(v) & 0x7fffffu) | 0x800000u;
@@ -37,59 +37,76 @@ struct ChainSum {
     __device__ __forceinline__ float after(uint32_t add) const {
         return add == 0 ? s : __uint_as_float(((uint32_t)(ex + 126) << 23) | ((m + add) & 0x7fffffu));
     }
-    // Rounded ulps of one term, added to `ulps` (saturating well above 2^24); false if the term
-    // has to be added by itself.
-    __device__ __forceinline__ bool take(double x, uint32_t &ulps) const {
+    // Rounded ulps of one term; false if the term has to be added by itself.
+    __device__ __forceinline__ bool ulps(double x, uint32_t &r) const {
+        r = 0;
         if (!normal) return x == 0.0 && s >= 0.0f;
         const double t = __dmul_rn(x, inv_u);
         if (!(t >= 0.0 && t < 0x1p24)) return false;
-        const double r = rint(t);
-        const double half = fabs(__dsub_rn(t, r));  // exact
-        ulps = min(ulps + (uint32_t)__double2uint_rn(r), 1u << 25);
-        return half < 0.5 - 0x1p-20;
+        const double w = rint(t);
+        r = (uint32_t)__double2uint_rn(w);
+        return fabs(__dsub_rn(t, w)) < 0.5 - 0x1p-20;  // the difference is exact
     }
 };
 
-// One warp: the chain over terms 0..n-1, `per` consecutive terms a lane. term(k) is term k in
-// double, step(s, k) the reference's own addition. Every lane gets the sum.
-template <int kPer, class Term, class Step>
-__device__ float warp_chain(float s, int n, const Term &term, const Step &step) {
+// Terms of warp_chain lie in its batches' order: four consecutive ones a lane, without bank
+// conflicts.
+constexpr int kChainPer = 4, kChainBatch = 32 * kChainPer, kChainHead = 12;
+__device__ __forceinline__ int chain_slot(int k) {
+    return (k & ~(kChainBatch - 1)) + (k & (kChainPer - 1)) * 32 + ((k & (kChainBatch - 1)) / kChainPer);
+}
+__host__ __device__ constexpr uint32_t chain_slots(uint32_t n) {
+    return (n + kChainBatch - 1) / kChainBatch * kChainBatch;
+}
+
+// One warp: the chain over n terms, term k at x[chain_slot(k)]. step(s, k) is the reference's own
+// addition. Every lane gets the sum. A pass takes what is left of the batch up to the first term
+// that leaves the binade or ties, and that term.
+template <class Step>
+__device__ __forceinline__ float warp_chain(const double *x, int n, const Step &step) {
     const int lane = threadIdx.x & 31;
-    for (int b = 0; b < n; b += 32 * kPer) {
-        const int k0 = b + lane * kPer, k1 = min(k0 + kPer, n);
-        double x[kPer];
+    float s = 0.0f;
+    // The sum leaves its binade at every other of the first terms: those are added as they are.
+    const int head = min(n, kChainHead);
+    for (int k = 0; k < head; k++) s = step(s, k);
+    for (int b = 0; b < n; b += kChainBatch) {
+        double v[kChainPer];
 #pragma unroll
-        for (int i = 0; i < kPer; i++) x[i] = k0 + i < n ? term(k0 + i) : 0.0;
-        int from = 0;  // lanes below are done
+        for (int i = 0; i < kChainPer; i++) v[i] = b + lane * kChainPer + i < n ? x[b + i * 32 + lane] : 0.0;
+        int done = b == 0 ? head : 0;  // terms of the batch already added
         while (true) {
             const ChainSum c(s);
-            uint32_t ulps = 0;
-            bool ok = true;
-            if (lane >= from) {
+            uint32_t r[kChainPer], sum = 0;
+            bool ok[kChainPer];
 #pragma unroll
-                for (int i = 0; i < kPer; i++) ok = c.take(x[i], ulps) && ok;
+            for (int i = 0; i < kChainPer; i++) {
+                ok[i] = c.ulps(v[i], r[i]);
+                if (lane * kChainPer + i < done) ok[i] = true, r[i] = 0;
+                sum += r[i];  // r <= 2^24
             }
-            ulps = min(ulps, 1u << 24);
-            uint32_t incl = ulps;
+            uint32_t incl = sum;  // <= 32 * 2^26
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += y;
             }
-            ok = ok && (!c.normal || c.m + incl < (1u << 24));
-            const unsigned bad = __ballot_sync(0xffffffffu, !ok);
-            const int f = bad ? __ffs(bad) - 1 : 31;
-            const float upto = c.normal ? c.after(__shfl_sync(0xffffffffu, bad ? incl - ulps : incl, f)) : s;
-            if (!bad) {
-                s = upto;
-                break;
+            // Within the lane: the first term that cannot be taken, and the sum before it.
+            uint32_t acc = incl - sum;
+            int at = kChainPer;
+#pragma unroll
+            for (int i = 0; i < kChainPer; i++) {
+                if (at != kChainPer) continue;
+                if (!ok[i] || (c.normal && c.m + acc + r[i] >= (1u << 24))) at = i;
+                else acc += r[i];
             }
-            float v = upto;
-            if (lane == f)
-                for (int k = k0; k < k1; k++) v = step(v, k);
-            s = __shfl_sync(0xffffffffu, v, f);
-            from = f + 1;
-            if (from == 32) break;
+            const unsigned bad = __ballot_sync(0xffffffffu, at != kChainPer);
+            const int f = bad ? __ffs(bad) - 1 : 31;
+            s = c.after(__shfl_sync(0xffffffffu, acc, f));
+            if (!bad) break;
+            const int k = f * kChainPer + __shfl_sync(0xffffffffu, at, f);
+            s = step(s, b + k);  // the same on every lane
+            done = k + 1;
+            if (b + done >= n) break;
         }
     }
     return s;
@@ -123,7 +140,11 @@ __device__ float block_chain(ChainShared &sh, float s, uint64_t n, const Load &l
             bool ok = true;
             if (tid >= from) {
 #pragma unroll
-                for (int i = 0; i < kPer; i++) ok = c.take(__dmul_rn((double)x[i], (double)x[i]), ulps) && ok;
+                for (int i = 0; i < kPer; i++) {
+                    uint32_t r;
+                    ok = c.ulps(__dmul_rn((double)x[i], (double)x[i]), r) && ok;
+                    ulps += r;
+                }
             }
             ulps = min(ulps, 1u << 24);
             uint32_t incl = ulps;
@@ -149,11 +170,11 @@ __device__ float block_chain(ChainShared &sh, float s, uint64_t n, const Load &l
             const uint32_t f = __reduce_min_sync(0xffffffffu, sh.first[parity][lane]);
             parity ^= 1;
             if (f == kT) {
-                if (c.normal) s = c.after(all);
+                s = c.after(all);
                 break;
             }
             if (tid == f) {
-                float v = c.normal ? c.after(before + incl - ulps) : s;
+                float v = c.after(before + incl - ulps);
 #pragma unroll
                 for (int i = 0; i < kPer; i++)
                     if (k0 + i < n) v = step(v, x[i]);

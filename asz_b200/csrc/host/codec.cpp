@@ -742,15 +742,21 @@ uint32_t exact_cap() {
         int dev = 0, lim = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        uint32_t c = 2048;
-        while (c > 64 && exact_smem_bytes(c) + 2048 > (uint32_t)lim) c -= 64;
+        uint32_t c = 4096;
+        while (c > 64 && exact_smem_bytes(c) + kExactStatic > (uint32_t)lim) c -= 64;
         cap = c;
     }
     return cap;
 }
 
-// Bytes of one CTA's slice of the global scratch for exact replays of up to cap samples.
-u64 exact_global_stride(uint32_t cap) { return ((u64)exact_smem_bytes(cap) + 255) / 256 * 256; }
+// Global scratch of exact replays of up to cap samples: at most 148 slices and 512 MiB in all, and
+// the bytes of one slice, with room for the evaluations side by side where 148 of those fit.
+constexpr u64 kExactScratch = 512ull << 20;
+u64 exact_global_stride(uint32_t cap) {
+    u64 b = exact_smem_bytes(cap);
+    if (cap < kExactFullMost && (u64)exact_full_bytes(cap) * 148 <= kExactScratch) b = exact_full_bytes(cap);
+    return (b + 255) / 256 * 256;
+}
 
 // AB maps larger than shared memory holds (dm->boxes, dm->evals uploaded): the exact kernel with
 // each box's working set in global scratch, a CTA per box. done is false when a box needs the
@@ -916,7 +922,7 @@ int abmap_exact_global(asz_ctx *ctx, uint32_t ne, const float *field, u64 n1n2, 
     MiscLayout *dm = ctx->misc.as<MiscLayout>();
     cudaStream_t st = ctx->stream;
     const u64 stride = exact_global_stride(cap);
-    CK(ctx->gscratch.reserve(nb * stride));
+    CK(ctx->gscratch.reserve((u64)nb * slope_batches(ne) * stride));
     CK(cudaMemsetAsync(&dm->err, 0, 4, st));
     {
         ProfScope ps(ctx, prof_name, 0);
@@ -1040,7 +1046,7 @@ int default_slope_on(asz_ctx *ctx, const float *field, const uint64_t fdims[3], 
         {
             ProfScope ps_slope(ctx, "slope", 0);
             CK(launch_slope_exact(dm->boxes, dm->evals, ne, d_in, dims[1] * dims[2], dims[2], ctx->log2arena.as<float>(),
-                                  R * R, dm->h1, dm->x, dm->m, &dm->err, exact_cap(), 3, ctx->stream));
+                                  R * R, dm->h1, dm->x, dm->m, &dm->err, exact_cap(), cap, 3, ctx->stream));
         }
         uint32_t e1 = 0;
         CK(cudaMemcpyAsync(&e1, &dm->err, 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1237,7 +1243,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
                     {
                         ProfScope ps_(ctx, "plan_abmap", 0);
                         CK(launch_slope_exact(dm->boxes, dm->evals, ne, d_in, dims[1] * dims[2], dims[2], ctx->log2arena.as<float>(),
-                                              R * R, dm->h1, dm->x, dm->m, &dm->err, exact_cap(), nb, st));
+                                              R * R, dm->h1, dm->x, dm->m, &dm->err, exact_cap(), cap, nb, st));
                     }
                     uint32_t e1 = 0;
                     CK(cudaMemcpyAsync(&e1, &dm->err, 4, cudaMemcpyDeviceToHost, st));
@@ -1596,7 +1602,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
     const u64 gstride = exact_global_stride(capmax);
     unsigned ggrid = 0;
     if (capmax > exact_cap()) {
-        ggrid = (unsigned)std::max<u64>(1, std::min<u64>(148, (512ull << 20) / gstride));
+        ggrid = (unsigned)std::max<u64>(1, std::min<u64>(148, kExactScratch / gstride));
         CK(ctx->gscratch.reserve(ggrid * gstride));
         CK(ctx->spill2.reserve(G.nblocks * sizeof(uint32_t)));
     }
@@ -1840,7 +1846,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
                                              d_tval, d_tint, &dm->fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap,
                                              &dm->amb_count, ctx->overrides.as<uint32_t>(), nov,
                                              ctx->proxies.as<float>() + G.nblocks * l * 10, d_bail + G.nblocks * l,
-                                             &dm->list_count[l], d_spill, d_scount, exact_cap(), 148, st));
+                                             &dm->list_count[l], d_spill, d_scount, exact_cap(), G.cap[l], 148, st));
                     }
                     {
                         ProfScope ps(ctx, "tsel_serial", 0);
@@ -1914,7 +1920,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
                 CK(launch_tsel_exact(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default, d_tval,
                                      d_tint, &dm->fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->amb_count,
                                      ctx->overrides.as<uint32_t>(), nov, ctx->proxies.as<float>() + G.nblocks * l * 10,
-                                     d_list, d_lcount, d_spill, d_scount, exact_cap(), 148, st));
+                                     d_list, d_lcount, d_spill, d_scount, exact_cap(), G.cap[l], 148, st));
             }
             // Groups larger than shared memory holds: the same replay with global scratch, a CTA
             // per group; only what that cannot take (keys outside int32) reaches the serial kernel.
@@ -3518,6 +3524,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     const std::vector<float> cand = candidate_t(p);
     u64 nb_total = 0, ent_total = 0, tint_total = 0, qb_total = 0;
     uint32_t capmax = 1;
+    std::vector<uint32_t> cap_round(L, 1);  // largest group of each round over the fields
     for (uint32_t f = 0; f < nf; f++) {
         BatchItem &b = B[f];
         const std::string tag = "field " + std::to_string(f) + ": ";
@@ -3545,6 +3552,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
             for (auto &ci : b.G.classes[l])
                 if (ci.n) ci.log2_off = log2_table(ctx, ci.n);
             capmax = std::max(capmax, b.G.cap[l]);
+            cap_round[l] = std::max(cap_round[l], b.G.cap[l]);
         }
         b.o_rec = b.o_qb = qb_total;
         qb_total += b.N;
@@ -3584,7 +3592,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     const u64 gstride = exact_global_stride(capmax);
     unsigned ggrid = 0;
     if (capmax > exact_cap()) {
-        ggrid = (unsigned)std::max<u64>(1, std::min<u64>(148, (512ull << 20) / gstride));
+        ggrid = (unsigned)std::max<u64>(1, std::min<u64>(148, kExactScratch / gstride));
         CK(ctx->gscratch.reserve(ggrid * gstride));
         CK(ctx->b_spill2.reserve(std::max<u64>(nb_total, 1) * sizeof(unsigned long long)));
     }
@@ -3690,7 +3698,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
             CK(launch_tsel_fast_batch(dF, d_goff, nf, (uint32_t)l, ctx->log2arena.as<float>(), t_default, q, d_hand, q + 2,
                                       148 * sh[0], st));
             CK(launch_tsel_exact_batch(dF, (uint32_t)l, ctx->log2arena.as<float>(), t_default, d_hand, q + 2, d_spill, q + 3,
-                                       exact_cap(), 148, st));
+                                       exact_cap(), cap_round[l], 148, st));
             unsigned long long *d_left = d_spill;
             uint32_t *d_lcnt = q + 3;
             if (ggrid) {

@@ -11,12 +11,27 @@
 //     is its position in the previous stage's list if it was present at the rehash, else its
 //     insertion index. So each stage is a parallel rank computation (atomics, one scan);
 //  4. per evaluation: quantised errors in map order, the qb_map's own order (same method, identity
-//     hash), then the two order-dependent float sums, one thread each, all evaluations at once.
+//     hash), then the two order-dependent float sums.
 // The result is the reference's float h1 and log10f argument bit for bit; the t decision then
 // uses the same certified log10 step as the serial kernel.
+//
+// A launch has a few groups (tens in a round, three boxes for the default slope), so what counts is
+// how long one group takes, and that is a chain of short dependent steps, not work. Hence:
+// - the CTA splits into up to five teams of warps, an evaluation each, so a group takes as long as
+//   one evaluation and not as five (as many teams as the shared memory holds the tables of);
+// - tables are sized by the group and not by the largest group;
+// - a rehash stage has the threads it needs: a warp up to 31 nodes, four (or the team's three) up to
+//   127, and then a node a thread in registers;
+// - the serial float sums go to a warp each (float_chain.cuh) instead of a thread, a step of which
+//   takes a double fused add and two conversions in a row.
+// Default slope of a 512^3 field (three boxes, ten evaluations): 84 -> 39 us; the nine rounds' groups
+// of a 161x257x349 quintic field at 1e-4: 1.13 -> 0.52 ms; the plan search's AB maps at 100x500x500:
+// 3.2 -> 0.79 ms. What is left of one group is spread over all phases (363 samples: sampling 4 us,
+// map order 6, evaluation maps 6, sums 7), each a few dozen dependent shared-memory round trips.
 #include <cuda_runtime.h>
 
 #include "dev_common.cuh"
+#include "float_chain.cuh"
 #include "launch.h"
 #include "listsim.cuh"
 #include "tsel.cuh"
@@ -24,7 +39,8 @@
 namespace asz {
 namespace {
 
-constexpr int kThreads = 512;  // 16 warps: 5 run the sum chains, 11 build the qb maps
+constexpr int kThreads = 512;
+constexpr int kTeams = 5;      // evaluations side by side, where their tables fit
 constexpr int kMaxEvals = 22;  // default slope: 11 t values x 2 error bounds
 
 __device__ __forceinline__ int class_of(uint64_t b, uint64_t nb) { return b == 0 ? 0 : (b == nb - 1 ? 2 : 1); }
@@ -38,33 +54,38 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
     return x;
 }
 
-// A set of whole warps that synchronise on their own hardware barrier (bar 0 is the CTA's).
+// A set of whole warps that synchronise on their own hardware barrier (bar 0 is the CTA's). A team
+// of one warp needs none.
 struct Team {
     int tid, size, bar;
-    __device__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(size) : "memory"); }
+    __device__ __forceinline__ void sync() const {
+        if (size == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(size) : "memory");
+    }
 };
+
+__device__ __forceinline__ int warp_incl_scan(int v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    return v;
+}
 
 // Exclusive scan of one value per team thread; total in *tot. warp_sums holds 32 ints.
 __device__ int team_excl_scan(const Team &T, int v, int *warp_sums, int *tot) {
     const int lane = T.tid & 31, w = T.tid >> 5, nw = T.size >> 5;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
+    const int x = warp_incl_scan(v);
+    if (nw == 1) {
+        if (tot) *tot = __shfl_sync(0xffffffffu, x, 31);
+        return x - v;
     }
     if (lane == 31) warp_sums[w] = x;
     T.sync();
-    if (w == 0) {
-        int s = lane < nw ? warp_sums[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        warp_sums[lane] = s;  // inclusive
-    }
-    T.sync();
-    int base = w ? warp_sums[w - 1] : 0;
-    int total = warp_sums[nw - 1];
+    const int s = warp_incl_scan(lane < nw ? warp_sums[lane] : 0);  // every warp, so no second barrier
+    const int base = w ? __shfl_sync(0xffffffffu, s, w - 1) : 0, total = __shfl_sync(0xffffffffu, s, nw - 1);
     T.sync();
     if (tot) *tot = total;
     return base + x - v;
@@ -87,52 +108,110 @@ __device__ int team_scan_array(const Team &T, int *a, int n, int *warp_sums) {
     return tot;
 }
 
-// Iteration order of a std::unordered_map filled by inserting distinct elements 0..m-1 in order
-// (stage method, see the file comment). code(e) is the element's hash. Writes ord[m].
-// Scratch: tim, pos, ebk, nxt (m each), ctm, bsz, hed (buckets), arr (m+1).
-template <class Code>
-__device__ void map_order(const Team &T, int m, Code code, int *tim, int *pos, int *ebk, int *nxt, int *ctm, int *bsz,
-                          int *hed, int *arr, int *ord, int *warp_sums) {
-    int stage = 0;
-    while (stage < kSchedLen && sched_at(stage) <= (uint64_t)m) {
-        const int r = (int)sched_at(stage);
-        const uint64_t beta = sched_bkt(stage);
-        const int end = (stage + 1 < kSchedLen && sched_at(stage + 1) <= (uint64_t)m) ? (int)sched_at(stage + 1) - 1 : m;
-        for (int e = T.tid; e < end; e += T.size) tim[e] = (stage == 0 || e >= r - 1) ? e : pos[e];
-        for (uint64_t b = T.tid; b < beta; b += T.size) {
-            ctm[b] = INT32_MAX;
-            bsz[b] = 0;
-            hed[b] = -1;
-        }
-        for (int t = T.tid; t < end; t += T.size) arr[t] = 0;
-        T.sync();
-        for (int e = T.tid; e < end; e += T.size) {
-            int b = (int)(code(e) % beta);
-            ebk[e] = b;
-            atomicMin(&ctm[b], tim[e]);
-            atomicAdd(&bsz[b], 1);
-            nxt[e] = atomicExch(&hed[b], e);
-        }
-        T.sync();
-        // arr[end-1-t] = size of the run whose bucket was created at time t.
-        for (int e = T.tid; e < end; e += T.size) {
-            int b = ebk[e];
-            if (ctm[b] == tim[e]) arr[end - 1 - tim[e]] = bsz[b];
-        }
-        T.sync();
-        team_scan_array(T, arr, end, warp_sums);  // arr[end-1-t] = nodes in runs created after t
-        for (int e = T.tid; e < end; e += T.size) {
-            int b = ebk[e], te = tim[e];
-            int rank = 0, guard = 0;
-            for (int x = hed[b]; x >= 0 && guard <= end; x = nxt[x], guard++)
-                if (tim[x] > te) rank++;
-            pos[e] = arr[end - 1 - ctm[b]] + rank;
-        }
-        T.sync();
-        stage++;
+// Working arrays of one map's order: heads (one int a bucket), next, after, first, rank, moved (one a
+// node).
+struct OrderScratch {
+    int *heads, *next, *after, *first, *rank, *moved;
+};
+
+// h mod the stage's bucket count: the quotient by the reciprocal is at most two short.
+__device__ __forceinline__ int bucket_of(uint64_t h, uint32_t beta, uint64_t magic) {
+    uint64_t r = h - __umul64hi(h, magic) * beta;
+    if (r >= beta) r -= beta;
+    if (r >= beta) r -= beta;
+    return (int)r;
+}
+
+// A bucket's chain from `head`, as times of its nodes in no order: the first of them, how many they
+// are, and how many are later than t.
+__device__ __forceinline__ void walk(const int *next, int head, int t, int limit, int &first, int &count, int &later) {
+    first = t;
+    count = later = 0;
+    for (int x = head; x >= 0 && count < limit; x = next[x]) {
+        first = min(first, x);
+        count++;
+        later += x > t;
     }
-    for (int e = T.tid; e < m; e += T.size) ord[pos[e]] = e;
+}
+
+// One rehash stage over nodes [0, end): ord[] is the list before it for the first `fresh` nodes (the
+// others come in the order of their index) and the list after it at the end. A node's time is its
+// place in that sequence, thread or iteration t has the node of time t, and its new place is the
+// number of nodes in runs opened after its own plus those of its run that are later than it.
+__device__ __forceinline__ void map_stage(const Team T, int stage, int end, int fresh, const uint64_t *hash, const OrderScratch S,
+                                       int *ord, int *warp_sums) {
+    const uint32_t beta = (uint32_t)sched_bkt(stage);
+    const uint64_t magic = sched_magic(stage);
+    const int lane = T.tid & 31, w = T.tid >> 5, nw = T.size >> 5;
+    for (uint32_t b = T.tid; b < beta; b += T.size) S.heads[b] = -1;
+    if (end <= T.size) {  // a node a thread, in registers
+        const int t = T.tid;
+        const bool in = t < end;
+        const int e = t < fresh ? ord[t] : t;
+        const int b = in ? bucket_of(hash[e], beta, magic) : 0;
+        T.sync();
+        if (in) S.next[t] = atomicExch(&S.heads[b], t);
+        T.sync();
+        int first = t, count = 0, later = 0;
+        if (in) walk(S.next, S.heads[b], t, end, first, count, later);
+        const int opened = first == t ? count : 0;  // the run's nodes, at the time it was opened
+        int sum = opened;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_down_sync(0xffffffffu, sum, o);
+            if (lane + o < 32) sum += y;
+        }
+        int behind = 0;
+        if (nw > 1) {
+            if (lane == 0) warp_sums[w] = sum;
+            T.sync();
+            behind = __reduce_add_sync(0xffffffffu, lane > w && lane < nw ? warp_sums[lane] : 0);
+        }
+        if (in && opened) S.after[t] = behind + sum - opened;
+        T.sync();
+        if (in) ord[S.after[first] + later] = e;
+        T.sync();
+        return;
+    }
     T.sync();
+    for (int t = T.tid; t < end; t += T.size) {
+        const int e = t < fresh ? ord[t] : t;
+        const int b = bucket_of(hash[e], beta, magic);
+        S.moved[t] = e;
+        S.rank[t] = b;
+        S.next[t] = atomicExch(&S.heads[b], t);
+    }
+    T.sync();
+    for (int t = T.tid; t < end; t += T.size) {
+        int first, count, later;
+        walk(S.next, S.heads[S.rank[t]], t, end, first, count, later);
+        S.first[t] = first;
+        S.rank[t] = later;
+        S.after[end - 1 - t] = first == t ? count : 0;
+    }
+    T.sync();
+    team_scan_array(T, S.after, end, warp_sums);
+    for (int t = T.tid; t < end; t += T.size) ord[S.after[end - 1 - S.first[t]] + S.rank[t]] = S.moved[t];
+    T.sync();
+}
+
+// Iteration order of a std::unordered_map filled by inserting distinct elements 0..m-1 (m >= 1) with
+// the given hashes in order (stage method, see the file comment). Writes ord[m]. The stages of up to
+// 31 nodes are the team's first warp's, those of up to 127 the first `few` threads', which
+// synchronise on barrier `few_bar` (few == the team's size: on the team's).
+__device__ __forceinline__ void map_order(const Team &T, int few, int few_bar, int m, const uint64_t *hash, const OrderScratch &S, int *ord,
+                          int *warp_sums) {
+    int had = 32;  // threads that have the list
+    for (int stage = 0; stage < kSchedLen && sched_at(stage) <= (uint64_t)m; stage++) {
+        const int fresh = stage == 0 ? 0 : (int)sched_at(stage) - 1;
+        const int end = (stage + 1 < kSchedLen && sched_at(stage + 1) <= (uint64_t)m) ? (int)sched_at(stage + 1) - 1 : m;
+        const Team U{T.tid, end < 32 ? 32 : end < 128 ? few : T.size, end < 128 ? few_bar : T.bar};
+        if (T.tid >= U.size) continue;
+        if (U.size != had) U.sync();
+        had = U.size;
+        map_stage(U, stage, end, fresh, hash, S, ord, warp_sums);
+    }
+    if (had != T.size) T.sync();
 }
 
 struct ExactGroup {
@@ -140,57 +219,80 @@ struct ExactGroup {
     uint32_t n;
 };
 
-// Shared-memory layout for groups of up to `cap` samples (offsets in bytes). The distinct
-// entries and the AB map order persist; the sampling/de-duplication arrays and the later stage and
-// qb_map arrays share one region.
+// Layout of the working set of a group of up to n samples with `teams` evaluations side by side
+// (offsets in bytes), made on the host. The distinct entries and the AB map's order persist;
+// sampling and de-duplication, the AB map's stages and the teams' tables follow one another in one
+// region. In a team's slice, beside its distinct values, their counts and their order, one area
+// holds its hash table, then its map's stages, then the terms of its sums.
 struct Layout {
-    uint32_t tcap, bmax;
-    uint32_t ekey, ecnt, ord;                         // persistent
-    uint32_t key, tkey, tfirst, tcnt, sslot;          // phase 1-3
-    uint32_t tim, pos, ebk, nxt, ctm, bsz, hed, arr;  // phase 4-7 (stage scratch)
-    uint32_t qtab, qfirst, qsum, qslot, qval, qc, qord;
+    uint32_t n, teams;
+    uint32_t ekey, ecnt, ord;                 // persistent
+    uint32_t key, tkey, tfirst, tcnt, sslot;  // phases 1-2
+    uint32_t hash, order;                     // phase 3
+    uint32_t team, team_stride;               // phase 4
+    uint32_t qval, qc, qord, work;            // in a team's slice
+    uint32_t qtab, qfirst, qsum, qslot;       // in its work area
     uint32_t total;
-    __host__ __device__ Layout(uint32_t cap) {
-        tcap = 16;
-        while (tcap < 2 * cap) tcap <<= 1;
-        bmax = (uint32_t)sched_buckets(cap);
-        uint32_t off = 0;
+    __host__ Layout(uint32_t n_, uint32_t teams_) : n(n_), teams(teams_) {
+        const uint32_t hcap = hash_slots(n);
+        uint32_t off = 0, top = 0;
         auto take = [&](uint32_t bytes) {
-            uint32_t o = off;
+            const uint32_t o = off;
             off += (bytes + 15) & ~15u;
+            top = off > top ? off : top;
             return o;
         };
-        ekey = take(8 * cap);
-        ecnt = take(4 * cap);
-        ord = take(4 * cap);
+        ekey = take(8 * n);
+        ecnt = take(4 * n);
+        ord = take(4 * n);
         const uint32_t u = off;
-        key = take(8 * cap);
-        tkey = take(8 * tcap);
-        tfirst = take(4 * tcap);
-        tcnt = take(4 * tcap);
-        sslot = take(4 * cap);
-        const uint32_t end_a = off;
+        key = take(8 * n);
+        tkey = take(8 * hcap);
+        tfirst = take(4 * hcap);
+        tcnt = take(4 * hcap);
+        sslot = take(4 * n);
         off = u;
-        tim = take(4 * cap);
-        pos = take(4 * cap);
-        ebk = take(4 * cap);
-        nxt = take(4 * cap);
-        ctm = take(4 * bmax);
-        bsz = take(4 * bmax);
-        hed = take(4 * bmax);
-        arr = take(4 * (cap + 1));
-        qtab = take(4 * tcap);
-        qfirst = take(4 * tcap);
-        qsum = take(4 * tcap);
-        qslot = take(4 * cap);
-        qval = take(4 * cap);
-        qc = take(4 * cap);
-        qord = take(4 * cap);
-        total = off > end_a ? off : end_a;
+        hash = take(8 * n);
+        order = take(order_bytes(n));
+        off = 0;
+        uint32_t own = top;
+        top = 0;
+        qval = take(8 * n);
+        qc = take(4 * n);
+        qord = take(4 * n);
+        work = take(order_bytes(n));
+        off = work;
+        take(16 * chain_slots(n) + 12 * n);
+        off = work;
+        qtab = take(4 * hcap);
+        qfirst = take(4 * hcap);
+        qsum = take(4 * hcap);
+        qslot = take(4 * n);
+        team = u;
+        team_stride = top;
+        total = u + teams * team_stride > own ? u + teams * team_stride : own;
+    }
+    __host__ __device__ static uint32_t hash_slots(uint32_t n) { return n + n / 2 + 16; }
+    __host__ static uint32_t order_bytes(uint32_t n) {
+        return 4 * (5 * ((n + 3) & ~3u) + (uint32_t)sched_buckets(n));
+    }
+    __device__ OrderScratch order_at(uint8_t *p) const {
+        const uint32_t an = (n + 3) & ~3u;
+        int *q = (int *)p;
+        return OrderScratch{q + 5 * an, q, q + an, q + 2 * an, q + 3 * an, q + 4 * an};
     }
 };
 
-constexpr int kChainWarps = 5;  // warps 0..4: one mse chain each; the rest build qb maps
+// The layout of a launch whose groups have up to n samples, in `bytes` of memory: five teams of
+// three warps, two of eight, or the whole CTA. The last fits where exact_smem_bytes(n) does.
+Layout exact_layout(uint32_t n, uint64_t bytes) {
+    if (n < kExactFullMost)
+        for (uint32_t teams : {(uint32_t)kTeams, 2u}) {
+            const Layout l(n, teams);
+            if (l.total <= bytes) return l;
+        }
+    return Layout(n, 1);
+}
 
 // Quantised error of an entry for one evaluation (get_h_psnr.tpp:14-19 as emitted).
 __device__ __forceinline__ void entry_err(uint64_t kk, float t2, float stat_eb, float neg, float eb2, int &q, float &d) {
@@ -201,37 +303,32 @@ __device__ __forceinline__ void entry_err(uint64_t kk, float t2, float stat_eb, 
     d = __fmaf_rn(-__ll2float_rn(q64), eb2, err);
 }
 
-// Evaluations of one group: h1 and the log10f argument for each (t, abs_eb).
-// Returns false if the group does not fit `cap` or has keys outside int32.
+__device__ __forceinline__ uint32_t hash_slot(uint64_t k, uint32_t cap) { return __umulhi((uint32_t)(mix64(k) >> 32), cap); }
+
+// Evaluations of one group: h1 and the log10f argument for each (t, abs_eb), in the working set at
+// `mem`. Returns false if the group is larger than the layout or has keys outside int32.
 __device__ bool exact_eval(const ExactGroup &eg, const float *__restrict__ ref, const float *__restrict__ x0, uint64_t n1n2,
                            uint64_t n2, const ProxyEval *evals, int n_evals, float R2, const float *__restrict__ log2tab,
-                           uint8_t *smem, uint32_t cap, float *h1_out, float *x_out, uint32_t *m_out) {
-    const uint32_t n = eg.n;
-    if (n > cap || blockDim.x != (unsigned)kThreads) return false;
-    const Layout Lo(cap);
-    __shared__ int warp_sums[2][32];
-    __shared__ int flag_wide, m_sh;
-    __shared__ float h1_sh[5], mse_sh[5];
-    __shared__ int mq_sh;
+                           uint8_t *mem, const Layout &Lo, float *h1_out, float *x_out, uint32_t *m_out) {
+    const uint32_t n = eg.n, hcap = Layout::hash_slots(n);
+    if (n > Lo.n || blockDim.x != (unsigned)kThreads) return false;
+    const int teams = (int)Lo.teams;
+    __shared__ int warp_sums[kTeams][32], all_sums[32];
+    __shared__ int flag_wide;
     const Team all{(int)threadIdx.x, (int)blockDim.x, 0};
-    uint64_t *key = (uint64_t *)(smem + Lo.key), *tkey = (uint64_t *)(smem + Lo.tkey), *ekey = (uint64_t *)(smem + Lo.ekey);
-    int *tfirst = (int *)(smem + Lo.tfirst), *tcnt = (int *)(smem + Lo.tcnt), *sslot = (int *)(smem + Lo.sslot);
-    int *ecnt = (int *)(smem + Lo.ecnt), *ord = (int *)(smem + Lo.ord);
-    int *tim = (int *)(smem + Lo.tim), *pos = (int *)(smem + Lo.pos), *ebk = (int *)(smem + Lo.ebk),
-        *nxt = (int *)(smem + Lo.nxt), *ctm = (int *)(smem + Lo.ctm), *bsz = (int *)(smem + Lo.bsz),
-        *hed = (int *)(smem + Lo.hed), *arr = (int *)(smem + Lo.arr);
-    int *qtab = (int *)(smem + Lo.qtab), *qfirst = (int *)(smem + Lo.qfirst), *qsum = (int *)(smem + Lo.qsum),
-        *qslot = (int *)(smem + Lo.qslot), *qval = (int *)(smem + Lo.qval), *qc = (int *)(smem + Lo.qc),
-        *qord = (int *)(smem + Lo.qord);
+    uint64_t *key = (uint64_t *)(mem + Lo.key), *tkey = (uint64_t *)(mem + Lo.tkey), *ekey = (uint64_t *)(mem + Lo.ekey);
+    int *tfirst = (int *)(mem + Lo.tfirst), *tcnt = (int *)(mem + Lo.tcnt), *sslot = (int *)(mem + Lo.sslot);
+    int *ecnt = (int *)(mem + Lo.ecnt), *ord = (int *)(mem + Lo.ord);
     if (threadIdx.x == 0) flag_wide = 0;
     const uint64_t EMPTY = 0x8000000000000000ull;  // a = INT32_MIN: rejected below, so never a key
-    for (uint32_t i = threadIdx.x; i < Lo.tcap; i += blockDim.x) {
+    for (uint32_t i = threadIdx.x; i < hcap; i += blockDim.x) {
         tkey[i] = EMPTY;
         tfirst[i] = INT32_MAX;
         tcnt[i] = 0;
     }
     all.sync();
-    // 1. Sample keys in get_AB_map's scan order.
+    // 1. Sample keys in get_AB_map's scan order, into the hash table: first occurrence and count
+    // per distinct key.
     const SampleBox &b = eg.box;
     uint32_t c[3];
     for (int a = 0; a < 3; a++) c[a] = b.hi[a] > b.lo[a] ? (uint32_t)((b.hi[a] - b.lo[a] + b.step[a] - 1) / b.step[a]) : 0;
@@ -244,139 +341,138 @@ __device__ bool exact_eval(const ExactGroup &eg, const float *__restrict__ ref, 
         float S4 = __fadd_rn(__fadd_rn(p1, p3), __fadd_rn(m1, m3));
         float Bf = __double2float_rn(__fma_rn((double)S4, 0.25, -(double)x0[p]));
         int64_t ak = lround_f(__fmul_rn(Af, b.neg_2_stat_eb)), bk = lround_f(__fmul_rn(Bf, b.neg_2_stat_eb));
-        if (ak <= INT32_MIN || ak > INT32_MAX || bk < INT32_MIN || bk > INT32_MAX) flag_wide = 1;
-        key[s] = ((uint64_t)(uint32_t)(int32_t)ak << 32) | (uint32_t)(int32_t)bk;
-    }
-    all.sync();
-    if (flag_wide) return false;
-    // 2. De-duplicate; first occurrence and count per distinct key.
-    for (uint32_t s = threadIdx.x; s < n; s += blockDim.x) {
-        uint64_t k = key[s];
-        uint32_t slot = (uint32_t)(mix64(k) & (Lo.tcap - 1));
-        for (uint32_t probe = 0; probe < Lo.tcap; probe++) {
+        if (ak <= INT32_MIN || ak > INT32_MAX || bk < INT32_MIN || bk > INT32_MAX) {
+            flag_wide = 1;
+            sslot[s] = 0;
+            continue;
+        }
+        const uint64_t k = ((uint64_t)(uint32_t)(int32_t)ak << 32) | (uint32_t)(int32_t)bk;
+        key[s] = k;
+        uint32_t slot = hash_slot(k, hcap);
+        for (uint32_t probe = 0; probe < hcap; probe++) {
             unsigned long long prev = atomicCAS((unsigned long long *)&tkey[slot], (unsigned long long)EMPTY, (unsigned long long)k);
             if (prev == EMPTY || prev == k) break;
-            slot = (slot + 1) & (Lo.tcap - 1);
+            if (++slot == hcap) slot = 0;
         }
         sslot[s] = (int)slot;
         atomicMin(&tfirst[slot], (int)s);
         atomicAdd(&tcnt[slot], 1);
     }
     all.sync();
-    // 3. Distinct keys in first-occurrence order.
+    if (flag_wide) return false;
+    // 2. Distinct keys in first-occurrence order.
+    int m;
     {
         const uint32_t per = (n + blockDim.x - 1) / blockDim.x, beg = threadIdx.x * per, end = min(beg + per, n);
         int local = 0;
         for (uint32_t s = beg; s < end; s++) local += tfirst[sslot[s]] == (int)s;
-        int tot;
-        int off = team_excl_scan(all, local, warp_sums[0], &tot);
+        int off = team_excl_scan(all, local, all_sums, &m);
         for (uint32_t s = beg; s < end; s++)
             if (tfirst[sslot[s]] == (int)s) {
                 ekey[off] = key[s];
                 ecnt[off] = tcnt[sslot[s]];
                 off++;
             }
-        if (threadIdx.x == 0) m_sh = tot;
     }
     all.sync();
-    const int m = m_sh;
+    // hash = a*1145141919810 + b (asz_param.hpp:22-40); its array lies over the hash table
+    uint64_t *hash = (uint64_t *)(mem + Lo.hash);
+    for (int e = threadIdx.x; e < m; e += blockDim.x) {
+        const uint64_t k = ekey[e];
+        hash[e] = (uint64_t)(int64_t)(int32_t)(uint32_t)(k >> 32) * 1145141919810ull + (uint64_t)(int64_t)(int32_t)(uint32_t)k;
+    }
+    all.sync();
     if (m_out && threadIdx.x == 0) *m_out = (uint32_t)m;
     if (m == 0) return true;
-    // 4. AB map order; hash = a*1145141919810 + b (asz_param.hpp:22-40).
-    auto abcode = [&](int e) {
-        uint64_t k = ekey[e];
-        int64_t a = (int32_t)(uint32_t)(k >> 32), bb = (int32_t)(uint32_t)k;
-        return (uint64_t)a * 1145141919810ull + (uint64_t)bb;
-    };
-    map_order(all, m, abcode, tim, pos, ebk, nxt, ctm, bsz, hed, arr, ord, warp_sums[0]);
-    // 5-7. Evaluations in batches of five: warps 0-4 run the mse chains while the other warps build
-    // each evaluation's qb_map and run its h1 chain.
+    // 3. AB map order.
+    map_order(all, 128, kTeams + 1, m, (const uint64_t *)(mem + Lo.hash), Lo.order_at(mem + Lo.order), ord, all_sums);
+    // 4. Evaluations, a team each; the warps past the last whole team have none.
     const float nf = __ull2float_rn((uint64_t)n), rn = __fdiv_rn(1.0f, nf);
-    for (int e0 = 0; e0 < n_evals; e0 += 5) {
-        const int ne = min(5, n_evals - e0);
-        const int warp = threadIdx.x >> 5;
-        if (warp < kChainWarps) {
-            // mse chain (get_h_psnr.tpp:12-22) in map order.
-            if ((threadIdx.x & 31) == 0 && warp < ne) {
-                const ProxyEval ev = evals[e0 + warp];
-                const float neg = __fdiv_rn(0.5f, ev.abs_eb), t2 = __fadd_rn(ev.t, ev.t), eb2 = __fadd_rn(ev.abs_eb, ev.abs_eb);
-                float mse = 0.0f;
-                for (int k = 0; k < m; k++) {
-                    const int e = ord[k];
-                    int q;
-                    float dv;
-                    entry_err(ekey[e], t2, b.stat_eb, neg, eb2, q, dv);
-                    double dd = (double)dv;
-                    mse = __double2float_rn(__fma_rn((double)ecnt[e], __dmul_rn(dd, dd), (double)mse));
-                }
-                mse_sh[warp] = mse;
+    const int team_size = (kThreads / 32 / teams) * 32, t = threadIdx.x / team_size;
+    if (t < teams) {
+        const Team qt{(int)threadIdx.x - t * team_size, team_size, t + 1};
+        const int few = min(team_size, 128), few_bar = team_size > 128 ? kTeams + 2 + t : qt.bar;
+        uint8_t *const tm = mem + Lo.team + t * Lo.team_stride;
+        int *qtab = (int *)(tm + Lo.qtab), *qfirst = (int *)(tm + Lo.qfirst), *qsum = (int *)(tm + Lo.qsum),
+            *qslot = (int *)(tm + Lo.qslot), *qc = (int *)(tm + Lo.qc), *qord = (int *)(tm + Lo.qord);
+        uint64_t *qval = (uint64_t *)(tm + Lo.qval);  // sign-extended: the identity hash
+        double *xh = (double *)(tm + Lo.work), *xm = xh + chain_slots(n);
+        float2 *pl = (float2 *)(xm + chain_slots(n));
+        float *dev = (float *)(pl + n);
+        for (int j = t; j < n_evals; j += teams) {
+            const ProxyEval ev = evals[j];
+            const float neg = __fdiv_rn(0.5f, ev.abs_eb), t2 = __fadd_rn(ev.t, ev.t), eb2 = __fadd_rn(ev.abs_eb, ev.abs_eb);
+            for (uint32_t i = qt.tid; i < hcap; i += qt.size) {
+                qtab[i] = INT32_MIN;
+                qfirst[i] = INT32_MAX;
+                qsum[i] = 0;
             }
-        } else {
-            const Team qt{(int)threadIdx.x - kChainWarps * 32, (int)blockDim.x - kChainWarps * 32, 1};
-            for (int j = 0; j < ne; j++) {
-                const ProxyEval ev = evals[e0 + j];
-                const float neg = __fdiv_rn(0.5f, ev.abs_eb), t2 = __fadd_rn(ev.t, ev.t), eb2 = __fadd_rn(ev.abs_eb, ev.abs_eb);
-                for (uint32_t i = qt.tid; i < Lo.tcap; i += qt.size) {
-                    qtab[i] = INT32_MIN;
-                    qfirst[i] = INT32_MAX;
-                    qsum[i] = 0;
+            qt.sync();
+            // Distinct q values, first occurrence in map order, summed counts.
+            for (int k = qt.tid; k < m; k += qt.size) {
+                const int e = ord[k];
+                int q;
+                float dv;
+                entry_err(ekey[e], t2, b.stat_eb, neg, eb2, q, dv);
+                uint32_t slot = hash_slot((uint64_t)(uint32_t)q, hcap);
+                for (uint32_t probe = 0; probe < hcap; probe++) {
+                    int prev = atomicCAS(&qtab[slot], INT32_MIN, q);
+                    if (prev == INT32_MIN || prev == q) break;
+                    if (++slot == hcap) slot = 0;
                 }
-                qt.sync();
-                // Distinct q values, first occurrence in map order, summed counts.
-                for (int k = qt.tid; k < m; k += qt.size) {
-                    const int e = ord[k];
-                    int q;
-                    float dv;
-                    entry_err(ekey[e], t2, b.stat_eb, neg, eb2, q, dv);
-                    uint32_t slot = (uint32_t)(mix64((uint64_t)(uint32_t)q) & (Lo.tcap - 1));
-                    for (uint32_t probe = 0; probe < Lo.tcap; probe++) {
-                        int prev = atomicCAS(&qtab[slot], INT32_MIN, q);
-                        if (prev == INT32_MIN || prev == q) break;
-                        slot = (slot + 1) & (Lo.tcap - 1);
+                qslot[k] = (int)slot;
+                atomicMin(&qfirst[slot], k);
+                atomicAdd(&qsum[slot], ecnt[e]);
+            }
+            qt.sync();
+            int mq;
+            {
+                const int per = (m + qt.size - 1) / qt.size, beg = qt.tid * per, end = min(beg + per, m);
+                int local = 0;
+                for (int k = beg; k < end; k++) local += qfirst[qslot[k]] == k;
+                int off = team_excl_scan(qt, local, warp_sums[t], &mq);
+                for (int k = beg; k < end; k++)
+                    if (qfirst[qslot[k]] == k) {
+                        qval[off] = (uint64_t)(int64_t)qtab[qslot[k]];
+                        qc[off] = qsum[qslot[k]];
+                        off++;
                     }
-                    qslot[k] = (int)slot;
-                    atomicMin(&qfirst[slot], k);
-                    atomicAdd(&qsum[slot], ecnt[e]);
-                }
-                qt.sync();
-                {
-                    const int per = (m + qt.size - 1) / qt.size, beg = qt.tid * per, end = min(beg + per, m);
-                    int local = 0;
-                    for (int k = beg; k < end; k++) local += qfirst[qslot[k]] == k;
-                    int tot;
-                    int off = team_excl_scan(qt, local, warp_sums[1], &tot);
-                    for (int k = beg; k < end; k++)
-                        if (qfirst[qslot[k]] == k) {
-                            qval[off] = qtab[qslot[k]];
-                            qc[off] = qsum[qslot[k]];
-                            off++;
-                        }
-                    if (qt.tid == 0) mq_sh = tot;
-                }
-                qt.sync();
-                const int mq = mq_sh;
-                auto qcode = [&](int e) { return (uint64_t)(int64_t)qval[e]; };
-                map_order(qt, mq, qcode, tim, pos, ebk, nxt, ctm, bsz, hed, arr, qord, warp_sums[1]);
+            }
+            qt.sync();
+            map_order(qt, few, few_bar, mq, qval, Lo.order_at(tm + Lo.work), qord, warp_sums[t]);
+            // The terms of both sums in their order (the stages' arrays are free now).
+            for (int k = qt.tid; k < m; k += qt.size) {
+                const int e = ord[k];
+                int q;
+                float dv;
+                entry_err(ekey[e], t2, b.stat_eb, neg, eb2, q, dv);
+                dev[k] = dv;
+                xm[chain_slot(k)] = __dmul_rn((double)ecnt[e], __dmul_rn((double)dv, (double)dv));
+            }
+            for (int k = qt.tid; k < mq; k += qt.size) {
+                const int cnt = qc[qord[k]];
+                const float2 v = make_float2(__fmul_rn(__ull2float_rn((uint64_t)cnt), rn), log2tab[cnt]);
+                pl[k] = v;
+                xh[chain_slot(k)] = __dmul_rn(-(double)v.x, (double)v.y);
+            }
+            qt.sync();
+            const int w = qt.tid >> 5;
+            if (w == 0) {
                 // h1 chain (get_h_psnr.tpp:23-28).
-                if (qt.tid == 0) {
-                    float h1 = 0.0f;
-                    for (int k = 0; k < mq; k++) {
-                        int cnt = qc[qord[k]];
-                        float pr = __fmul_rn(__ull2float_rn((uint64_t)cnt), rn);
-                        h1 = __fmaf_rn(-pr, log2tab[cnt], h1);
-                    }
-                    h1_sh[j] = h1;
-                }
-                qt.sync();
+                const float h1 = warp_chain(xh, mq, [&](float s, int k) { return __fmaf_rn(-pl[k].x, pl[k].y, s); });
+                if (qt.tid == 0) h1_out[j] = h1;
+            } else if (w == 1) {
+                // mse chain (get_h_psnr.tpp:12-22) in map order.
+                const float mse = warp_chain(xm, m, [&](float s, int k) {
+                    const double dd = (double)dev[k];
+                    return __double2float_rn(__fma_rn((double)ecnt[ord[k]], __dmul_rn(dd, dd), (double)s));
+                });
+                if (qt.tid == 32) x_out[j] = __fmul_rn(__fdiv_rn(R2, mse), nf);
             }
+            qt.sync();
         }
-        all.sync();
-        if ((int)threadIdx.x < ne) {
-            h1_out[e0 + threadIdx.x] = h1_sh[threadIdx.x];
-            x_out[e0 + threadIdx.x] = __fmul_rn(__fdiv_rn(R2, mse_sh[threadIdx.x]), nf);
-        }
-        all.sync();
     }
+    all.sync();
     return true;
 }
 
@@ -415,8 +511,8 @@ __device__ void exact_one(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, 
                           const float *__restrict__ rec, const float *__restrict__ orig, const float *__restrict__ log2arena,
                           float R2, float t_default, float *__restrict__ tval, int64_t *__restrict__ t_int, uint32_t *fb_count,
                           AmbiguousRecord *amb, uint32_t amb_cap, uint32_t *amb_count, const uint32_t *__restrict__ overrides,
-                          uint32_t n_overrides, float *__restrict__ proxies, uint64_t g, uint8_t *smem, uint32_t cap,
-                          float *h1v, float *xv, uint32_t &m_sh, const Spill &spill) {
+                          uint32_t n_overrides, float *__restrict__ proxies, uint64_t g, uint8_t *smem,
+                          const Layout &Lo, float *h1v, float *xv, uint32_t &m_sh, const Spill &spill) {
     const uint64_t nblocks = fg.block_num[0] * fg.block_num[1] * fg.block_num[2];
     const float cand[5] = {1.0f / 16, 1.0f / 4, 9.0f / 32, 5.0f / 16, 11.0f / 32};
     if (g >= nblocks) return;
@@ -443,12 +539,15 @@ __device__ void exact_one(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, 
     eg.box.neg_2_stat_eb = rg.neg_2_stat_eb;
     eg.box.stat_eb = rg.stat_eb;
     eg.n = ci.n;
-    ProxyEval ev[5];
-    for (int c = 0; c < 5; c++) ev[c] = ProxyEval{cand[c], rg.eb};
+    __shared__ ProxyEval ev[5];
+    __shared__ Band band[5];
+    if (threadIdx.x < 5) ev[threadIdx.x] = ProxyEval{cand[threadIdx.x], rg.eb};
     if (threadIdx.x == 0) m_sh = 0;
     __syncthreads();
-    bool ok = exact_eval(eg, rec, orig, fg.n[1] * fg.n[2], fg.n[2], ev, 5, R2, log2arena + ci.log2_off, smem, cap, h1v,
+    bool ok = exact_eval(eg, rec, orig, fg.n[1] * fg.n[2], fg.n[2], ev, 5, R2, log2arena + ci.log2_off, smem, Lo, h1v,
                          xv, &m_sh);
+    __syncthreads();
+    if (ok && threadIdx.x < 5) band[threadIdx.x] = psnr_band(xv[threadIdx.x]);
     __syncthreads();
     if (!ok) {
         if (threadIdx.x == 0) spill(g);
@@ -479,7 +578,7 @@ __device__ void exact_one(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, 
                 if (__float_as_uint(xv[c]) == __float_as_uint(xv[best]) && isfinite(xv[c]) && xv[c] > 0.0f) {
                     accept = __fmaf_rn(d_h1, rg.slope, 0.0f) > 0.0f;
                 } else {
-                    Band pc = psnr_band(xv[c]), pb = psnr_band(xv[best]);
+                    const Band pc = band[c], pb = band[best];
                     float s_mid = __fmaf_rn(d_h1, rg.slope, __fsub_rn(pc.mid, pb.mid));
                     float s_lo = __fmaf_rn(d_h1, rg.slope, __fsub_rn(pc.lo, pb.hi));
                     float s_hi = __fmaf_rn(d_h1, rg.slope, __fsub_rn(pc.hi, pb.lo));
@@ -515,14 +614,14 @@ struct ListSpill {
     __device__ void operator()(uint64_t g) const { list[atomicAdd(count, 1u)] = (uint32_t)g; }
 };
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     tsel_exact_kernel(FieldGeom fg, RoundGeom rg, uint32_t l, const ClassInfo *__restrict__ classes,
                       const float *__restrict__ rec, const float *__restrict__ orig, const float *__restrict__ log2arena,
                       float R2, float t_default, float *__restrict__ tval, int64_t *__restrict__ t_int,
                       uint32_t *__restrict__ fb_count, AmbiguousRecord *amb, uint32_t amb_cap, uint32_t *amb_count,
                       const uint32_t *__restrict__ overrides, uint32_t n_overrides, float *__restrict__ proxies,
                       const uint32_t *__restrict__ list, const uint32_t *__restrict__ list_count, uint32_t *spill,
-                      uint32_t *spill_count, uint32_t smem_bytes, uint32_t cap) {
+                      uint32_t *spill_count, const __grid_constant__ Layout Lo) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t items = *list_count;
     __shared__ float h1v[kMaxEvals], xv[kMaxEvals];
@@ -530,7 +629,7 @@ __global__ void __launch_bounds__(kThreads)
     const ListSpill sp{spill, spill_count};
     for (uint32_t it = blockIdx.x; it < items; it += gridDim.x)
         exact_one(fg, rg, l, classes, rec, orig, log2arena, R2, t_default, tval, t_int, fb_count, amb, amb_cap, amb_count,
-                  overrides, n_overrides, proxies, list[it], smem, cap, h1v, xv, m_sh, sp);
+                  overrides, n_overrides, proxies, list[it], smem, Lo, h1v, xv, m_sh, sp);
 }
 
 // Batched form: the (field << 32 | group) entries that the batched fast path handed off, for all
@@ -542,10 +641,10 @@ struct PairSpill {
     __device__ void operator()(uint64_t g) const { list[atomicAdd(count, 1u)] = ((unsigned long long)f << 32) | g; }
 };
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     tsel_exact_batch_kernel(const BatchField *__restrict__ F, uint32_t l, const float *__restrict__ log2arena,
                             float t_default, const unsigned long long *__restrict__ list, const uint32_t *__restrict__ list_count,
-                            unsigned long long *spill, uint32_t *spill_count, uint32_t cap) {
+                            unsigned long long *spill, uint32_t *spill_count, const __grid_constant__ Layout Lo) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t items = *list_count;
     __shared__ float h1v[kMaxEvals], xv[kMaxEvals];
@@ -558,18 +657,18 @@ __global__ void __launch_bounds__(kThreads)
         const PairSpill sp{spill, spill_count, f};
         exact_one(B.fg, B.rounds[l], l, B.classes + 27 * l, B.rec, B.in, log2arena, B.R2, t_default, B.tval, B.tint, &B.cnt->fb,
                   B.amb, B.amb_cap, &B.cnt->amb_count, nullptr, 0, B.proxies ? B.proxies + nb * l * 10 : nullptr,
-                  e & 0xffffffffull, smem, cap, h1v, xv, m_sh, sp);
+                  e & 0xffffffffull, smem, Lo, h1v, xv, m_sh, sp);
     }
 }
 
 // Batched form of tsel_exact_global_kernel: the entries the batched exact kernel spilled (groups
 // above its shared-memory capacity), a CTA per group in its slice of global scratch; what this
 // cannot take (keys outside int32) goes on to `spill` for the serial kernel.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     tsel_exact_global_batch_kernel(const BatchField *__restrict__ F, uint32_t l, const float *__restrict__ log2arena,
                                    float t_default, const unsigned long long *__restrict__ list,
                                    const uint32_t *__restrict__ list_count, unsigned long long *spill, uint32_t *spill_count,
-                                   uint8_t *scratch, uint64_t stride, uint32_t cap) {
+                                   uint8_t *scratch, uint64_t stride, const __grid_constant__ Layout Lo) {
     uint8_t *mine = scratch + blockIdx.x * stride;
     const uint32_t items = *list_count;
     __shared__ float h1v[kMaxEvals], xv[kMaxEvals];
@@ -582,27 +681,28 @@ __global__ void __launch_bounds__(kThreads)
         const PairSpill sp{spill, spill_count, f};
         exact_one(B.fg, B.rounds[l], l, B.classes + 27 * l, B.rec, B.in, log2arena, B.R2, t_default, B.tval, B.tint, &B.cnt->fb,
                   B.amb, B.amb_cap, &B.cnt->amb_count, nullptr, 0, B.proxies ? B.proxies + nb * l * 10 : nullptr,
-                  e & 0xffffffffull, mine, cap, h1v, xv, m_sh, sp);
+                  e & 0xffffffffull, mine, Lo, h1v, xv, m_sh, sp);
     }
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     slope_exact_kernel(const SampleBox *__restrict__ boxes, const ProxyEval *__restrict__ evals, uint32_t n_evals,
                        const float *__restrict__ orig, uint64_t n1n2, uint64_t n2, const float *__restrict__ log2arena,
                        float R2, float *__restrict__ h1_out, float *__restrict__ x_out, uint32_t *__restrict__ m_out,
-                       uint32_t *__restrict__ err_word, uint32_t smem_bytes, uint32_t cap) {
+                       uint32_t *__restrict__ err_word, const __grid_constant__ Layout Lo) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ float h1v[kMaxEvals], xv[kMaxEvals];
-    // Box blockIdx.x, evaluations [5 * blockIdx.y, 5 * blockIdx.y + 5): exact_eval runs five
-    // evaluations side by side, so each CTA rebuilds the box's map and runs one batch of them.
-    const uint32_t g = blockIdx.x, e0 = 5 * blockIdx.y;
+    // Box blockIdx.x, evaluations [kTeams * blockIdx.y, + kTeams): each CTA rebuilds the box's map
+    // and runs one batch of evaluations side by side.
+    const uint32_t g = blockIdx.x, e0 = kTeams * blockIdx.y;
     if (e0 >= n_evals) return;
-    const uint32_t ne = min(5u, n_evals - e0);
+    const uint32_t ne = min((uint32_t)kTeams, n_evals - e0);
     ExactGroup eg;
     eg.box = boxes[g];
     eg.n = eg.box.n;
     uint32_t m = 0;
-    bool ok = exact_eval(eg, orig, orig, n1n2, n2, evals + e0, (int)ne, R2, log2arena + eg.box.log2_off, smem, cap, h1v, xv, &m);
+    bool ok = exact_eval(eg, orig, orig, n1n2, n2, evals + e0, (int)ne, R2, log2arena + eg.box.log2_off, smem, Lo,
+                         h1v, xv, &m);
     __syncthreads();
     if (!ok) {
         if (threadIdx.x == 0) atomicOr(err_word, 2u);
@@ -619,7 +719,7 @@ __global__ void __launch_bounds__(kThreads)
 // slice of a global scratch arena (stride bytes, L2-resident) instead of shared memory, so a group
 // of up to `cap` samples is still replayed by a whole CTA rather than by one thread. Groups it
 // cannot take (more samples than cap, keys outside int32) go to `spill` for the serial kernel.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     tsel_exact_global_kernel(FieldGeom fg, RoundGeom rg, uint32_t l, const ClassInfo *__restrict__ classes,
                              const float *__restrict__ rec, const float *__restrict__ orig,
                              const float *__restrict__ log2arena, float R2, float t_default, float *__restrict__ tval,
@@ -627,7 +727,7 @@ __global__ void __launch_bounds__(kThreads)
                              uint32_t amb_cap, uint32_t *amb_count, const uint32_t *__restrict__ overrides,
                              uint32_t n_overrides, float *__restrict__ proxies, const uint32_t *__restrict__ list,
                              const uint32_t *__restrict__ list_count, uint32_t *spill, uint32_t *spill_count,
-                             uint8_t *scratch, uint64_t stride, uint32_t cap) {
+                             uint8_t *scratch, uint64_t stride, const __grid_constant__ Layout Lo) {
     uint8_t *mine = scratch + blockIdx.x * stride;
     const uint32_t items = *list_count;
     __shared__ float h1v[kMaxEvals], xv[kMaxEvals];
@@ -635,36 +735,57 @@ __global__ void __launch_bounds__(kThreads)
     const ListSpill sp{spill, spill_count};
     for (uint32_t it = blockIdx.x; it < items; it += gridDim.x)
         exact_one(fg, rg, l, classes, rec, orig, log2arena, R2, t_default, tval, t_int, fb_count, amb, amb_cap, amb_count,
-                  overrides, n_overrides, proxies, list[it], mine, cap, h1v, xv, m_sh, sp);
+                  overrides, n_overrides, proxies, list[it], mine, Lo, h1v, xv, m_sh, sp);
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 1)
     slope_exact_global_kernel(const SampleBox *__restrict__ boxes, const ProxyEval *__restrict__ evals, uint32_t n_evals,
                               const float *__restrict__ orig, uint64_t n1n2, uint64_t n2,
                               const float *__restrict__ log2arena, float R2, float *__restrict__ h1_out,
                               float *__restrict__ x_out, uint32_t *__restrict__ m_out, uint32_t *__restrict__ err_word,
-                              uint8_t *scratch, uint64_t stride, uint32_t cap) {
+                              uint8_t *scratch, uint64_t stride, const __grid_constant__ Layout Lo) {
     __shared__ float h1v[kMaxEvals], xv[kMaxEvals];
-    const uint32_t g = blockIdx.x;
+    const uint32_t g = blockIdx.x, e0 = kTeams * blockIdx.y;  // as slope_exact_kernel
+    if (e0 >= n_evals) return;
+    const uint32_t ne = min((uint32_t)kTeams, n_evals - e0);
     ExactGroup eg;
     eg.box = boxes[g];
     eg.n = eg.box.n;
-    bool ok = exact_eval(eg, orig, orig, n1n2, n2, evals, (int)n_evals, R2, log2arena + eg.box.log2_off,
-                         scratch + g * stride, cap, h1v, xv, m_out + g);
+    uint32_t m = 0;
+    bool ok = exact_eval(eg, orig, orig, n1n2, n2, evals + e0, (int)ne, R2, log2arena + eg.box.log2_off,
+                         scratch + (blockIdx.y * gridDim.x + g) * stride, Lo, h1v, xv, &m);
     __syncthreads();
     if (!ok) {
         if (threadIdx.x == 0) atomicOr(err_word, 2u);
         return;
     }
-    for (uint32_t e = threadIdx.x; e < n_evals; e += blockDim.x) {
-        h1_out[g * n_evals + e] = h1v[e];
-        x_out[g * n_evals + e] = xv[e];
+    if (threadIdx.x == 0 && blockIdx.y == 0) m_out[g] = m;
+    for (uint32_t e = threadIdx.x; e < ne; e += blockDim.x) {
+        h1_out[g * n_evals + e0 + e] = h1v[e];
+        x_out[g * n_evals + e0 + e] = xv[e];
     }
 }
 
-// Shared-memory bytes the exact kernels need for groups of up to `cap` samples (also the size of
-// a global-scratch slice).
-uint32_t exact_smem_bytes(uint32_t cap) { return Layout(cap).total; }
+// Working-set bytes of groups of up to n samples: with one evaluation at a time (what a kernel
+// needs at least), and with as many side by side as are worth having.
+uint32_t exact_smem_bytes(uint32_t n) { return Layout(n, 1).total; }
+uint32_t exact_full_bytes(uint32_t n) { return Layout(n, kTeams).total; }
+uint32_t slope_batches(uint32_t n_evals) { return (n_evals + kTeams - 1) / kTeams; }
+
+namespace {
+
+// Shared memory of a launch whose largest group has `most` samples and whose kernel takes groups of
+// up to `cap`: the side-by-side tables where they fit.
+cudaError_t exact_shared(const void *kernel, uint32_t cap, uint32_t most, Layout &lo) {
+    int dev = 0, lim = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    lo = exact_layout(most < cap ? most : cap, (uint32_t)lim - kExactStatic);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lo.total);
+}
+
+}  // namespace
 
 cudaError_t launch_tsel_exact_global(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, const ClassInfo *classes,
                                      const float *rec, const float *orig, const float *log2arena, float R2, float t_default,
@@ -675,7 +796,8 @@ cudaError_t launch_tsel_exact_global(const FieldGeom &fg, const RoundGeom &rg, u
     if (grid == 0) return cudaSuccess;
     tsel_exact_global_kernel<<<grid, kThreads, 0, st>>>(fg, rg, l, classes, rec, orig, log2arena, R2, t_default, tval, t_int,
                                                         fb_count, amb, amb_cap, amb_count, overrides, n_overrides, proxies,
-                                                        list, list_count, spill, spill_count, scratch, stride, cap);
+                                                        list, list_count, spill, spill_count, scratch, stride,
+                                                        exact_layout(cap, stride));
     count_launch();
     return cudaGetLastError();
 }
@@ -685,8 +807,8 @@ cudaError_t launch_slope_exact_global(const SampleBox *boxes, const ProxyEval *e
                                       uint32_t *m_out, uint32_t *err, uint8_t *scratch, uint64_t stride, uint32_t cap,
                                       uint32_t nboxes, cudaStream_t st) {
     if (nboxes == 0) return cudaSuccess;
-    slope_exact_global_kernel<<<nboxes, kThreads, 0, st>>>(boxes, evals, n_evals, orig, n1n2, n2, log2arena, R2, h1, x, m_out,
-                                                           err, scratch, stride, cap);
+    slope_exact_global_kernel<<<dim3(nboxes, slope_batches(n_evals)), kThreads, 0, st>>>(boxes, evals, n_evals, orig, n1n2, n2, log2arena, R2, h1, x, m_out,
+                                                           err, scratch, stride, exact_layout(cap, stride));
     count_launch();
     return cudaGetLastError();
 }
@@ -696,13 +818,13 @@ cudaError_t launch_tsel_exact(const FieldGeom &fg, const RoundGeom &rg, uint32_t
                               int64_t *t_int, uint32_t *fb_count, AmbiguousRecord *amb, uint32_t amb_cap,
                               uint32_t *amb_count, const uint32_t *overrides, uint32_t n_overrides, float *proxies,
                               const uint32_t *list, const uint32_t *list_count, uint32_t *spill, uint32_t *spill_count,
-                              uint32_t cap, unsigned grid, cudaStream_t st) {
-    uint32_t smem = exact_smem_bytes(cap);
-    cudaError_t e = cudaFuncSetAttribute(tsel_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                              uint32_t cap, uint32_t most, unsigned grid, cudaStream_t st) {
+    Layout lo(1, 1);
+    cudaError_t e = exact_shared((const void *)tsel_exact_kernel, cap, most, lo);
     if (e != cudaSuccess) return e;
-    tsel_exact_kernel<<<grid, kThreads, smem, st>>>(fg, rg, l, classes, rec, orig, log2arena, R2, t_default, tval, t_int,
+    tsel_exact_kernel<<<grid, kThreads, lo.total, st>>>(fg, rg, l, classes, rec, orig, log2arena, R2, t_default, tval, t_int,
                                                      fb_count, amb, amb_cap, amb_count, overrides, n_overrides, proxies, list,
-                                                     list_count, spill, spill_count, smem, cap);
+                                                     list_count, spill, spill_count, lo);
     count_launch();
     return cudaGetLastError();
 }
@@ -713,32 +835,33 @@ cudaError_t launch_tsel_exact_global_batch(const BatchField *F, uint32_t l, cons
                                            uint32_t cap, unsigned grid, cudaStream_t st) {
     if (grid == 0) return cudaSuccess;
     tsel_exact_global_batch_kernel<<<grid, kThreads, 0, st>>>(F, l, log2arena, t_default, list, list_count, spill, spill_count,
-                                                              scratch, stride, cap);
+                                                              scratch, stride, exact_layout(cap, stride));
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_tsel_exact_batch(const BatchField *F, uint32_t l, const float *log2arena, float t_default,
                                     const unsigned long long *list, const uint32_t *list_count, unsigned long long *spill,
-                                    uint32_t *spill_count, uint32_t cap, unsigned grid, cudaStream_t st) {
-    uint32_t smem = exact_smem_bytes(cap);
-    cudaError_t e = cudaFuncSetAttribute(tsel_exact_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                    uint32_t *spill_count, uint32_t cap, uint32_t most, unsigned grid, cudaStream_t st) {
+    Layout lo(1, 1);
+    cudaError_t e = exact_shared((const void *)tsel_exact_batch_kernel, cap, most, lo);
     if (e != cudaSuccess) return e;
-    tsel_exact_batch_kernel<<<grid, kThreads, smem, st>>>(F, l, log2arena, t_default, list, list_count, spill, spill_count, cap);
+    tsel_exact_batch_kernel<<<grid, kThreads, lo.total, st>>>(F, l, log2arena, t_default, list, list_count, spill, spill_count, lo);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_slope_exact(const SampleBox *boxes, const ProxyEval *evals, uint32_t n_evals, const float *orig,
                                uint64_t n1n2, uint64_t n2, const float *log2arena, float R2, float *h1, float *x,
-                               uint32_t *m_out, uint32_t *err, uint32_t cap, uint32_t nboxes, cudaStream_t st) {
+                               uint32_t *m_out, uint32_t *err, uint32_t cap, uint32_t most, uint32_t nboxes,
+                               cudaStream_t st) {
     if (nboxes == 0) return cudaSuccess;
-    uint32_t smem = exact_smem_bytes(cap);
-    cudaError_t e = cudaFuncSetAttribute(slope_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    Layout lo(1, 1);
+    cudaError_t e = exact_shared((const void *)slope_exact_kernel, cap, most, lo);
     if (e != cudaSuccess) return e;
-    const dim3 grid(nboxes, (n_evals + 4) / 5);
-    slope_exact_kernel<<<grid, kThreads, smem, st>>>(boxes, evals, n_evals, orig, n1n2, n2, log2arena, R2, h1, x, m_out, err,
-                                                  smem, cap);
+    const dim3 grid(nboxes, slope_batches(n_evals));
+    slope_exact_kernel<<<grid, kThreads, lo.total, st>>>(boxes, evals, n_evals, orig, n1n2, n2, log2arena, R2, h1, x, m_out, err,
+                                                      lo);
     count_launch();
     return cudaGetLastError();
 }

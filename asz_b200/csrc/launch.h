@@ -64,7 +64,7 @@ cudaError_t launch_tsel_fast_batch(const BatchField *F, const uint64_t *goff, ui
                                    uint32_t grid, cudaStream_t st);
 cudaError_t launch_tsel_exact_batch(const BatchField *F, uint32_t l, const float *log2arena, float t_default,
                                     const unsigned long long *list, const uint32_t *list_count, unsigned long long *spill,
-                                    uint32_t *spill_count, uint32_t cap, unsigned grid, cudaStream_t st);
+                                    uint32_t *spill_count, uint32_t cap, uint32_t most, unsigned grid, cudaStream_t st);
 // Groups the batched exact kernel spilled (above its shared-memory capacity), a CTA each in a
 // `stride`-byte slice of global scratch; what it cannot take goes to `spill`.
 cudaError_t launch_tsel_exact_global_batch(const BatchField *F, uint32_t l, const float *log2arena, float t_default,
@@ -141,15 +141,24 @@ cudaError_t launch_tsel_fast(const FieldGeom &fg, const RoundGeom &rg, uint32_t 
                              int64_t *t_int, uint32_t *fb_count, uint32_t *list_out, uint32_t *list_count,
                              const uint32_t *overrides, uint32_t n_overrides, uint32_t *why, cudaStream_t st,
                              uint32_t common_samples);
-uint32_t exact_smem_bytes(uint32_t cap);
+// Working set of an exact replay of up to n samples, one evaluation at a time or all side by side
+// (the latter only below kExactFullMost samples), what the kernels need beside it in shared memory,
+// and the CTAs a box that n_evals evaluations take.
+constexpr uint32_t kExactFullMost = 1u << 20;
+constexpr uint32_t kExactStatic = 2048;
+uint32_t exact_smem_bytes(uint32_t n);
+uint32_t exact_full_bytes(uint32_t n);
+uint32_t slope_batches(uint32_t n_evals);
+// cap: the largest group the launch takes (the others are spilled); most: the largest it can meet.
 cudaError_t launch_tsel_exact(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, const ClassInfo *classes, const float *rec,
                               const float *orig, const float *log2arena, float R2, float t_default, float *tval,
                               int64_t *t_int, uint32_t *fb_count, AmbiguousRecord *amb, uint32_t amb_cap,
                               uint32_t *amb_count, const uint32_t *overrides, uint32_t n_overrides, float *proxies,
                               const uint32_t *list, const uint32_t *list_count, uint32_t *spill, uint32_t *spill_count,
-                              uint32_t cap, unsigned grid, cudaStream_t st);
+                              uint32_t cap, uint32_t most, unsigned grid, cudaStream_t st);
 // The exact replay with each CTA's working set in a slice of `scratch` (stride bytes, at least
-// exact_smem_bytes(cap)) instead of shared memory, for groups of up to cap samples.
+// exact_smem_bytes(cap)) instead of shared memory, for groups of up to cap samples. The slope form
+// takes nboxes * slope_batches(n_evals) slices.
 cudaError_t launch_tsel_exact_global(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, const ClassInfo *classes,
                                      const float *rec, const float *orig, const float *log2arena, float R2, float t_default,
                                      float *tval, int64_t *t_int, uint32_t *fb_count, AmbiguousRecord *amb, uint32_t amb_cap,
@@ -171,7 +180,7 @@ cudaError_t launch_plan_sample(const float *d, uint64_t n1, uint64_t n2, const P
 cudaError_t launch_plan_mse(const PlanCand *cands, uint32_t ncands, const float *e, float *mse, cudaStream_t st);
 cudaError_t launch_slope_exact(const SampleBox *boxes, const ProxyEval *evals, uint32_t n_evals, const float *orig,
                                uint64_t n1n2, uint64_t n2, const float *log2arena, float R2, float *h1, float *x,
-                               uint32_t *m_out, uint32_t *err, uint32_t cap, uint32_t nboxes, cudaStream_t st);
+                               uint32_t *m_out, uint32_t *err, uint32_t cap, uint32_t most, uint32_t nboxes, cudaStream_t st);
 cudaError_t launch_slope_v0(const FieldGeom &fg, const SampleBox *boxes, const ProxyEval *evals, uint32_t n_evals,
                             const float *orig, const float *log2arena, float R2, uint8_t *scratch, uint64_t scratch_stride,
                             uint32_t cap, uint32_t bcap, uint32_t tcap, float *h1, float *x, uint32_t *m_out, uint32_t *err,

@@ -40,6 +40,18 @@ ASZ_HD uint64_t sched_bkt(int i) {
 #endif
 }
 
+#ifdef __CUDACC__
+// floor((2^64 - 1) / buckets) of each stage, to reduce a hash without a division.
+struct SchedMagic {
+    uint64_t v[kSchedLen];
+    constexpr SchedMagic() : v{} {
+        for (int i = 0; i < kSchedLen; i++) v[i] = ~0ull / kSchedBkt[i];
+    }
+};
+static __constant__ SchedMagic d_sched_magic = SchedMagic();
+__device__ __forceinline__ uint64_t sched_magic(int i) { return d_sched_magic.v[i]; }
+#endif
+
 // Bucket count in use after `m` insertions.
 ASZ_HD uint64_t sched_buckets(uint64_t m) {
     uint64_t b = 1;
