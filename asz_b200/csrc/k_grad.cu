@@ -22,7 +22,8 @@
 // triangle kernel gives dH/dq_s = (h'(p_{k0+1}) - h'(p_{k0})) / n with k0 = floor(q_s) and
 // h'(p) = -(log2(p + 1e-6) + p / ((p + 1e-6) ln 2)).
 //
-// One CTA per group, its soft histogram (513 bins) in shared memory; sums in double.
+// A warp per group in the forward and backward kernels (a CTA for the largest groups and in the
+// tuner), its soft histogram (513 bins) in shared memory; sums in double.
 #include <cuda_runtime.h>
 
 #include "dev_common.cuh"
@@ -67,12 +68,15 @@ constexpr int kTeamWarps = kMaxTeam / 32;
 constexpr int kJudgeBins = 2048;              // judge window (quantised-error values)
 constexpr uint32_t kMaxJudgeWindows = 128;    // beyond 128 * 2048 bins the judge keeps the default
 
-struct TeamShared {
+struct PassShared {
     float hist[kBins];   // soft histogram
     float hp[kBins];     // h'(p) per bin
-    uint32_t counts[2][kJudgeBins];  // judge: one window of quantised-error counts per candidate
     double red[kTeamWarps][4];
     int imn[kTeamWarps], imx[kTeamWarps];
+};
+
+struct TeamShared : PassShared {
+    uint32_t counts[2][kJudgeBins];  // judge: one window of quantised-error counts per candidate
     long long lmn[kTeamWarps], lmx[kTeamWarps];
 };
 
@@ -90,7 +94,7 @@ __device__ void team_sum4(TeamShared &sh, double (&v)[4]) {
     __syncthreads();
 }
 
-__device__ void team_sum3(TeamShared &sh, double &a, double &b, double &c) {
+__device__ void team_sum3(PassShared &sh, double &a, double &b, double &c) {
     for (int o = 16; o; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
         b += __shfl_xor_sync(0xffffffffu, b, o);
@@ -134,7 +138,7 @@ __device__ void team_minmax(T (&mn)[kTeamWarps], T (&mx)[kTeamWarps], T &lo, T &
 
 // Soft histogram of the group's samples at t and the sums. keep: leave the histogram for
 // group_grad (which clears it); otherwise it is cleared here.
-__device__ Sums group_pass(TeamShared &sh, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
+__device__ Sums group_pass(PassShared &sh, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
                            const Meta &mt, float t, bool keep) {
     const float inv2eb = 0.5f / mt.eb;
     double m = 0.0, ra = 0.0, H = 0.0;
@@ -171,9 +175,16 @@ __device__ __forceinline__ double objective(const Sums &S, const Meta &mt, float
     return (double)mt.slope * S.H - 10.0 * log10((double)R2 / mse);
 }
 
+// dJ/dt from the sums and the samples' sum of dH/dq dq/dt.
+__device__ __forceinline__ double gradient(const Sums &S, double gh, uint32_t n, const Meta &mt) {
+    const double c = (double)mt.eb * mt.eb / 3.0;
+    const double dlog = S.m > 0.0 ? c / (S.m * (S.m + c)) : 0.0;
+    return (double)mt.slope * (gh / n) + kTenOverLn10 * dlog * 2.0 * S.ra;
+}
+
 // dJ/dt after group_pass(keep) at the same t, from the h' values it left (the barriers of its
 // final reduction made them visible).
-__device__ double group_grad(TeamShared &sh, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
+__device__ double group_grad(PassShared &sh, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
                              const Meta &mt, float t, const Sums &S) {
     const float inv2eb = 0.5f / mt.eb;
     double gh = 0.0, u0 = 0.0, u1 = 0.0;
@@ -186,10 +197,7 @@ __device__ double group_grad(TeamShared &sh, const float *__restrict__ A, const 
         if (!cl) gh += (double)(sh.hp[k0 + 1] - sh.hp[k0]) * (double)(a * inv2eb);
     }
     team_sum3(sh, gh, u0, u1);  // its barriers end the reads of h'
-    gh /= n;
-    const double c = (double)mt.eb * mt.eb / 3.0;
-    const double dlog = S.m > 0.0 ? c / (S.m * (S.m + c)) : 0.0;
-    return (double)mt.slope * gh + kTenOverLn10 * dlog * 2.0 * S.ra;
+    return gradient(S, gh, n, mt);
 }
 
 __device__ __forceinline__ Meta load_meta(const float4 *meta, uint64_t g) {
@@ -205,40 +213,138 @@ __device__ __forceinline__ void team_clear(TeamShared &sh) {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kMaxTeam)
-    forward_kernel(const float *__restrict__ A, const float *__restrict__ B, const uint32_t *__restrict__ off,
-                   const float4 *__restrict__ meta, float R2, const float *__restrict__ t, uint64_t groups,
-                   float *__restrict__ J) {
-    __shared__ TeamShared sh;
-    team_clear(sh);
-    for (uint64_t g = blockIdx.x; g < groups; g += gridDim.x) {
-        const uint32_t o = off[g], n = off[g + 1] - o;
-        if (n == 0) {
-            if (threadIdx.x == 0) J[g] = 0.0f;
-            continue;
+// J (kGrad false) or dJ/dt times its incoming gradient (true) of every group, a warp per group.
+//
+// A group is 3 to 1600 samples in the plans met in use: a CTA of 256 threads spent its time at the
+// barriers between its passes, ten groups one after another, and on float atomics in shared memory,
+// which are compare-and-swap loops (256^3 field, 12k groups, 38 MB of samples: 100 us forward, 122
+// backward). A warp per group needs no barrier and has 40 groups an SM under way; the histogram is
+// in fixed point, whose atomics are single instructions, with the scale that n samples of weight 1
+// just fit 32 bits in (at least 2^20, finer than a float's ulp once a bin holds 16 samples), so its
+// sums are exact in any order: 29 us forward, 43 backward, the same without the atomics or the double
+// sums, so what is left is the latency of a group's chain of loads; sixteen in flight a lane and five
+// CTAs an SM were the best of 8 and 16 loads, 4 to 8 CTAs (37 and 55 us with eight loads). Above
+// kWarpMost samples a group is a CTA's.
+constexpr uint32_t kWarpMost = 4095;
+constexpr int kProxyThreads = 256;
+constexpr int kInFlight = 8;  // samples a lane loads ahead (two words each)
+
+template <bool kGrad>
+__device__ double warp_proxy(uint32_t *hist, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
+                             const Meta &mt, float t, float R2) {
+    const int lane = threadIdx.x & 31;
+    const float inv2eb = 0.5f / mt.eb;
+    const int frac = __clz(n);  // n < 2^(32 - frac): n 2^frac fits 32 bits
+    const float one = __uint_as_float((uint32_t)(127 + frac) << 23);
+    const uint32_t unit = 1u << frac;
+    double m = 0.0, ra = 0.0, H = 0.0;
+    int klo = kBins, khi = -1;
+    for (uint32_t s0 = lane; s0 < n; s0 += 32 * kInFlight) {
+        float a[kInFlight], b[kInFlight];
+#pragma unroll
+        for (int i = 0; i < kInFlight; i++) {
+            const uint32_t s = s0 + 32 * i;
+            a[i] = s < n ? A[s] : 0.0f;
+            b[i] = s < n ? B[s] : 0.0f;
         }
-        const Meta mt = load_meta(meta, g);
-        const Sums S = group_pass(sh, A + o, B + o, n, mt, t[g], false);
-        if (threadIdx.x == 0) J[g] = (float)objective(S, mt, R2);
+#pragma unroll
+        for (int i = 0; i < kInFlight; i++) {
+            if (s0 + 32 * i >= n) break;
+            const float r = fmaf(a[i], t, b[i]);
+            float f;
+            int k0;
+            bool cl;
+            bin_of(r, inv2eb, f, k0, cl);
+            const uint32_t w = __float2uint_rn(f * one);
+            atomicAdd(&hist[k0], unit - w);
+            atomicAdd(&hist[k0 + 1], w);
+            klo = min(klo, k0);
+            khi = max(khi, k0 + 1);
+            m = fma((double)r, (double)r, m);
+            ra = fma((double)r, (double)a[i], ra);
+        }
     }
+    klo = __reduce_min_sync(0xffffffffu, klo);
+    khi = __reduce_max_sync(0xffffffffu, khi);
+    __syncwarp();
+    const float inv_n = 1.0f / ((float)n * one);
+    for (int i = klo + lane; i <= khi; i += 32) {
+        const float p = (float)hist[i] * inv_n;
+        const float l2 = log2f(p + kEps);
+        H -= (double)p * (double)l2;
+        // h'(p) takes the bin's place until the gradient's pass
+        hist[i] = kGrad ? __float_as_uint(-(l2 + p / (p + kEps) * kInvLn2)) : 0u;
+    }
+    for (int o = 16; o; o >>= 1) {
+        m += __shfl_xor_sync(0xffffffffu, m, o);
+        ra += __shfl_xor_sync(0xffffffffu, ra, o);
+        if (!kGrad) H += __shfl_xor_sync(0xffffffffu, H, o);
+    }
+    const Sums S{m / n, ra / n, H, klo, khi};
+    __syncwarp();
+    if (!kGrad) return objective(S, mt, R2);
+    double gh = 0.0;
+    for (uint32_t s0 = lane; s0 < n; s0 += 32 * kInFlight) {
+        float a[kInFlight], b[kInFlight];
+#pragma unroll
+        for (int i = 0; i < kInFlight; i++) {
+            const uint32_t s = s0 + 32 * i;
+            a[i] = s < n ? A[s] : 0.0f;
+            b[i] = s < n ? B[s] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kInFlight; i++) {
+            if (s0 + 32 * i >= n) break;
+            float f;
+            int k0;
+            bool cl;
+            bin_of(fmaf(a[i], t, b[i]), inv2eb, f, k0, cl);
+            if (!cl)
+                gh = fma((double)(__uint_as_float(hist[k0 + 1]) - __uint_as_float(hist[k0])), (double)(a[i] * inv2eb), gh);
+        }
+    }
+    for (int o = 16; o; o >>= 1) gh += __shfl_xor_sync(0xffffffffu, gh, o);
+    __syncwarp();
+    for (int i = klo + lane; i <= khi; i += 32) hist[i] = 0u;
+    __syncwarp();
+    return gradient(S, gh, n, mt);
 }
 
-__global__ void __launch_bounds__(kMaxTeam)
-    backward_kernel(const float *__restrict__ A, const float *__restrict__ B, const uint32_t *__restrict__ off,
-                    const float4 *__restrict__ meta, float R2, const float *__restrict__ t, const float *__restrict__ gJ,
-                    uint64_t groups, float *__restrict__ gt) {
-    __shared__ TeamShared sh;
-    team_clear(sh);
+template <bool kGrad>
+__global__ void __launch_bounds__(kProxyThreads, 5)
+    proxy_kernel(const float *__restrict__ A, const float *__restrict__ B, const uint32_t *__restrict__ off,
+                 const float4 *__restrict__ meta, float R2, const float *__restrict__ t, const float *__restrict__ gJ,
+                 uint64_t groups, float *__restrict__ out) {
+    constexpr uint32_t kWarps = kProxyThreads / 32;
+    __shared__ union Both {
+        uint32_t warp[kWarps][kBins];
+        PassShared team;
+        __device__ Both() {}
+    } sh;
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = lane; i < kBins; i += 32) sh.warp[w][i] = 0u;
+    __syncwarp();
+    for (uint64_t g = blockIdx.x * (uint64_t)kWarps + w; g < groups; g += (uint64_t)gridDim.x * kWarps) {
+        const uint32_t o = off[g], n = off[g + 1] - o;
+        if (n > kWarpMost) continue;
+        double v = 0.0;
+        if (n) v = warp_proxy<kGrad>(sh.warp[w], A + o, B + o, n, load_meta(meta, g), t[g], R2);
+        if (lane == 0) out[g] = n == 0 ? 0.0f : kGrad ? (float)(v * (double)gJ[g]) : (float)v;
+    }
+    bool cleared = false;
     for (uint64_t g = blockIdx.x; g < groups; g += gridDim.x) {
         const uint32_t o = off[g], n = off[g + 1] - o;
-        if (n == 0) {
-            if (threadIdx.x == 0) gt[g] = 0.0f;
-            continue;
+        if (n <= kWarpMost) continue;
+        if (!cleared) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < kBins; i += blockDim.x) sh.team.hist[i] = 0.0f;
+            __syncthreads();
+            cleared = true;
         }
         const Meta mt = load_meta(meta, g);
-        const Sums S = group_pass(sh, A + o, B + o, n, mt, t[g], true);
-        const double d = group_grad(sh, A + o, B + o, n, mt, t[g], S);
-        if (threadIdx.x == 0) gt[g] = (float)(d * (double)gJ[g]);
+        const Sums S = group_pass(sh.team, A + o, B + o, n, mt, t[g], kGrad);
+        const double v = kGrad ? group_grad(sh.team, A + o, B + o, n, mt, t[g], S) * (double)gJ[g] : objective(S, mt, R2);
+        if (threadIdx.x == 0) out[g] = (float)v;
     }
 }
 
@@ -450,7 +556,10 @@ unsigned grid_for(uint64_t items, unsigned per_cta) {
     return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
-// Grid of the per-group kernels: one group per CTA at a time, up to 16 CTAs per SM.
+// Grid of the forward and backward kernels: a group a warp, eight CTAs an SM.
+unsigned proxy_grid(uint64_t groups) { return grid_for(groups, kProxyThreads / 32); }
+
+// Grid of the gather and the tuner: one group per CTA at a time, up to 16 CTAs per SM.
 unsigned group_grid(uint64_t groups) {
     const uint64_t cap = 148ull * 16;
     return (unsigned)(groups < 1 ? 1 : (groups > cap ? cap : groups));
@@ -474,7 +583,8 @@ extern "C" int asz_grad_forward(const float *A, const float *B, const uint32_t *
                                 const float *t, uint64_t groups, float *J, void *cuda_stream) {
     if (groups == 0) return 0;
     if (!A || !B || !offsets || !meta || !t || !J) return 1;
-    grad::forward_kernel<<<grad::group_grid(groups), grad::kTeam, 0, (cudaStream_t)cuda_stream>>>(A, B, offsets, (const float4 *)meta, R2, t, groups, J);
+    grad::proxy_kernel<false><<<grad::proxy_grid(groups), grad::kProxyThreads, 0, (cudaStream_t)cuda_stream>>>(
+        A, B, offsets, (const float4 *)meta, R2, t, nullptr, groups, J);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? 0 : 7;
 }
@@ -483,7 +593,8 @@ extern "C" int asz_grad_backward(const float *A, const float *B, const uint32_t 
                                  const float *t, const float *grad_J, uint64_t groups, float *grad_t, void *cuda_stream) {
     if (groups == 0) return 0;
     if (!A || !B || !offsets || !meta || !t || !grad_J || !grad_t) return 1;
-    grad::backward_kernel<<<grad::group_grid(groups), grad::kTeam, 0, (cudaStream_t)cuda_stream>>>(A, B, offsets, (const float4 *)meta, R2, t, grad_J, groups, grad_t);
+    grad::proxy_kernel<true><<<grad::proxy_grid(groups), grad::kProxyThreads, 0, (cudaStream_t)cuda_stream>>>(
+        A, B, offsets, (const float4 *)meta, R2, t, grad_J, groups, grad_t);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? 0 : 7;
 }
