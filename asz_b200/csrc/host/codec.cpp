@@ -265,6 +265,7 @@ struct asz_ctx {
     PinnedBuf pre_zstd;   // the last compress call's stream before zstd
     PinnedBuf batch_pre[2];  // batches: two chunks of fields' streams, one encoding while one is compressed
     PinnedBuf raw_in;     // decompress: the stream after zstd
+    PinnedBuf words;      // a few result words of a call
     bool have_last = false;
     // Profiling (asz_profile_*).
     bool prof = false;
@@ -856,6 +857,7 @@ void asz_destroy(asz_ctx *c) {
     c->batch_pre[0].release();
     c->batch_pre[1].release();
     c->raw_in.release();
+    c->words.release();
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
     asz::host::sweep_release(c->sweep);
     for (ZSTD_CCtx *z : c->zfree) ZSTD_freeCCtx(z);
@@ -896,7 +898,9 @@ struct MiscLayout {  // small device words, one allocation
     int32_t range[2];
     unsigned long long nonfinite;
     unsigned long long zfirst, zlast;
-    uint32_t err;
+    uint32_t dec_err;      // batched Huffman decoding: error bits
+    uint32_t dec_changed;  // batched Huffman decoding: a run's first chunk starts elsewhere
+    uint32_t err;          // the three words of a decompression are read together
     uint32_t fb;
     uint32_t amb_count;
     uint32_t changed;
@@ -905,8 +909,6 @@ struct MiscLayout {  // small device words, one allocation
     uint32_t spill2_count[64];  // groups the global-scratch exact kernel left to the serial one
     uint32_t all_count;
     uint32_t why[3];  // fast path: [0] handed off (bins too spread), [1] handed off (undecided), [2] settled window by window
-    uint32_t dec_err;      // batched Huffman decoding: error bits
-    uint32_t dec_changed;  // batched Huffman decoding: a chunk start moved in the last pass
     uint32_t resume_count;  // fused axis-2 compression: columns waiting for the exact path
     int32_t qb_range[2 * 64];
     uint32_t hist_over[64];  // round l: a QB of its stream fell outside the histogram window
@@ -2826,17 +2828,27 @@ struct DecodeJob {
     bool wide;
 };
 
-// Decode every stream of a .asz in one batched launch per pass (k_huff.cu). The stream bytes are
-// on the device at d_base (256-byte aligned, padded by kDecodePad). Errors of the payloads are
-// left in dm->dec_err for the caller to read with its final synchronisation.
-int gpu_decode_all(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8_t *d_base, MiscLayout *dm, cudaStream_t st) {
-    const u64 C = 1024;  // chunk bits
+// The decoding of every stream of a .asz, in batched launches (k_huff.cu).
+struct DecodeRun {
+    const uint8_t *base = nullptr;
+    const DecStream *ds = nullptr;
+    const uint32_t *ts = nullptr, *lut = nullptr, *lut2 = nullptr, *child = nullptr;
+    u64 *start = nullptr, *end = nullptr, *cnt = nullptr, *off = nullptr;
+    uint32_t *moved = nullptr;
+    uint32_t nst = 0, max_lut_bits = 1;
+    u64 ntiles = 0, nchunks = 0;
+};
+constexpr u64 kChunkBits = 1024;
+
+// Tables and descriptors to the device, and the first synchronisation pass. The stream bytes are on
+// the device at d_base (256-byte aligned, padded by kDecodePad).
+int decode_begin(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8_t *d_base, MiscLayout *dm, cudaStream_t st,
+                 DecodeRun &r) {
+    const u64 C = kChunkBits;
     std::vector<DecStream> ds;
     std::vector<uint32_t> tile_stream;
-    std::vector<LutEntry> luts;
-    std::vector<uint32_t> childs;
+    std::vector<uint32_t> luts, lut2s, childs;
     u64 nchunks = 0;
-    uint32_t max_lut_bits = 1;
     for (const DecodeJob &j : jobs) {
         const HuffParsed &hp = *j.hp;
         if (!j.count) continue;
@@ -2853,6 +2865,7 @@ int gpu_decode_all(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8
         d.nchunks = std::max<u64>(1, (hp.payload_bits + C - 1) / C);
         d.tile0 = tile_stream.size();
         d.lut_off = luts.size();
+        d.lut2_off = lut2s.size();
         d.child_off = childs.size();
         d.count = j.count;
         d.offset = hp.offset;
@@ -2860,64 +2873,103 @@ int gpu_decode_all(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8
         d.lut_bits = hp.lut_bits;
         d.wide = j.wide ? 1 : 0;
         luts.insert(luts.end(), hp.lut.begin(), hp.lut.end());
+        luts.resize((luts.size() + 3) & ~size_t(3));
+        lut2s.insert(lut2s.end(), hp.lut2.begin(), hp.lut2.end());
         childs.insert(childs.end(), hp.child.begin(), hp.child.end());
         const u64 tiles = (d.nchunks + kDecodeTile - 1) / kDecodeTile;
         tile_stream.insert(tile_stream.end(), tiles, (uint32_t)ds.size());
         nchunks += d.nchunks;
-        max_lut_bits = std::max(max_lut_bits, hp.lut_bits);
+        r.max_lut_bits = std::max(r.max_lut_bits, hp.lut_bits);
         ds.push_back(d);
     }
-    CK(cudaMemsetAsync(&dm->dec_err, 0, 4, st));
+    CK(cudaMemsetAsync(&dm->dec_err, 0, 8, st));  // and dec_changed
     if (ds.empty()) return ASZ_OK;
     if (childs.empty()) childs.push_back(0);
     // Tables and descriptors in one upload.
-    const u64 ds_bytes = ds.size() * sizeof(DecStream), ts_bytes = tile_stream.size() * 4, lut_bytes = luts.size() * sizeof(LutEntry),
-              ch_bytes = childs.size() * 4;
-    auto al = [](u64 x) { return (x + 255) & ~255ull; };
-    const u64 o_ts = al(ds_bytes), o_lut = o_ts + al(ts_bytes), o_ch = o_lut + al(lut_bytes), total = o_ch + al(ch_bytes);
+    u64 total = 0;
+    auto place = [&](u64 bytes) {
+        const u64 o = total;
+        total = (total + bytes + 255) & ~255ull;
+        return o;
+    };
+    const u64 o_ds = place(ds.size() * sizeof(DecStream)), o_ts = place(tile_stream.size() * 4), o_lut = place(luts.size() * 4),
+              o_lut2 = place(lut2s.size() * 4), o_ch = place(childs.size() * 4);
     std::vector<uint8_t> blob(total);
-    std::memcpy(blob.data(), ds.data(), ds_bytes);
-    std::memcpy(blob.data() + o_ts, tile_stream.data(), ts_bytes);
-    std::memcpy(blob.data() + o_lut, luts.data(), lut_bytes);
-    std::memcpy(blob.data() + o_ch, childs.data(), ch_bytes);
+    std::memcpy(blob.data() + o_ds, ds.data(), ds.size() * sizeof(DecStream));
+    std::memcpy(blob.data() + o_ts, tile_stream.data(), tile_stream.size() * 4);
+    std::memcpy(blob.data() + o_lut, luts.data(), luts.size() * 4);
+    std::memcpy(blob.data() + o_lut2, lut2s.data(), lut2s.size() * 4);
+    std::memcpy(blob.data() + o_ch, childs.data(), childs.size() * 4);
     CK(ctx->codes.reserve(total));
     uint8_t *dc = ctx->codes.as<uint8_t>();
     CK(cudaMemcpyAsync(dc, blob.data(), total, cudaMemcpyHostToDevice, st));
-    const DecStream *d_ds = (const DecStream *)dc;
-    const uint32_t *d_ts = (const uint32_t *)(dc + o_ts);
-    const LutEntry *d_lut = (const LutEntry *)(dc + o_lut);
-    const uint32_t *d_ch = (const uint32_t *)(dc + o_ch);
+    r.base = d_base;
+    r.ds = (const DecStream *)(dc + o_ds);
+    r.ts = (const uint32_t *)(dc + o_ts);
+    r.lut = (const uint32_t *)(dc + o_lut);
+    r.lut2 = (const uint32_t *)(dc + o_lut2);
+    r.child = (const uint32_t *)(dc + o_ch);
     // Per-chunk arrays: start, end, count, off (count + 1 entries for the scan), moved (u32).
     CK(ctx->chunks.reserve(4 * (nchunks + 1) * 8 + (nchunks + 1) * 4 + 64));
-    u64 *d_start = ctx->chunks.as<u64>(), *d_end = d_start + nchunks + 1, *d_cnt = d_end + nchunks + 1, *d_off = d_cnt + nchunks + 1;
-    uint32_t *d_moved = reinterpret_cast<uint32_t *>(d_off + nchunks + 1);
-    CK(cudaMemsetAsync(d_cnt + nchunks, 0, 8, st));
-    const uint32_t nst = (uint32_t)ds.size();
-    const u64 ntiles = tile_stream.size();
-    for (u64 it = 0;; it++) {
-        {
-            ProfScope ps(ctx, "huff_decode_sync", 0);
-            CK(launch_decode_sync(d_base, C, d_ds, d_ts, ntiles, max_lut_bits, d_lut, d_ch, it == 0 ? 1 : 0, d_start, d_end, d_cnt,
-                                  d_moved, &dm->dec_err, st));
-        }
+    r.start = ctx->chunks.as<u64>(), r.end = r.start + nchunks + 1, r.cnt = r.end + nchunks + 1, r.off = r.cnt + nchunks + 1;
+    r.moved = reinterpret_cast<uint32_t *>(r.off + nchunks + 1);
+    r.nst = (uint32_t)ds.size();
+    r.ntiles = tile_stream.size();
+    r.nchunks = nchunks;
+    CK(cudaMemsetAsync(r.cnt + nchunks, 0, 8, st));
+    ProfScope ps(ctx, "huff_decode_sync", 0);
+    CK(launch_decode_sync(r.base, C, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 1, r.start, r.end, r.cnt, r.moved,
+                          &dm->dec_err, st));
+    // A second pass where a run's guess is likely to miss somewhere (it costs about 10 us; finding out
+    // at the end costs the whole decoding and reconstruction again). The bits until a wrong start
+    // falls in step are geometrically distributed, their mean about 1.8 b^2 at b bits a symbol
+    // (simulated for normal and Laplace symbols, 4 to 11 bits).
+    double misses = 0;
+    for (const DecStream &d : ds) {
+        const double b = (double)(d.bit_end - d.bit_begin) / (double)d.count;
+        misses += (double)(d.nchunks / kDecodeRun) * std::exp(-(double)(kDecodeHalo * C) / (1.8 * b * b));
+    }
+    if (misses > 0.01) {
+        CK(launch_decode_restart(r.ds, r.nst, nchunks, r.end, r.start, r.moved, &dm->dec_changed, st));
+        CK(launch_decode_sync(r.base, C, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 0, r.start, r.end, r.cnt,
+                              r.moved, &dm->dec_err, st));
         CK(cudaMemsetAsync(&dm->dec_changed, 0, 4, st));
-        CK(launch_decode_restart(d_ds, nst, nchunks, d_end, d_start, d_moved, &dm->dec_changed, st));
+    }
+    return ASZ_OK;
+}
+
+// The values, from the starts as they are. Errors of the payloads (dm->dec_err) and a start that
+// the check found moved (dm->dec_changed) are left for the caller to read with its final
+// synchronisation; with the latter the values are not the stream's.
+int decode_values(asz_ctx *ctx, const DecodeRun &r, MiscLayout *dm, cudaStream_t st) {
+    if (!r.nst) return ASZ_OK;
+    size_t tb = 0;
+    CK(launch_scan_u64(r.cnt, r.off, r.nchunks + 1, nullptr, tb, st));
+    CK(ctx->cubtmp.reserve(tb));
+    tb = ctx->cubtmp.cap;
+    CK(launch_scan_u64(r.cnt, r.off, r.nchunks + 1, ctx->cubtmp.p, tb, st));
+    CK(launch_decode_check(r.ds, r.nst, r.ts, r.ntiles, r.off, r.start, r.end, &dm->dec_err, &dm->dec_changed, st));
+    ProfScope ps_w(ctx, "huff_decode_write", 0);
+    CK(launch_decode_write(r.base, kChunkBits, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, r.start, r.off, &dm->dec_err,
+                           st));
+    return ASZ_OK;
+}
+
+// Passes until no run's first chunk moves (the first one's guess missed somewhere).
+int decode_settle(asz_ctx *ctx, const DecodeRun &r, MiscLayout *dm, cudaStream_t st) {
+    for (u64 it = 0;; it++) {
+        CK(cudaMemsetAsync(&dm->dec_err, 0, 8, st));
+        CK(launch_decode_restart(r.ds, r.nst, r.nchunks, r.end, r.start, r.moved, &dm->dec_changed, st));
         uint32_t changed;
         CK(cudaMemcpyAsync(&changed, &dm->dec_changed, 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if (!changed) break;
-        // Every pass that moves a start fixes at least one more chunk, so this ends.
-        if (it > nchunks + 2) return fail(ctx, ASZ_E_DATA, "Huffman payload does not synchronise");
+        if (!changed) return ASZ_OK;
+        // Every pass that moves a start fixes at least one more run, so this ends.
+        if (it > r.ntiles * (kDecodeTile / kDecodeRun) + 2) return fail(ctx, ASZ_E_DATA, "Huffman payload does not synchronise");
+        ProfScope ps(ctx, "huff_decode_sync", 0);
+        CK(launch_decode_sync(r.base, kChunkBits, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 0, r.start, r.end, r.cnt,
+                              r.moved, &dm->dec_err, st));
     }
-    size_t tb = 0;
-    CK(launch_scan_u64(d_cnt, d_off, nchunks + 1, nullptr, tb, st));
-    CK(ctx->cubtmp.reserve(tb));
-    tb = ctx->cubtmp.cap;
-    CK(launch_scan_u64(d_cnt, d_off, nchunks + 1, ctx->cubtmp.p, tb, st));
-    CK(launch_decode_check(d_ds, nst, d_off, d_end, &dm->dec_err, st));
-    ProfScope ps_w(ctx, "huff_decode_write", 0);
-    CK(launch_decode_write(d_base, C, d_ds, d_ts, ntiles, max_lut_bits, d_lut, d_ch, d_start, d_off, &dm->dec_err, st));
-    return ASZ_OK;
 }
 
 }  // namespace
@@ -3066,18 +3118,17 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     CK(ctx->qb.reserve(std::max<u64>(qtot, 1) * 4));
     std::optional<HostScope> hs_dec(std::in_place, ctx, "host:huffman_decode");
     MiscLayout *dm = ctx->misc.as<MiscLayout>();
+    DecodeRun run;
     {
         std::vector<DecodeJob> jobs;
         jobs.push_back({&hp[0], counts[0], ctx->tint.p, true});
         for (u64 s = 0; s <= L; s++) jobs.push_back({&hp[s + 1], counts[s + 1], ctx->qb.as<int32_t>() + qoff[s], false});
-        rc = gpu_decode_all(ctx, jobs, ctx->pre.as<uint8_t>(), dm, st);
+        rc = decode_begin(ctx, jobs, ctx->pre.as<uint8_t>(), dm, st, run);
         if (rc) return rc;
     }
     hs_dec.reset();
-    R.huffman_s = secs(t_h, clk::now());
-    // Reconstruction.
-    auto t_core = clk::now();
-    std::optional<HostScope> hs_rec(std::in_place, ctx, "host:reconstruct");
+    // Reconstruction, behind the decoding: the host waits once, and reads then whether the decoding
+    // settled in its first pass. If not, it is settled and the rest runs again.
     float *d_out = out;
     if (!out_on_device) {
         CK(ctx->rec.reserve(N * sizeof(float)));
@@ -3086,37 +3137,49 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     CK(ctx->axis.reserve(std::max<size_t>(G.ent.size(), 1) * sizeof(AxisEntry)));
     const AxisEntry *d_ent = ctx->axis.as<AxisEntry>();
     CK(cudaMemcpyAsync(ctx->axis.p, G.ent.data(), G.ent.size() * sizeof(AxisEntry), cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(&dm->err, 0, 4, st));
-    {
-        ProfScope ps(ctx, "pivot_decompress", G.pivots * 8);
-        CK(launch_pivot_decompress(G.pg, ctx->qb.as<int32_t>() + qoff[0], d_out, st));
-    }
-    if (const uint32_t line_bytes = ctx->tsel_mode == 2 ? lines_smem_bytes(G) : 0) {
-        // Every round along axis 2: all rounds fused per column of lines (k_lines.cu).
-        const u64 rbytes = L * sizeof(RoundGeom);
-        CK(ctx->rounds_dev.reserve(rbytes + (L + 1) * sizeof(u64)));
-        uint8_t *rd = ctx->rounds_dev.as<uint8_t>();
-        CK(cudaMemcpyAsync(rd, G.rounds.data(), rbytes, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(rd + rbytes, qoff.data(), (L + 1) * sizeof(u64), cudaMemcpyHostToDevice, st));
-        u64 tgt = 0;
-        for (u64 l = 0; l < L; l++) tgt += G.rounds[l].targets;
-        // Algorithmic bytes: the field loaded and stored once, one QB read per target.
-        ProfScope ps(ctx, "lines_decompress", N * 8 + tgt * 4);
-        for (const LinesLaunch &ll : lines_launches(G, line_bytes))
-            CK(launch_lines_decompress(G.fg, (const RoundGeom *)rd, d_ent, (const u64 *)(rd + rbytes),
-                                       ctx->tint.as<int64_t>(), ctx->qb.as<int32_t>(), d_out, &dm->err, ll.set, ll.bytes, st));
-    } else {
-        for (u64 l = 0; l < L; l++) {
-            ProfScope ps(ctx, "round_decompress", G.rounds[l].targets * 8);
-            CK(launch_round_decompress(G.fg, G.rounds[l], (uint32_t)l, d_ent, ctx->tint.as<int64_t>(),
-                                       ctx->qb.as<int32_t>() + qoff[l + 1], d_out, &dm->err, st));
+    CK(ctx->words.reserve(64));
+    const volatile uint32_t *words = (const volatile uint32_t *)ctx->words.p;  // dec_err, dec_changed, err
+    auto t_core = clk::now();
+    for (int attempt = 0;; attempt++) {
+        rc = decode_values(ctx, run, dm, st);
+        if (rc) return rc;
+        if (attempt == 0) R.huffman_s = secs(t_h, clk::now());
+        t_core = clk::now();
+        HostScope hs_rec(ctx, "host:reconstruct");
+        CK(cudaMemsetAsync(&dm->err, 0, 4, st));
+        {
+            ProfScope ps(ctx, "pivot_decompress", G.pivots * 8);
+            CK(launch_pivot_decompress(G.pg, ctx->qb.as<int32_t>() + qoff[0], d_out, st));
         }
+        if (const uint32_t line_bytes = ctx->tsel_mode == 2 ? lines_smem_bytes(G) : 0) {
+            // Every round along axis 2: all rounds fused per column of lines (k_lines.cu).
+            const u64 rbytes = L * sizeof(RoundGeom);
+            CK(ctx->rounds_dev.reserve(rbytes + (L + 1) * sizeof(u64)));
+            uint8_t *rd = ctx->rounds_dev.as<uint8_t>();
+            CK(cudaMemcpyAsync(rd, G.rounds.data(), rbytes, cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(rd + rbytes, qoff.data(), (L + 1) * sizeof(u64), cudaMemcpyHostToDevice, st));
+            u64 tgt = 0;
+            for (u64 l = 0; l < L; l++) tgt += G.rounds[l].targets;
+            // Algorithmic bytes: the field loaded and stored once, one QB read per target.
+            ProfScope ps(ctx, "lines_decompress", N * 8 + tgt * 4);
+            for (const LinesLaunch &ll : lines_launches(G, line_bytes))
+                CK(launch_lines_decompress(G.fg, (const RoundGeom *)rd, d_ent, (const u64 *)(rd + rbytes),
+                                           ctx->tint.as<int64_t>(), ctx->qb.as<int32_t>(), d_out, &dm->err, ll.set, ll.bytes, st));
+        } else {
+            for (u64 l = 0; l < L; l++) {
+                ProfScope ps(ctx, "round_decompress", G.rounds[l].targets * 8);
+                CK(launch_round_decompress(G.fg, G.rounds[l], (uint32_t)l, d_ent, ctx->tint.as<int64_t>(),
+                                           ctx->qb.as<int32_t>() + qoff[l + 1], d_out, &dm->err, st));
+            }
+        }
+        CK(cudaMemcpyAsync(ctx->words.p, &dm->dec_err, 12, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (!words[1]) break;
+        if (attempt) return fail(ctx, ASZ_E_DEVICE, "Huffman decoding did not settle");
+        rc = decode_settle(ctx, run, dm, st);
+        if (rc) return rc;
     }
-    uint32_t errw, decw;
-    CK(cudaMemcpyAsync(&errw, &dm->err, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&decw, &dm->dec_err, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    hs_rec.reset();
+    const uint32_t decw = words[0], errw = words[2];
     // Payload errors first: the reconstruction ran on whatever was decoded (bounded, no faults).
     if (decw & (8u | 16u)) return fail(ctx, ASZ_E_DATA, "corrupt Huffman payload");
     if (decw & 128u) return fail(ctx, ASZ_E_DATA, "Huffman payload ends inside a code");

@@ -2,6 +2,7 @@
 #include "huffman_host.h"
 
 #include <algorithm>
+#include <cstring>
 
 #include <queue>
 #include <utility>
@@ -172,6 +173,88 @@ void write_len_word(const HuffCode &c, uint8_t *dst) {
     put_be64(dst, (c.maxval == 1 ? c.count : c.bits) ^ 0x1234abcdull);
 }
 
+namespace {
+
+// Bits of buf[0, len) by position, LSB-first.
+struct TreeBits {
+    const uint8_t *buf;
+    uint64_t len, avail;
+    uint64_t pos = 0;
+    // The next n bits (n <= 63; false past the end).
+    bool read(unsigned n, uint64_t &v) {
+        if (pos + n > avail) return false;
+        const uint64_t byte = pos >> 3;
+        const unsigned sh = (unsigned)(pos & 7);
+        if (byte + 9 <= len) {
+            uint64_t w;
+            std::memcpy(&w, buf + byte, 8);
+            w >>= sh;
+            if (sh) w |= (uint64_t)buf[byte + 8] << (64 - sh);
+            v = w & ((1ull << n) - 1);
+        } else {
+            v = 0;
+            for (unsigned j = 0; j < n; j++) v |= (uint64_t)((buf[(pos + j) >> 3] >> ((pos + j) & 7)) & 1) << j;
+        }
+        pos += n;
+        return true;
+    }
+    // The number of zero bits before the next one, at most `most` + 1 of them, all consumed but the one.
+    bool zeros(unsigned most, unsigned &count) {
+        count = 0;
+        uint64_t v;
+        while (count <= most) {
+            const unsigned n = (unsigned)std::min<uint64_t>(32, avail - pos);
+            if (n == 0 || !read(n, v)) return false;
+            const unsigned z = v ? (unsigned)__builtin_ctzll(v) : n;
+            count += z;
+            if (v) {
+                pos -= n - z;
+                return true;
+            }
+        }
+        return true;
+    }
+};
+
+constexpr uint32_t kLutBits = 12, kLut2Bits = 10, kLutValueBits = 27, kLut2Most = 1u << 20;
+
+struct LongLeaf {
+    uint32_t code, len, sym;
+};
+
+constexpr uint32_t lut_entry(uint32_t len, uint32_t v) { return len << kLutValueBits | v; }
+
+// The second table, for the codes longer than the first one (in preorder, so those of one prefix lie
+// together), and the first one's entries that lead there.
+bool fill_lut2(const std::vector<LongLeaf> &leaves, uint32_t sub_bits, HuffParsed &o) {
+    o.lut2.clear();
+    for (size_t i = 0; i < leaves.size();) {
+        const uint32_t prefix = leaves[i].code & ((1u << kLutBits) - 1);
+        size_t j = i;
+        uint32_t most = 0;
+        for (; j < leaves.size() && (leaves[j].code & ((1u << kLutBits) - 1)) == prefix; j++) most = std::max(most, leaves[j].len);
+        const uint32_t bits = std::min(most - kLutBits, sub_bits), off = (uint32_t)o.lut2.size();
+        if (off + (1u << bits) > kLut2Most) return false;
+        o.lut2.resize(off + (1u << bits));
+        uint32_t *t = o.lut2.data() + off;
+        for (; i < j; i++) {
+            const LongLeaf &l = leaves[i];
+            const uint32_t rest = l.code >> kLutBits, len = l.len - kLutBits;
+            if (len <= bits) {
+                for (uint32_t k = rest; k < (1u << bits); k += 1u << len) t[k] = lut_entry(l.len, l.sym);
+            } else {  // the tree node after the table's bits
+                uint32_t node = 0;
+                for (uint32_t k = 0; k < kLutBits + bits; k++) node = o.child[2 * (size_t)node + ((l.code >> k) & 1)];
+                t[rest & ((1u << bits) - 1)] = lut_entry(0, node);
+            }
+        }
+        o.lut[prefix] = lut_entry(0, off << 4 | bits);
+    }
+    return true;
+}
+
+}  // namespace
+
 bool parse_stream(const uint8_t *buf, uint64_t len, uint64_t &pos, HuffParsed &o, std::string &err) {
     o = HuffParsed();
     if (len - pos < 25 || pos > len) {
@@ -195,94 +278,86 @@ bool parse_stream(const uint8_t *buf, uint64_t len, uint64_t &pos, HuffParsed &o
             err = "corrupt Huffman tree header";
             return false;
         }
-        // Rebuild the tree from its preorder bits, starting after the root's bit.
-        struct N {
-            int32_t c[2] = {-1, -1};
-            int64_t sym = -1;
-            uint32_t depth = 0;
-        };
-        std::vector<N> nodes(1);
-        std::vector<int32_t> st{0};
-        uint64_t i = 1;
-        const uint64_t avail_bits = (len - pos) * 8;
-        auto rd = [&](uint64_t k, unsigned &v) {
-            if (k >= avail_bits) return false;
-            v = (buf[pos + (k >> 3)] >> (k & 7)) & 1;
-            return true;
-        };
-        uint64_t leaves = 0;
+        // The tree from its preorder bits, starting after the root's bit: internal nodes in their
+        // order, a leaf in its parent's branch. The open nodes are the path to the next one; `turn`
+        // has its branches (bit d: the branch taken at depth d).
+        TreeBits in{buf + pos, len - pos, (len - pos) * 8, 1};
+        o.child.reserve(2 * std::min<uint64_t>(o.n, len));
+        o.child.assign(2, 0);
+        o.lut.assign(1u << kLutBits, 0);
+        std::vector<LongLeaf> longer;
+        std::vector<uint32_t> open{0};
+        uint64_t turn = 0, leaves = 0, nodes = 1;
         uint32_t max_len = 0;
-        while (!st.empty()) {
-            int32_t u = st.back();
-            unsigned bit;
-            if (!rd(i++, bit)) {
+        bool in_range = true, fits = true;
+        while (!open.empty()) {
+            unsigned inner;
+            if (!in.zeros(48, inner)) {
                 err = "truncated Huffman tree";
                 return false;
             }
-            N nd;
-            nd.depth = nodes[u].depth + 1;
-            if (bit == 0) {
-                nodes.push_back(nd);
-                int32_t id = (int32_t)nodes.size() - 1;
-                if (nodes[u].c[0] < 0) nodes[u].c[0] = id;
-                else nodes[u].c[1] = id;
-                st.push_back(id);
-            } else {
-                uint64_t s = 0;
-                for (unsigned j = 0; j < o.mbft; j++) {
-                    unsigned v;
-                    if (!rd(i++, v)) {
-                        err = "truncated Huffman tree";
-                        return false;
-                    }
-                    s |= (uint64_t)v << j;
+            for (unsigned k = 0; k < inner; k++) {  // each the first branch of the one before
+                const uint32_t id = (uint32_t)(o.child.size() / 2), d = (uint32_t)open.size() - 1;
+                if (++nodes > 2 * o.n + 1 || open.size() > 40) {
+                    err = "corrupt Huffman tree";
+                    return false;
                 }
-                nd.sym = (int64_t)s;
-                nodes.push_back(nd);
-                int32_t id = (int32_t)nodes.size() - 1;
-                if (nodes[u].c[0] < 0) nodes[u].c[0] = id;
-                else nodes[u].c[1] = id;
-                leaves++;
-                max_len = std::max(max_len, nd.depth);
-                while (!st.empty() && nodes[st.back()].c[1] >= 0) st.pop_back();
+                o.child[2 * (size_t)open.back() + ((turn >> d) & 1)] = id;
+                o.child.resize(o.child.size() + 2);
+                open.push_back(id);
             }
-            if (nodes.size() > 2 * o.n + 1 || nd.depth > 40) {
+            uint64_t one, sym;
+            if (!in.read(1, one) || !in.read(o.mbft, sym)) {
+                err = "truncated Huffman tree";
+                return false;
+            }
+            const uint32_t d = (uint32_t)open.size() - 1, l = d + 1;
+            if (++nodes > 2 * o.n + 1 || l > 40) {
                 err = "corrupt Huffman tree";
                 return false;
             }
+            o.child[2 * (size_t)open.back() + ((turn >> d) & 1)] = 0x80000000u | (uint32_t)sym;
+            leaves++;
+            max_len = std::max(max_len, l);
+            in_range = in_range && (sym < std::max<uint64_t>(o.maxval, 1) || o.maxval >= (1ull << 31));
+            fits = fits && sym < (1ull << kLutValueBits);
+            if (l <= kLutBits) {
+                const uint32_t e = lut_entry(l, (uint32_t)sym & ((1u << kLutValueBits) - 1));
+                for (uint32_t i = (uint32_t)turn; i < o.lut.size(); i += 1u << l) o.lut[i] = e;
+            } else if (l <= 32) {
+                longer.push_back({(uint32_t)turn, l, (uint32_t)sym});
+            }
+            // On to the second branch of the deepest node that has not had it.
+            while (!open.empty() && (turn >> (open.size() - 1)) & 1) {
+                turn &= ~(1ull << (open.size() - 1));
+                open.pop_back();
+            }
+            if (!open.empty()) turn |= 1ull << (open.size() - 1);
         }
         if (leaves != o.n) {
             err = "Huffman tree does not match its symbol count";
             return false;
         }
-        pos += (i + 7) >> 3;
+        pos += (in.pos + 7) >> 3;
         if (max_len > 32) {
             err = "Huffman code longer than 32 bits";
             return false;
         }
-        o.lut_bits = std::min<uint32_t>(max_len, 12);
-        o.child.assign(2 * nodes.size(), 0);
-        auto ref = [&](int32_t id) -> uint32_t {
-            return nodes[id].sym >= 0 ? (0x80000000u | (uint32_t)nodes[id].sym) : (uint32_t)id;
-        };
-        for (size_t u = 0; u < nodes.size(); u++)
-            if (nodes[u].sym < 0) {
-                o.child[2 * u] = ref(nodes[u].c[0]);
-                o.child[2 * u + 1] = ref(nodes[u].c[1]);
-            }
-        for (size_t u = 0; u < nodes.size(); u++)
-            if (nodes[u].sym >= 0 && (uint64_t)nodes[u].sym >= std::max<uint64_t>(o.maxval, 1) && o.maxval < (1ull << 31)) {
-                err = "Huffman symbol outside its range";
-                return false;
-            }
-        o.lut.resize(1ull << o.lut_bits);
-        for (uint64_t pre = 0; pre < o.lut.size(); pre++) {
-            int32_t u = 0;
-            uint32_t l = 0;
-            while (l < o.lut_bits && nodes[u].sym < 0) u = nodes[u].c[(pre >> l++) & 1];
-            if (nodes[u].sym >= 0) o.lut[pre] = LutEntry{(uint32_t)nodes[u].sym, l};
-            else o.lut[pre] = LutEntry{(uint32_t)u, 0};
+        if (!in_range) {
+            err = "Huffman symbol outside its range";
+            return false;
         }
+        o.lut_bits = std::min(max_len, kLutBits);
+        o.lut.resize(1ull << o.lut_bits);  // a shorter table's entries are the first ones
+        uint32_t sub = kLut2Bits;
+        fits = fits && o.child.size() / 2 < (1ull << kLutValueBits);
+        while (fits && !fill_lut2(longer, sub, o)) fits = sub-- > 0;
+        if (!fits) {  // every code is walked from the root
+            o.lut_bits = 0;
+            o.lut.assign(1, lut_entry(0, 0));
+            o.lut2.assign(1, lut_entry(0, 0));
+        }
+        if (o.lut2.empty()) o.lut2.assign(1, 0);
     } else {
         o.single = true;
     }

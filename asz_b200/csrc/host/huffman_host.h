@@ -50,8 +50,11 @@ struct HuffParsed {
     uint64_t payload_bits = 0;     // from the length word
     uint64_t single_count = 0;     // from the length word when single
     uint64_t payload_off = 0;      // byte offset of the payload in the stream buffer
-    std::vector<LutEntry> lut;
-    std::vector<uint32_t> child;   // 2 per internal node
+    // Lookup tables, entries of a length (top 5 bits) and a value. lut: by the next lut_bits bits, a
+    // code's length and symbol, or length 0 and (offset << 4 | bits) of a table in lut2 by the bits
+    // after those. lut2: a code's length and symbol, or length 0 and the tree node to walk on from.
+    std::vector<uint32_t> lut, lut2;
+    std::vector<uint32_t> child;   // 2 per node: a node, or a symbol with the top bit set
     uint32_t lut_bits = 0;
 };
 

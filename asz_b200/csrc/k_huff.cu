@@ -4,8 +4,9 @@
 // The reference decodes serially (huffman.hpp:383-526). Here the payload is cut into chunks
 // of a fixed number of bits, and one thread decodes each chunk from a guessed codeword boundary.
 // Huffman codes resynchronise after a few codewords, so a chunk decoded from the true start of
-// its predecessor's last codeword ends at the same place as the guess. Passes repeat until no
-// chunk start changes. A final pass writes the symbols at offsets from a scan of per-chunk counts.
+// its predecessor's last codeword ends at the same place as the guess. A warp settles a run of
+// chunks and a check compares the runs' ends and starts (passes repeat while one moves). A final
+// pass writes the symbols at offsets from a scan of per-chunk counts.
 // Every loop is bounded by the chunk length plus the longest code.
 #include <cuda_runtime.h>
 
@@ -268,96 +269,70 @@ __global__ void __launch_bounds__(kEncThreads, 4)
 }
 
 // ---------------------------------------------------------------------------------------------
-// Decoding. The host builds a lookup table of 2^lut_bits entries indexed by the next lut_bits
-// payload bits (LSB-first): len>0 gives a complete code of that length and its symbol index;
-// len==0 means the code is longer, and `node` is the tree node reached after lut_bits bits.
-// Longer codes continue through child[2*node+bit] (a value >= 0x80000000 marks a leaf whose
-// symbol index is the low bits).
+// Decoding. The host builds two tables per stream (huffman_host.h): one indexed by the next lut_bits
+// payload bits (LSB-first), staged in shared memory, and, for longer codes, one by up to ten bits
+// more, read through L1. Entries carry the code's length in the top 5 bits and its symbol; length 0
+// leads on to the second table, and from there to the tree: child[2*node+bit] (a value >= 0x80000000
+// marks a leaf whose symbol index is the low bits).
+//
+// A symbol is a dependent chain of a few shared-memory reads, so a kernel decodes as fast as its
+// warps issue. A tile's payload is therefore staged in shared memory too, where the next 32 bits of
+// any position are two words and a funnel shift; a queue of words in each thread's registers, refilled
+// by 16-byte loads, had the threads of a warp refill at different symbols, so that every symbol of
+// the warp ran all the refill's branches (512^3 at 1e-3, 6.6 bits a symbol: 0.75 ms to synchronise and
+// 0.82 to write, now 0.47 and 0.49).
 
-// Bit reader with read-ahead: `buf` holds the next `nb` payload bits (LSB-first) and is topped up
-// to at least 32 bits (the longest code) before each codeword from a queue of 32-bit words. The
-// queue is fed by 16-byte loads issued one block ahead, so a load's latency overlaps the decoding
-// of the ~128 bits before it is needed. `payload` is 16-byte aligned; reads run at most 48 bytes
-// past the current position and the stream buffer is padded for that.
-struct BitReader {
-    const uint4 *p;
-    uint64_t idx;      // next 16-byte block to request
-    uint4 nxt;         // requested block
-    uint64_t c0, c1;   // current block, words consumed from the low end
-    uint32_t cw;       // words left in (c0, c1)
-    uint64_t buf;
-    uint32_t nb;
-
-    __device__ __forceinline__ void load_cur(const uint4 &v) {
-        c0 = (uint64_t)v.x | ((uint64_t)v.y << 32);
-        c1 = (uint64_t)v.z | ((uint64_t)v.w << 32);
-        cw = 4;
-    }
-    __device__ __forceinline__ uint32_t take() {
-        const uint32_t w = (uint32_t)c0;
-        c0 = (c0 >> 32) | (c1 << 32);
-        c1 >>= 32;
-        if (--cw == 0) {
-            load_cur(nxt);
-            nxt = __ldg(p + idx++);
-        }
-        return w;
-    }
-    __device__ __forceinline__ void init(const uint8_t *payload, uint64_t bit) {
-        p = reinterpret_cast<const uint4 *>(payload);
-        idx = bit >> 7;
-        load_cur(__ldg(p + idx));
-        nxt = __ldg(p + idx + 1);
-        idx += 2;
-        for (uint32_t i = (uint32_t)((bit >> 5) & 3); i; i--) take();
-        const uint32_t skip = (uint32_t)(bit & 31);
-        buf = (uint64_t)(take() >> skip);
-        nb = 32 - skip;
-        refill();
-    }
-    __device__ __forceinline__ void refill() {
-        if (nb < 32) {
-            buf |= (uint64_t)take() << nb;
-            nb += 32;
-        }
-    }
-    __device__ __forceinline__ void drop(uint32_t n) {
-        buf >>= n;
-        nb -= n;
-    }
+// A stream's tables, the first in shared memory.
+struct DecodeTables {
+    const uint32_t *lut, *lut2, *child;
+    uint32_t lut_bits;
 };
 
-// Decode one codeword through the shared-memory table `lut`; returns the symbol index, or
-// 0xffffffff for a path that leaves the tree. Advances `bit` by the code length.
-__device__ __forceinline__ uint32_t decode_sym(BitReader &br, uint64_t &bit, const LutEntry *lut, uint32_t lut_bits,
-                                               const uint32_t *__restrict__ child) {
-    br.refill();
-    const LutEntry e = lut[br.buf & ((1u << lut_bits) - 1)];
-    if (e.len) {
-        br.drop(e.len);
-        bit += e.len;
-        return e.sym;
-    }
-    uint32_t node = e.sym;
-    uint32_t used = lut_bits;
-    uint64_t b = br.buf >> lut_bits;
-    // Codes are at most 32 bits and the buffer holds at least 32.
-    while (true) {
-        const uint32_t c = __ldg(child + 2 * node + (uint32_t)(b & 1));
-        b >>= 1;
-        used++;
-        if (c & 0x80000000u) {
-            br.drop(used);
-            bit += used;
-            return c & 0x7fffffffu;
+// A chunk's words: 32 of its own after a lead of up to 31 bits, and two more that its last codeword
+// may reach. The odd stride keeps a warp's reads, at about the same place of its chunks, on
+// different banks.
+constexpr uint32_t kSlotWords = 35;
+constexpr uint32_t kDecodeSlotBytes = ((kDecodeTile + kDecodeHalo) * kSlotWords * 4 + 15) / 16 * 16;
+
+// The 32 payload bits from bit `pos` of a slot on.
+__device__ __forceinline__ uint32_t peek(const uint32_t *slot, uint32_t pos) {
+    const uint32_t i = pos >> 5;
+    return __funnelshift_r(slot[i], slot[i + 1], pos & 31);
+}
+
+// Decode the codeword at `pos`; returns the symbol index and advances pos by the code length. A path
+// that leaves the tree moves pos past every limit (kBadPath).
+constexpr uint32_t kBadPath = 1u << 30;
+
+__device__ __forceinline__ uint32_t decode_sym(const uint32_t *slot, uint32_t &pos, const DecodeTables &T) {
+    const uint32_t v = peek(slot, pos);
+    uint32_t e = T.lut[v & ((1u << T.lut_bits) - 1)], len = e >> 27;
+    e &= 0x7ffffffu;
+    if (len == 0) {
+        const uint32_t sub = e & 15u;
+        const uint32_t e2 = __ldg(T.lut2 + (e >> 4) + ((v >> T.lut_bits) & ((1u << sub) - 1)));
+        len = e2 >> 27;
+        e = e2 & 0x7ffffffu;
+        if (len == 0) {  // codes are at most 32 bits
+            uint32_t node = e, used = T.lut_bits + sub;
+            while (true) {
+                const uint32_t c = __ldg(T.child + 2 * (uint64_t)node + ((v >> used) & 1));
+                used++;
+                if (c & 0x80000000u) {
+                    e = c & 0x7fffffffu;
+                    break;
+                }
+                node = c;
+                if (used >= 32) {  // impossible for a validated tree; stop instead of running on
+                    used = kBadPath;
+                    break;
+                }
+            }
+            len = used;
         }
-        node = c;
-        if (used >= 32) {  // impossible for a validated tree; stop instead of running on
-            br.drop(used);
-            bit += used;
-            return 0xffffffffu;
-        }
     }
+    pos += len;
+    return e;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -366,53 +341,144 @@ __device__ __forceinline__ uint32_t decode_sym(BitReader &br, uint64_t &bit, con
 // so a CTA stages one stream's lookup table for a tile. Bit positions are absolute from the
 // 16-byte aligned stream buffer `base`.
 
-__device__ __forceinline__ void stage_lut(LutEntry *lut_sh, const LutEntry *__restrict__ lut, uint32_t lut_bits) {
-    for (uint32_t i = threadIdx.x; i < (1u << lut_bits); i += blockDim.x) lut_sh[i] = lut[i];
+__device__ __forceinline__ void stage_lut(uint4 *lut_sh, const uint32_t *__restrict__ lut, uint32_t lut_bits) {
+    const uint4 *v = reinterpret_cast<const uint4 *>(lut);
+    for (uint32_t i = threadIdx.x; i < ((1u << lut_bits) + 3) / 4; i += blockDim.x) lut_sh[i] = __ldg(v + i);
 }
 
-// Pass A over all tiles: chunk k decodes from its start until it reaches the next chunk's first
-// bit, recording where it stopped (end[k]) and how many values it produced (count[k]). On the
-// first pass the start is the chunk's first bit; later passes start where chunk k-1 ended, and a
-// chunk whose start did not move (moved[k] == 0) keeps its end and count without decoding.
-__global__ void __launch_bounds__(256)
-    decode_sync_kernel(const uint8_t *__restrict__ base, uint64_t chunk_bits, const DecStream *__restrict__ streams,
-                       const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const LutEntry *__restrict__ luts,
-                       const uint32_t *__restrict__ childs, int first_pass, uint64_t *__restrict__ start,
-                       uint64_t *__restrict__ end, uint64_t *__restrict__ count, const uint32_t *__restrict__ moved,
-                       uint32_t *err_word) {
-    extern __shared__ LutEntry lut_sh[];
-    uint32_t staged = 0xffffffffu;
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t si = tile_stream[tile];
-        const DecStream d = streams[si];
-        if (si != staged) {
-            __syncthreads();
-            stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
-            __syncthreads();
-            staged = si;
+// The words of kSlots chunks from chunk `first` of the stream on (negative: none there) into their
+// slots. Words outside the payload read as zero.
+template <uint32_t kSlots>
+__device__ __forceinline__ void stage_payload(uint32_t *slots, const uint8_t *__restrict__ base, const DecStream &d, int64_t first) {
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(base);
+    const int64_t lo = (int64_t)(d.bit_begin >> 5), hi = (int64_t)(d.bit_end >> 5) + 1;  // kDecodePad lies behind
+    const int64_t w0 = lo + first * 32;
+    constexpr uint32_t kWords = kSlots * 32 + 2, kUnroll = 8;
+    for (uint32_t i0 = threadIdx.x; i0 < kWords; i0 += kUnroll * kDecodeThreads) {
+        uint32_t v[kUnroll];
+#pragma unroll
+        for (uint32_t u = 0; u < kUnroll; u++) {
+            const int64_t g = w0 + i0 + u * kDecodeThreads;
+            v[u] = g >= lo && g <= hi && i0 + u * kDecodeThreads < kWords ? __ldg(words + g) : 0u;
         }
-        const uint64_t kl = (tile - d.tile0) * blockDim.x + threadIdx.x;
-        if (kl >= d.nchunks) continue;
-        const uint64_t k = d.chunk0 + kl;
-        if (!first_pass && !moved[k]) continue;
-        uint64_t bit = first_pass ? d.bit_begin + kl * chunk_bits : start[k];
-        if (first_pass) start[k] = bit;
-        const uint64_t lim = min(d.bit_begin + (kl + 1) * chunk_bits, d.bit_end);
-        uint64_t c = 0;
-        if (bit < lim) {
-            BitReader br;
-            br.init(base, bit);
-            while (bit < lim) {
-                const uint32_t sym = decode_sym(br, bit, lut_sh, d.lut_bits, childs + d.child_off);
-                if (sym == 0xffffffffu) {
-                    atomicOr(err_word, 8u);
-                    break;
+#pragma unroll
+        for (uint32_t u = 0; u < kUnroll; u++) {
+            const uint32_t i = i0 + u * kDecodeThreads, slot = i >> 5, j = i & 31;
+            if (slot < kSlots) slots[slot * kSlotWords + j] = v[u];
+            if (j < 2 && slot && slot <= kSlots) slots[(slot - 1) * kSlotWords + 32 + j] = v[u];
+        }
+    }
+}
+
+// One chunk's decoding, in bits from its slot's start: where it stopped and how many values it met.
+// marks[j * kDecodeThreads] keeps the first codeword's start from 128 (j + 1) bits after `lead` on, with
+// the values before it in the upper half. A chunk that has to start elsewhere is read until it meets
+// one of them (codewords fall in step after a geometrically distributed number of bits, about 30 at 4
+// bits a symbol and 130 at 10; from there on it is decoded already).
+constexpr uint32_t kMarkBits = 128, kMarks = 7;
+
+struct ChunkRun {
+    uint32_t end = 0, count = 0;
+
+    __device__ __forceinline__ void decode(const uint32_t *slot, uint32_t lead, uint32_t pos, uint32_t lim, const DecodeTables &T,
+                                           uint32_t *marks, uint32_t *err_word) {
+        uint32_t c = 0, mark = lead + kMarkBits, j = 0;
+        while (pos < lim) {
+            decode_sym(slot, pos, T);
+            c++;
+            if (pos >= mark) {
+                if (j >= kMarks || pos >= kBadPath) continue;
+                const uint32_t old = marks[j * kDecodeThreads];
+                marks[j * kDecodeThreads] = c << 16 | pos;
+                if ((old & 0xffffu) == pos) {
+                    const uint32_t more = c - (old >> 16);  // modulo 2^16, as the marks
+                    for (uint32_t i = j + 1; i < kMarks; i++) marks[i * kDecodeThreads] += more << 16;
+                    count += (uint32_t)(int32_t)(int16_t)more;
+                    return;  // the same end
                 }
-                c++;
+                j++;
+                mark += kMarkBits;
             }
         }
-        end[k] = bit;
-        count[k] = c;
+        if (pos >= kBadPath) atomicOr(err_word, 8u);
+        end = pos;
+        count = c;
+        for (; j < kMarks; j++) marks[j * kDecodeThreads] = 0;  // not reached: no position
+    }
+};
+
+// Synchronisation. Chunk k decodes from its start until it reaches the next chunk's first bit,
+// recording where it stopped (end[k]) and how many values it produced (count[k]). First pass: every
+// chunk starts at its first bit, and then, within its warp, where its predecessor ended, until no
+// start moves. A warp's first chunk has its predecessor in another warp, so a warp's first
+// kDecodeHalo lanes decode the chunks before its own as well: a wrong guess nearly always meets the
+// true codewords within those 2048 bits (a 161x257x349 quintic stream at 1e-4 needed five passes
+// over all chunks, with the host waiting for each; now it is this one). What it nearly always is,
+// decode_check_kernel checks; a warp whose first chunk did start elsewhere is settled by the later
+// passes, which start at start[] and decode only from a moved first chunk on (moved[k] != 0).
+__global__ void __launch_bounds__(kDecodeThreads, 4)
+    decode_sync_kernel(const uint8_t *__restrict__ base, uint64_t chunk_bits, const DecStream *__restrict__ streams,
+                       const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const uint32_t *__restrict__ luts,
+                       const uint32_t *__restrict__ lut2s, const uint32_t *__restrict__ childs, int first_pass,
+                       uint64_t *__restrict__ start, uint64_t *__restrict__ end, uint64_t *__restrict__ count,
+                       const uint32_t *__restrict__ moved, uint32_t *err_word) {
+    extern __shared__ uint4 dec_smem[];
+    __shared__ uint32_t marks_sh[kMarks * kDecodeThreads];
+    uint32_t *const slots = reinterpret_cast<uint32_t *>(dec_smem);
+    uint4 *const lut_sh = dec_smem + kDecodeSlotBytes / 16;
+    uint32_t staged = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t *const marks = marks_sh + threadIdx.x;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint32_t si = tile_stream[tile];
+        const DecStream &d = streams[si];
+        const int64_t kl0 = (int64_t)((tile - d.tile0) * kDecodeTile) - (int)kDecodeHalo;
+        if (!first_pass) {
+            const uint64_t mine = (uint64_t)(tile - d.tile0) * kDecodeTile + threadIdx.x;
+            if (!__syncthreads_or(threadIdx.x < kDecodeTile && mine < d.nchunks && moved[d.chunk0 + mine])) continue;
+        }
+        __syncthreads();  // the tile before is done with the shared memory
+        if (si != staged) stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
+        stage_payload<kDecodeTile + kDecodeHalo>(slots, base, d, kl0);
+        for (uint32_t j = 0; j < kMarks; j++) marks[j * kDecodeThreads] = 0;
+        __syncthreads();
+        staged = si;
+        const DecodeTables T{reinterpret_cast<const uint32_t *>(lut_sh), lut2s + d.lut2_off, childs + d.child_off, d.lut_bits};
+        const int at_slot = warp * (int)kDecodeRun + lane;
+        const int64_t kl = kl0 + at_slot;
+        const uint32_t *slot = slots + at_slot * kSlotWords;
+        const bool own = lane >= (int)kDecodeHalo && kl < (int64_t)d.nchunks;
+        const bool in = first_pass ? kl >= 0 && kl < (int64_t)d.nchunks : own;
+        const bool after = in && lane > (first_pass ? 0 : (int)kDecodeHalo) && kl > 0;  // has a predecessor here
+        const uint64_t k = d.chunk0 + (uint64_t)kl;
+        // Positions relative to the chunk's slot.
+        const uint32_t lead = (uint32_t)(d.bit_begin & 31), span = (uint32_t)chunk_bits;
+        const uint64_t first = d.bit_begin + (uint64_t)kl * chunk_bits, origin = first - lead;
+        const uint32_t lim = in ? lead + (uint32_t)min((uint64_t)span, d.bit_end - first) : 0;
+        uint32_t s = lead;
+        ChunkRun run;
+        bool need = in;
+        if (in && !first_pass) {
+            s = (uint32_t)(start[k] - origin);
+            run.end = (uint32_t)(end[k] - origin);
+            run.count = (uint32_t)count[k];
+            need = moved[k] != 0;
+        }
+        // Each turn makes at least one more chunk of the warp final.
+        for (uint32_t turn = 0; turn <= 32; turn++) {
+            if (need) run.decode(slot, lead, s, lim, T, marks, err_word);
+            __syncwarp();
+            const uint32_t before = __shfl_up_sync(0xffffffffu, run.end, 1);
+            const uint32_t at = after ? before - span : s;
+            need = at != s;
+            s = at;
+            if (!__any_sync(0xffffffffu, need)) break;
+        }
+        if (own) {
+            start[k] = origin + s;
+            end[k] = origin + run.end;
+            count[k] = run.count;
+        }
     }
 }
 
@@ -445,14 +511,24 @@ __global__ void decode_restart_kernel(const DecStream *__restrict__ streams, uin
     }
 }
 
-// Per stream, once the starts are stable: the values decoded must equal the stream's count and
-// the last chunk must end exactly at the payload's last bit. off[] is the exclusive scan of
-// count[] over all chunks (nchunks + 1 entries).
-__global__ void decode_check_kernel(const DecStream *__restrict__ streams, uint32_t nstreams, const uint64_t *__restrict__ off,
-                                    const uint64_t *__restrict__ end, uint32_t *err_word) {
-    const uint32_t si = blockIdx.x * blockDim.x + threadIdx.x;
-    if (si >= nstreams) return;
-    const DecStream d = streams[si];
+// Per warp of a tile: whether its first chunk started where the one before it ended (`changed` if
+// not). Per stream, once the starts are stable: the values decoded must equal the stream's count and the last
+// chunk must end exactly at the payload's last bit. off[] is the exclusive scan of count[] over all
+// chunks (nchunks + 1 entries).
+__global__ void decode_check_kernel(const DecStream *__restrict__ streams, uint32_t nstreams,
+                                    const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const uint64_t *__restrict__ off,
+                                    const uint64_t *__restrict__ start, const uint64_t *__restrict__ end, uint32_t *err_word,
+                                    uint32_t *changed) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    constexpr uint32_t kRuns = kDecodeTile / kDecodeRun;
+    if (i < ntiles * kRuns) {
+        const uint64_t tile = i / kRuns;
+        const DecStream &d = streams[tile_stream[tile]];
+        const uint64_t kl = (tile - d.tile0) * kDecodeTile + i % kRuns * kDecodeRun, k = d.chunk0 + kl;
+        if (kl && kl < d.nchunks && start[k] != end[k - 1]) *changed = 1u;
+    }
+    if (i >= nstreams) return;
+    const DecStream d = streams[i];
     const uint64_t got = off[d.chunk0 + d.nchunks] - off[d.chunk0];
     if (got < d.count) atomicOr(err_word, 32u);
     if (got > d.count) atomicOr(err_word, 64u);
@@ -461,70 +537,77 @@ __global__ void decode_check_kernel(const DecStream *__restrict__ streams, uint3
 
 // Pass B over all tiles: write the values (symbol index + offset) of chunk k at its offset in its
 // stream's output (int64 for the t stream, int32 for QB streams).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kDecodeThreads, 4)
     decode_write_kernel(const uint8_t *__restrict__ base, uint64_t chunk_bits, const DecStream *__restrict__ streams,
-                        const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const LutEntry *__restrict__ luts,
-                        const uint32_t *__restrict__ childs, const uint64_t *__restrict__ start,
-                        const uint64_t *__restrict__ off, uint32_t *err_word) {
-    extern __shared__ LutEntry lut_sh[];
+                        const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const uint32_t *__restrict__ luts,
+                        const uint32_t *__restrict__ lut2s, const uint32_t *__restrict__ childs,
+                        const uint64_t *__restrict__ start, const uint64_t *__restrict__ off, uint32_t *err_word) {
+    extern __shared__ uint4 dec_smem[];
+    uint32_t *const slots = reinterpret_cast<uint32_t *>(dec_smem);
+    uint4 *const lut_sh = dec_smem + kDecodeSlotBytes / 16;
     uint32_t staged = 0xffffffffu;
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint32_t si = tile_stream[tile];
-        const DecStream d = streams[si];
-        if (si != staged) {
-            __syncthreads();
-            stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
-            __syncthreads();
-            staged = si;
-        }
-        const uint64_t kl = (tile - d.tile0) * blockDim.x + threadIdx.x;
-        if (kl >= d.nchunks) continue;
+        const DecStream &d = streams[si];
+        const uint64_t kl0 = (tile - d.tile0) * kDecodeTile, kl = kl0 + threadIdx.x;
+        __syncthreads();
+        if (si != staged) stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
+        stage_payload<kDecodeTile>(slots, base, d, (int64_t)kl0);
+        __syncthreads();
+        staged = si;
+        if (threadIdx.x >= kDecodeTile || kl >= d.nchunks) continue;
+        const DecodeTables T{reinterpret_cast<const uint32_t *>(lut_sh), lut2s + d.lut2_off, childs + d.child_off, d.lut_bits};
+        const uint32_t *slot = slots + threadIdx.x * kSlotWords;
         const uint64_t k = d.chunk0 + kl;
-        uint64_t bit = start[k];
-        const uint64_t lim = min(d.bit_begin + (kl + 1) * chunk_bits, d.bit_end);
-        if (bit >= lim) continue;
-        uint64_t o = off[k] - off[d.chunk0];
-        BitReader br;
-        br.init(base, bit);
-        if (d.wide) {
-            while (bit < lim) {
-                const uint32_t sym = decode_sym(br, bit, lut_sh, d.lut_bits, childs + d.child_off);
-                if (sym == 0xffffffffu || o >= d.count) {
-                    atomicOr(err_word, 16u);
-                    break;
-                }
-                static_cast<int64_t *>(d.out)[o++] = (int64_t)sym + d.offset;
-            }
+        const uint32_t lead = (uint32_t)(d.bit_begin & 31);
+        const uint64_t first = d.bit_begin + kl * chunk_bits;
+        uint32_t pos = (uint32_t)(start[k] - (first - lead));
+        const uint32_t lim = lead + (uint32_t)min(chunk_bits, d.bit_end - first);
+        if (pos >= lim) continue;
+        const uint64_t o0 = off[k] - off[d.chunk0], count = d.count;
+        if (o0 >= count) {
+            atomicOr(err_word, 16u);
             continue;
         }
-        // int32 values go out four at a time as one 16-byte store once the position is aligned:
-        // whole sectors leave the thread instead of one value per store.
-        int32_t *out = static_cast<int32_t *>(d.out);
-        int32_t b0 = 0, b1 = 0, b2 = 0;
-        uint32_t nb = 0;  // values held, to be stored from out + o
-        while (bit < lim) {
-            const uint32_t sym = decode_sym(br, bit, lut_sh, d.lut_bits, childs + d.child_off);
-            if (sym == 0xffffffffu || o + nb >= d.count) {
-                atomicOr(err_word, 16u);
-                break;
-            }
-            const int32_t v = (int32_t)((int64_t)sym + d.offset);
-            if (nb == 0 && ((uintptr_t)(out + o) & 15u) != 0) {
-                out[o++] = v;
-            } else if (nb == 3) {
-                *reinterpret_cast<int4 *>(out + o) = make_int4(b0, b1, b2, v);
+        const uint32_t room = (uint32_t)min(count - o0, (uint64_t)0xffffffffu);  // values left of the stream
+        uint32_t o = 0;
+        if (d.wide) {
+            int64_t *out = static_cast<int64_t *>(d.out) + o0;
+            const int64_t offset = d.offset;
+            while (pos < lim && o < room) out[o++] = (int64_t)decode_sym(slot, pos, T) + offset;
+        } else {
+            // int32 values go out four at a time as one 16-byte store once the position is aligned:
+            // whole sectors leave the thread instead of one value per store.
+            int32_t *out = static_cast<int32_t *>(d.out) + o0;
+            const uint32_t offset = (uint32_t)(int32_t)d.offset;
+            const uint32_t head = min(room, (uint32_t)(-(intptr_t)((uintptr_t)out >> 2) & 3));  // up to the alignment
+            while (pos < lim && o < head) out[o++] = (int32_t)(decode_sym(slot, pos, T) + offset);
+            while (pos < lim && o + 4 <= room) {
+                int4 v;
+                v.x = (int32_t)(decode_sym(slot, pos, T) + offset);
+                if (pos >= lim) {
+                    out[o++] = v.x;
+                    break;
+                }
+                v.y = (int32_t)(decode_sym(slot, pos, T) + offset);
+                if (pos >= lim) {
+                    out[o] = v.x, out[o + 1] = v.y;
+                    o += 2;
+                    break;
+                }
+                v.z = (int32_t)(decode_sym(slot, pos, T) + offset);
+                if (pos >= lim) {
+                    out[o] = v.x, out[o + 1] = v.y, out[o + 2] = v.z;
+                    o += 3;
+                    break;
+                }
+                v.w = (int32_t)(decode_sym(slot, pos, T) + offset);
+                *reinterpret_cast<int4 *>(out + o) = v;
                 o += 4;
-                nb = 0;
-            } else {
-                if (nb == 0) b0 = v;
-                else if (nb == 1) b1 = v;
-                else b2 = v;
-                nb++;
             }
+            while (pos < lim && o < room) out[o++] = (int32_t)(decode_sym(slot, pos, T) + offset);
         }
-        if (nb > 0) out[o] = b0;
-        if (nb > 1) out[o + 1] = b1;
-        if (nb > 2) out[o + 2] = b2;
+        if (pos < lim || pos >= kBadPath) atomicOr(err_word, 16u);
     }
 }
 
@@ -670,15 +753,22 @@ template cudaError_t launch_encode_tiles<int32_t>(const EncStream *, uint32_t, c
 template cudaError_t launch_encode_tiles<int64_t>(const EncStream *, uint32_t, const uint64_t *, uint64_t, uint64_t *, uint64_t *,
                                                   void *, size_t &, cudaStream_t);
 
-// Persistent decode grid: up to 6 CTAs of 256 threads per SM (a table takes up to 32 KB).
-static unsigned decode_grid(uint64_t ntiles) { return (unsigned)(ntiles < 148 * 6 ? (ntiles ? ntiles : 1) : 148 * 6); }
+// Persistent decode grid: up to 4 CTAs of 256 threads per SM, each with a tile's payload and a table
+// of up to 16 KB.
+static unsigned decode_grid(uint64_t ntiles) { return (unsigned)(ntiles < 148 * 4 ? (ntiles ? ntiles : 1) : 148 * 4); }
+static size_t decode_smem(uint32_t max_lut_bits) {
+    return kDecodeSlotBytes + std::max<size_t>(((size_t)1 << max_lut_bits) * 4, 16);
+}
 
 cudaError_t launch_decode_sync(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
-                               uint64_t ntiles, uint32_t max_lut_bits, const LutEntry *luts, const uint32_t *childs,
+                               uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
+                               const uint32_t *childs,
                                int first_pass, uint64_t *start, uint64_t *end, uint64_t *count, const uint32_t *moved,
                                uint32_t *err, cudaStream_t st) {
-    const size_t sh = ((size_t)1 << max_lut_bits) * sizeof(LutEntry);
-    decode_sync_kernel<<<decode_grid(ntiles), kDecodeTile, sh, st>>>(base, chunk_bits, streams, tile_stream, ntiles, luts,
+    const size_t sh = decode_smem(max_lut_bits);
+    const cudaError_t e = cudaFuncSetAttribute(decode_sync_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    if (e != cudaSuccess) return e;
+    decode_sync_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, chunk_bits, streams, tile_stream, ntiles, luts, lut2s,
                                                                       childs, first_pass, start, end, count, moved, err);
     count_launch();
     return cudaGetLastError();
@@ -693,18 +783,24 @@ cudaError_t launch_decode_restart(const DecStream *streams, uint32_t nstreams, u
     return cudaGetLastError();
 }
 
-cudaError_t launch_decode_check(const DecStream *streams, uint32_t nstreams, const uint64_t *off, const uint64_t *end,
-                                uint32_t *err, cudaStream_t st) {
-    decode_check_kernel<<<(nstreams + 63) / 64, 64, 0, st>>>(streams, nstreams, off, end, err);
+cudaError_t launch_decode_check(const DecStream *streams, uint32_t nstreams, const uint32_t *tile_stream, uint64_t ntiles,
+                                const uint64_t *off, const uint64_t *start, const uint64_t *end, uint32_t *err,
+                                uint32_t *changed, cudaStream_t st) {
+    const uint64_t n = std::max<uint64_t>(ntiles * (kDecodeTile / kDecodeRun), nstreams);
+    decode_check_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(streams, nstreams, tile_stream, ntiles, off, start, end, err,
+                                                                      changed);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_decode_write(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
-                                uint64_t ntiles, uint32_t max_lut_bits, const LutEntry *luts, const uint32_t *childs,
+                                uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
+                               const uint32_t *childs,
                                 const uint64_t *start, const uint64_t *off, uint32_t *err, cudaStream_t st) {
-    const size_t sh = ((size_t)1 << max_lut_bits) * sizeof(LutEntry);
-    decode_write_kernel<<<decode_grid(ntiles), kDecodeTile, sh, st>>>(base, chunk_bits, streams, tile_stream, ntiles, luts, childs,
+    const size_t sh = decode_smem(max_lut_bits);
+    const cudaError_t e = cudaFuncSetAttribute(decode_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    if (e != cudaSuccess) return e;
+    decode_write_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, chunk_bits, streams, tile_stream, ntiles, luts, lut2s, childs,
                                                                        start, off, err);
     count_launch();
     return cudaGetLastError();

@@ -21,24 +21,22 @@ struct CodeEntry {
     uint32_t len;
 };
 
-struct LutEntry {
-    uint32_t sym;   // symbol index (value - offset), or tree node when len == 0
-    uint32_t len;
-};
-
 // One stream of a batched decode (see k_huff.cu). Chunks of the stream are chunk0 .. chunk0 +
 // nchunks - 1 in the global numbering; its tiles start at tile0.
 struct DecStream {
     uint64_t bit_begin, bit_end;   // payload bits, absolute from the stream buffer base
     uint64_t chunk0, nchunks, tile0;
-    uint64_t lut_off, child_off;   // entries into the batched table arenas
+    uint64_t lut_off, lut2_off, child_off;   // entries into the batched table arenas (lut_off a multiple of 4)
     uint64_t count;                // values the stream must produce
     int64_t offset;                // added to each symbol index
     void *out;                     // int64 values when wide, else int32
     uint32_t lut_bits, wide;
 };
 
-constexpr uint32_t kDecodeTile = 256;  // chunks per tile (threads per decode CTA)
+// A decode CTA has a tile of chunks, a run of them a warp, whose first lanes decode the chunks before
+// its run as well.
+constexpr uint32_t kDecodeThreads = 256, kDecodeHalo = 2, kDecodeRun = 32 - kDecodeHalo,
+                   kDecodeTile = kDecodeThreads / 32 * kDecodeRun;
 
 // One candidate predictor of a plan-search layer (generate_config.tpp:526-604): its sample lattice
 // (start, stride and count per axis; loop nest ax[0] outer .. ax[2] inner), stencil geometry along
@@ -213,15 +211,18 @@ cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uin
                                 uint64_t *err, void *tmp, size_t &tmp_bytes, cudaStream_t st);
 cudaError_t launch_scan_u64(const uint64_t *in, uint64_t *out, uint64_t n, void *tmp, size_t &tmp_bytes, cudaStream_t st);
 cudaError_t launch_decode_sync(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
-                               uint64_t ntiles, uint32_t max_lut_bits, const LutEntry *luts, const uint32_t *childs,
+                               uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
+                               const uint32_t *childs,
                                int first_pass, uint64_t *start, uint64_t *end, uint64_t *count, const uint32_t *moved,
                                uint32_t *err, cudaStream_t st);
 cudaError_t launch_decode_restart(const DecStream *streams, uint32_t nstreams, uint64_t nchunks, const uint64_t *end,
                                   uint64_t *start, uint32_t *moved, uint32_t *changed, cudaStream_t st);
-cudaError_t launch_decode_check(const DecStream *streams, uint32_t nstreams, const uint64_t *off, const uint64_t *end,
-                                uint32_t *err, cudaStream_t st);
+cudaError_t launch_decode_check(const DecStream *streams, uint32_t nstreams, const uint32_t *tile_stream, uint64_t ntiles,
+                                const uint64_t *off, const uint64_t *start, const uint64_t *end, uint32_t *err,
+                                uint32_t *changed, cudaStream_t st);
 cudaError_t launch_decode_write(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
-                                uint64_t ntiles, uint32_t max_lut_bits, const LutEntry *luts, const uint32_t *childs,
+                                uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
+                               const uint32_t *childs,
                                 const uint64_t *start, const uint64_t *off, uint32_t *err, cudaStream_t st);
 template <class T>
 cudaError_t launch_fill(T *out, uint64_t n, T v, cudaStream_t st);
