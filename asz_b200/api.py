@@ -122,6 +122,8 @@ def lib():
     L.asz_decompress.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.POINTER(C.c_uint64), C.c_float,
                                  C.POINTER(Params), C.c_void_p, C.c_int, C.POINTER(Report)]
     L.asz_free.argtypes = [C.c_void_p]
+    L.asz_copy_output.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t]
+    L.asz_copy_output.restype = None
     L.asz_compress_stats.argtypes = [C.c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_double)]
     for name, elem in (("asz_debug_qb", None), ("asz_debug_t", None), ("asz_debug_recon", None),
                        ("asz_debug_pre_zstd", None)):
@@ -165,6 +167,13 @@ def _dims(shape):
     if len(shape) != 3:
         raise ValueError("fields are three-dimensional")
     return (C.c_uint64 * 3)(*[int(s) for s in shape])
+
+
+# A new bytes object of n bytes, and where they lie; they are written once, before anyone else sees it.
+_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.argtypes, _new_bytes.restype = [C.c_void_p, C.c_ssize_t], C.py_object
+_bytes_at = C.pythonapi.PyBytes_AsString
+_bytes_at.argtypes, _bytes_at.restype = [C.py_object], C.c_void_p
 
 
 def _is_cuda_tensor(x):
@@ -237,6 +246,18 @@ class Context:
         if rc != 0:
             raise AszError(rc, self._L.asz_last_error(self._c).decode())
 
+    def _take(self, out, n: int) -> bytes:
+        """The bytes of a library output, which is released. A large one is copied on the library's worker
+        threads: its pages are fresh, and one thread maps and fills them at a few GB/s."""
+        try:
+            if n <= 32 << 20:
+                return C.string_at(out, n)
+            blob = _new_bytes(None, n)
+            self._L.asz_copy_output(self._c, _bytes_at(blob), out, n)
+            return blob
+        finally:
+            self._L.asz_free(out)
+
     def _use_torch_stream(self, x):
         import torch
         self._L.asz_set_stream(self._c, C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream))
@@ -259,11 +280,7 @@ class Context:
             rc = self._L.asz_compress(self._c, C.c_void_p(a.ctypes.data), 0, _dims(a.shape), C.c_float(rel_eb),
                                       C.byref(p), plan.encode() if plan else None, C.byref(out), C.byref(n), C.byref(rep))
         self._check(rc)
-        try:
-            blob = C.string_at(out, n.value)
-        finally:
-            self._L.asz_free(out)
-        return blob, rep
+        return self._take(out, n.value), rep
 
     def decompress(self, blob: bytes, shape, rel_eb: float, params: Params | None = None, out=None):
         """Decompress .asz bytes; returns a NumPy array, or fills the CUDA tensor `out`."""
@@ -276,16 +293,17 @@ class Context:
             if not _is_cuda_tensor(out):
                 raise ValueError("out must be a CUDA tensor (omit it to get a NumPy array)")
             _check_device_field(out, self.device, "out", numel)
-        buf = C.create_string_buffer(bytes(blob), len(blob))
+        data = bytes(blob)  # itself, when it is bytes: the library reads it in place
+        buf = C.c_void_p(_bytes_at(data))
         if out is not None:
             self._use_torch_stream(out)
-            rc = self._L.asz_decompress(self._c, buf, len(blob), _dims(shape), C.c_float(rel_eb), C.byref(p),
+            rc = self._L.asz_decompress(self._c, buf, len(data), _dims(shape), C.c_float(rel_eb), C.byref(p),
                                         C.c_void_p(out.data_ptr()), 1, C.byref(rep))
             self._L.asz_set_stream(self._c, None)
             self._check(rc)
             return out, rep
         res = np.empty(tuple(int(s) for s in shape), dtype=np.float32)
-        rc = self._L.asz_decompress(self._c, buf, len(blob), _dims(shape), C.c_float(rel_eb), C.byref(p),
+        rc = self._L.asz_decompress(self._c, buf, len(data), _dims(shape), C.c_float(rel_eb), C.byref(p),
                                     C.c_void_p(res.ctypes.data), 0, C.byref(rep))
         self._check(rc)
         return res, rep
@@ -314,11 +332,7 @@ class Context:
                                              C.byref(p), plan.encode(), C.c_void_p(codes.ctypes.data), codes.size,
                                              C.byref(out), C.byref(n), C.byref(rep))
         self._check(rc)
-        try:
-            blob = C.string_at(out, n.value)
-        finally:
-            self._L.asz_free(out)
-        return blob, rep
+        return self._take(out, n.value), rep
 
     def compress_batch(self, fields, rel_eb: float, plan: str, family: str = "cubic", params: Params | None = None,
                        t_tables=None):
@@ -371,8 +385,7 @@ class Context:
         self._check(rc)
         blobs = []
         for i in range(n):
-            blobs.append(C.string_at(outs[i], lens[i]))
-            self._L.asz_free(outs[i])
+            blobs.append(self._take(outs[i], lens[i]))
         return blobs, list(reps), br
 
     def set_tsel_mode(self, mode: int):

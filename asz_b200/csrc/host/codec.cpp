@@ -13,6 +13,7 @@
 // them, so the host values are the reference's on the same machine.
 #include <cuda_runtime.h>
 #include <immintrin.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <chrono>
@@ -40,12 +41,14 @@
 #include "../listsim.cuh"
 #include "../../../include/asz_b200.h"
 #include "buffers.h"
+#include "host_pool.h"
 #include "huffman_host.h"
 #include "internal.h"
 #include "zstd_api.h"
 
 using namespace asz;
 using asz::host::DevBuf;
+using asz::host::HostPool;
 using asz::host::PinnedBuf;
 
 namespace {
@@ -106,67 +109,6 @@ struct Geometry {
     u64 pivots = 0, nblocks = 0;
 };
 
-}  // namespace
-
-namespace {
-// Worker threads kept for a context's host-side parallel loops: run(n, f) calls f(0..n-1) on the
-// workers and the calling thread, and returns when all calls have returned.
-class HostPool {
-public:
-    explicit HostPool(unsigned workers) {
-        for (unsigned i = 0; i < workers; i++) th_.emplace_back([this] { loop(); });
-    }
-    ~HostPool() {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            stop_ = true;
-        }
-        cv_.notify_all();
-        for (auto &t : th_) t.join();
-    }
-    void run(uint64_t n, const std::function<void(uint64_t)> &f) {
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            fn_ = &f;
-            n_ = n;
-            next_ = 0;
-            active_ = th_.size();
-            ++gen_;
-        }
-        cv_.notify_all();
-        work();
-        std::unique_lock<std::mutex> l(mu_);
-        done_.wait(l, [&] { return active_ == 0; });
-        fn_ = nullptr;
-    }
-
-private:
-    void work() {
-        for (uint64_t j; (j = next_.fetch_add(1)) < n_;) (*fn_)(j);
-    }
-    void loop() {
-        uint64_t seen = 0;
-        for (;;) {
-            {
-                std::unique_lock<std::mutex> l(mu_);
-                cv_.wait(l, [&] { return stop_ || gen_ != seen; });
-                if (stop_) return;
-                seen = gen_;
-            }
-            work();
-            std::lock_guard<std::mutex> g(mu_);
-            if (--active_ == 0) done_.notify_one();
-        }
-    }
-    std::vector<std::thread> th_;
-    std::mutex mu_;
-    std::condition_variable cv_, done_;
-    const std::function<void(uint64_t)> *fn_ = nullptr;
-    std::atomic<uint64_t> next_{0};
-    uint64_t n_ = 0, gen_ = 0;
-    size_t active_ = 0;
-    bool stop_ = false;
-};
 }  // namespace
 
 namespace {
@@ -266,6 +208,14 @@ struct asz_ctx {
     PinnedBuf batch_pre[2];  // batches: two chunks of fields' streams, one encoding while one is compressed
     PinnedBuf raw_in;     // decompress: the stream after zstd
     PinnedBuf words;      // a few result words of a call
+    PinnedBuf enc_host;   // encoding: histograms on their way here, code tables on theirs there
+    // Transfers of large pageable host buffers: pinned slots, and the events of the copies that use them.
+    PinnedBuf stage;
+    std::vector<cudaEvent_t> stage_ev;
+    // Plan search: per candidate, its framed stream and zstd output (kept, so that their pages are
+    // mapped once).
+    std::vector<std::array<std::vector<uint8_t>, 2>> plan_bufs;
+    PinnedBuf plan_host;
     bool have_last = false;
     // Profiling (asz_profile_*).
     bool prof = false;
@@ -402,6 +352,15 @@ std::mutex g_out_mu;
 std::vector<uint8_t *> g_out_cache;  // block starts (header), oldest first
 uint64_t g_out_cached = 0;
 
+// Large pages for a fresh block so large that malloc maps it by itself (a page fault each 2 MiB
+// instead of each 4 KiB). Smaller ones come from the heap, whose pages are mapped already.
+constexpr size_t kOwnMapping = 32u << 20;
+void advise_huge(void *p, size_t n) {
+    constexpr uintptr_t kHuge = 2u << 20;
+    const uintptr_t b = ((uintptr_t)p + kHuge - 1) / kHuge * kHuge, e = ((uintptr_t)p + n) / kHuge * kHuge;
+    if (n > kOwnMapping && e > b) madvise((void *)b, e - b, MADV_HUGEPAGE);
+}
+
 uint8_t *out_alloc(size_t n) {
     {
         std::lock_guard<std::mutex> g(g_out_mu);
@@ -419,6 +378,7 @@ uint8_t *out_alloc(size_t n) {
     }
     uint8_t *b = (uint8_t *)std::malloc(kOutHeader + (n ? n : 1));
     if (!b) return nullptr;
+    advise_huge(b, kOutHeader + n);
     *reinterpret_cast<OutHeader *>(b) = OutHeader{kOutMagic, (uint64_t)(n ? n : 1)};
     return b + kOutHeader;
 }
@@ -440,6 +400,99 @@ void out_release(uint8_t *p) {
         cudaError_t e_ = (call);                                                    \
         if (e_ != cudaSuccess) return fail(ctx, ASZ_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
+
+HostPool &host_pool(asz_ctx *ctx) {
+    if (!ctx->pool) ctx->pool = std::make_unique<HostPool>(std::min(15u, std::max(1u, std::thread::hardware_concurrency()) - 1));
+    return *ctx->pool;
+}
+
+// Copies on the worker threads, in pieces: one thread moves about 10 GB/s, and less into pages that
+// are not mapped yet.
+constexpr size_t kCopyPiece = 512 << 10;
+void parallel_copy(asz_ctx *ctx, void *dst, const void *src, size_t n) {
+    if (n <= 2 * kCopyPiece) {
+        std::memcpy(dst, src, n);
+        return;
+    }
+    host_pool(ctx).run((n + kCopyPiece - 1) / kCopyPiece, [&](uint64_t k) {
+        const size_t o = k * kCopyPiece;
+        std::memcpy((uint8_t *)dst + o, (const uint8_t *)src + o, std::min(kCopyPiece, n - o));
+    });
+}
+
+// Host memory to and from the device. A large buffer that is not pinned goes through pinned slots,
+// filled (or emptied) by the worker threads while the slot before is on its way: the driver's own
+// staging of pageable memory is one thread (100 MB in: 9.0 ms, now 3.7; the same out into fresh
+// pages: 21 ms, now 6.1). Small or pinned buffers are copied as they are.
+constexpr size_t kStageSlot = 8 << 20, kStageSlots = 3, kStageLeast = 4 << 20;
+
+int stage_ready(asz_ctx *ctx, const void *host, size_t bytes, bool &staged) {
+    staged = false;
+    if (bytes < kStageLeast) return ASZ_OK;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        cudaGetLastError();
+        return ASZ_OK;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return ASZ_OK;
+    CK(ctx->stage.reserve(kStageSlots * kStageSlot));
+    while (ctx->stage_ev.size() < kStageSlots) {
+        cudaEvent_t e;
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ctx->stage_ev.push_back(e);
+    }
+    for (cudaEvent_t e : ctx->stage_ev) CK(cudaEventSynchronize(e));  // an earlier call's copies
+    staged = true;
+    return ASZ_OK;
+}
+
+// The copy is in flight on `st` on return; `src` has been read unless it is pinned.
+int copy_in(asz_ctx *ctx, void *d_dst, const void *src, size_t bytes, cudaStream_t st) {
+    bool staged;
+    int rc = stage_ready(ctx, src, bytes, staged);
+    if (rc) return rc;
+    if (!staged) {
+        CK(cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, st));
+        return ASZ_OK;
+    }
+    for (size_t o = 0, k = 0; o < bytes; o += kStageSlot, k = (k + 1) % kStageSlots) {
+        const size_t n = std::min(kStageSlot, bytes - o);
+        uint8_t *slot = ctx->stage.p + k * kStageSlot;
+        if (o >= kStageSlots * kStageSlot) CK(cudaEventSynchronize(ctx->stage_ev[k]));
+        parallel_copy(ctx, slot, (const uint8_t *)src + o, n);
+        CK(cudaMemcpyAsync((uint8_t *)d_dst + o, slot, n, cudaMemcpyHostToDevice, st));
+        CK(cudaEventRecord(ctx->stage_ev[k], st));
+    }
+    return ASZ_OK;
+}
+
+// The data is in `dst` on return.
+int copy_out(asz_ctx *ctx, void *dst, const void *d_src, size_t bytes, cudaStream_t st) {
+    bool staged;
+    int rc = stage_ready(ctx, dst, bytes, staged);
+    if (rc) return rc;
+    if (!staged) {
+        CK(cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        return ASZ_OK;
+    }
+    const size_t slots = (bytes + kStageSlot - 1) / kStageSlot;
+    auto size_of = [&](size_t i) { return std::min(kStageSlot, bytes - i * kStageSlot); };
+    for (size_t i = 0; i < slots + kStageSlots - 1; i++) {
+        if (i < slots) {
+            CK(cudaMemcpyAsync(ctx->stage.p + i % kStageSlots * kStageSlot, (const uint8_t *)d_src + i * kStageSlot, size_of(i),
+                               cudaMemcpyDeviceToHost, st));
+            CK(cudaEventRecord(ctx->stage_ev[i % kStageSlots], st));
+        }
+        if (i + 1 < kStageSlots) continue;
+        const size_t k = i + 1 - kStageSlots;
+        if (k >= slots) break;
+        CK(cudaEventSynchronize(ctx->stage_ev[k % kStageSlots]));
+        parallel_copy(ctx, (uint8_t *)dst + k * kStageSlot, ctx->stage.p + k % kStageSlots * kStageSlot, size_of(k));
+    }
+    return ASZ_OK;
+}
+
 
 int validate(asz_ctx *ctx, const asz_params &p, bool compress_side) {
     // validate_parameters (s1_compress.cpp:49-99) and s1_decompress.cpp:112-125.
@@ -858,6 +911,10 @@ void asz_destroy(asz_ctx *c) {
     c->batch_pre[1].release();
     c->raw_in.release();
     c->words.release();
+    c->enc_host.release();
+    c->stage.release();
+    c->plan_host.release();
+    for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
     asz::host::sweep_release(c->sweep);
     for (ZSTD_CCtx *z : c->zfree) ZSTD_freeCCtx(z);
@@ -878,6 +935,19 @@ void asz_free(void *p) {
     if (!p) return;
     // Every buffer this library hands out is an output block (out_alloc).
     out_release(static_cast<uint8_t *>(p));
+}
+
+void asz_copy_output(asz_ctx *ctx, void *dst, const void *src, size_t n) {
+    if (!ctx || !dst || !src) return;
+    // Up to kOwnMapping one thread is the better one: 13 MB take it 0.7 ms against 0.1, but zstd then
+    // writes the next stream into lines that the other cores share, which cost it 1 ms. 110 MB into
+    // fresh pages: 45 ms by one thread, 4 by all.
+    if (n <= kOwnMapping) {
+        std::memcpy(dst, src, n);
+        return;
+    }
+    advise_huge(dst, n);
+    parallel_copy(ctx, dst, src, n);
 }
 
 void asz_release_output_cache(void) {
@@ -1407,11 +1477,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
                 sym_lo[c] = (int64_t)ranges[2 * c] + (int64_t)a;
                 code_ok[c] = build_code(hh, sym_lo[c], (int64_t)ranges[2 * c] + (int64_t)b - 1, num[c], false, codes[c], code_err[c]);
             };
-            std::vector<std::thread> pool;
-            for (uint32_t c = 1; c < nc; c++)
-                if (num[c]) pool.emplace_back(build_one, c);
-            build_one(0);
-            for (auto &t : pool) t.join();
+            host_pool(ctx).run(nc, [&](uint64_t c) { build_one((uint32_t)c); });
         }
         for (uint32_t c = 0; c < nc; c++)
             if (!code_ok[c]) return fail(ctx, ASZ_E_UNSUPPORTED, code_err[c]);
@@ -1444,8 +1510,10 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
             CK(launch_encode<int32_t>(d_qb + pc[c].off, num[c], sym_lo[c], ctx->codes.as<CodeEntry>() + code_off[c],
                                       ctx->bitoff.as<u64>(), ctx->cubtmp.p, tb, ctx->plan_pay.as<uint32_t>() + word_off[c], st));
         }
-        std::vector<uint32_t> pay(std::max<u64>(words, 1));
-        CK(cudaMemcpyAsync(pay.data(), ctx->plan_pay.p, std::max<u64>(words, 1) * 4, cudaMemcpyDeviceToHost, st));
+        CK(ctx->plan_host.reserve(std::max<u64>(words, 1) * 4));
+        if (ctx->plan_bufs.size() < nc) ctx->plan_bufs.resize(nc);
+        const uint32_t *pay = (const uint32_t *)ctx->plan_host.p;
+        CK(cudaMemcpyAsync(ctx->plan_host.p, ctx->plan_pay.p, std::max<u64>(words, 1) * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         std::vector<u64> zlen(nc, 0);
         std::vector<char> z_ok(nc, 1);
@@ -1453,20 +1521,18 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
             auto zstd_one = [&](uint32_t c) {
                 if (!num[c]) return;
                 const HuffCode &hc = codes[c];
-                std::vector<uint8_t> bs(hc.save_size() + hc.encode_size());
+                const size_t len = hc.save_size() + hc.encode_size(), bound = ZSTD_compressBound(len);
+                std::vector<uint8_t> &bs = ctx->plan_bufs[c][0], &z = ctx->plan_bufs[c][1];
+                if (bs.size() < len) bs.resize(len);
+                if (z.size() < bound) z.resize(bound);
                 write_tree(hc, bs.data());
                 write_len_word(hc, bs.data() + hc.save_size());
-                if (hc.maxval != 1) std::memcpy(bs.data() + hc.save_size() + 8, pay.data() + word_off[c], (hc.bits + 7) >> 3);
-                std::vector<uint8_t> z(ZSTD_compressBound(bs.size()));
-                size_t zl = zstd3(ctx, z.data(), z.size(), bs.data(), bs.size());
+                if (hc.maxval != 1) std::memcpy(bs.data() + hc.save_size() + 8, pay + word_off[c], (hc.bits + 7) >> 3);
+                size_t zl = zstd3(ctx, z.data(), bound, bs.data(), len);
                 if (ZSTD_isError(zl)) z_ok[c] = 0;
                 else zlen[c] = zl;
             };
-            std::vector<std::thread> pool;
-            for (uint32_t c = 1; c < nc; c++)
-                if (num[c]) pool.emplace_back(zstd_one, c);
-            zstd_one(0);
-            for (auto &t : pool) t.join();
+            host_pool(ctx).run(nc, [&](uint64_t c) { zstd_one((uint32_t)c); });
         }
         for (uint32_t c = 0; c < nc; c++)
             if (!z_ok[c]) return fail(ctx, ASZ_E_DATA, "ZSTD_compress failed in the plan search");
@@ -2246,7 +2312,7 @@ struct EncodeArgs {
     const asz_params *p;
     const int64_t *t_given;    // a caller's t table, or nullptr
     u64 t_len, N;
-    const std::vector<PreCode> *pre = nullptr;  // QB streams' codes built during the rounds
+    std::vector<PreCode> *pre = nullptr;  // QB streams' codes built during the rounds (taken)
 };
 
 // Entropy stage of several fields at once: ranges, histograms, code builds (host threads over all
@@ -2293,11 +2359,11 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
             so[s2 + 1].lo = ranges[f][2 * s2];
             so[s2 + 1].hi = ranges[f][2 * s2 + 1];
             if (a.pre && s2 < a.pre->size() && (*a.pre)[s2].ok && so[s2 + 1].count) {
-                const PreCode &pc = (*a.pre)[s2];
+                PreCode &pc = (*a.pre)[s2];
                 so[s2 + 1].prebuilt = true;
                 so[s2 + 1].lo = pc.lo;
                 so[s2 + 1].hi = pc.hi;
-                so[s2 + 1].code = pc.code;
+                so[s2 + 1].code = std::move(pc.code);
             }
         }
         for (auto &o : so) {
@@ -2325,8 +2391,9 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
                                              (u64)(so[s2 + 1].hi - so[s2 + 1].lo) + 1, d_hist + so[s2 + 1].hist_off, st));
     }
     std::optional<HostScope> hs_h(std::in_place, ctx, "host:codes_hist_d2h");
-    std::vector<u64> hist(hist_total);
-    if (hist_total) CK(cudaMemcpyAsync(hist.data(), d_hist, hist_total * 8, cudaMemcpyDeviceToHost, st));
+    CK(ctx->enc_host.reserve(std::max<u64>(hist_total, 1) * 8));
+    const u64 *hist = (const u64 *)ctx->enc_host.p;
+    if (hist_total) CK(cudaMemcpyAsync(ctx->enc_host.p, d_hist, hist_total * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     hs_h.reset();
     std::optional<HostScope> hs_b(std::in_place, ctx, "host:codes_build");
@@ -2340,7 +2407,7 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
     auto build_one = [&](u64 j) {
         StreamOut &o = SO[jobs[j].first][jobs[j].second];
         u64 range = (u64)(o.hi - o.lo) + 1;
-        const u64 *h = hist.data() + o.hist_off;
+        const u64 *h = hist + o.hist_off;
         // Trim to the symbols present so the code's offset and range match the reference.
         u64 a0 = 0, b0 = range;
         while (a0 < b0 && h[a0] == 0) a0++;
@@ -2355,8 +2422,7 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
     u64 job_symbols = 0;
     for (auto &j : jobs) job_symbols += (u64)(SO[j.first][j.second].hi - SO[j.first][j.second].lo) + 1;
     if (jobs.size() > 2 && job_symbols > 4096) {
-        if (!ctx->pool) ctx->pool = std::make_unique<HostPool>(std::min(15u, std::max(1u, std::thread::hardware_concurrency()) - 1));
-        ctx->pool->run(jobs.size(), build_one);
+        host_pool(ctx).run(jobs.size(), build_one);
     } else {
         for (u64 j = 0; j < jobs.size(); j++) build_one(j);
     }
@@ -2377,13 +2443,15 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
         }
     }
     hs_b.reset();
-    std::vector<CodeEntry> codes(std::max<u64>(code_total, 1));
+    const u64 code_bytes = std::max<u64>(code_total, 1) * sizeof(CodeEntry);
+    CK(ctx->enc_host.reserve(code_bytes));
+    CodeEntry *codes = (CodeEntry *)ctx->enc_host.p;
     for (u64 f = 0; f < nf; f++)
         for (u64 s2 = 0; s2 < SO[f].size(); s2++)
             if (SO[f][s2].count)
-                std::copy(SO[f][s2].code.table.begin(), SO[f][s2].code.table.end(), codes.begin() + code_off[f][s2]);
-    CK(ctx->codes.reserve(codes.size() * sizeof(CodeEntry)));
-    CK(cudaMemcpyAsync(ctx->codes.p, codes.data(), codes.size() * sizeof(CodeEntry), cudaMemcpyHostToDevice, st));
+                std::copy(SO[f][s2].code.table.begin(), SO[f][s2].code.table.end(), codes + code_off[f][s2]);
+    CK(ctx->codes.reserve(code_bytes));
+    CK(cudaMemcpyAsync(ctx->codes.p, codes, code_bytes, cudaMemcpyHostToDevice, st));
     CK(ctx->payload.reserve(std::max<u64>(words_total, 1) * 4));
     CK(cudaMemsetAsync(ctx->payload.p, 0, std::max<u64>(words_total, 1) * 4, st));
     uint32_t *d_pay = ctx->payload.as<uint32_t>();
@@ -2467,6 +2535,8 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
     auto t_d2h = clk::now();
     {
         HostScope hs(ctx, "host:assembly");
+        std::vector<std::pair<const HuffCode *, uint8_t *>> trees;
+        u64 leaves = 0;
         for (u64 f = 0; f < nf; f++) {
             const EncodeArgs &a = A[f];
             const Plan &plan = *a.plan;
@@ -2486,7 +2556,8 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
                 for (int i = 0; i < 8; i++) w[i] = (uint8_t)(o.count >> (8 * i));
                 w += 8;
                 if (!o.count) continue;
-                write_tree(o.code, w);
+                trees.push_back({&o.code, w});
+                leaves += o.code.n;
                 w += o.code.save_size();
                 write_len_word(o.code, w);
                 w += 8;
@@ -2498,6 +2569,11 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
             }
             if ((u64)(w - bs0) != span[f].second) return fail(ctx, ASZ_E_DEVICE, "Huffman encoded size mismatch");
         }
+        // The trees while the payloads arrive; a few small ones are not worth waking the workers.
+        auto tree_one = [&](uint64_t k) { write_tree(*trees[k].first, trees[k].second); };
+        if (leaves > 8192) host_pool(ctx).run(trees.size(), tree_one);
+        else
+            for (u64 k = 0; k < trees.size(); k++) tree_one(k);
         CK(cudaStreamSynchronize(st));
     }
     const double d2h = secs(t_d2h, clk::now()), huff = secs(t_huff, clk::now());
@@ -2545,7 +2621,8 @@ static int compress_entry(asz_ctx *ctx, const float *in, int in_on_device, const
     auto t0 = clk::now();
     if (!in_on_device) {
         CK(ctx->in.reserve(N * sizeof(float)));
-        CK(cudaMemcpyAsync(ctx->in.p, in, N * sizeof(float), cudaMemcpyHostToDevice, st));
+        rc = copy_in(ctx, ctx->in.p, in, N * sizeof(float), st);
+        if (rc) return rc;
         d_in = ctx->in.as<float>();
     }
     CK(cudaStreamSynchronize(st));
@@ -2725,7 +2802,8 @@ extern "C" int asz_grad_setup(asz_ctx *ctx, const float *in, int in_on_device, c
     const float *d_in = in;
     if (!in_on_device) {
         CK(ctx->in.reserve(N * sizeof(float)));
-        CK(cudaMemcpyAsync(ctx->in.p, in, N * sizeof(float), cudaMemcpyHostToDevice, st));
+        rc = copy_in(ctx, ctx->in.p, in, N * sizeof(float), st);
+        if (rc) return rc;
         d_in = ctx->in.as<float>();
     }
     float mn, mx;
@@ -3081,8 +3159,7 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
             pok[s] = parse_stream(bsp, raw, at, hp[s], perr[s]) && at == send[s];
             if (!pok[s] && perr[s].empty()) perr[s] = "corrupt Huffman stream";
         };
-        if (!ctx->pool) ctx->pool = std::make_unique<HostPool>(std::min(15u, std::max(1u, std::thread::hardware_concurrency()) - 1));
-        ctx->pool->run(L + 2, parse_one);
+        host_pool(ctx).run(L + 2, parse_one);
         for (u64 s = 0; s < L + 2; s++) {
             if (!pok[s]) return fail(ctx, ASZ_E_DATA, perr[s]);
             // Every code is at least one bit, and a single-symbol stream still has to fit the
@@ -3189,8 +3266,8 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     R.core_s = secs(t_core, clk::now());
     if (!out_on_device) {
         auto t1 = clk::now();
-        CK(cudaMemcpyAsync(out, d_out, N * sizeof(float), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        rc = copy_out(ctx, out, d_out, N * sizeof(float), st);
+        if (rc) return rc;
         R.d2h_s = secs(t1, clk::now());
     }
     if (rep) {
@@ -3575,7 +3652,8 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     if (!in_on_device) {
         CK(ctx->b_in.reserve(in_total * sizeof(float)));
         for (uint32_t f = 0; f < nf; f++) {
-            CK(cudaMemcpyAsync(ctx->b_in.as<float>() + B[f].o_in, in[f], B[f].N * sizeof(float), cudaMemcpyHostToDevice, st));
+            rc = copy_in(ctx, ctx->b_in.as<float>() + B[f].o_in, in[f], B[f].N * sizeof(float), st);
+            if (rc) return rc;
             B[f].d_in = ctx->b_in.as<float>() + B[f].o_in;
         }
         CK(cudaStreamSynchronize(st));
@@ -4757,10 +4835,11 @@ int ctx_range(asz_ctx *ctx, const float *d_in, uint64_t n, bool first_max, float
 
 int ctx_upload(asz_ctx *ctx, const float *in, uint64_t n, const float **d_in) {
     CK(ctx->in.reserve(n * sizeof(float)));
-    CK(cudaMemcpyAsync(ctx->in.p, in, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     *d_in = ctx->in.as<float>();
-    return ASZ_OK;
+    return copy_in(ctx, ctx->in.p, in, n * sizeof(float), ctx->stream);
 }
+
+void ctx_parallel(asz_ctx *c, uint64_t n, const std::function<void(uint64_t)> &f) { host_pool(c).run(n, f); }
 
 void *&ctx_sweep_state(asz_ctx *c) { return c->sweep; }
 

@@ -101,28 +101,32 @@ bool build_code(const std::vector<uint64_t> &hist, int64_t min_sym, int64_t max_
         ifreq.push_back(fu + fv);
     }
     c.root = c.left.size() - 1;
-    // dfs_vec (huffman.hpp:80-95): bit k of the code is the branch taken at depth k+1.
-    struct Item {
-        uint64_t node;
-        uint32_t len;
+    // dfs_vec (huffman.hpp:80-95): bit k of the code is the branch taken at depth k+1. A node's
+    // children come before it, so one pass from the root down meets every parent first.
+    struct Path {
         uint64_t code;
+        uint32_t len;
     };
-    std::vector<Item> st{{c.root, 0, 0}};
-    while (!st.empty()) {
-        Item it = st.back();
-        st.pop_back();
-        if (it.node < n) {
-            if (it.len > 32) {
-                err = "Huffman code longer than 32 bits";
-                return false;
-            }
-            c.table[c.leaf_sym[it.node]] = CodeEntry{(uint32_t)it.code, it.len};
-            c.max_len = std::max(c.max_len, it.len);
-            c.bits += freq[it.node] * it.len;
-            continue;
+    std::vector<Path> path(n - 1);  // of the internal nodes
+    path[c.root - n] = Path{0, 0};
+    for (uint64_t k = c.root; k >= n; k--) {
+        const Path p = path[k - n];
+        if (p.len >= 32) {
+            err = "Huffman code longer than 32 bits";
+            return false;
         }
-        st.push_back({(uint64_t)c.right[it.node], it.len + 1, it.code | (1ull << it.len)});
-        st.push_back({(uint64_t)c.left[it.node], it.len + 1, it.code});
+        const uint64_t child[2] = {(uint64_t)c.left[k], (uint64_t)c.right[k]};
+        for (int i = 0; i < 2; i++) {
+            const uint64_t code = p.code | (uint64_t)i << p.len;
+            const uint32_t len = p.len + 1;
+            if (child[i] >= n) {
+                path[child[i] - n] = Path{code, len};
+                continue;
+            }
+            c.table[c.leaf_sym[child[i]]] = CodeEntry{(uint32_t)code, len};
+            c.max_len = std::max(c.max_len, len);
+            c.bits += freq[child[i]] * len;
+        }
     }
     return true;
 }
@@ -146,27 +150,36 @@ void write_tree(const HuffCode &c, uint8_t *dst) {
     put_be64(p, c.maxval);
     p += 8;
     if (c.n <= 1) return;
-    // Preorder: internal node -> 0, leaf -> 1 followed by mbft bits of its symbol, LSB-first.
-    uint64_t nbits = c.n * (uint64_t)(c.mbft + 2) - 1;
-    std::fill(p, p + ((nbits + 7) >> 3), 0);
-    uint64_t bit = 0;
-    auto put = [&](unsigned v) {
-        if (v) p[bit >> 3] |= (uint8_t)(1u << (bit & 7));
-        bit++;
-    };
-    std::vector<uint64_t> st{c.root};
-    while (!st.empty()) {
-        uint64_t u = st.back();
-        st.pop_back();
-        if (u < c.n) {
-            put(1);
-            for (unsigned j = 0; j < c.mbft; j++) put((unsigned)((c.leaf_sym[u] >> j) & 1));
-        } else {
-            put(0);
-            st.push_back((uint64_t)c.right[u]);
-            st.push_back((uint64_t)c.left[u]);
+    // Preorder: internal node -> 0, leaf -> 1 followed by mbft bits of its symbol, LSB-first; written
+    // by 64-bit words.
+    uint64_t word = 0;
+    unsigned have = 0;
+    auto put = [&](uint64_t v, unsigned n) {  // n <= 63
+        word |= v << have;
+        if (have + n < 64) {
+            have += n;
+            return;
         }
+        std::memcpy(p, &word, 8);
+        p += 8;
+        word = have ? v >> (64 - have) : 0;
+        have = have + n - 64;
+    };
+    std::vector<uint32_t> st{(uint32_t)c.root};
+    while (!st.empty()) {
+        uint32_t u = st.back();
+        st.pop_back();
+        unsigned inner = 0;
+        for (; u >= c.n; inner++) {
+            st.push_back((uint32_t)c.right[u]);
+            u = (uint32_t)c.left[u];
+        }
+        for (; inner > 32; inner -= 32) put(0, 32);
+        put(0, inner);
+        put(1, 1);
+        put(c.leaf_sym[u], c.mbft);
     }
+    for (unsigned i = 0; i < have; i += 8) *p++ = (uint8_t)(word >> i);
 }
 
 void write_len_word(const HuffCode &c, uint8_t *dst) {

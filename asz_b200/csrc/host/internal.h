@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <string>
 
 struct asz_ctx;
@@ -19,6 +20,8 @@ int ctx_fail(asz_ctx *c, int code, const std::string &m);
 int ctx_range(asz_ctx *c, const float *d_in, uint64_t n, bool first_max, float &mn, float &mx);
 // Copies a host input into the context's input buffer (asynchronously on the context's stream).
 int ctx_upload(asz_ctx *c, const float *in, uint64_t n, const float **d_in);
+// f(0..n-1) on the context's worker threads and the calling one.
+void ctx_parallel(asz_ctx *c, uint64_t n, const std::function<void(uint64_t)> &f);
 // The sweep's state, created and released by host/sweep.cpp.
 void *&ctx_sweep_state(asz_ctx *c);
 void sweep_release(void *state);

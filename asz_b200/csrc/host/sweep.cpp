@@ -15,13 +15,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <climits>
 #include <cmath>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <unordered_map>
 #include <utility>
 #include <vector>
@@ -42,7 +40,7 @@ namespace {
 using u64 = uint64_t;
 using clk = std::chrono::steady_clock;
 
-// Per host worker: the framed stream, the zstd output and a zstd context, kept across rows and
+// Per stream of a batch: the framed stream, the zstd output and a zstd context, kept across rows and
 // calls so that their pages are mapped once (first writes to fresh pages cost as much as zstd).
 struct WorkerScratch {
     std::vector<uint8_t> buf, z;
@@ -217,25 +215,6 @@ void finish_row(asz_sweep_row &r, double range) {  // s2_many_prediction.cpp:423
     r.rmse = std::sqrt(r.rmse_sum / S);
     r.mae = r.mae_sum / S;
     r.psnr = 10 * std::log10((range * range / r.mse_sum) * S);
-}
-
-u64 host_workers() { return std::max(1u, std::thread::hardware_concurrency()); }
-
-// f(i, w) for i in [0, n) on up to host_workers() threads; w is the calling worker's index.
-template <class F>
-void parallel_for(u64 n, F f) {
-    const u64 nt = std::min<u64>(host_workers(), n);
-    if (nt <= 1) {
-        for (u64 i = 0; i < n; i++) f(i, 0);
-        return;
-    }
-    std::atomic<u64> next{0};
-    std::vector<std::thread> th;
-    for (u64 t = 0; t < nt; t++)
-        th.emplace_back([&, t] {
-            for (u64 i; (i = next.fetch_add(1)) < n;) f(i, t);
-        });
-    for (auto &t : th) t.join();
 }
 
 constexpr u64 kMaxSymbolRange = 1ull << 27;
@@ -413,7 +392,7 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
             std::vector<double> h1(kc);
             std::vector<std::string> cerr(kc);
             std::vector<char> ok(kc, 1);
-            parallel_for(kc, [&](u64 k, u64) {
+            host::ctx_parallel(ctx, kc, [&](u64 k) {
                 const u64 r = hoff[k + 1] - hoff[k];
                 std::vector<u64> hv(h_hist + hoff[k], h_hist + hoff[k] + r);
                 ok[k] = build_code(hv, h_mm[2 * k], h_mm[2 * k + 1], S, true, code[k], cerr[k]);
@@ -467,10 +446,10 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
             // Frame each stream (save + encode, huffman.hpp) and compress it with zstd level 3.
             std::vector<u64> hb(kc), zb(kc);
             std::vector<char> zok(kc, 1);
-            if (W.ws.size() < host_workers()) W.ws.resize(host_workers());
-            parallel_for(kc, [&](u64 k, u64 w) {
+            if (W.ws.size() < kc) W.ws.resize(kc);
+            host::ctx_parallel(ctx, kc, [&](u64 k) {
                 const HuffCode &c = code[k];
-                WorkerScratch &sc = W.ws[w];
+                WorkerScratch &sc = W.ws[k];
                 const u64 pay = c.maxval == 1 ? 0 : (c.bits + 7) / 8, len = c.save_size() + 8 + pay;
                 if (sc.buf.size() < len) sc.buf.resize(len);
                 write_tree(c, sc.buf.data());

@@ -273,6 +273,11 @@ int asz_compress_slab(asz_ctx *ctx, const asz_comm *comm, const float *planes, i
 int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const uint64_t dims[3], float rel_eb,
                    const asz_params *p, float *out, int out_on_device, asz_report *rep);
 
+/* Copies n bytes of an output into memory of the caller's on the context's worker threads (one thread
+ * writes fresh pages at a few GB/s): for bindings whose objects own their bytes. No reference
+ * counterpart. */
+void asz_copy_output(asz_ctx *ctx, void *dst, const void *src, size_t n);
+
 void asz_free(void *ptr);
 /* asz_free keeps released output buffers (at most 64 of them, 2 GiB in all) for later outputs of
  * the same or smaller size, whose memory is then already mapped. This frees them. No reference
