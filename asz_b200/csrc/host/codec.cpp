@@ -964,6 +964,18 @@ void asz_release_output_cache(void) {
 
 namespace {
 
+// What the rounds of a compression count and record, reset by one copy before them and read by one
+// copy after them.
+struct RoundWords {
+    uint32_t err, fb, amb_count, changed;
+    uint32_t why[4];  // fast path: [0] handed off (bins too spread), [1] handed off (undecided), [2] settled window by window
+    uint32_t list_count[64];
+    uint32_t spill_count[64];
+    uint32_t spill2_count[64];  // groups the global-scratch exact kernel left to the serial one
+    uint32_t hist_over[64];     // round l: a QB of its stream fell outside the histogram window
+    int32_t qb_range[2 * 64];
+};
+
 struct MiscLayout {  // small device words, one allocation
     int32_t range[2];
     unsigned long long nonfinite;
@@ -971,23 +983,71 @@ struct MiscLayout {  // small device words, one allocation
     uint32_t dec_err;      // batched Huffman decoding: error bits
     uint32_t dec_changed;  // batched Huffman decoding: a run's first chunk starts elsewhere
     uint32_t err;          // the three words of a decompression are read together
-    uint32_t fb;
-    uint32_t amb_count;
-    uint32_t changed;
-    uint32_t list_count[64];
-    uint32_t spill_count[64];
-    uint32_t spill2_count[64];  // groups the global-scratch exact kernel left to the serial one
     uint32_t all_count;
-    uint32_t why[3];  // fast path: [0] handed off (bins too spread), [1] handed off (undecided), [2] settled window by window
     uint32_t resume_count;  // fused axis-2 compression: columns waiting for the exact path
-    int32_t qb_range[2 * 64];
-    uint32_t hist_over[64];  // round l: a QB of its stream fell outside the histogram window
+    uint32_t pad;
+    RoundWords rw;
+    // Proxies of up to three boxes: what a launch needs (from m on) and what it gives (up to perr)
+    // are a copy each.
     float h1[3 * 64];
     float x[3 * 64];
     uint32_t m[3];
+    uint32_t perr;
     SampleBox boxes[3];
     ProxyEval evals[64];
 };
+
+// Pinned words of a context: the rounds' start values, and results on their way here.
+struct HostWords {
+    RoundWords rounds0;  // never changes
+    RoundWords rounds;
+    MiscLayout misc;
+    uint32_t dec[4];
+    unsigned long long enc_err[2];
+};
+
+int host_words(asz_ctx *ctx, HostWords *&w) {
+    if (!ctx->words.p) {
+        CK(ctx->words.reserve(sizeof(HostWords)));
+        RoundWords &r = ((HostWords *)ctx->words.p)->rounds0;
+        std::memset(&r, 0, sizeof(r));
+        for (int s = 0; s < 64; s++) {
+            r.qb_range[2 * s] = INT32_MAX;
+            r.qb_range[2 * s + 1] = INT32_MIN;
+        }
+    }
+    w = (HostWords *)ctx->words.p;
+    return ASZ_OK;
+}
+
+// Uploads the boxes and evaluations of a proxy launch, with its error word and counts cleared.
+int proxy_upload(asz_ctx *ctx, const SampleBox *boxes, uint32_t nb, const ProxyEval *evals, uint32_t ne) {
+    HostWords *w;
+    int rc = host_words(ctx, w);
+    if (rc) return rc;
+    MiscLayout &h = w->misc;
+    std::memset(h.m, 0, sizeof(h.m));
+    h.perr = 0;
+    std::copy(boxes, boxes + nb, h.boxes);
+    std::copy(evals, evals + ne, h.evals);
+    MiscLayout *dm = ctx->misc.as<MiscLayout>();
+    CK(cudaMemcpyAsync(dm->m, h.m, offsetof(MiscLayout, evals) + ne * sizeof(ProxyEval) - offsetof(MiscLayout, m),
+                       cudaMemcpyHostToDevice, ctx->stream));
+    return ASZ_OK;
+}
+
+// The launch's results, waited for.
+int proxy_results(asz_ctx *ctx, const MiscLayout *&h) {
+    HostWords *w;
+    int rc = host_words(ctx, w);
+    if (rc) return rc;
+    MiscLayout *dm = ctx->misc.as<MiscLayout>();
+    CK(cudaMemcpyAsync(w->misc.h1, dm->h1, offsetof(MiscLayout, boxes) - offsetof(MiscLayout, h1), cudaMemcpyDeviceToHost,
+                       ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    h = &w->misc;
+    return ASZ_OK;
+}
 
 int abmap_exact_global(asz_ctx *ctx, uint32_t ne, const float *field, u64 n1n2, u64 n2, float R2, uint32_t cap, uint32_t nb,
                        const char *prof_name, bool &done) {
@@ -995,36 +1055,98 @@ int abmap_exact_global(asz_ctx *ctx, uint32_t ne, const float *field, u64 n1n2, 
     cudaStream_t st = ctx->stream;
     const u64 stride = exact_global_stride(cap);
     CK(ctx->gscratch.reserve((u64)nb * slope_batches(ne) * stride));
-    CK(cudaMemsetAsync(&dm->err, 0, 4, st));
+    CK(cudaMemsetAsync(&dm->perr, 0, 4, st));
     {
         ProfScope ps(ctx, prof_name, 0);
         CK(launch_slope_exact_global(dm->boxes, dm->evals, ne, field, n1n2, n2, ctx->log2arena.as<float>(), R2, dm->h1, dm->x,
-                                     dm->m, &dm->err, ctx->gscratch.as<uint8_t>(), stride, cap, nb, st));
+                                     dm->m, &dm->perr, ctx->gscratch.as<uint8_t>(), stride, cap, nb, st));
     }
-    uint32_t e1 = 0;
-    CK(cudaMemcpyAsync(&e1, &dm->err, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    done = e1 == 0;
-    if (!done) CK(cudaMemsetAsync(&dm->err, 0, 4, st));
+    const MiscLayout *h;
+    int rc = proxy_results(ctx, h);
+    if (rc) return rc;
+    done = h->perr == 0;
+    if (!done) CK(cudaMemsetAsync(&dm->perr, 0, 4, st));
+    return ASZ_OK;
+}
+
+// Encodes streams of int32 ([0]) and int64 ([1]) symbols, a launch a type; their outputs are zero. The
+// error words go to the context's host words, to be looked at after the caller's synchronisation.
+struct EncodeSet {
+    std::vector<EncStream> es[2];
+    std::vector<u64> toff[2] = {{0}, {0}};  // tiles before each stream
+    void add(int wide, const EncStream &e) {
+        const u64 tile = wide ? enc_tile<int64_t>() : enc_tile<int32_t>();
+        es[wide].push_back(e);
+        toff[wide].push_back(toff[wide].back() + (e.n + tile - 1) / tile);
+    }
+};
+
+int launch_encode_set(asz_ctx *ctx, const EncodeSet &set, cudaStream_t st) {
+    HostWords *hw;
+    int rc = host_words(ctx, hw);
+    if (rc) return rc;
+    hw->enc_err[0] = hw->enc_err[1] = 0;
+    if (set.toff[0].back() + set.toff[1].back() == 0) return ASZ_OK;
+    // Layout in ctx->enc: the stream records and tile prefixes of both types (one upload), the error
+    // words, and the tiles' states (cleared together).
+    u64 at[2][2], st_at[2], bytes = 0;
+    auto place = [&](u64 n) {
+        const u64 o = bytes;
+        bytes += (n + 15) / 16 * 16;
+        return o;
+    };
+    for (int k = 0; k < 2; k++) {
+        at[k][0] = place(set.es[k].size() * sizeof(EncStream));
+        at[k][1] = place(set.toff[k].size() * sizeof(u64));
+    }
+    const u64 upload = bytes, err_at = place(2 * sizeof(u64));
+    for (int k = 0; k < 2; k++) st_at[k] = place((set.toff[k].back() + 1) * sizeof(u64));
+    CK(ctx->enc.reserve(bytes));
+    uint8_t *eb = ctx->enc.as<uint8_t>();
+    std::vector<uint8_t> up(upload);
+    for (int k = 0; k < 2; k++) {
+        if (!set.es[k].empty()) std::memcpy(up.data() + at[k][0], set.es[k].data(), set.es[k].size() * sizeof(EncStream));
+        std::memcpy(up.data() + at[k][1], set.toff[k].data(), set.toff[k].size() * sizeof(u64));
+    }
+    CK(cudaMemcpyAsync(eb, up.data(), upload, cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(eb + err_at, 0, bytes - err_at, st));
+    for (int k = 0; k < 2; k++) {
+        const EncStream *E = (const EncStream *)(eb + at[k][0]);
+        const u64 *T = (const u64 *)(eb + at[k][1]);
+        u64 *state = (u64 *)(eb + st_at[k]), *err = (u64 *)(eb + err_at) + k;
+        const uint32_t n = (uint32_t)set.es[k].size();
+        if (k == 0) CK(launch_encode_tiles<int32_t>(E, n, T, set.toff[k].back(), state, err, st));
+        else CK(launch_encode_tiles<int64_t>(E, n, T, set.toff[k].back(), state, err, st));
+    }
+    CK(cudaMemcpyAsync(hw->enc_err, eb + err_at, 2 * sizeof(u64), cudaMemcpyDeviceToHost, st));
+    return ASZ_OK;
+}
+
+int encode_set_done(asz_ctx *ctx) {  // after the synchronisation
+    const HostWords *hw = (const HostWords *)ctx->words.p;
+    if (hw->enc_err[0] | hw->enc_err[1]) return fail(ctx, ASZ_E_DEVICE, "Huffman encoder: a tile's wait for the tiles before it timed out");
     return ASZ_OK;
 }
 
 // first_max: a zero maximum takes the sign of the first largest element (std::max_element)
 // instead of the last one (std::minmax_element).
 int compute_range(asz_ctx *ctx, const float *d_in, u64 N, float &mn, float &mx, bool first_max = false) {
-    MiscLayout init{};
-    init.range[0] = INT32_MAX;
-    init.range[1] = INT32_MIN;
-    init.zfirst = ~0ull;
-    init.zlast = 0;
+    struct {
+        int32_t range[2];
+        unsigned long long nonfinite, zfirst, zlast;
+    } const init{{INT32_MAX, INT32_MIN}, 0, ~0ull, 0};
+    static_assert(sizeof(init) == offsetof(MiscLayout, dec_err), "the range's words come first");
     MiscLayout *dm = ctx->misc.as<MiscLayout>();
-    CK(cudaMemcpyAsync(dm, &init, sizeof(MiscLayout), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(dm, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
     {
         ProfScope ps(ctx, "range", N * 4);
         CK(launch_range(d_in, N, dm->range, &dm->nonfinite, ctx->stream));
     }
-    MiscLayout h;
-    CK(cudaMemcpyAsync(&h, dm, offsetof(MiscLayout, err), cudaMemcpyDeviceToHost, ctx->stream));
+    HostWords *hw;
+    int rc = host_words(ctx, hw);
+    if (rc) return rc;
+    const MiscLayout &h = hw->misc;
+    CK(cudaMemcpyAsync(&hw->misc, dm, offsetof(MiscLayout, dec_err), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (h.nonfinite) return fail(ctx, ASZ_E_DATA, "input contains a nonfinite value");
     auto tof = [](int32_t k) {
@@ -1107,25 +1229,24 @@ int default_slope_on(asz_ctx *ctx, const float *field, const uint64_t fdims[3], 
     u64 sstride;
     scratch_dims(cap, bcap, tcap, sstride);
     CK(ctx->scratch.reserve(3 * sstride));
-    CK(cudaMemcpyAsync(dm->boxes, boxes, 3 * sizeof(SampleBox), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(dm->evals, evals, sizeof(ProxyEval) * ne, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemsetAsync(&dm->err, 0, 4, ctx->stream));
+    rc = proxy_upload(ctx, boxes, 3, evals, ne);
+    if (rc) return rc;
     const float R = mx - mn;
     // The shared-memory exact kernel when the maps fit, else the same kernel with global scratch;
     // the serial kernel when a key exceeds int32 (the exact kernels then report error bit 2).
     bool serial = cap > exact_cap();
+    const MiscLayout *res = nullptr;
     if (!serial) {
         {
             ProfScope ps_slope(ctx, "slope", 0);
             CK(launch_slope_exact(dm->boxes, dm->evals, ne, d_in, dims[1] * dims[2], dims[2], ctx->log2arena.as<float>(),
-                                  R * R, dm->h1, dm->x, dm->m, &dm->err, exact_cap(), cap, 3, ctx->stream));
+                                  R * R, dm->h1, dm->x, dm->m, &dm->perr, exact_cap(), cap, 3, ctx->stream));
         }
-        uint32_t e1 = 0;
-        CK(cudaMemcpyAsync(&e1, &dm->err, 4, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (e1) {
+        rc = proxy_results(ctx, res);
+        if (rc) return rc;
+        if (res->perr) {
             serial = true;
-            CK(cudaMemsetAsync(&dm->err, 0, 4, ctx->stream));
+            CK(cudaMemsetAsync(&dm->perr, 0, 4, ctx->stream));
         }
     }
     if (serial) {
@@ -1137,16 +1258,17 @@ int default_slope_on(asz_ctx *ctx, const float *field, const uint64_t fdims[3], 
     if (serial) {
         ProfScope ps_slope(ctx, "slope_serial", 0);
         CK(launch_slope_v0(fg, dm->boxes, dm->evals, ne, d_in, ctx->log2arena.as<float>(), R * R, ctx->scratch.as<uint8_t>(),
-                           sstride, cap, bcap, tcap, dm->h1, dm->x, dm->m, &dm->err, 3, ctx->stream));
+                           sstride, cap, bcap, tcap, dm->h1, dm->x, dm->m, &dm->perr, 3, ctx->stream));
     }
-    std::vector<float> h1(3 * ne), x(3 * ne);
-    uint32_t m[3], errw;
-    CK(cudaMemcpyAsync(h1.data(), dm->h1, 4 * 3 * ne, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(x.data(), dm->x, 4 * 3 * ne, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(m, dm->m, 12, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&errw, &dm->err, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (errw) return fail(ctx, ASZ_E_DEVICE, "default-slope kernel reported an internal error");
+    if (serial) {
+        rc = proxy_results(ctx, res);
+        if (rc) return rc;
+    } else {
+        res = &((HostWords *)ctx->words.p)->misc;  // read with the last launch's error word
+    }
+    const float *h1 = res->h1, *x = res->x;
+    const uint32_t *m = res->m;
+    if (res->perr) return fail(ctx, ASZ_E_DEVICE, "default-slope kernel reported an internal error");
     float avg_h1[2] = {0, 0}, avg_psnr[2] = {0, 0};
     u64 valid[2] = {0, 0};
     for (int d = 0; d < 3; d++) {
@@ -1306,23 +1428,21 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
                 for (uint32_t k = 0; k < ne; k++) evals[k] = ProxyEval{cand_t[k], layer_eb};
                 int rc = upload_log2(ctx);
                 if (rc) return rc;
-                CK(cudaMemcpyAsync(dm->boxes, boxes, sizeof(SampleBox) * nb, cudaMemcpyHostToDevice, st));
-                CK(cudaMemcpyAsync(dm->evals, evals, sizeof(ProxyEval) * ne, cudaMemcpyHostToDevice, st));
-                CK(cudaMemsetAsync(&dm->err, 0, 4, st));
-                CK(cudaMemsetAsync(dm->m, 0, sizeof(dm->m), st));
+                rc = proxy_upload(ctx, boxes, nb, evals, ne);
+                if (rc) return rc;
+                const MiscLayout *res = nullptr;
                 bool serial = cap > exact_cap();
                 if (!serial) {
                     {
                         ProfScope ps_(ctx, "plan_abmap", 0);
                         CK(launch_slope_exact(dm->boxes, dm->evals, ne, d_in, dims[1] * dims[2], dims[2], ctx->log2arena.as<float>(),
-                                              R * R, dm->h1, dm->x, dm->m, &dm->err, exact_cap(), cap, nb, st));
+                                              R * R, dm->h1, dm->x, dm->m, &dm->perr, exact_cap(), cap, nb, st));
                     }
-                    uint32_t e1 = 0;
-                    CK(cudaMemcpyAsync(&e1, &dm->err, 4, cudaMemcpyDeviceToHost, st));
-                    CK(cudaStreamSynchronize(st));
-                    if (e1) {
+                    rc = proxy_results(ctx, res);
+                    if (rc) return rc;
+                    if (res->perr) {
                         serial = true;
-                        CK(cudaMemsetAsync(&dm->err, 0, 4, st));
+                        CK(cudaMemsetAsync(&dm->perr, 0, 4, st));
                     }
                 }
                 if (serial) {
@@ -1339,17 +1459,18 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
                     CK(ctx->scratch.reserve(3 * sstride));
                     ProfScope ps_(ctx, "plan_abmap_serial", 0);
                     CK(launch_slope_v0(fg, dm->boxes, dm->evals, ne, d_in, ctx->log2arena.as<float>(), R * R,
-                                       ctx->scratch.as<uint8_t>(), sstride, cap, bcap, tcap, dm->h1, dm->x, dm->m, &dm->err, nb,
+                                       ctx->scratch.as<uint8_t>(), sstride, cap, bcap, tcap, dm->h1, dm->x, dm->m, &dm->perr, nb,
                                        st));
                 }
-                std::vector<float> h1(nb * ne), x(nb * ne);
-                uint32_t m[3], errw;
-                CK(cudaMemcpyAsync(h1.data(), dm->h1, 4 * nb * ne, cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(x.data(), dm->x, 4 * nb * ne, cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(m, dm->m, 12, cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(&errw, &dm->err, 4, cudaMemcpyDeviceToHost, st));
-                CK(cudaStreamSynchronize(st));
-                if (errw) return fail(ctx, ASZ_E_DEVICE, "plan-search AB-map kernel reported an internal error");
+                if (serial) {
+                    rc = proxy_results(ctx, res);
+                    if (rc) return rc;
+                } else {
+                    res = &((HostWords *)ctx->words.p)->misc;  // read with the last launch's error word
+                }
+                const float *h1 = res->h1, *x = res->x;
+                const uint32_t *m = res->m;
+                if (res->perr) return fail(ctx, ASZ_E_DEVICE, "plan-search AB-map kernel reported an internal error");
                 for (uint32_t bi = 0; bi < nb; bi++) {
                     if (m[bi] == 0) continue;  // empty map: t stays 1/4
                     auto score = [&](uint32_t k) {
@@ -1600,6 +1721,7 @@ struct CoreOut {
     Geometry G;
     std::vector<u64> qb_off, qb_len;
     std::vector<PreCode> pre;  // index s: QB stream s (0: pivots, 1..L: rounds)
+    std::vector<int32_t> range;  // [min, max] per QB stream
 };
 
 int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
@@ -1684,7 +1806,13 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
     }
     const float Rg = mx - mn, R2 = Rg * Rg;
     const float t_default = 4.0f / 16;  // insufficient_sample_t (asz_param.hpp:206)
-    int32_t init_range[2] = {INT32_MAX, INT32_MIN};
+    HostWords *hw;
+    rc = host_words(ctx, hw);
+    if (rc) return rc;
+    // The serial kernel takes groups that the exact ones leave (keys outside int32): none, nearly
+    // always, so the rounds go without its launches and are repeated with them where one is left.
+    // (Ranks of a slab take their rounds together, so they do not repeat them one by one.)
+    bool with_serial = ctx->tsel_mode == 2 || a.before_round || a.agree;
     std::vector<uint32_t> overrides;  // (block, round, t bits) settled by host replays
     std::vector<AmbiguousRecord> ambs;
     uint32_t fb_total = 0;
@@ -1738,16 +1866,12 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
     const bool prebuild = a.prebuild && !line_bytes && !a.probe && !a.origin && L > 0;
     unsigned long long *d_hwin = nullptr;
     u64 *h_hist = nullptr;
-    int32_t *h_rng = nullptr;
-    uint32_t *h_over = nullptr;
     o.pre.assign(L + 1, PreCode{});
     if (prebuild) {
         CK(ctx->hwin.reserve(L * kHistWin * 8));
-        CK(ctx->hwin_host.reserve(L * kHistWin * 8 + L * 8 + L * 4 + 8 + G.pivots * 4));
+        CK(ctx->hwin_host.reserve(L * kHistWin * 8 + G.pivots * 4));
         d_hwin = ctx->hwin.as<unsigned long long>();
         h_hist = (u64 *)ctx->hwin_host.p;
-        h_rng = (int32_t *)(h_hist + L * kHistWin);
-        h_over = (uint32_t *)(h_rng + 2 * L);
         while (ctx->round_ev.size() < 2 * L) {
             cudaEvent_t e;
             CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1768,31 +1892,28 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
         CK(cudaEventRecord(ev_r, st));
         CK(cudaStreamWaitEvent(ctx->side, ev_r, 0));
         CK(cudaMemcpyAsync(h_hist + l * kHistWin, d_hwin + l * kHistWin, kHistWin * 8, cudaMemcpyDeviceToHost, ctx->side));
-        CK(cudaMemcpyAsync(h_rng + 2 * l, &dm->qb_range[2 * (l + 1)], 8, cudaMemcpyDeviceToHost, ctx->side));
-        CK(cudaMemcpyAsync(h_over + l, &dm->hist_over[l], 4, cudaMemcpyDeviceToHost, ctx->side));
         CK(cudaEventRecord(ev_c, ctx->side));
         const u64 count = qb_len[l + 1];
         PreCode *pc = &o.pre[l + 1];
         const int dev = ctx->device;
-        const u64 *hl = h_hist + l * kHistWin;
-        const int32_t *rl = h_rng + 2 * l;
-        const uint32_t *ol = h_over + l;
+        const u64 *h = h_hist + l * kHistWin;
         ctx->builder->submit([=]() {
             cudaSetDevice(dev);
             if (cudaEventSynchronize(ev_c) != cudaSuccess) return;
-            const int32_t lo = rl[0], hi = rl[1];
-            if (*ol || count == 0 || lo > hi || lo < -(int32_t)kHistHalf || hi >= (int32_t)kHistHalf) return;
-            const u64 *h = hl + (int64_t)lo + kHistHalf;
-            u64 a0 = 0, b0 = (u64)(hi - lo) + 1;
-            while (a0 < b0 && h[a0] == 0) a0++;
-            while (b0 > a0 && h[b0 - 1] == 0) b0--;
+            u64 inside = 0;
+            for (u64 i = 0; i < kHistWin; i++) inside += h[i];
+            if (count == 0 || inside != count) return;  // QBs outside the window
+            u64 a0 = 0, b0 = kHistWin;
+            while (h[a0] == 0) a0++;
+            while (h[b0 - 1] == 0) b0--;
+            const int64_t lo = -(int64_t)kHistHalf;
             std::vector<u64> hh(h + a0, h + b0);
             std::string err;
             HuffCode code;
-            if (!build_code(hh, (int64_t)lo + (int64_t)a0, (int64_t)lo + (int64_t)b0 - 1, count, false, code, err)) return;
+            if (!build_code(hh, lo + (int64_t)a0, lo + (int64_t)b0 - 1, count, false, code, err)) return;
             pc->code = std::move(code);
-            pc->lo = (int64_t)lo + (int64_t)a0;
-            pc->hi = (int64_t)lo + (int64_t)b0 - 1;
+            pc->lo = lo + (int64_t)a0;
+            pc->hi = lo + (int64_t)b0 - 1;
             pc->ok = true;
         });
         return ASZ_OK;
@@ -1801,8 +1922,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
     // range is known only then, and it is small: one value per pivot).
     auto schedule_pivot_code = [&]() -> int {
         if (!prebuild || G.pivots == 0) return ASZ_OK;
-        int32_t *h_prng = (int32_t *)(h_over + L);
-        int32_t *h_piv = h_prng + 2;
+        int32_t *h_piv = (int32_t *)(h_hist + L * kHistWin);
         if (ctx->round_ev.size() < 2 * L + 2) {
             for (int k = 0; k < 2; k++) {
                 cudaEvent_t e;
@@ -1814,7 +1934,6 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
         CK(cudaEventRecord(ev_r, st));
         CK(cudaStreamWaitEvent(ctx->side, ev_r, 0));
         CK(cudaMemcpyAsync(h_piv, d_qb + qb_off[0], G.pivots * 4, cudaMemcpyDeviceToHost, ctx->side));
-        CK(cudaMemcpyAsync(h_prng, &dm->qb_range[0], 8, cudaMemcpyDeviceToHost, ctx->side));
         CK(cudaEventRecord(ev_c, ctx->side));
         const u64 count = G.pivots;
         PreCode *pc = &o.pre[0];
@@ -1822,8 +1941,8 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
         ctx->builder->submit([=]() {
             cudaSetDevice(dev);
             if (cudaEventSynchronize(ev_c) != cudaSuccess) return;
-            const int32_t lo = h_prng[0], hi = h_prng[1];
-            if (lo > hi || (u64)((int64_t)hi - lo) >= (1ull << 24)) return;
+            const int32_t lo = *std::min_element(h_piv, h_piv + count), hi = *std::max_element(h_piv, h_piv + count);
+            if ((u64)((int64_t)hi - lo) >= (1ull << 24)) return;
             std::vector<u64> h((u64)((int64_t)hi - lo) + 1, 0);
             for (u64 i = 0; i < count; i++) {
                 const int64_t v = (int64_t)h_piv[i] - lo;
@@ -1848,12 +1967,8 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
             ctx->builder->wait();  // builds of a previous attempt
             for (PreCode &pc : o.pre) pc = PreCode{};
             CK(cudaMemsetAsync(d_hwin, 0, L * kHistWin * 8, st));
-            CK(cudaMemsetAsync(dm->hist_over, 0, sizeof(dm->hist_over), st));
         }
-        CK(cudaMemsetAsync(&dm->err, 0, 3 * sizeof(uint32_t), st));
-        CK(cudaMemsetAsync(dm->why, 0, sizeof(dm->why), st));
-        for (u64 s = 0; s <= L; s++)
-            CK(cudaMemcpyAsync(&dm->qb_range[2 * s], init_range, 8, cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(&dm->rw, &hw->rounds0, sizeof(RoundWords), cudaMemcpyHostToDevice, st));
         if (!overrides.empty()) {
             CK(ctx->overrides.reserve(overrides.size() * sizeof(uint32_t)));
             CK(cudaMemcpyAsync(ctx->overrides.p, overrides.data(), overrides.size() * sizeof(uint32_t),
@@ -1862,7 +1977,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
         // Pivots (compress.tpp:162-175).
         {
             ProfScope ps(ctx, "pivot_compress", G.pivots * 12);
-            CK(launch_pivot_compress(G.pg, d_in, d_rec, d_qb + qb_off[0], &dm->qb_range[0], st));
+            CK(launch_pivot_compress(G.pg, d_in, d_rec, d_qb + qb_off[0], &dm->rw.qb_range[0], st));
         }
         rc = schedule_pivot_code();
         if (rc) return rc;
@@ -1876,10 +1991,10 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
             uint32_t n_resume = 0;
             int cur = 0;
             lines_exact = lines_serial = 0;
-            CK(cudaMemsetAsync(dm->spill_count, 0, sizeof(dm->spill_count), st));
+            CK(cudaMemsetAsync(dm->rw.spill_count, 0, sizeof(dm->rw.spill_count), st));
             for (u64 pass = 0;; pass++) {
                 if (pass > L) return fail(ctx, ASZ_E_DEVICE, "fused rounds did not finish");
-                CK(cudaMemsetAsync(dm->list_count, 0, sizeof(dm->list_count), st));
+                CK(cudaMemsetAsync(dm->rw.list_count, 0, sizeof(dm->rw.list_count), st));
                 CK(cudaMemsetAsync(&dm->resume_count, 0, 4, st));
                 {
                     ProfScope ps(ctx, "lines_compress", pass ? 0 : lines_alg_bytes);
@@ -1887,42 +2002,42 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
                     if (pass) lls = {{kColumnsAll, line_bytes}};  // resumptions list column indices
                     for (const LinesLaunch &ll : lls)
                         CK(launch_lines_compress(G.fg, d_rounds, d_ent, d_qoff, ctx->classes.as<ClassInfo>(), d_in, d_rec,
-                                                 ctx->log2arena.as<float>(), R2, t_default, d_tval, d_tint, &dm->fb, d_qb,
-                                                 dm->qb_range, ctx->overrides.as<uint32_t>(), nov, dm->why,
-                                                 pass ? d_res[cur] : nullptr, n_resume, d_bail, dm->list_count,
-                                                 d_res[cur ^ 1], &dm->resume_count, &dm->err, ll.set, ll.bytes, st));
+                                                 ctx->log2arena.as<float>(), R2, t_default, d_tval, d_tint, &dm->rw.fb, d_qb,
+                                                 dm->rw.qb_range, ctx->overrides.as<uint32_t>(), nov, dm->rw.why,
+                                                 pass ? d_res[cur] : nullptr, n_resume, d_bail, dm->rw.list_count,
+                                                 d_res[cur ^ 1], &dm->resume_count, &dm->rw.err, ll.set, ll.bytes, st));
                 }
                 uint32_t bails[64], spills[64], nres = 0;
-                CK(cudaMemcpyAsync(bails, dm->list_count, sizeof(bails), cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(spills, dm->spill_count, sizeof(spills), cudaMemcpyDeviceToHost, st));
+                CK(cudaMemcpyAsync(bails, dm->rw.list_count, sizeof(bails), cudaMemcpyDeviceToHost, st));
+                CK(cudaMemcpyAsync(spills, dm->rw.spill_count, sizeof(spills), cudaMemcpyDeviceToHost, st));
                 CK(cudaMemcpyAsync(&nres, &dm->resume_count, 4, cudaMemcpyDeviceToHost, st));
                 CK(cudaStreamSynchronize(st));
                 for (u64 l = 0; l < L; l++) lines_serial += spills[l];
                 if (nres == 0) break;
                 if (nres > ncols) return fail(ctx, ASZ_E_DEVICE, "fused rounds listed too many columns");
-                CK(cudaMemsetAsync(dm->spill_count, 0, sizeof(dm->spill_count), st));
+                CK(cudaMemsetAsync(dm->rw.spill_count, 0, sizeof(dm->rw.spill_count), st));
                 for (u64 l = 0; l < L; l++) {
                     if (!bails[l]) continue;
                     if (bails[l] > G.nblocks) return fail(ctx, ASZ_E_DEVICE, "fused rounds listed too many blocks");
                     lines_exact += bails[l];
                     const RoundGeom &rg = G.rounds[l];
                     const ClassInfo *cls = ctx->classes.as<ClassInfo>() + 27 * l;
-                    uint32_t *d_spill = ctx->spill.as<uint32_t>(), *d_scount = &dm->spill_count[l];
+                    uint32_t *d_spill = ctx->spill.as<uint32_t>(), *d_scount = &dm->rw.spill_count[l];
                     {
                         ProfScope ps(ctx, "tsel_exact", 0);
                         CK(launch_tsel_exact(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default,
-                                             d_tval, d_tint, &dm->fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap,
-                                             &dm->amb_count, ctx->overrides.as<uint32_t>(), nov,
+                                             d_tval, d_tint, &dm->rw.fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap,
+                                             &dm->rw.amb_count, ctx->overrides.as<uint32_t>(), nov,
                                              ctx->proxies.as<float>() + G.nblocks * l * 10, d_bail + G.nblocks * l,
-                                             &dm->list_count[l], d_spill, d_scount, exact_cap(), G.cap[l], 148, st));
+                                             &dm->rw.list_count[l], d_spill, d_scount, exact_cap(), G.cap[l], 148, st));
                     }
                     {
                         ProfScope ps(ctx, "tsel_serial", 0);
                         CK(launch_tsel_v0(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default,
-                                          ctx->scratch.as<uint8_t>(), sstride, capmax, bcap, tcap, d_tval, d_tint, &dm->fb,
-                                          ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->amb_count,
+                                          ctx->scratch.as<uint8_t>(), sstride, capmax, bcap, tcap, d_tval, d_tint, &dm->rw.fb,
+                                          ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->rw.amb_count,
                                           ctx->overrides.as<uint32_t>(), nov, ctx->proxies.as<float>() + G.nblocks * l * 10,
-                                          d_spill, d_scount, slots, &dm->err, st));
+                                          d_spill, d_scount, slots, &dm->rw.err, st));
                     }
                 }
                 n_resume = nres;
@@ -1942,15 +2057,14 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
                 CK(launch_tval_from_codes(d_tint, G.nblocks, (uint32_t)L, (uint32_t)l, (float)p.t_precision, d_tval, st));
                 ProfScope ps(ctx, "round_compress", rg.targets * 12);
                 CK(launch_round_compress(G.fg, rg, d_ent, d_tval, d_in, d_rec, d_qb + qb_off[l + 1],
-                                         &dm->qb_range[2 * (l + 1)], &dm->err, 0, nullptr, st,
-                                         prebuild ? d_hwin + l * kHistWin : nullptr, prebuild ? &dm->hist_over[l] : nullptr));
+                                         &dm->rw.qb_range[2 * (l + 1)], &dm->rw.err, 0, nullptr, st,
+                                         prebuild ? d_hwin + l * kHistWin : nullptr, prebuild ? &dm->rw.hist_over[l] : nullptr));
                 rc = schedule_code(l);
                 if (rc) return rc;
                 continue;
             }
-            uint32_t *d_list = ctx->tlist.as<uint32_t>(), *d_lcount = &dm->list_count[l % 64];
-            uint32_t *d_spill = ctx->spill.as<uint32_t>(), *d_scount = &dm->spill_count[l % 64];
-            CK(cudaMemsetAsync(d_scount, 0, 4, st));
+            uint32_t *d_list = ctx->tlist.as<uint32_t>(), *d_lcount = &dm->rw.list_count[l % 64];
+            uint32_t *d_spill = ctx->spill.as<uint32_t>(), *d_scount = &dm->rw.spill_count[l % 64];
             if (tsel_mode == 0) {
                 // Blocks per class (first, middle, last along each axis), for the algorithmic bytes
                 // (one read of the 5 operands, 4 neighbours + original, per sample) and the group
@@ -1975,9 +2089,8 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
                     }
                 }
                 ProfScope ps(ctx, "tsel_fast", sample_bytes);
-                CK(cudaMemsetAsync(d_lcount, 0, 4, st));
                 CK(launch_tsel_fast(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default, d_tval,
-                                    d_tint, &dm->fb, d_list, d_lcount, ctx->overrides.as<uint32_t>(), nov, dm->why, st,
+                                    d_tint, &dm->rw.fb, d_list, d_lcount, ctx->overrides.as<uint32_t>(), nov, dm->rw.why, st,
                                     common_samples));
             } else {
                 d_list = ctx->iota.as<uint32_t>();
@@ -1986,7 +2099,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
             {
                 ProfScope ps(ctx, "tsel_exact", 0);
                 CK(launch_tsel_exact(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default, d_tval,
-                                     d_tint, &dm->fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->amb_count,
+                                     d_tint, &dm->rw.fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->rw.amb_count,
                                      ctx->overrides.as<uint32_t>(), nov, ctx->proxies.as<float>() + G.nblocks * l * 10,
                                      d_list, d_lcount, d_spill, d_scount, exact_cap(), G.cap[l], 148, st));
             }
@@ -1995,40 +2108,38 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
             uint32_t *d_left = d_spill, *d_lcnt = d_scount;
             if (G.cap[l] > exact_cap()) {
                 d_left = ctx->spill2.as<uint32_t>();
-                d_lcnt = &dm->spill2_count[l % 64];
-                CK(cudaMemsetAsync(d_lcnt, 0, 4, st));
+                d_lcnt = &dm->rw.spill2_count[l % 64];
                 ProfScope ps(ctx, "tsel_exact_global", 0);
                 CK(launch_tsel_exact_global(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default,
-                                            d_tval, d_tint, &dm->fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap,
-                                            &dm->amb_count, ctx->overrides.as<uint32_t>(), nov,
+                                            d_tval, d_tint, &dm->rw.fb, ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap,
+                                            &dm->rw.amb_count, ctx->overrides.as<uint32_t>(), nov,
                                             ctx->proxies.as<float>() + G.nblocks * l * 10, d_spill, d_scount, d_left, d_lcnt,
                                             ctx->gscratch.as<uint8_t>(), gstride, G.cap[l], ggrid, st));
             }
-            {
+            if (with_serial) {
                 ProfScope ps(ctx, "tsel_serial", 0);
                 CK(launch_tsel_v0(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default,
-                                  ctx->scratch.as<uint8_t>(), sstride, capmax, bcap, tcap, d_tval, d_tint, &dm->fb,
-                                  ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->amb_count,
+                                  ctx->scratch.as<uint8_t>(), sstride, capmax, bcap, tcap, d_tval, d_tint, &dm->rw.fb,
+                                  ctx->amb.as<AmbiguousRecord>(), (uint32_t)amb_cap, &dm->rw.amb_count,
                                   ctx->overrides.as<uint32_t>(), nov, ctx->proxies.as<float>() + G.nblocks * l * 10, d_left,
-                                  d_lcnt, slots, &dm->err, st));
+                                  d_lcnt, slots, &dm->rw.err, st));
             }
             ProfScope ps(ctx, "round_compress", rg.targets * 12);
             CK(launch_round_compress(G.fg, rg, d_ent, d_tval, d_in, d_rec, d_qb + qb_off[l + 1],
-                                     &dm->qb_range[2 * (l + 1)], &dm->err, a.probe ? 1 : 0, a.pred_out, st,
-                                     prebuild ? d_hwin + l * kHistWin : nullptr, prebuild ? &dm->hist_over[l] : nullptr));
+                                     &dm->rw.qb_range[2 * (l + 1)], &dm->rw.err, a.probe ? 1 : 0, a.pred_out, st,
+                                     prebuild ? d_hwin + l * kHistWin : nullptr, prebuild ? &dm->rw.hist_over[l] : nullptr));
             rc = schedule_code(l);
             if (rc) return rc;
         }
-        uint32_t words[3];
-        uint32_t lcounts[64], scounts[64];
-        CK(cudaMemcpyAsync(words, &dm->err, sizeof(words), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(lcounts, dm->list_count, sizeof(lcounts), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(scounts, dm->spill_count, sizeof(scounts), cudaMemcpyDeviceToHost, st));
-        uint32_t s2counts[64];
-        CK(cudaMemcpyAsync(s2counts, dm->spill2_count, sizeof(s2counts), cudaMemcpyDeviceToHost, st));
-        uint32_t why[3];
-        CK(cudaMemcpyAsync(why, dm->why, sizeof(why), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&hw->rounds, &dm->rw, sizeof(RoundWords), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        const RoundWords &rw = hw->rounds;
+        const uint32_t *lcounts = rw.list_count, *why = rw.why;
+        auto left_of = [&](u64 l) { return !line_bytes && G.cap[l] > exact_cap() ? rw.spill2_count[l] : rw.spill_count[l]; };
+        if (!with_serial) {
+            for (u64 l = 0; l < L; l++) with_serial = with_serial || left_of(l) != 0;
+            if (with_serial) continue;
+        }
         R.exact_window = why[0];
         R.exact_undecided = why[1];
         R.wide_groups = why[2];
@@ -2036,15 +2147,15 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
         R.serial_groups = 0;
         for (u64 l = 0; l < L && l < 64; l++) {
             if (tsel_mode == 0) R.exact_groups += lcounts[l];
-            R.serial_groups += !line_bytes && G.cap[l] > exact_cap() ? s2counts[l] : scounts[l];
+            R.serial_groups += left_of(l);
         }
         if (line_bytes) {
             R.exact_groups = lines_exact;
             R.serial_groups = lines_serial;
         }
-        if (words[0]) return fail(ctx, ASZ_E_DEVICE, "round kernels reported an internal error " + std::to_string(words[0]));
-        fb_total = words[1];
-        uint32_t namb = words[2];
+        if (rw.err) return fail(ctx, ASZ_E_DEVICE, "round kernels reported an internal error " + std::to_string(rw.err));
+        fb_total = rw.fb;
+        uint32_t namb = rw.amb_count;
         if (namb > amb_cap) return fail(ctx, ASZ_E_UNSUPPORTED, "too many ambiguous coefficient decisions");
         ambs.resize(namb);
         if (namb) CK(cudaMemcpy(ambs.data(), ctx->amb.p, namb * sizeof(AmbiguousRecord), cudaMemcpyDeviceToHost));
@@ -2069,6 +2180,7 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
         if (!changed) break;
         if (++reruns > 16) return fail(ctx, ASZ_E_DEVICE, "coefficient decisions did not settle");
     }
+    o.range.assign(hw->rounds.qb_range, hw->rounds.qb_range + 2 * (L + 1));
     R.reruns = (u64)reruns;
     R.t_fallback_count = fb_total;
     hs_rounds.reset();
@@ -2312,6 +2424,7 @@ struct EncodeArgs {
     const asz_params *p;
     const int64_t *t_given;    // a caller's t table, or nullptr
     u64 t_len, N;
+    const int32_t *h_ranges = nullptr;  // the same on the host, where they are there already
     std::vector<PreCode> *pre = nullptr;  // QB streams' codes built during the rounds (taken)
 };
 
@@ -2332,9 +2445,10 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
         const u64 L = A[f].plan->pred.size();
         SO[f].resize(L + 2);  // index 0: t stream, 1..L+1: QB streams
         ranges[f].resize(2 * (L + 1));
-        CK(cudaMemcpyAsync(ranges[f].data(), A[f].d_ranges, ranges[f].size() * 4, cudaMemcpyDeviceToHost, st));
+        if (A[f].h_ranges) std::copy(A[f].h_ranges, A[f].h_ranges + ranges[f].size(), ranges[f].begin());
+        else CK(cudaMemcpyAsync(ranges[f].data(), A[f].d_ranges, ranges[f].size() * 4, cudaMemcpyDeviceToHost, st));
     }
-    CK(cudaStreamSynchronize(st));
+    if (!A[0].h_ranges) CK(cudaStreamSynchronize(st));
     u64 hist_total = 0;
     for (u64 f = 0; f < nf; f++) {
         const EncodeArgs &a = A[f];
@@ -2457,63 +2571,24 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
     uint32_t *d_pay = ctx->payload.as<uint32_t>();
     CodeEntry *d_codes = ctx->codes.as<CodeEntry>();
     hs_codes.reset();
-    u64 enc_err[2] = {0, 0};  // the encoder's error words, read back with the sync below
     {
         // Every stream of every field in two launches, one per symbol type (the t streams are
         // int64, the QB streams int32).
-        std::vector<EncStream> es[2];
-        std::vector<u64> toff[2] = {{0}, {0}};
+        EncodeSet set;
         u64 enc_bytes = 0;
         for (u64 f = 0; f < nf; f++) {
             const EncodeArgs &a = A[f];
             for (u64 s2 = 0; s2 < SO[f].size(); s2++) {
                 StreamOut &o = SO[f][s2];
                 if (!o.count || o.code.maxval == 1) continue;
-                const int k = s2 == 0 ? 1 : 0;
                 const void *sym = s2 == 0 ? (const void *)a.d_tint : (const void *)(a.d_qb + (*a.qb_off)[s2 - 1]);
-                es[k].push_back(EncStream{sym, o.count, o.lo, d_codes + code_off[f][s2], d_pay + o.payload_word_off});
-                const u64 tile = k ? enc_tile<int64_t>() : enc_tile<int32_t>();
-                toff[k].push_back(toff[k].back() + (o.count + tile - 1) / tile);
+                set.add(s2 == 0, EncStream{sym, o.count, o.lo, d_codes + code_off[f][s2], d_pay + o.payload_word_off});
                 enc_bytes += o.count * (s2 == 0 ? 8 : 4) + (o.code.bits + 7) / 8;
             }
         }
-        // Layout in ctx->enc: per type the stream records, the tile prefix, tile_bits, tile_scan.
-        u64 off[2][4], bytes = 0;
-        auto place = [&](u64 n) {
-            const u64 o = bytes;
-            bytes += (n + 15) / 16 * 16;
-            return o;
-        };
-        size_t tmp_bytes = 0;
-        for (int k = 0; k < 2; k++) {
-            const u64 nt = toff[k].back();
-            off[k][0] = place(es[k].size() * sizeof(EncStream));
-            off[k][1] = place(toff[k].size() * sizeof(u64));
-            off[k][2] = place((nt + 1) * sizeof(u64));
-            off[k][3] = place((nt + 1) * sizeof(u64));
-            size_t tb = 0;
-            if (k == 0) CK(launch_encode_tiles<int32_t>(nullptr, 0, nullptr, nt, nullptr, nullptr, nullptr, tb, st));
-            else CK(launch_encode_tiles<int64_t>(nullptr, 0, nullptr, nt, nullptr, nullptr, nullptr, tb, st));
-            tmp_bytes = std::max(tmp_bytes, tb);
-        }
-        CK(ctx->enc.reserve(std::max<u64>(bytes, 16)));
-        CK(ctx->cubtmp.reserve(std::max<size_t>(tmp_bytes, 16)));
-        uint8_t *eb = ctx->enc.as<uint8_t>();
         ProfScope ps(ctx, "huff_encode", enc_bytes);
-        for (int k = 0; k < 2; k++) {
-            const u64 nt = toff[k].back();
-            if (!nt) continue;
-            CK(cudaMemcpyAsync(eb + off[k][0], es[k].data(), es[k].size() * sizeof(EncStream), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(eb + off[k][1], toff[k].data(), toff[k].size() * sizeof(u64), cudaMemcpyHostToDevice, st));
-            CK(cudaMemsetAsync(eb + off[k][2] + nt * sizeof(u64), 0, sizeof(u64), st));  // the scan's total
-            size_t tb = ctx->cubtmp.cap;
-            const EncStream *E = (const EncStream *)(eb + off[k][0]);
-            const u64 *T = (const u64 *)(eb + off[k][1]);
-            u64 *tbits = (u64 *)(eb + off[k][2]), *tscan = (u64 *)(eb + off[k][3]);
-            if (k == 0) CK(launch_encode_tiles<int32_t>(E, (uint32_t)es[k].size(), T, nt, tbits, tscan, ctx->cubtmp.p, tb, st));
-            else CK(launch_encode_tiles<int64_t>(E, (uint32_t)es[k].size(), T, nt, tbits, tscan, ctx->cubtmp.p, tb, st));
-            CK(cudaMemcpyAsync(&enc_err[k], tscan, sizeof(u64), cudaMemcpyDeviceToHost, st));
-        }
+        const int rc = launch_encode_set(ctx, set, st);
+        if (rc) return rc;
     }
     // Stream assembly (compress.tpp:233-291) in pinned memory: the host writes the headers and
     // code trees while each payload is copied from the device straight into its place.
@@ -2531,7 +2606,7 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
     // The encoding launches finish before the copy timer starts, so that d2h_s holds the copies
     // (and the host's header writing between them) and none of the kernels' time.
     CK(cudaStreamSynchronize(st));
-    if (enc_err[0] | enc_err[1]) return fail(ctx, ASZ_E_DEVICE, "Huffman encoder: a tile's wait for the tiles before it timed out");
+    if (const int rc = encode_set_done(ctx)) return rc;
     auto t_d2h = clk::now();
     {
         HostScope hs(ctx, "host:assembly");
@@ -2694,7 +2769,8 @@ static int compress_entry(asz_ctx *ctx, const float *in, int in_on_device, const
     std::vector<u64> &qb_off = co.qb_off, &qb_len = co.qb_len;
     {
         const std::vector<EncodeArgs> ea{EncodeArgs{&G, &qb_off, &qb_len, ctx->qb.as<int32_t>(), ctx->tint.as<int64_t>(),
-                                                    dm->qb_range, mn, mx, quintic, &plan, &p, t_given, t_len, N, &co.pre}};
+                                                    dm->rw.qb_range, mn, mx, quintic, &plan, &p, t_given, t_len, N, co.range.data(),
+                                                    &co.pre}};
         std::vector<asz_report *> rs{&R};
         std::vector<std::pair<u64, u64>> span;
         rc = encode_fields(ctx, ea, rs, span, ctx->pre_zstd);
@@ -3214,8 +3290,10 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     CK(ctx->axis.reserve(std::max<size_t>(G.ent.size(), 1) * sizeof(AxisEntry)));
     const AxisEntry *d_ent = ctx->axis.as<AxisEntry>();
     CK(cudaMemcpyAsync(ctx->axis.p, G.ent.data(), G.ent.size() * sizeof(AxisEntry), cudaMemcpyHostToDevice, st));
-    CK(ctx->words.reserve(64));
-    const volatile uint32_t *words = (const volatile uint32_t *)ctx->words.p;  // dec_err, dec_changed, err
+    HostWords *hw;
+    rc = host_words(ctx, hw);
+    if (rc) return rc;
+    const volatile uint32_t *words = hw->dec;  // dec_err, dec_changed, err
     auto t_core = clk::now();
     for (int attempt = 0;; attempt++) {
         rc = decode_values(ctx, run, dm, st);
@@ -3249,7 +3327,7 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
                                            ctx->qb.as<int32_t>() + qoff[l + 1], d_out, &dm->err, st));
             }
         }
-        CK(cudaMemcpyAsync(ctx->words.p, &dm->dec_err, 12, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(hw->dec, &dm->dec_err, 12, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (!words[1]) break;
         if (attempt) return fail(ctx, ASZ_E_DEVICE, "Huffman decoding did not settle");
@@ -3820,8 +3898,9 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     uint32_t *d_queue = ctx->b_queue.as<uint32_t>();
     unsigned long long *d_hand = ctx->b_hand.as<unsigned long long>(), *d_spill = ctx->b_spill.as<unsigned long long>();
     // The whole sequence: counters and ranges reset, pivots, then per round the batched fast
-    // selection, exact replay, serial spill and prediction.
-    auto enqueue = [&](const BatchShape &sh) -> int {
+    // selection, exact replay, serial spill (with `serial`: nearly always nothing is left for it) and
+    // prediction.
+    auto enqueue = [&](const BatchShape &sh, bool serial) -> int {
         CK(cudaMemcpyAsync(ctx->b_range.p, ctx->b_range0.p, (u64)nf * 2 * (L + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice,
                            st));
         CK(cudaMemsetAsync(ctx->b_cnt.p, 0, (u64)nf * sizeof(BatchCounters), st));
@@ -3848,7 +3927,8 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
                 CK(launch_tsel_exact_global_batch(dF, (uint32_t)l, ctx->log2arena.as<float>(), t_default, d_spill, q + 3, d_left,
                                                   d_lcnt, ctx->gscratch.as<uint8_t>(), gstride, capmax, ggrid, st));
             }
-            CK(launch_tsel_v0_batch(dF, (uint32_t)l, ctx->log2arena.as<float>(), t_default, ctx->scratch.as<uint8_t>(), sstride,
+            if (serial)
+                CK(launch_tsel_v0_batch(dF, (uint32_t)l, ctx->log2arena.as<float>(), t_default, ctx->scratch.as<uint8_t>(), sstride,
                                     capmax, bcap, tcap, d_left, d_lcnt, slots, st));
             CK(launch_round_compress_batch(dF, d_ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * sh[1], st));
         }
@@ -3878,7 +3958,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
                     }
                     const BatchShape sh{fast, round, shift};
                     CK(cudaEventRecord(e0, st));
-                    rc = enqueue(sh);
+                    rc = enqueue(sh, false);
                     if (rc) return rc;
                     CK(cudaEventRecord(e1, st));
                     CK(cudaEventSynchronize(e1));
@@ -3900,10 +3980,10 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     BR.tpl_shift = best[2];
     rc = upload_shape(best[2]);
     if (rc) return rc;
-    // ---- The round sequence as a CUDA graph (captured once per batch layout).
+    // ---- The round sequence as a CUDA graph (captured once per batch layout; the inputs' addresses are
+    // in the fields' records, which every call uploads).
     std::vector<uint64_t> graph_key = shape_key;
     graph_key.insert(graph_key.end(), best.begin(), best.end());
-    for (uint32_t f = 0; f < nf; f++) graph_key.push_back((uint64_t)(uintptr_t)B[f].d_in);
     for (DevBuf *d : {&ctx->b_rec, &ctx->b_qb, &ctx->b_tval, &ctx->b_tint, &ctx->b_ent, &ctx->b_cls, &ctx->b_rounds,
                       &ctx->b_qoff, &ctx->b_range, &ctx->b_range0, &ctx->b_prox, &ctx->b_amb, &ctx->b_cnt, &ctx->b_fields,
                       &ctx->b_goff, &ctx->b_poff, &ctx->b_ioff, &ctx->b_queue, &ctx->b_hand, &ctx->b_spill, &ctx->scratch,
@@ -3921,7 +4001,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
         const bool prof = ctx->prof;
         ctx->prof = false;  // no event records inside the capture
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        const int erc = enqueue(best);
+        const int erc = enqueue(best, false);
         const cudaError_t ce = cudaStreamEndCapture(st, &graph);
         ctx->prof = prof;
         if (erc) {
@@ -3943,8 +4023,20 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     CK(cudaGraphLaunch(ctx->batch_graph, st));
     CK(cudaEventRecord(r1, st));
     std::vector<BatchCounters> cnt(nf);
-    CK(cudaMemcpyAsync(cnt.data(), ctx->b_cnt.p, nf * sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    std::vector<uint32_t> queues(5 * L);
+    auto counters = [&]() -> int {
+        CK(cudaMemcpyAsync(cnt.data(), ctx->b_cnt.p, nf * sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(queues.data(), d_queue, queues.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        return ASZ_OK;
+    };
+    if ((rc = counters())) return rc;
+    bool left = false;  // a group for the serial kernel: the sequence again, with its launches
+    for (u64 l = 0; l < L; l++) left = left || queues[5 * l + (ggrid ? 4 : 3)] != 0;
+    if (left) {
+        if ((rc = enqueue(best, true))) return rc;
+        if ((rc = counters())) return rc;
+    }
     {
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, r0, r1));
@@ -4358,7 +4450,7 @@ int slab_encode(asz_ctx *ctx, SlabComm &cm, const CoreOut &co, const Plan &plan,
     std::vector<StreamOut> so(NS);
     std::vector<u64> local(NS), global(NS);
     std::vector<int32_t> rng(2 * (L + 1));
-    CK(cudaMemcpyAsync(rng.data(), dm->qb_range, rng.size() * 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(rng.data(), dm->rw.qb_range, rng.size() * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     std::vector<int32_t> rlo(L + 1), rhi(L + 1);
     for (u64 s = 0; s <= L; s++) {
@@ -4453,53 +4545,14 @@ int slab_encode(asz_ctx *ctx, SlabComm &cm, const CoreOut &co, const Plan &plan,
     CK(cudaMemsetAsync(ctx->payload.p, 0, std::max<u64>(words_total, 1) * 4, st));
     uint32_t *d_pay = ctx->payload.as<uint32_t>();
     CodeEntry *d_codes = ctx->codes.as<CodeEntry>();
-    u64 enc_err[2] = {0, 0};  // the encoder's error words, read back with the pieces
     {
-        std::vector<EncStream> es[2];
-        std::vector<u64> toff[2] = {{0}, {0}};
+        EncodeSet set;
         for (u64 s = 0; s < NS; s++) {
             if (!so[s].count || so[s].code.maxval == 1 || !local[s]) continue;
-            const int k = s == 0 ? 1 : 0;
             const void *sym = s == 0 ? (const void *)ctx->tint.as<int64_t>() : (const void *)(ctx->qb.as<int32_t>() + co.qb_off[s - 1]);
-            es[k].push_back(EncStream{sym, local[s], so[s].lo, d_codes + code_off[s], d_pay + word_off[s]});
-            const u64 tile = k ? enc_tile<int64_t>() : enc_tile<int32_t>();
-            toff[k].push_back(toff[k].back() + (local[s] + tile - 1) / tile);
+            set.add(s == 0, EncStream{sym, local[s], so[s].lo, d_codes + code_off[s], d_pay + word_off[s]});
         }
-        u64 off[2][4], bytes = 0;
-        auto place = [&](u64 n) {
-            const u64 o = bytes;
-            bytes += (n + 15) / 16 * 16;
-            return o;
-        };
-        size_t tmp_bytes = 0;
-        for (int k = 0; k < 2; k++) {
-            const u64 nt = toff[k].back();
-            off[k][0] = place(es[k].size() * sizeof(EncStream));
-            off[k][1] = place(toff[k].size() * sizeof(u64));
-            off[k][2] = place((nt + 1) * sizeof(u64));
-            off[k][3] = place((nt + 1) * sizeof(u64));
-            size_t tb = 0;
-            if (k == 0) CK(launch_encode_tiles<int32_t>(nullptr, 0, nullptr, nt, nullptr, nullptr, nullptr, tb, st));
-            else CK(launch_encode_tiles<int64_t>(nullptr, 0, nullptr, nt, nullptr, nullptr, nullptr, tb, st));
-            tmp_bytes = std::max(tmp_bytes, tb);
-        }
-        CK(ctx->enc.reserve(std::max<u64>(bytes, 16)));
-        CK(ctx->cubtmp.reserve(std::max<size_t>(tmp_bytes, 16)));
-        uint8_t *eb = ctx->enc.as<uint8_t>();
-        for (int k = 0; k < 2; k++) {
-            const u64 nt = toff[k].back();
-            if (!nt) continue;
-            CK(cudaMemcpyAsync(eb + off[k][0], es[k].data(), es[k].size() * sizeof(EncStream), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(eb + off[k][1], toff[k].data(), toff[k].size() * sizeof(u64), cudaMemcpyHostToDevice, st));
-            CK(cudaMemsetAsync(eb + off[k][2] + nt * sizeof(u64), 0, sizeof(u64), st));
-            size_t tb = ctx->cubtmp.cap;
-            const EncStream *E = (const EncStream *)(eb + off[k][0]);
-            const u64 *T = (const u64 *)(eb + off[k][1]);
-            u64 *tbits = (u64 *)(eb + off[k][2]), *tscan = (u64 *)(eb + off[k][3]);
-            if (k == 0) CK(launch_encode_tiles<int32_t>(E, (uint32_t)es[k].size(), T, nt, tbits, tscan, ctx->cubtmp.p, tb, st));
-            else CK(launch_encode_tiles<int64_t>(E, (uint32_t)es[k].size(), T, nt, tbits, tscan, ctx->cubtmp.p, tb, st));
-            CK(cudaMemcpyAsync(&enc_err[k], tscan, sizeof(u64), cudaMemcpyDeviceToHost, st));
-        }
+        if ((rc = launch_encode_set(ctx, set, st))) return rc;
     }
     // This rank's pieces, back on the host: per stream its bits, then the bytes.
     u64 piece_bytes = 0;
@@ -4513,8 +4566,7 @@ int slab_encode(asz_ctx *ctx, SlabComm &cm, const CoreOut &co, const Plan &plan,
             w += nb;
         }
         CK(cudaStreamSynchronize(st));
-        if (enc_err[0] | enc_err[1])
-            return fail(ctx, ASZ_E_DEVICE, "Huffman encoder: a tile's wait for the tiles before it timed out");
+        if ((rc = encode_set_done(ctx))) return rc;
     }
     auto t_d2h = clk::now();
     if (rank != 0) {

@@ -48,7 +48,7 @@ struct WorkerScratch {
 };
 
 struct SweepState {
-    DevBuf coef, qb, part, sums, mm, hist, first, tab, pay, enc, cub;
+    DevBuf coef, qb, part, sums, mm, hist, first, tab, pay, enc;
     PinnedBuf small, counts, payload;
     std::vector<WorkerScratch> ws;
 };
@@ -232,7 +232,7 @@ namespace asz::host {
 void sweep_release(void *state) {
     SweepState *s = (SweepState *)state;
     if (!s) return;
-    for (DevBuf *b : {&s->coef, &s->qb, &s->part, &s->sums, &s->mm, &s->hist, &s->first, &s->tab, &s->pay, &s->enc, &s->cub})
+    for (DevBuf *b : {&s->coef, &s->qb, &s->part, &s->sums, &s->mm, &s->hist, &s->first, &s->tab, &s->pay, &s->enc})
         b->release();
     s->small.release();
     s->counts.release();
@@ -424,21 +424,17 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
             if (nt) {
                 CK(cudaMemcpyAsync(W.tab.p, h_tab, tab_tot * sizeof(CodeEntry), cudaMemcpyHostToDevice, st));
                 CK(cudaMemsetAsync(W.pay.p, 0, word_off[kc] * 4, st));
-                size_t tb = 0;
-                CK(launch_encode_tiles<int64_t>(nullptr, 0, nullptr, nt, nullptr, nullptr, nullptr, tb, st));
-                const u64 o_es = 0, o_toff = (es.size() * sizeof(EncStream) + 15) / 16 * 16,
-                          o_bits = o_toff + (toff.size() * 8 + 15) / 16 * 16, o_scan = o_bits + (nt + 1) * 8 + 8;
-                CK(W.enc.reserve(o_scan + (nt + 1) * 8 + 8));
-                CK(W.cub.reserve(std::max<size_t>(tb, 16)));
+                const u64 o_toff = (es.size() * sizeof(EncStream) + 15) / 16 * 16,
+                          o_err = o_toff + (toff.size() * 8 + 15) / 16 * 16, o_state = o_err + 16, end = o_state + (nt + 1) * 8;
+                CK(W.enc.reserve(end));
                 uint8_t *eb = W.enc.as<uint8_t>();
-                CK(cudaMemcpyAsync(eb + o_es, es.data(), es.size() * sizeof(EncStream), cudaMemcpyHostToDevice, st));
+                CK(cudaMemcpyAsync(eb, es.data(), es.size() * sizeof(EncStream), cudaMemcpyHostToDevice, st));
                 CK(cudaMemcpyAsync(eb + o_toff, toff.data(), toff.size() * 8, cudaMemcpyHostToDevice, st));
-                CK(cudaMemsetAsync(eb + o_bits + nt * 8, 0, 8, st));
-                tb = W.cub.cap;
-                CK(launch_encode_tiles<int64_t>((const EncStream *)(eb + o_es), (uint32_t)es.size(), (const u64 *)(eb + o_toff),
-                                                nt, (u64 *)(eb + o_bits), (u64 *)(eb + o_scan), W.cub.p, tb, st));
+                CK(cudaMemsetAsync(eb + o_err, 0, end - o_err, st));
+                CK(launch_encode_tiles<int64_t>((const EncStream *)eb, (uint32_t)es.size(), (const u64 *)(eb + o_toff), nt,
+                                                (u64 *)(eb + o_state), (u64 *)(eb + o_err), st));
                 u64 enc_err = 0;
-                CK(cudaMemcpyAsync(&enc_err, eb + o_scan, sizeof(u64), cudaMemcpyDeviceToHost, st));
+                CK(cudaMemcpyAsync(&enc_err, eb + o_err, sizeof(u64), cudaMemcpyDeviceToHost, st));
                 CK(cudaMemcpyAsync(W.payload.p, W.pay.p, word_off[kc] * 4, cudaMemcpyDeviceToHost, st));
                 CK(cudaStreamSynchronize(st));
                 if (enc_err) return host::ctx_fail(ctx, ASZ_E_DEVICE, "Huffman encoder: a tile's wait for the tiles before it timed out");

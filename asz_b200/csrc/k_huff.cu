@@ -728,15 +728,9 @@ cudaError_t launch_encode(const T *s, uint64_t n, int64_t offset, const CodeEntr
 
 template <class T>
 cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uint64_t *toff, uint64_t ntiles, uint64_t *tile_state,
-                                uint64_t *err, void *tmp, size_t &tmp_bytes, cudaStream_t st) {
-    if (tmp == nullptr) {
-        tmp_bytes = 0;
-        return cudaSuccess;
-    }
+                                uint64_t *err, cudaStream_t st) {
     if (ntiles == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(tile_state, 0, (ntiles + 1) * sizeof(uint64_t), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(uint64_t), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     constexpr uint32_t kTile = enc_tile<T>();
     const int smem = (int)(2 * (kTile + kEncThreads) * sizeof(T) + (kTile + 2) * sizeof(uint32_t));
     e = cudaFuncSetAttribute(encode_tiles_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -749,9 +743,9 @@ cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uin
 }
 
 template cudaError_t launch_encode_tiles<int32_t>(const EncStream *, uint32_t, const uint64_t *, uint64_t, uint64_t *, uint64_t *,
-                                                  void *, size_t &, cudaStream_t);
+                                                  cudaStream_t);
 template cudaError_t launch_encode_tiles<int64_t>(const EncStream *, uint32_t, const uint64_t *, uint64_t, uint64_t *, uint64_t *,
-                                                  void *, size_t &, cudaStream_t);
+                                                  cudaStream_t);
 
 // Persistent decode grid: up to 4 CTAs of 256 threads per SM, each with a tile's payload and a table
 // of up to 16 KB.

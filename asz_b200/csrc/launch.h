@@ -192,10 +192,9 @@ cudaError_t launch_encode(const T *s, uint64_t n, int64_t offset, const CodeEntr
                           size_t &tmp_bytes, uint32_t *out, cudaStream_t st);
 // Tiled encoding of several streams of one symbol type in one launch (k_huff.cu). toff: exclusive
 // prefix of the streams' tile counts (ns + 1 entries, tiles of enc_tile<T>() symbols);
-// tile_state needs ntiles + 1 entries and err one, both cleared here; each stream's out is zeroed
-// beforehand. After the launch *err is nonzero if a tile's wait for the bit counts before it ran
-// out (the payload is then not valid). With tmp == nullptr, only sets tmp_bytes (no temporary
-// space is used).
+// tile_state needs ntiles + 1 entries and err one, both zero before the launch, as each stream's out.
+// After it *err is nonzero if a tile's wait for the bit counts before it ran out (the payload is
+// then not valid).
 constexpr uint32_t kEncThreads = 256;
 template <class T>
 ASZ_HD constexpr uint32_t enc_tile() { return sizeof(T) == 4 ? 4096u : 2048u; }
@@ -208,7 +207,7 @@ struct EncStream {
 };
 template <class T>
 cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uint64_t *toff, uint64_t ntiles, uint64_t *tile_state,
-                                uint64_t *err, void *tmp, size_t &tmp_bytes, cudaStream_t st);
+                                uint64_t *err, cudaStream_t st);
 cudaError_t launch_scan_u64(const uint64_t *in, uint64_t *out, uint64_t n, void *tmp, size_t &tmp_bytes, cudaStream_t st);
 cudaError_t launch_decode_sync(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
                                uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
