@@ -177,7 +177,7 @@ struct asz_ctx {
     std::unique_ptr<SerialWorker> builder;
     std::string err;
     // Device buffers.
-    DevBuf in, rec, qb, tval, tint, misc, scratch, log2arena, hist, codes, bitoff, cubtmp, payload, amb, overrides,
+    DevBuf in, rec, qb, tval, tint, misc, scratch, log2arena, hist, codes, cubtmp, payload, amb, overrides,
         classes, axis, pre, chunks, out, proxies, tlist, spill, iota, plan_qb, plan_e, plan_aux, plan_pay, probe_in, probe_pred,
         rounds_dev, lines_bail, lines_resume, enc;
     // Batches (asz_compress_batch): per-field slices of these arenas, the captured round sequence
@@ -215,7 +215,7 @@ struct asz_ctx {
     // Plan search: per candidate, its framed stream and zstd output (kept, so that their pages are
     // mapped once).
     std::vector<std::array<std::vector<uint8_t>, 2>> plan_bufs;
-    PinnedBuf plan_host;
+    PinnedBuf plan_host, plan_words;
     bool have_last = false;
     // Profiling (asz_profile_*).
     bool prof = false;
@@ -899,7 +899,7 @@ void asz_destroy(asz_ctx *c) {
     c->gscratch.release();
     c->spill2.release();
     for (DevBuf *b : {&c->in, &c->rec, &c->qb, &c->tval, &c->tint, &c->misc, &c->scratch, &c->log2arena, &c->hist, &c->codes,
-                      &c->bitoff, &c->cubtmp, &c->payload, &c->amb, &c->overrides, &c->classes, &c->axis, &c->pre, &c->chunks,
+                      &c->cubtmp, &c->payload, &c->amb, &c->overrides, &c->classes, &c->axis, &c->pre, &c->chunks,
                       &c->out, &c->proxies, &c->tlist, &c->spill, &c->iota, &c->plan_qb, &c->plan_e, &c->plan_aux,
                       &c->plan_pay, &c->probe_in, &c->probe_pred, &c->rounds_dev, &c->lines_bail,
                       &c->lines_resume, &c->enc, &c->b_in, &c->b_rec, &c->b_qb, &c->b_tval, &c->b_tint, &c->b_ent, &c->b_cls,
@@ -914,6 +914,7 @@ void asz_destroy(asz_ctx *c) {
     c->enc_host.release();
     c->stage.release();
     c->plan_host.release();
+    c->plan_words.release();
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
     asz::host::sweep_release(c->sweep);
@@ -1374,6 +1375,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
     for (int a = 0; a < 3; a++) fg.n[a] = dims[a];
     u64 ps[3] = {1, 1, 1};
     out = PlanSearchOut();
+    int rc;
     for (u64 layer = 0; layer < p.max_layer_num; layer++) {
         const float layer_eb = (float)((double)abs_eb * std::pow((double)p.eb_ratio, (double)layer));
         const float neg_2_layer_eb = 0.5f / layer_eb;
@@ -1426,7 +1428,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
                 const uint32_t ne = (uint32_t)cand_t.size();
                 ProxyEval evals[64];
                 for (uint32_t k = 0; k < ne; k++) evals[k] = ProxyEval{cand_t[k], layer_eb};
-                int rc = upload_log2(ctx);
+                rc = upload_log2(ctx);
                 if (rc) return rc;
                 rc = proxy_upload(ctx, boxes, nb, evals, ne);
                 if (rc) return rc;
@@ -1532,56 +1534,68 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         for (uint32_t c = 0; c < nc; c++) num[c] = pc[c].cnt[0] * pc[c].cnt[1] * pc[c].cnt[2];
         CK(ctx->plan_qb.reserve(std::max<u64>(total, 1) * 4));
         CK(ctx->plan_e.reserve(std::max<u64>(total, 1) * 4));
-        const u64 aux_cands = 0, aux_range = (nc * sizeof(PlanCand) + 255) & ~255ull, aux_mse = aux_range + 256;
-        CK(ctx->plan_aux.reserve(aux_mse + 256));
-        uint8_t *aux = ctx->plan_aux.as<uint8_t>();
-        CK(cudaMemcpyAsync(aux + aux_cands, pc.data(), nc * sizeof(PlanCand), cudaMemcpyHostToDevice, st));
-        std::vector<int32_t> rinit(2 * nc);
+        // Upload: the candidates and their ranges' start values. Counted on the device: ranges and
+        // histogram windows. On the way back beside them: the error sums.
+        const u64 cand_bytes = (nc * sizeof(PlanCand) + 255) & ~255ull, range_bytes = 256, win_bytes = (u64)nc * kPlanWin * 8;
+        const u64 at_range = cand_bytes, at_win = at_range + range_bytes, at_mse = at_win + win_bytes;
+        CK(ctx->plan_aux.reserve(at_mse + 256));
+        CK(ctx->plan_host.reserve(at_mse + 256));
+        uint8_t *aux = ctx->plan_aux.as<uint8_t>(), *haux = ctx->plan_host.p;
+        std::memcpy(haux, pc.data(), nc * sizeof(PlanCand));
+        int32_t *ranges = (int32_t *)(haux + at_range);
         for (uint32_t c = 0; c < nc; c++) {
-            rinit[2 * c] = INT32_MAX;
-            rinit[2 * c + 1] = INT32_MIN;
+            ranges[2 * c] = INT32_MAX;
+            ranges[2 * c + 1] = INT32_MIN;
         }
-        CK(cudaMemcpyAsync(aux + aux_range, rinit.data(), rinit.size() * 4, cudaMemcpyHostToDevice, st));
-        const PlanCand *d_pc = (const PlanCand *)(aux + aux_cands);
+        CK(cudaMemcpyAsync(aux, haux, at_win, cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(aux + at_win, 0, win_bytes, st));
+        const PlanCand *d_pc = (const PlanCand *)aux;
         int32_t *d_qb = ctx->plan_qb.as<int32_t>();
         {
             ProfScope ps_(ctx, "plan_sample", total * 8);
-            CK(launch_plan_sample(d_in, dims[1], dims[2], d_pc, nc, most, d_qb, ctx->plan_e.as<float>(), (int32_t *)(aux + aux_range),
-                                  st));
+            CK(launch_plan_sample(d_in, dims[1], dims[2], d_pc, nc, most, d_qb, ctx->plan_e.as<float>(), (int32_t *)(aux + at_range),
+                                  (unsigned long long *)(aux + at_win), st));
         }
-        {
-            ProfScope ps_(ctx, "plan_mse", total * 4);
-            CK(launch_plan_mse(d_pc, nc, ctx->plan_e.as<float>(), (float *)(aux + aux_mse), st));
+        // The error sums, a long chain of a few CTAs, run beside the coding on the side stream.
+        if (ctx->round_ev.size() < 2) {
+            ctx->round_ev.resize(2, nullptr);
+            for (cudaEvent_t &e : ctx->round_ev)
+                if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
-        std::vector<int32_t> ranges(2 * nc);
-        std::vector<float> mse(nc);
-        CK(cudaMemcpyAsync(ranges.data(), aux + aux_range, ranges.size() * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(mse.data(), aux + aux_mse, nc * 4, cudaMemcpyDeviceToHost, st));
+        CK(cudaEventRecord(ctx->round_ev[0], st));
+        CK(cudaStreamWaitEvent(ctx->side, ctx->round_ev[0], 0));
+        CK(launch_plan_mse(d_pc, nc, ctx->plan_e.as<float>(), (float *)(aux + at_mse), ctx->side));
+        CK(cudaMemcpyAsync(haux + at_mse, aux + at_mse, nc * 4, cudaMemcpyDeviceToHost, ctx->side));
+        CK(cudaEventRecord(ctx->round_ev[1], ctx->side));
+        struct SideDone {  // no return leaves the side stream at work on these buffers
+            cudaEvent_t e;
+            ~SideDone() { cudaEventSynchronize(e); }
+        } side_done{ctx->round_ev[1]};
+        CK(cudaMemcpyAsync(haux + at_range, aux + at_range, range_bytes + win_bytes, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         out.sample_s += secs(t_sample, clk::now());
         // ---- Huffman code of each candidate's QBs (device histogram and encoding), zstd on the host.
         auto t_lossless = clk::now();
-        std::vector<u64> hist_off(nc, 0);
-        u64 hist_total = 0;
+        // Candidates with QBs outside their window are counted over their whole range.
+        const u64 *win = (const u64 *)(haux + at_win);
+        std::vector<std::vector<u64>> wide(nc);
         for (uint32_t c = 0; c < nc; c++) {
             if (!num[c]) continue;
             const u64 range = (u64)((int64_t)ranges[2 * c + 1] - (int64_t)ranges[2 * c]) + 1;
             if (range > (1ull << 27)) return fail(ctx, ASZ_E_UNSUPPORTED, "QB range too wide for the dense histogram");
-            hist_off[c] = hist_total;
-            hist_total += range;
+            u64 inside = 0;
+            for (uint32_t i = 0; i < kPlanWin; i++) inside += win[(u64)c * kPlanWin + i];
+            if (inside == num[c]) continue;
+            CK(ctx->hist.reserve(range * 8));
+            CK(cudaMemsetAsync(ctx->hist.p, 0, range * 8, st));
+            {
+                ProfScope ps_(ctx, "plan_histogram", num[c] * 4);
+                CK(launch_histogram<int32_t>(d_qb + pc[c].off, num[c], ranges[2 * c], range, ctx->hist.as<unsigned long long>(), st));
+            }
+            wide[c].resize(range);
+            CK(cudaMemcpyAsync(wide[c].data(), ctx->hist.p, range * 8, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
         }
-        CK(ctx->hist.reserve(std::max<u64>(hist_total, 1) * 8));
-        CK(cudaMemsetAsync(ctx->hist.p, 0, std::max<u64>(hist_total, 1) * 8, st));
-        unsigned long long *d_hist = ctx->hist.as<unsigned long long>();
-        for (uint32_t c = 0; c < nc; c++) {
-            if (!num[c]) continue;
-            const u64 range = (u64)((int64_t)ranges[2 * c + 1] - (int64_t)ranges[2 * c]) + 1;
-            ProfScope ps_(ctx, "plan_histogram", num[c] * 4);
-            CK(launch_histogram<int32_t>(d_qb + pc[c].off, num[c], ranges[2 * c], range, d_hist + hist_off[c], st));
-        }
-        std::vector<u64> hist(hist_total);
-        if (hist_total) CK(cudaMemcpyAsync(hist.data(), d_hist, hist_total * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
         std::vector<HuffCode> codes(nc);
         std::vector<int64_t> sym_lo(nc, 0);
         std::vector<std::string> code_err(nc);
@@ -1589,14 +1603,14 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         {
             auto build_one = [&](uint32_t c) {
                 if (!num[c]) return;
-                const u64 range = (u64)((int64_t)ranges[2 * c + 1] - (int64_t)ranges[2 * c]) + 1;
-                const u64 *h = hist.data() + hist_off[c];
-                u64 a = 0, b = range;
+                const u64 *h = wide[c].empty() ? win + (u64)c * kPlanWin : wide[c].data();
+                const int64_t lo = wide[c].empty() ? -(int64_t)(kPlanWin / 2) : ranges[2 * c];
+                u64 a = 0, b = wide[c].empty() ? kPlanWin : wide[c].size();
                 while (a < b && h[a] == 0) a++;
                 while (b > a && h[b - 1] == 0) b--;
                 std::vector<u64> hh(h + a, h + b);
-                sym_lo[c] = (int64_t)ranges[2 * c] + (int64_t)a;
-                code_ok[c] = build_code(hh, sym_lo[c], (int64_t)ranges[2 * c] + (int64_t)b - 1, num[c], false, codes[c], code_err[c]);
+                sym_lo[c] = lo + (int64_t)a;
+                code_ok[c] = build_code(hh, sym_lo[c], lo + (int64_t)b - 1, num[c], false, codes[c], code_err[c]);
             };
             host_pool(ctx).run(nc, [&](uint64_t c) { build_one((uint32_t)c); });
         }
@@ -1604,14 +1618,13 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
             if (!code_ok[c]) return fail(ctx, ASZ_E_UNSUPPORTED, code_err[c]);
         // Encode all candidates into one payload arena.
         std::vector<u64> word_off(nc, 0), code_off(nc, 0);
-        u64 words = 0, ncode = 0, max_count = 0;
+        u64 words = 0, ncode = 0;
         for (uint32_t c = 0; c < nc; c++) {
             if (!num[c]) continue;
             word_off[c] = words;
             words += (codes[c].bits + 31) / 32 + 2;
             code_off[c] = ncode;
             ncode += codes[c].table.size();
-            max_count = std::max(max_count, num[c]);
         }
         std::vector<CodeEntry> ctab(std::max<u64>(ncode, 1));
         for (uint32_t c = 0; c < nc; c++)
@@ -1620,22 +1633,21 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         CK(cudaMemcpyAsync(ctx->codes.p, ctab.data(), ctab.size() * sizeof(CodeEntry), cudaMemcpyHostToDevice, st));
         CK(ctx->plan_pay.reserve(std::max<u64>(words, 1) * 4));
         CK(cudaMemsetAsync(ctx->plan_pay.p, 0, std::max<u64>(words, 1) * 4, st));
-        CK(ctx->bitoff.reserve(std::max<u64>(max_count, 1) * 8));
-        size_t tmp_bytes = 0;
-        CK(launch_encode<int32_t>(nullptr, max_count, 0, nullptr, ctx->bitoff.as<u64>(), nullptr, tmp_bytes, nullptr, st));
-        CK(ctx->cubtmp.reserve(tmp_bytes));
-        for (uint32_t c = 0; c < nc; c++) {
-            if (!num[c] || codes[c].maxval == 1) continue;
-            size_t tb = ctx->cubtmp.cap;
-            ProfScope ps_(ctx, "plan_encode", num[c] * 4);
-            CK(launch_encode<int32_t>(d_qb + pc[c].off, num[c], sym_lo[c], ctx->codes.as<CodeEntry>() + code_off[c],
-                                      ctx->bitoff.as<u64>(), ctx->cubtmp.p, tb, ctx->plan_pay.as<uint32_t>() + word_off[c], st));
+        {
+            EncodeSet set;
+            for (uint32_t c = 0; c < nc; c++)
+                if (num[c] && codes[c].maxval != 1)
+                    set.add(0, EncStream{d_qb + pc[c].off, num[c], sym_lo[c], ctx->codes.as<CodeEntry>() + code_off[c],
+                                         ctx->plan_pay.as<uint32_t>() + word_off[c]});
+            ProfScope ps_(ctx, "plan_encode", total * 4);
+            if ((rc = launch_encode_set(ctx, set, st))) return rc;
         }
-        CK(ctx->plan_host.reserve(std::max<u64>(words, 1) * 4));
+        CK(ctx->plan_words.reserve(std::max<u64>(words, 1) * 4));
         if (ctx->plan_bufs.size() < nc) ctx->plan_bufs.resize(nc);
-        const uint32_t *pay = (const uint32_t *)ctx->plan_host.p;
-        CK(cudaMemcpyAsync(ctx->plan_host.p, ctx->plan_pay.p, std::max<u64>(words, 1) * 4, cudaMemcpyDeviceToHost, st));
+        const uint32_t *pay = (const uint32_t *)ctx->plan_words.p;
+        CK(cudaMemcpyAsync(ctx->plan_words.p, ctx->plan_pay.p, std::max<u64>(words, 1) * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if ((rc = encode_set_done(ctx))) return rc;
         std::vector<u64> zlen(nc, 0);
         std::vector<char> z_ok(nc, 1);
         {
@@ -1657,6 +1669,8 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         }
         for (uint32_t c = 0; c < nc; c++)
             if (!z_ok[c]) return fail(ctx, ASZ_E_DATA, "ZSTD_compress failed in the plan search");
+        CK(cudaEventSynchronize(ctx->round_ev[1]));
+        const float *mse = (const float *)(haux + at_mse);
         out.lossless_s += secs(t_lossless, clk::now());
         // ---- Choose the layer's predictor.
         int best = -1;

@@ -60,29 +60,6 @@ __global__ void histogram_kernel(const T *__restrict__ s, uint64_t n, int64_t of
     }
 }
 
-// Code table entries (launch.h): length in bits and the code, LSB-first (bit k = branch at depth k+1).
-
-template <class T>
-__global__ void code_len_kernel(const T *__restrict__ s, uint64_t n, int64_t offset, const CodeEntry *__restrict__ tab,
-                                uint64_t *__restrict__ len) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        len[i] = tab[(uint64_t)((int64_t)s[i] - offset)].len;
-}
-
-// Writes each symbol's code at its bit offset. out is zero-initialised; codes are <= 32 bits.
-template <class T>
-__global__ void encode_kernel(const T *__restrict__ s, uint64_t n, int64_t offset, const CodeEntry *__restrict__ tab,
-                              const uint64_t *__restrict__ bitoff, uint32_t *__restrict__ out) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        CodeEntry e = tab[(uint64_t)((int64_t)s[i] - offset)];
-        uint64_t o = bitoff[i];
-        uint64_t v = (uint64_t)e.code << (o & 31);
-        uint64_t w = o >> 5;
-        if ((uint32_t)v) atomicOr(&out[w], (uint32_t)v);
-        if ((o & 31) + e.len > 32 && (uint32_t)(v >> 32)) atomicOr(&out[w + 1], (uint32_t)(v >> 32));
-    }
-}
-
 // ---------------------------------------------------------------------------------------------
 // Tiled encoding of several streams in one launch: tiles of enc_tile<T>() symbols, a stream's
 // tiles consecutive. A CTA takes tiles in order from a ticket counter and copies the next tile's
@@ -712,21 +689,6 @@ cudaError_t launch_scan_u64(const uint64_t *in, uint64_t *out, uint64_t n, void 
 }
 
 template <class T>
-cudaError_t launch_encode(const T *s, uint64_t n, int64_t offset, const CodeEntry *tab, uint64_t *bitoff, void *tmp,
-                          size_t &tmp_bytes, uint32_t *out, cudaStream_t st) {
-    if (tmp == nullptr) return launch_scan_u64(bitoff, bitoff, n, nullptr, tmp_bytes, st);
-    if (n == 0) return cudaSuccess;
-    uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 148 * 16);
-    code_len_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(s, n, offset, tab, bitoff);
-    count_launch();
-    cudaError_t e = launch_scan_u64(bitoff, bitoff, n, tmp, tmp_bytes, st);
-    if (e != cudaSuccess) return e;
-    encode_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(s, n, offset, tab, bitoff, out);
-    count_launch();
-    return cudaGetLastError();
-}
-
-template <class T>
 cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uint64_t *toff, uint64_t ntiles, uint64_t *tile_state,
                                 uint64_t *err, cudaStream_t st) {
     if (ntiles == 0) return cudaSuccess;
@@ -811,10 +773,6 @@ cudaError_t launch_fill(T *out, uint64_t n, T v, cudaStream_t st) {
 
 template cudaError_t launch_histogram<int32_t>(const int32_t *, uint64_t, int64_t, uint64_t, unsigned long long *, cudaStream_t);
 template cudaError_t launch_histogram<int64_t>(const int64_t *, uint64_t, int64_t, uint64_t, unsigned long long *, cudaStream_t);
-template cudaError_t launch_encode<int32_t>(const int32_t *, uint64_t, int64_t, const CodeEntry *, uint64_t *, void *, size_t &,
-                                            uint32_t *, cudaStream_t);
-template cudaError_t launch_encode<int64_t>(const int64_t *, uint64_t, int64_t, const CodeEntry *, uint64_t *, void *, size_t &,
-                                            uint32_t *, cudaStream_t);
 template cudaError_t launch_fill<int32_t>(int32_t *, uint64_t, int32_t, cudaStream_t);
 template cudaError_t launch_fill<int64_t>(int64_t *, uint64_t, int64_t, cudaStream_t);
 

@@ -18,11 +18,17 @@ namespace {
 // extremes are reduced in the CTA before they reach the candidate's two words: one pair of atomics
 // a CTA. Every thread's own pair, on the same two words, was most of the kernel (100x500x500, the
 // search's 14 layers, nine candidates of 0.5 M samples in the first: 11.1 ms with it, 0.24 without).
+// The QBs are counted on the way, in a window of kPlanWin bins around zero (hist: a window a
+// candidate, zero before); a candidate whose counts do not add up has QBs outside it and is counted
+// by the host's own launch. A window's set-up and fold are 4096 shared words a CTA, so a CTA has some
+// thousand samples.
 constexpr int kSampleThreads = 256;
 
 __global__ void __launch_bounds__(kSampleThreads)
     plan_sample_kernel(const float *__restrict__ d, uint64_t n1, uint64_t n2, const PlanCand *__restrict__ cands,
-                       int32_t *__restrict__ qb_out, float *__restrict__ e_out, int32_t *__restrict__ qb_range) {
+                       int32_t *__restrict__ qb_out, float *__restrict__ e_out, int32_t *__restrict__ qb_range,
+                       unsigned long long *__restrict__ hist) {
+    __shared__ uint32_t hsh[kPlanWin];
     __shared__ int32_t rlo[kSampleThreads / 32], rhi[kSampleThreads / 32];
     const PlanCand &c = cands[blockIdx.y];
     const uint64_t n = c.cnt[0] * c.cnt[1] * c.cnt[2];
@@ -38,6 +44,8 @@ __global__ void __launch_bounds__(kSampleThreads)
     float *const eo = e_out + c.off;
     const uint64_t hs = c.hs, right = c.right, dist = c.dist;
     const bool narrow = n < (1ull << 32);
+    for (uint32_t i = threadIdx.x; i < kPlanWin; i += blockDim.x) hsh[i] = 0u;
+    __syncthreads();
     int32_t lo = INT32_MAX, hi = INT32_MIN;
     for (uint64_t kl = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; kl < n; kl += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t k0, k1, k2;
@@ -80,6 +88,8 @@ __global__ void __launch_bounds__(kSampleThreads)
         eo[kl] = __fmaf_rn(-eb, q2, diff);
         lo = min(lo, q);
         hi = max(hi, q);
+        const uint32_t bin = (uint32_t)q + kPlanWin / 2;
+        if (bin < kPlanWin) atomicAdd(&hsh[bin], 1u);
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
@@ -98,6 +108,8 @@ __global__ void __launch_bounds__(kSampleThreads)
             atomicMax(&qb_range[2 * blockIdx.y + 1], hi);
         }
     }
+    for (uint32_t i = threadIdx.x; i < kPlanWin; i += blockDim.x)
+        if (hsh[i]) atomicAdd(&hist[(uint64_t)blockIdx.y * kPlanWin + i], (unsigned long long)hsh[i]);
 }
 
 // mse = fmaf(e, e, mse) over each candidate's samples in loop order, the reference's float sum
@@ -131,12 +143,12 @@ __global__ void __launch_bounds__(1024) plan_mse_kernel(const PlanCand *__restri
 }  // namespace
 
 cudaError_t launch_plan_sample(const float *d, uint64_t n1, uint64_t n2, const PlanCand *cands, uint32_t ncands, uint64_t most,
-                               int32_t *qb, float *e, int32_t *qb_range, cudaStream_t st) {
+                               int32_t *qb, float *e, int32_t *qb_range, unsigned long long *hist, cudaStream_t st) {
     if (most == 0 || ncands == 0) return cudaSuccess;
-    // CTAs a candidate: enough for its samples, and about 16 an SM over all candidates.
-    const uint64_t want = (most + kSampleThreads - 1) / kSampleThreads, share = (148 * 16 + ncands - 1) / ncands;
+    // CTAs a candidate: 1024 samples each, and about 8 an SM over all candidates.
+    const uint64_t want = (most + 4 * kSampleThreads - 1) / (4 * kSampleThreads), share = (148 * 8 + ncands - 1) / ncands;
     plan_sample_kernel<<<dim3((unsigned)(want < share ? want : share), ncands), kSampleThreads, 0, st>>>(d, n1, n2, cands, qb, e,
-                                                                                                        qb_range);
+                                                                                                        qb_range, hist);
     count_launch();
     return cudaGetLastError();
 }

@@ -172,9 +172,11 @@ cudaError_t launch_copy_box(const float *in, const uint64_t n[3], const uint64_t
 // out[k] = in[idx[k]] for k < n.
 cudaError_t launch_gather(const float *in, const uint64_t *idx, uint64_t n, float *out, cudaStream_t st);
 // most: samples of the largest candidate. The candidates' offsets are multiples of kPlanAlign.
+// hist: kPlanWin counts a candidate, of the QBs from -kPlanWin / 2 on.
 constexpr uint64_t kPlanAlign = 64;
+constexpr uint32_t kPlanWin = 2048;
 cudaError_t launch_plan_sample(const float *d, uint64_t n1, uint64_t n2, const PlanCand *cands, uint32_t ncands, uint64_t most,
-                               int32_t *qb, float *e, int32_t *qb_range, cudaStream_t st);
+                               int32_t *qb, float *e, int32_t *qb_range, unsigned long long *hist, cudaStream_t st);
 cudaError_t launch_plan_mse(const PlanCand *cands, uint32_t ncands, const float *e, float *mse, cudaStream_t st);
 cudaError_t launch_slope_exact(const SampleBox *boxes, const ProxyEval *evals, uint32_t n_evals, const float *orig,
                                uint64_t n1n2, uint64_t n2, const float *log2arena, float R2, float *h1, float *x,
@@ -187,9 +189,6 @@ cudaError_t launch_slope_v0(const FieldGeom &fg, const SampleBox *boxes, const P
 template <class T>
 cudaError_t launch_histogram(const T *s, uint64_t n, int64_t offset, uint64_t range, unsigned long long *hist,
                              cudaStream_t st);
-template <class T>
-cudaError_t launch_encode(const T *s, uint64_t n, int64_t offset, const CodeEntry *tab, uint64_t *bitoff, void *tmp,
-                          size_t &tmp_bytes, uint32_t *out, cudaStream_t st);
 // Tiled encoding of several streams of one symbol type in one launch (k_huff.cu). toff: exclusive
 // prefix of the streams' tile counts (ns + 1 entries, tiles of enc_tile<T>() symbols);
 // tile_state needs ntiles + 1 entries and err one, both zero before the launch, as each stream's out.
