@@ -121,12 +121,27 @@ struct BatchField {
     int32_t *qb;                    // QB streams, pivots first
     const uint64_t *qoff;           // stream offsets (layer_num + 1)
     int32_t *qb_range;              // [min, max] per stream
+    float *pred;                    // the targets' predictions (predictor-family probes only)
     float *proxies;                 // exact path's proxies, 10 per (block, round)
     AmbiguousRecord *amb;           // ambiguous decisions for the host replay
     uint32_t amb_cap;
     BatchCounters *cnt;
     float R2;                       // (max - min)^2
     uint32_t tpl_log2[64];          // threads per target line (log2), per round
+};
+
+// One round's targets of a probe frame's target block, in the block's loop order, and what the host's
+// reductions need of each.
+struct ProbeSpan {
+    const float *in, *rec, *pred;
+    const int32_t *qb;              // the block's QB box
+    uint64_t left[3], step[3], cnt[3];
+    uint64_t n1n2, n2;
+    uint64_t out;                   // first point
+};
+struct ProbePoint {
+    float pred, rec, orig;
+    int32_t qb;
 };
 
 #ifdef __CUDACC__

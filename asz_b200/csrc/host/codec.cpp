@@ -216,6 +216,8 @@ struct asz_ctx {
     // mapped once).
     std::vector<std::array<std::vector<uint8_t>, 2>> plan_bufs;
     PinnedBuf plan_host, plan_words;
+    DevBuf fam_tab, fam_mem, fam_points;  // predictor-family probes: tables, frames, the targets' points
+    PinnedBuf fam_host;
     bool have_last = false;
     // Profiling (asz_profile_*).
     bool prof = false;
@@ -915,6 +917,8 @@ void asz_destroy(asz_ctx *c) {
     c->stage.release();
     c->plan_host.release();
     c->plan_words.release();
+    for (DevBuf *b : {&c->fam_tab, &c->fam_mem, &c->fam_points}) b->release();
+    c->fam_host.release();
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
     asz::host::sweep_release(c->sweep);
@@ -2240,6 +2244,8 @@ long double family_entropy(const std::vector<int32_t> &qbs) {
     return h1;
 }
 
+constexpr uint32_t kBatchAmbCap = 1024;
+
 struct FamilyProbe {
     const float *d_in;
     const uint64_t *dims;
@@ -2249,88 +2255,78 @@ struct FamilyProbe {
     float mn, mx, abs_eb, slope;
 };
 
-int family_evaluate(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::array<u64, 3>> &targets, bool quintic,
-                    FamilyEval &out) {
-    cudaStream_t st = ctx->stream;
-    const u64 L = pr.plan.pred.size();
-    std::vector<std::vector<int32_t>> layer_qbs(L);
-    std::vector<long double> pred_sse(L, 0), rec_sse(L, 0);
-    std::vector<u64> counts(L, 0);
-    for (const auto &tb : targets) {
-        u64 cbb[3], cb[3], ce[3], hb[3], m[3], origin[3], tl[3];
+// A probe's frame: the target block with the blocks below it and a halo of input values.
+struct ProbeFrame {
+    u64 m[3], hb[3], origin[3], tl[3];  // extent, first plane in the field, frame origin, target block in the frame
+    ProbeFrame(const FamilyProbe &pr, const std::array<u64, 3> &tb) {
         for (int a = 0; a < 3; a++) {
-            cbb[a] = tb[a] ? tb[a] - 1 : 0;
-            cb[a] = cbb[a] * pr.shape[a];
-            ce[a] = std::min((tb[a] + 1) * pr.shape[a] + 1, pr.dims[a]);
-            const u64 left_halo = 5 * (pr.ps[a] / 2);
-            hb[a] = cb[a] > left_halo ? cb[a] - left_halo : 0;
-            m[a] = ce[a] - hb[a];
-            origin[a] = cb[a] - hb[a];
-            tl[a] = tb[a] - cbb[a];  // target block in the frame
-        }
-        const u64 n = m[0] * m[1] * m[2];
-        CK(ctx->probe_in.reserve(n * sizeof(float)));
-        CK(ctx->probe_pred.reserve(n * sizeof(float)));
-        CK(launch_copy_box(pr.d_in, pr.dims, hb, m, ctx->probe_in.as<float>(), st));
-        CoreOut co;
-        asz_report scratch{};
-        CoreArgs ca{ctx->probe_in.as<float>(), m, origin, &pr.plan, &pr.p, quintic, true, ctx->probe_pred.as<float>(),
-                    pr.mn, pr.mx, pr.abs_eb, pr.slope};
-        int rc = run_core(ctx, ca, co, scratch);
-        if (rc) return rc;
-        std::vector<float> orig(n), rec(n), pred(n);
-        u64 qtot = co.qb_off[L] + co.qb_len[L];
-        std::vector<int32_t> qb(qtot);
-        CK(cudaMemcpyAsync(orig.data(), ctx->probe_in.p, n * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(rec.data(), ctx->rec.p, n * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(pred.data(), ctx->probe_pred.p, n * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(qb.data(), ctx->qb.p, qtot * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        const Geometry &G = co.G;
-        for (u64 l = 0; l < L; l++) {
-            const RoundGeom &rg = G.rounds[l];
-            // The target block's targets in block_compress_impl's loop order (compress.tpp:67-86).
-            u64 lo[3], hi[3], left[3];
-            for (int a = 0; a < 3; a++) {
-                lo[a] = origin[a] + tl[a] * pr.shape[a];
-                hi[a] = std::min(lo[a] + pr.shape[a] + 1, m[a]);
-                left[a] = a == rg.dir ? lo[a] + rg.stride[a] / 2 : (lo[a] == 0 ? 0 : lo[a] + rg.stride[a]);
-            }
-            long double lp = 0, lr = 0;
-            u64 lc = 0;
-            for (u64 i0 = left[0]; i0 < hi[0]; i0 += rg.stride[0])
-                for (u64 i1 = left[1]; i1 < hi[1]; i1 += rg.stride[1])
-                    for (u64 i2 = left[2]; i2 < hi[2]; i2 += rg.stride[2]) {
-                        const u64 pos = (i0 * m[1] + i1) * m[2] + i2;
-                        const long double pe = (long double)pred[pos] - (long double)orig[pos];
-                        const long double re = (long double)rec[pos] - (long double)orig[pos];
-                        lp = lp + pe * pe;
-                        lr = lr + re * re;
-                        lc++;
-                    }
-            pred_sse[l] = pred_sse[l] + lp;
-            rec_sse[l] = rec_sse[l] + lr;
-            counts[l] += lc;
-            // Its QB box, in stream order.
-            u64 cc[3], pre[3];
-            for (int a = 0; a < 3; a++) {
-                cc[a] = G.tab_count[rg.axis_off[a] + tl[a]];
-                pre[a] = G.tab_prefix[rg.axis_off[a] + tl[a]];
-            }
-            const u64 base = pre[0] * rg.total[1] * rg.total[2] + cc[0] * pre[1] * rg.total[2] + cc[0] * cc[1] * pre[2];
-            const u64 size = cc[0] * cc[1] * cc[2];
-            if (size != lc || base + size > co.qb_len[l + 1]) return fail(ctx, ASZ_E_DEVICE, "predictor-family target count mismatch");
-            const int32_t *q = qb.data() + co.qb_off[l + 1] + base;
-            layer_qbs[l].insert(layer_qbs[l].end(), q, q + size);
+            const u64 cbb = tb[a] ? tb[a] - 1 : 0, cb = cbb * pr.shape[a];
+            const u64 ce = std::min((tb[a] + 1) * pr.shape[a] + 1, pr.dims[a]), left_halo = 5 * (pr.ps[a] / 2);
+            hb[a] = cb > left_halo ? cb - left_halo : 0;
+            m[a] = ce - hb[a];
+            origin[a] = cb - hb[a];
+            tl[a] = tb[a] - cbb;
         }
     }
+    u64 values() const { return m[0] * m[1] * m[2]; }
+};
+
+// The target block's targets of a round in block_compress_impl's loop order (compress.tpp:67-86), and
+// where its QB box starts in the round's stream. Returns its size.
+u64 probe_targets(const FamilyProbe &pr, const ProbeFrame &f, const Geometry &G, const RoundGeom &rg, ProbeSpan &s, u64 &qb_base) {
+    u64 cc[3], pre[3];
+    for (int a = 0; a < 3; a++) {
+        const u64 lo = f.origin[a] + f.tl[a] * pr.shape[a], hi = std::min(lo + pr.shape[a] + 1, f.m[a]);
+        s.left[a] = a == rg.dir ? lo + rg.stride[a] / 2 : (lo == 0 ? 0 : lo + rg.stride[a]);
+        s.step[a] = rg.stride[a];
+        s.cnt[a] = hi > s.left[a] ? (hi - s.left[a] + s.step[a] - 1) / s.step[a] : 0;
+        cc[a] = G.tab_count[rg.axis_off[a] + f.tl[a]];
+        pre[a] = G.tab_prefix[rg.axis_off[a] + f.tl[a]];
+    }
+    s.n1n2 = f.m[1] * f.m[2];
+    s.n2 = f.m[2];
+    qb_base = pre[0] * rg.total[1] * rg.total[2] + cc[0] * pre[1] * rg.total[2] + cc[0] * cc[1] * pre[2];
+    return cc[0] * cc[1] * cc[2];
+}
+
+// One family's figures from its targets' points, by target and round: sums per target and round on
+// the worker threads, added up in the targets' order.
+int family_figures(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::pair<const ProbePoint *, u64>> &points,
+                   FamilyEval &out) {
+    const u64 L = pr.plan.pred.size(), T = points.size() / L;
+    std::vector<long double> lp(points.size(), 0), lr(points.size(), 0), h1(L, 0);
+    host_pool(ctx).run(points.size() + L, [&](uint64_t j) {
+        if (j < points.size()) {
+            long double p = 0, r = 0;
+            for (u64 k = 0; k < points[j].second; k++) {
+                const ProbePoint &q = points[j].first[k];
+                const long double pe = (long double)q.pred - (long double)q.orig, re = (long double)q.rec - (long double)q.orig;
+                p = p + pe * pe;
+                r = r + re * re;
+            }
+            lp[j] = p;
+            lr[j] = r;
+            return;
+        }
+        std::vector<int32_t> qbs;
+        for (u64 t = 0, l = j - points.size(); t < T; t++)
+            for (u64 k = 0; k < points[t * L + l].second; k++) qbs.push_back(points[t * L + l].first[k].qb);
+        h1[j - points.size()] = family_entropy(qbs);
+    });
     out = FamilyEval();
     long double wh1 = 0, ptot = 0, rtot = 0;
     for (u64 l = 0; l < L; l++) {
-        out.points += counts[l];
-        ptot = ptot + pred_sse[l];
-        rtot = rtot + rec_sse[l];
-        wh1 = wh1 + family_entropy(layer_qbs[l]) * (long double)counts[l];
+        long double pred_sse = 0, rec_sse = 0;
+        u64 count = 0;
+        for (u64 t = 0; t < T; t++) {
+            pred_sse = pred_sse + lp[t * L + l];
+            rec_sse = rec_sse + lr[t * L + l];
+            count += points[t * L + l].second;
+        }
+        out.points += count;
+        ptot = ptot + pred_sse;
+        rtot = rtot + rec_sse;
+        wh1 = wh1 + h1[l] * (long double)count;
     }
     if (out.points == 0) return fail(ctx, ASZ_E_DATA, "predictor-family sample contains no target points");
     const long double rc = 1.0L / (long double)out.points;
@@ -2339,6 +2335,271 @@ int family_evaluate(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::
     const long double range = (long double)pr.mx - (long double)pr.mn;
     out.psnr = out.rec_mse == 0 ? (long double)INFINITY : x87_fyl2x(range * range / out.rec_mse, x87_lg2()) * 10.0L;
     out.h1 = wh1 * rc;
+    return ASZ_OK;
+}
+
+// Both families over all targets, frame by frame through the core: where the frames do not fit one
+// batch, or a coefficient decision needs the core's reruns.
+int family_by_frames(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::array<u64, 3>> &targets, FamilyEval (&out)[2]) {
+    cudaStream_t st = ctx->stream;
+    const u64 L = pr.plan.pred.size();
+    for (int fam = 0; fam < 2; fam++) {
+        std::vector<std::vector<ProbePoint>> held;  // a frame's points, round by round
+        std::vector<u64> sizes;
+        for (const auto &tb : targets) {
+            const ProbeFrame f(pr, tb);
+            const u64 n = f.values();
+            CK(ctx->probe_in.reserve(n * sizeof(float)));
+            CK(ctx->probe_pred.reserve(n * sizeof(float)));
+            CK(launch_copy_box(pr.d_in, pr.dims, f.hb, f.m, ctx->probe_in.as<float>(), st));
+            CoreOut co;
+            asz_report scratch{};
+            CoreArgs ca{ctx->probe_in.as<float>(), f.m, f.origin, &pr.plan, &pr.p, fam == 1, true, ctx->probe_pred.as<float>(),
+                        pr.mn, pr.mx, pr.abs_eb, pr.slope};
+            int rc = run_core(ctx, ca, co, scratch);
+            if (rc) return rc;
+            std::vector<ProbeSpan> spans(L);
+            u64 points = 0, most = 0;
+            for (u64 l = 0; l < L; l++) {
+                ProbeSpan &s = spans[l];
+                u64 base;
+                const u64 size = probe_targets(pr, f, co.G, co.G.rounds[l], s, base);
+                if (size != s.cnt[0] * s.cnt[1] * s.cnt[2] || base + size > co.qb_len[l + 1])
+                    return fail(ctx, ASZ_E_DEVICE, "predictor-family target count mismatch");
+                s.in = ctx->probe_in.as<float>();
+                s.rec = ctx->rec.as<float>();
+                s.pred = ctx->probe_pred.as<float>();
+                s.qb = ctx->qb.as<int32_t>() + co.qb_off[l + 1] + base;
+                s.out = points;
+                points += size;
+                most = std::max(most, size);
+                sizes.push_back(size);
+            }
+            held.emplace_back(points);
+            CK(ctx->fam_tab.reserve(L * sizeof(ProbeSpan)));
+            CK(ctx->fam_points.reserve(std::max<u64>(points, 1) * sizeof(ProbePoint)));
+            CK(cudaMemcpyAsync(ctx->fam_tab.p, spans.data(), L * sizeof(ProbeSpan), cudaMemcpyHostToDevice, st));
+            CK(launch_probe_points(ctx->fam_tab.as<ProbeSpan>(), (uint32_t)L, most, ctx->fam_points.as<ProbePoint>(), st));
+            CK(cudaMemcpyAsync(held.back().data(), ctx->fam_points.p, points * sizeof(ProbePoint), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+        }
+        std::vector<std::pair<const ProbePoint *, u64>> points;
+        for (u64 t = 0, j = 0; t < targets.size(); t++)
+            for (u64 l = 0, at = 0; l < L; l++, j++) {
+                points.push_back({held[t].data() + at, sizes[j]});
+                at += sizes[j];
+            }
+        const int rc = family_figures(ctx, pr, points, out[fam]);
+        if (rc) return rc;
+    }
+    return ASZ_OK;
+}
+
+// Both families over all targets as one batch: a launch per round of each batched kernel for all
+// frames, instead of sixteen cores one after another, each bound by its launches and waits
+// (100x500x500: 5.5 -> 0.7 ms). done is false where the frames have to go one by one.
+// The bounds keep the batch's memory at a few hundred MiB, and its frames within the kernels' tables.
+constexpr u64 kFamilyValues = 1ull << 24, kFamilyFrames = 256, kFamilyRounds = 64;
+
+int family_batch(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::array<u64, 3>> &targets, FamilyEval (&out)[2],
+                 bool &done) {
+    done = false;
+    cudaStream_t st = ctx->stream;
+    const u64 L = pr.plan.pred.size(), T = targets.size();
+    const uint32_t nf = (uint32_t)(2 * T);
+    std::vector<ProbeFrame> frames;
+    u64 values = 0;
+    for (const auto &tb : targets) {
+        frames.emplace_back(pr, tb);
+        values += 2 * frames.back().values();
+    }
+    if (ctx->tsel_mode == 1 || values > kFamilyValues || nf > kFamilyFrames || L > kFamilyRounds) return ASZ_OK;
+    // Geometry of every frame in both families (frame f of family q at q T + f).
+    std::vector<Geometry> G(nf);
+    std::vector<std::vector<u64>> qoff(nf);
+    u64 blocks = 0, pivots = 0, qbs = 0, ents = 0;
+    uint32_t capmax = 1;
+    std::vector<uint32_t> cap_round(L, 1);
+    for (uint32_t f = 0; f < nf; f++) {
+        const ProbeFrame &fr = frames[f % T];
+        Geometry &g = G[f];
+        build_geometry(fr.m, pr.plan, pr.p, pr.abs_eb, pr.slope, f >= T, g, fr.origin);
+        if (!kernel_limits_ok(g)) return fail(ctx, ASZ_E_UNSUPPORTED, "field too large for the round kernels' 32-bit line indexing");
+        qoff[f].push_back(0);
+        u64 acc = g.pivots;
+        for (u64 l = 0; l < L; l++) {
+            qoff[f].push_back(acc);
+            acc += g.rounds[l].qb_total;
+            cap_round[l] = std::max(cap_round[l], g.cap[l]);
+            capmax = std::max(capmax, g.cap[l]);
+            for (auto &ci : g.classes[l])
+                if (ci.n) ci.log2_off = log2_table(ctx, ci.n);
+        }
+        qoff[f].push_back(acc);
+        qbs += acc;
+        blocks += g.nblocks;
+        pivots += g.pivots;
+        ents += g.ent.size();
+    }
+    int rc = upload_log2(ctx);
+    if (rc) return rc;
+    // Device memory: tables (uploaded at once), data, and the counters (cleared).
+    u64 at = 0;
+    auto place = [&](u64 n) {
+        const u64 o = at;
+        at = (at + n + 255) & ~255ull;
+        return o;
+    };
+    const u64 t_fields = place(nf * sizeof(BatchField)), t_rounds = place(nf * L * sizeof(RoundGeom)),
+              t_ent = place(ents * sizeof(AxisEntry)), t_cls = place(nf * L * 27 * sizeof(ClassInfo)),
+              t_qoff = place(nf * (L + 2) * 8), t_goff = place((nf + 1) * 8), t_poff = place((nf + 1) * 8),
+              t_ioff = place(L * (nf + 1) * 8), t_spans = place(nf * L * sizeof(ProbeSpan)), tab = at;
+    at = 0;
+    const u64 d_in = place(values / 2 * 4), d_rec = place(values * 4), d_pred = place(values * 4), d_qb = place(qbs * 4),
+              d_tval = place(blocks * 4), d_tint = place(blocks * L * 8), d_range = place(nf * 2 * (L + 1) * 4),
+              d_amb = place((u64)nf * kBatchAmbCap * sizeof(AmbiguousRecord)), d_hand = place(blocks * 8),
+              d_spill = place(blocks * 8), d_spill2 = place(blocks * 8), d_cnt = place(nf * sizeof(BatchCounters)),
+              d_queue = place(5 * L * 4), mem = at;
+    CK(ctx->fam_tab.reserve(tab));
+    CK(ctx->fam_mem.reserve(mem));
+    CK(ctx->plan_host.reserve(std::max(tab, mem - d_cnt)));
+    uint8_t *const dt = ctx->fam_tab.as<uint8_t>(), *const dv = ctx->fam_mem.as<uint8_t>(), *const ht = ctx->plan_host.p;
+    u64 points = 0, most = 0;
+    std::vector<u64> sizes;
+    {
+        u64 o_val = 0, o_qb = 0, o_blk = 0, o_ent = 0;
+        u64 *goff = (u64 *)(ht + t_goff), *poff = (u64 *)(ht + t_poff), *ioff = (u64 *)(ht + t_ioff);
+        goff[0] = poff[0] = 0;
+        for (u64 l = 0; l < L; l++) ioff[l * (nf + 1)] = 0;
+        for (uint32_t f = 0; f < nf; f++) {
+            const Geometry &g = G[f];
+            const ProbeFrame &fr = frames[f % T];
+            if (f == T) o_val = 0;
+            BatchField x;
+            std::memset(&x, 0, sizeof(x));
+            x.fg = g.fg;
+            x.pg = g.pg;
+            x.rounds = (const RoundGeom *)(dt + t_rounds) + f * L;
+            x.ent = (const AxisEntry *)(dt + t_ent) + o_ent;
+            x.classes = (const ClassInfo *)(dt + t_cls) + f * L * 27;
+            x.in = (const float *)(dv + d_in) + o_val;
+            const u64 val = o_val + (f >= T ? values / 2 : 0);
+            x.rec = (float *)(dv + d_rec) + val;
+            x.pred = (float *)(dv + d_pred) + val;
+            x.tval = (float *)(dv + d_tval) + o_blk;
+            x.tint = (int64_t *)(dv + d_tint) + o_blk * L;
+            x.qb = (int32_t *)(dv + d_qb) + o_qb;
+            x.qoff = (const u64 *)(dt + t_qoff) + f * (L + 2);
+            x.qb_range = (int32_t *)(dv + d_range) + f * 2 * (L + 1);
+            x.amb = (AmbiguousRecord *)(dv + d_amb) + (u64)f * kBatchAmbCap;
+            x.amb_cap = kBatchAmbCap;
+            x.cnt = (BatchCounters *)(dv + d_cnt) + f;
+            x.R2 = (pr.mx - pr.mn) * (pr.mx - pr.mn);
+            std::memcpy(ht + t_rounds + f * L * sizeof(RoundGeom), g.rounds.data(), L * sizeof(RoundGeom));
+            std::memcpy(ht + t_ent + o_ent * sizeof(AxisEntry), g.ent.data(), g.ent.size() * sizeof(AxisEntry));
+            std::memcpy(ht + t_qoff + f * (L + 2) * 8, qoff[f].data(), (L + 2) * 8);
+            for (u64 l = 0; l < L; l++) {
+                const RoundGeom &rg = g.rounds[l];
+                std::memcpy(ht + t_cls + (f * L + l) * 27 * sizeof(ClassInfo), g.classes[l].data(), 27 * sizeof(ClassInfo));
+                x.tpl_log2[l] = round_tpl_log2(rg.tcount[2]);
+                ioff[l * (nf + 1) + f + 1] = ioff[l * (nf + 1) + f] + round_batch_items(rg, x.tpl_log2[l]);
+                ProbeSpan s{};
+                u64 base;
+                const u64 size = probe_targets(pr, fr, g, rg, s, base);
+                if (size != s.cnt[0] * s.cnt[1] * s.cnt[2] || base + size > rg.qb_total)
+                    return fail(ctx, ASZ_E_DEVICE, "predictor-family target count mismatch");
+                s.in = x.in;
+                s.rec = x.rec;
+                s.pred = x.pred;
+                s.qb = x.qb + qoff[f][l + 1] + base;
+                s.out = points;
+                points += size;
+                most = std::max(most, size);
+                sizes.push_back(size);
+                std::memcpy(ht + t_spans + (f * L + l) * sizeof(ProbeSpan), &s, sizeof(s));
+            }
+            std::memcpy(ht + t_fields + f * sizeof(BatchField), &x, sizeof(x));
+            goff[f + 1] = goff[f] + g.nblocks;
+            poff[f + 1] = poff[f] + g.pivots;
+            o_val += fr.values();
+            o_qb += qoff[f][L + 1];
+            o_blk += g.nblocks;
+            o_ent += g.ent.size();
+        }
+    }
+    CK(ctx->fam_points.reserve(std::max<u64>(points, 1) * sizeof(ProbePoint)));
+    CK(ctx->fam_host.reserve(std::max<u64>(points, 1) * sizeof(ProbePoint)));
+    const u64 gstride = exact_global_stride(capmax);
+    unsigned ggrid = 0;
+    if (capmax > exact_cap()) {
+        ggrid = (unsigned)std::max<u64>(1, std::min<u64>(148, kExactScratch / gstride));
+        CK(ctx->gscratch.reserve(ggrid * gstride));
+    }
+    CK(cudaMemcpyAsync(dt, ht, tab, cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(dv + d_cnt, 0, mem - d_cnt, st));
+    u64 o_val = 0;
+    for (const ProbeFrame &fr : frames) {
+        CK(launch_copy_box(pr.d_in, pr.dims, fr.hb, fr.m, (float *)(dv + d_in) + o_val, st));
+        o_val += fr.values();
+    }
+    // A frame's halo and unowned faces keep their input values (the reference starts from a copy).
+    for (u64 q = 0; q < 2; q++)
+        CK(cudaMemcpyAsync(dv + d_rec + q * values / 2 * 4, dv + d_in, values / 2 * 4, cudaMemcpyDeviceToDevice, st));
+    const BatchField *F = (const BatchField *)(dt + t_fields);
+    const u64 *goff = (const u64 *)(dt + t_goff), *ioff = (const u64 *)(dt + t_ioff);
+    unsigned long long *hand = (unsigned long long *)(dv + d_hand), *spill = (unsigned long long *)(dv + d_spill),
+                       *spill2 = (unsigned long long *)(dv + d_spill2);
+    const float t_default = 4.0f / 16, *log2 = ctx->log2arena.as<float>();
+    CK(launch_pivot_compress_batch(F, (const u64 *)(dt + t_poff), nf, pivots, st));
+    for (u64 l = 0; l < L; l++) {
+        uint32_t *q = (uint32_t *)(dv + d_queue) + 5 * l;
+        {
+            ProfScope ps(ctx, "tsel_fast", 0);
+            CK(launch_tsel_fast_batch(F, goff, nf, (uint32_t)l, log2, t_default, q, hand, q + 2,
+                                      (uint32_t)std::min<u64>(blocks, 148 * 16), st));
+        }
+        {
+            ProfScope ps(ctx, "tsel_exact", 0);
+            CK(launch_tsel_exact_batch(F, (uint32_t)l, log2, t_default, hand, q + 2, spill, q + 3, exact_cap(), cap_round[l], 148, st));
+        }
+        if (ggrid)
+            CK(launch_tsel_exact_global_batch(F, (uint32_t)l, log2, t_default, spill, q + 3, spill2, q + 4,
+                                              ctx->gscratch.as<uint8_t>(), gstride, capmax, ggrid, st));
+        ProfScope ps(ctx, "round_compress", 0);
+        CK(launch_round_compress_batch(F, ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * 5, true, st));
+    }
+    CK(launch_probe_points((const ProbeSpan *)(dt + t_spans), (uint32_t)(nf * L), most, ctx->fam_points.as<ProbePoint>(), st));
+    CK(cudaMemcpyAsync(ctx->fam_host.p, ctx->fam_points.p, points * sizeof(ProbePoint), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(ht, dv + d_cnt, mem - d_cnt, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    const BatchCounters *cnt = (const BatchCounters *)ht;
+    const uint32_t *queue = (const uint32_t *)(ht + (d_queue - d_cnt));
+    for (u64 l = 0; l < L; l++)
+        if (queue[5 * l + (ggrid ? 4 : 3)]) return ASZ_OK;  // a group for the serial kernel
+    std::vector<AmbiguousRecord> recs;
+    for (uint32_t f = 0; f < nf; f++) {
+        if (cnt[f].err)
+            return fail(ctx, ASZ_E_DEVICE, "round kernels reported an internal error " + std::to_string(cnt[f].err));
+        if (cnt[f].amb_count > kBatchAmbCap) return ASZ_OK;
+        if (!cnt[f].amb_count) continue;
+        recs.resize(cnt[f].amb_count);
+        CK(cudaMemcpyAsync(recs.data(), dv + d_amb + (u64)f * kBatchAmbCap * sizeof(AmbiguousRecord),
+                           recs.size() * sizeof(AmbiguousRecord), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (const AmbiguousRecord &r : recs)
+            if ((int32_t)host_lround_f(replay_decision(r, G[f].rounds[r.round].slope) * (float)pr.p.t_precision) != r.provisional)
+                return ASZ_OK;  // the replay changes a decision
+    }
+    const ProbePoint *pt = (const ProbePoint *)ctx->fam_host.p;
+    for (int fam = 0; fam < 2; fam++) {
+        std::vector<std::pair<const ProbePoint *, u64>> pts;
+        for (u64 j = 0; j < T * L; j++) {
+            pts.push_back({pt, sizes[fam * T * L + j]});
+            pt += pts.back().second;
+        }
+        if ((rc = family_figures(ctx, pr, pts, out[fam]))) return rc;
+    }
+    done = true;
     return ASZ_OK;
 }
 
@@ -2406,11 +2667,12 @@ int select_family(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const
         quintic = false;
         return ASZ_OK;
     }
-    FamilyEval c, q;
-    int rc = family_evaluate(ctx, pr, targets, false, c);
+    FamilyEval ev[2];
+    bool done;
+    int rc = family_batch(ctx, pr, targets, ev, done);
+    if (!rc && !done) rc = family_by_frames(ctx, pr, targets, ev);
     if (rc) return rc;
-    rc = family_evaluate(ctx, pr, targets, true, q);
-    if (rc) return rc;
+    const FamilyEval &c = ev[0], &q = ev[1];
     const long double score = (c.h1 - q.h1) * (long double)slope + (q.psnr - c.psnr);
     R.fam_points = c.points;
     R.fam_cubic_mse = c.pred_mse;
@@ -3687,8 +3949,6 @@ struct BatchItem {
     u64 o_in = 0, o_rec = 0, o_qb = 0, o_tval = 0, o_tint = 0, o_ent = 0, o_prox = 0;
 };
 
-constexpr uint32_t kBatchAmbCap = 1024;
-
 // Launch shapes that change no result: CTAs per SM of the persistent selection and round
 // kernels, and a shift of the threads per target line (fewer threads per line, more lines per CTA).
 using BatchShape = std::array<uint32_t, 3>;
@@ -3926,7 +4186,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
             if (t_tables) {
                 // The caller's t codes replace the coefficient selection.
                 CK(launch_tval_from_codes_batch(dF, d_goff, nf, nb_total, (uint32_t)l, st));
-                CK(launch_round_compress_batch(dF, d_ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * sh[1], st));
+                CK(launch_round_compress_batch(dF, d_ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * sh[1], false, st));
                 continue;
             }
             CK(launch_tsel_fast_batch(dF, d_goff, nf, (uint32_t)l, ctx->log2arena.as<float>(), t_default, q, d_hand, q + 2,
@@ -3944,7 +4204,7 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
             if (serial)
                 CK(launch_tsel_v0_batch(dF, (uint32_t)l, ctx->log2arena.as<float>(), t_default, ctx->scratch.as<uint8_t>(), sstride,
                                     capmax, bcap, tcap, d_left, d_lcnt, slots, st));
-            CK(launch_round_compress_batch(dF, d_ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * sh[1], st));
+            CK(launch_round_compress_batch(dF, d_ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * sh[1], false, st));
         }
         return ASZ_OK;
     };

@@ -467,6 +467,8 @@ __global__ void __launch_bounds__(256, 3)
 // kBatchChunks CTA-sized chunks of one field's target lines (256 >> tpl_log2 lines each).
 constexpr uint32_t kBatchChunks = 8;
 
+// kProbe: the fields are predictor-family probe frames (as round_compress_kernel's kProbe).
+template <bool kProbe>
 __global__ void __launch_bounds__(256, 5)
     round_compress_batch_kernel(const BatchField *__restrict__ F, const uint64_t *__restrict__ ioff, uint32_t nf, uint32_t l,
                                 uint32_t *queue) {
@@ -490,8 +492,8 @@ __global__ void __launch_bounds__(256, 5)
         for (uint32_t c = 0; c < kBatchChunks; c++) {
             const uint64_t line = (c0 + c) * m.lines_per_cta + m.row;
             if (line < lines)
-                compress_line<false>(B.fg, rg, B.ent, tpl, m.sub, (uint32_t)line, B.tval, B.in, B.rec, B.qb + B.qoff[l + 1],
-                                     &B.cnt->err, nullptr, ebd, eb2, rinv, r0, lo, hi);
+                compress_line<kProbe>(B.fg, rg, B.ent, tpl, m.sub, (uint32_t)line, B.tval, B.in, B.rec, B.qb + B.qoff[l + 1],
+                                      &B.cnt->err, B.pred, ebd, eb2, rinv, r0, lo, hi);
         }
         reduce_range(lo, hi, B.qb_range + 2 * (l + 1));
     }
@@ -732,8 +734,9 @@ uint64_t round_batch_items(const RoundGeom &rg, uint32_t tpl_log2) {
 }
 
 cudaError_t launch_round_compress_batch(const BatchField *F, const uint64_t *ioff, uint32_t nf, uint32_t l, uint32_t *queue,
-                                        uint32_t grid, cudaStream_t st) {
-    round_compress_batch_kernel<<<grid ? grid : 148 * 5, 256, 0, st>>>(F, ioff, nf, l, queue);
+                                        uint32_t grid, bool probe, cudaStream_t st) {
+    if (probe) round_compress_batch_kernel<true><<<grid ? grid : 148 * 5, 256, 0, st>>>(F, ioff, nf, l, queue);
+    else round_compress_batch_kernel<false><<<grid ? grid : 148 * 5, 256, 0, st>>>(F, ioff, nf, l, queue);
     count_launch();
     return cudaGetLastError();
 }
@@ -800,7 +803,24 @@ __global__ void copy_box_kernel(const float *__restrict__ in, uint64_t n1, uint6
         out[k] = in[((lo0 + i0) * n1 + lo1 + i1) * n2 + lo2 + i2];
     }
 }
+// grid y: spans, x: CTAs over a span's points.
+__global__ void probe_points_kernel(const ProbeSpan *__restrict__ spans, ProbePoint *__restrict__ out) {
+    const ProbeSpan &s = spans[blockIdx.y];
+    const uint64_t total = s.cnt[0] * s.cnt[1] * s.cnt[2];
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < total; k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t k2 = k % s.cnt[2], r = k / s.cnt[2], k1 = r % s.cnt[1], k0 = r / s.cnt[1];
+        const uint64_t pos = (s.left[0] + k0 * s.step[0]) * s.n1n2 + (s.left[1] + k1 * s.step[1]) * s.n2 + s.left[2] + k2 * s.step[2];
+        out[s.out + k] = ProbePoint{s.pred[pos], s.rec[pos], s.in[pos], s.qb[k]};
+    }
+}
 }  // namespace
+
+cudaError_t launch_probe_points(const ProbeSpan *spans, uint32_t nspans, uint64_t most, ProbePoint *out, cudaStream_t st) {
+    if (nspans == 0 || most == 0) return cudaSuccess;
+    probe_points_kernel<<<dim3(grid_for(most, 256, 148), nspans), 256, 0, st>>>(spans, out);
+    count_launch();
+    return cudaGetLastError();
+}
 
 // out[k] = in[idx[k]]: the default slope's sample neighbourhoods of a slab (asz_compress_slab).
 __global__ void gather_kernel(const float *__restrict__ in, const uint64_t *__restrict__ idx, uint64_t n,

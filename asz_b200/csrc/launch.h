@@ -79,7 +79,7 @@ cudaError_t launch_tval_from_codes_batch(const BatchField *F, const uint64_t *go
 uint32_t round_tpl_log2(uint64_t t2);
 uint64_t round_batch_items(const RoundGeom &rg, uint32_t tpl_log2);
 cudaError_t launch_round_compress_batch(const BatchField *F, const uint64_t *ioff, uint32_t nf, uint32_t l, uint32_t *queue,
-                                        uint32_t grid, cudaStream_t st);
+                                        uint32_t grid, bool probe, cudaStream_t st);
 
 // Open-loop AB samples of every (block, round) group for the gradient tuner (k_grad.cu).
 cudaError_t launch_grad_gather(const FieldGeom &fg, const RoundGeom *rounds, const ClassInfo *classes, const float *x,
@@ -167,6 +167,8 @@ cudaError_t launch_slope_exact_global(const SampleBox *boxes, const ProxyEval *e
                                       uint64_t n1n2, uint64_t n2, const float *log2arena, float R2, float *h1, float *x,
                                       uint32_t *m_out, uint32_t *err, uint8_t *scratch, uint64_t stride, uint32_t cap,
                                       uint32_t nboxes, cudaStream_t st);
+// The points of nspans spans of at most `most` points each (predictor-family probes).
+cudaError_t launch_probe_points(const ProbeSpan *spans, uint32_t nspans, uint64_t most, ProbePoint *out, cudaStream_t st);
 cudaError_t launch_copy_box(const float *in, const uint64_t n[3], const uint64_t lo[3], const uint64_t m[3], float *out,
                             cudaStream_t st);
 // out[k] = in[idx[k]] for k < n.
