@@ -3582,26 +3582,21 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
             ProfScope ps(ctx, "pivot_decompress", G.pivots * 8);
             CK(launch_pivot_decompress(G.pg, ctx->qb.as<int32_t>() + qoff[0], d_out, st));
         }
-        if (const uint32_t line_bytes = ctx->tsel_mode == 2 ? lines_smem_bytes(G) : 0) {
-            // Every round along axis 2: all rounds fused per column of lines (k_lines.cu).
-            const u64 rbytes = L * sizeof(RoundGeom);
-            CK(ctx->rounds_dev.reserve(rbytes + (L + 1) * sizeof(u64)));
-            uint8_t *rd = ctx->rounds_dev.as<uint8_t>();
-            CK(cudaMemcpyAsync(rd, G.rounds.data(), rbytes, cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(rd + rbytes, qoff.data(), (L + 1) * sizeof(u64), cudaMemcpyHostToDevice, st));
-            u64 tgt = 0;
-            for (u64 l = 0; l < L; l++) tgt += G.rounds[l].targets;
-            // Algorithmic bytes: the field loaded and stored once, one QB read per target.
-            ProfScope ps(ctx, "lines_decompress", N * 8 + tgt * 4);
-            for (const LinesLaunch &ll : lines_launches(G, line_bytes))
-                CK(launch_lines_decompress(G.fg, (const RoundGeom *)rd, d_ent, (const u64 *)(rd + rbytes),
-                                           ctx->tint.as<int64_t>(), ctx->qb.as<int32_t>(), d_out, &dm->err, ll.set, ll.bytes, st));
-        } else {
-            for (u64 l = 0; l < L; l++) {
-                ProfScope ps(ctx, "round_decompress", G.rounds[l].targets * 8);
-                CK(launch_round_decompress(G.fg, G.rounds[l], (uint32_t)l, d_ent, ctx->tint.as<int64_t>(),
-                                           ctx->qb.as<int32_t>() + qoff[l + 1], d_out, &dm->err, st));
+        for (u64 l = 0; l < L;) {
+            if (const u64 len = lines_run_length(G.fg, &G.rounds[l], (uint32_t)(L - l))) {
+                // Algorithmic bytes: the run's lines loaded and stored once, one QB read per target.
+                u64 tgt = 0;
+                for (u64 k = l; k < l + len; k++) tgt += G.rounds[k].targets;
+                ProfScope ps(ctx, "lines_decompress", tgt * 8);
+                CK(launch_lines_decompress(G.fg, &G.rounds[l], (uint32_t)len, (uint32_t)l, d_ent, qoff.data(),
+                                           ctx->tint.as<int64_t>(), ctx->qb.as<int32_t>(), d_out, &dm->err, st));
+                l += len;
+                continue;
             }
+            ProfScope ps(ctx, "round_decompress", G.rounds[l].targets * 8);
+            CK(launch_round_decompress(G.fg, G.rounds[l], (uint32_t)l, d_ent, ctx->tint.as<int64_t>(),
+                                       ctx->qb.as<int32_t>() + qoff[l + 1], d_out, &dm->err, st));
+            l++;
         }
         CK(cudaMemcpyAsync(hw->dec, &dm->dec_err, 12, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));

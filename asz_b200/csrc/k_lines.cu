@@ -1,6 +1,7 @@
-// Fused rounds for plans whose every round runs along axis 2 (e.g. "cubic2_012" on every level).
+// Fused rounds along axis 2: whole plans of them compressed (e.g. "cubic2_012" on every level), and runs
+// of consecutive ones decompressed.
 //
-// With all rounds on one axis, the pivot stride is 1 on the other two axes, so a block owns whole
+// Compression. With all rounds on one axis, the pivot stride is 1 on the other two axes, so a block owns whole
 // lines along axis 2 and every stencil read of a round stays on the target's own line. The lines of
 // a "column" (the blocks sharing one (block0, block1) pair) can therefore be held in shared memory
 // by one CTA for all rounds: the field is read and written once instead of once per round.
@@ -8,6 +9,8 @@
 // rounds run in the same order, and a round's coefficient selection sees the column after the
 // previous round, as the per-round kernels do.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "dev_common.cuh"
 #include "geometry.cuh"
@@ -83,59 +86,291 @@ __device__ __forceinline__ void store_lines(const FieldGeom &fg, const Column &c
 __host__ __device__ constexpr size_t align16(size_t b) { return (b + 15) & ~size_t(15); }
 
 // ---------------------------------------------------------------------------------------------
-// Decompression: every round of every column, from the pivots (already in rec) to the final
-// values. decompress.tpp:34: value = fma(-qb, 2eb, pred) in double, t = t_int / t_precision.
-struct DecShared {
-    float t[kMaxColumnBlocks];
+// Decompression: consecutive rounds along axis 2, a warp per line. Nothing crosses lines here (the t
+// codes are given), so a line needs only its own known points: the warp loads them, runs the rounds
+// in shared memory and stores the line once. decompress.tpp:34: value = fma(-qb, 2eb, pred) in
+// double, t = t_int / t_precision.
+//
+// A launch per round reads and writes the line's sectors again in every round of stride up to 8, and
+// costs a launch for the few targets of a coarse one. Here the traffic is the QBs read and the field
+// written once, and what bounds it is the instructions issued per target, so the parts that are the
+// same for a round or a line are kept out of the targets' loop and the QBs' offsets are 32-bit from
+// the line's base. A round's first QBs are loaded during the round before. One value in 32 is
+// padding: with it the lattices' power-of-two strides meet no bank twice. 512x512x512 in nine rounds:
+// 1.70 -> 0.72 ms (a table for the one block too, and a line a warp: 1.04), 75% of the issue slots and
+// 40% of the conversion units taken; 40x48x64 in five: 53 -> 13 us. Four CTAs of 64 registers: five
+// of 48 spill (0.82 ms).
+constexpr uint32_t kRunRounds = 16, kRunAhead = 4, kRunWarps = 8, kRunCtas = 4;
+constexpr uint64_t kRunSmem = 227 * 1024, kRunSm = 228 * 1024;  // shared memory of a CTA, of an SM
+
+struct RunRound {
+    double eb2;
+    uint64_t qoff, qb_total;  // the stream's first QB and its length
+    uint64_t ent2;            // axis 2's entries
+    uint32_t hs, count, first, total2, order, l;
+    uint32_t cubics, quintics;  // one block: targets [1, 1 + cubics) are cubic, but [2, 2 + quintics) quintic
+};
+struct LineRun {
+    RunRound r[kRunRounds];
+    uint64_t ent0, ent1, total1, n1n2;
+    uint32_t rounds, lines, T1, n2, nb1, nb2, layers, targets, known, step, tab_words, line_words;
+    float tp;
 };
 
-__global__ void __launch_bounds__(256)
-    lines_decompress_kernel(FieldGeom fg, const RoundGeom *__restrict__ rounds, const AxisEntry *__restrict__ ent,
-                            const uint64_t *__restrict__ qoff, const int64_t *__restrict__ t_int, const int32_t *__restrict__ qb,
-                            float *__restrict__ rec, uint32_t set, uint32_t items, uint32_t *err_word) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    DecShared &ds = *reinterpret_cast<DecShared *>(smem_raw);
-    float *sl = reinterpret_cast<float *>(smem_raw + align16(sizeof(DecShared)));
-    const uint32_t nb1 = (uint32_t)fg.block_num[1], nb2 = (uint32_t)fg.block_num[2];
-    const uint32_t n2 = (uint32_t)fg.n[2], L = fg.layer_num;
-    const float tp = (float)fg.t_precision;
-    for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
-        uint32_t b0, b1;
-        column_at(set, it, nb1, b0, b1);
-        const uint32_t c = b0 * nb1 + b1;
-        const Column col = column_of(fg, b0, b1);
-        const uint32_t nl = col.nl0 * col.nl1;
-        __syncthreads();
-        load_lines(fg, col, rec, sl);
-        for (uint32_t l = 0; l < L; l++) {
-            const RoundGeom &rg = rounds[l];
-            if (threadIdx.x < nb2)
-                ds.t[threadIdx.x] =
-                    __fdiv_rn(__ll2float_rn(t_int[((uint64_t)c * nb2 + threadIdx.x) * L + l]), tp);
-            __syncthreads();
-            const double eb2 = __dadd_rn((double)rg.eb, (double)rg.eb);
-            const uint32_t T2 = (uint32_t)rg.tcount[2], hs = (uint32_t)rg.hs;
-            const AxisEntry *e0t = ent + rg.ent_off[0], *e1t = ent + rg.ent_off[1], *e2t = ent + rg.ent_off[2];
-            const int32_t *qbl = qb + qoff[l + 1];
-            const uint32_t work = nl * T2;
-            for (uint32_t w = threadIdx.x; w < work; w += blockDim.x) {
-                const uint32_t line = w / T2, k = w - line * T2;
-                const uint32_t r0 = line / col.nl1;
-                const AxisEntry e0 = load_entry(e0t + col.lo0 + r0), e1 = load_entry(e1t + col.lo1 + (line - r0 * col.nl1));
-                const AxisEntry e2 = load_entry(e2t + k);
-                const uint64_t qi = qb_index(rg, e0, e1, e2);
-                if (qi >= rg.qb_total || e2.bb >= kMaxColumnBlocks) {
-                    atomicOr(err_word, 4u);
-                    continue;
-                }
-                float *ln = sl + line * n2;
-                const float t = e2.stencil == kStencilCubic ? ds.t[e2.bb] : 0.0f;
-                const float pred = predict_case(ln, e2.ii, hs, e2.stencil, t);
-                ln[e2.ii] = __double2float_rn(__fma_rn(-(double)qbl[qi], eb2, (double)pred));
-            }
-            __syncthreads();
+__device__ __forceinline__ uint32_t padded(uint32_t i) { return i + (i >> 5); }
+
+__device__ __forceinline__ float cubic(float m3, float m1, float p1, float p3, double c1, double c2) {
+    const float a = __double2float_rn(__dmul_rn((double)__fadd_rn(m3, p3), c1));
+    return __double2float_rn(__fma_rn(c2, (double)__fadd_rn(m1, p1), (double)a));
+}
+
+// The cases other than the cubic and the quintic one, without branches: neighbours that a case does
+// not use are read from the target's own place.
+__device__ __forceinline__ float predict_edge(const float *s, uint32_t i, uint32_t hs, uint32_t sc) {
+    const bool has_p1 = sc != kStencilLeft1 && sc != kStencilRight1, right = sc >= kStencilRight1;
+    const float m1 = s[padded(i - hs)], p1 = s[padded(has_p1 ? i + hs : i)], m3 = s[padded(right ? i - 3 * hs : i)],
+                p3 = s[padded(sc == kStencilLeft3 ? i + 3 * hs : i)];
+    float v = m1;
+    if (sc == kStencilLeft2) v = __fmul_rn(__fadd_rn(m1, p1), 0.5f);
+    if (sc == kStencilLeft3) v = __fmul_rn(__fsub_rn(__fmaf_rn(m1, 3.0f, __fmul_rn(p1, 6.0f)), p3), 0.125f);
+    if (sc == kStencilRight1) v = __fmul_rn(__fmaf_rn(m1, 3.0f, -m3), 0.5f);
+    if (sc == kStencilRight2) v = __fmul_rn(__fmaf_rn(p1, 3.0f, __fmaf_rn(m1, 6.0f, -m3)), 0.125f);
+    return v;
+}
+
+// A line: its place in the field, its blocks, and the parts of its QBs' offsets that no round changes.
+struct RunLine {
+    AxisEntry e0, e1;
+    float *g;
+    uint64_t blk, base;
+};
+
+__device__ __forceinline__ RunLine run_line(const LineRun &R, const AxisEntry *ent, float *rec, uint32_t line) {
+    RunLine l;
+    const uint32_t k0 = line / R.T1;
+    l.e0 = load_entry(ent + R.ent0 + k0);
+    l.e1 = load_entry(ent + R.ent1 + (line - k0 * R.T1));
+    l.g = rec + (uint64_t)l.e0.ii * R.n1n2 + (uint64_t)l.e1.ii * R.n2;
+    l.blk = ((uint64_t)l.e0.bb * R.nb1 + l.e1.bb) * R.nb2;
+    l.base = l.e0.pre * R.total1 + (uint64_t)l.e0.cc * l.e1.pre;
+    return l;
+}
+
+// A line's QBs in a round: where its part of the stream starts, and the factors of a target's offset,
+// mul * pre + (u * cc + jj) * w + x (get_qb_index).
+struct LineQBs {
+    const int32_t *q;
+    uint32_t limit;  // QBs from q to the stream's end
+    uint32_t mul, u, w, x;
+};
+
+__device__ __forceinline__ LineQBs line_qbs(const RunRound &m, const RunLine &l, const int32_t *qb) {
+    LineQBs L;
+    const uint64_t off = l.base * m.total2, left = off < m.qb_total ? m.qb_total - off : 0;
+    L.mul = l.e0.cc * l.e1.cc;
+    L.u = m.order == 2 ? l.e0.jj * l.e1.cc + l.e1.jj : m.order == 0 ? l.e1.jj : l.e0.jj;
+    L.w = m.order == 2 ? 1 : m.order == 0 ? l.e0.cc : l.e1.cc;
+    L.x = m.order == 2 ? 0 : m.order == 0 ? l.e0.jj : l.e1.jj;
+    L.q = qb + m.qoff + off;
+    L.limit = left < 0xffffffffu ? (uint32_t)left : 0xffffffffu;
+    return L;
+}
+
+__device__ __forceinline__ float run_t(const LineRun &R, const int64_t *t_int, uint64_t blk, uint32_t r) {
+    return __fdiv_rn(__ll2float_rn(__ldg(t_int + blk * R.layers + R.r[r].l)), R.tp);
+}
+
+// Several blocks along axis 2: a warp per line; the targets' block offsets, QB boxes and stencil cases
+// come from a table in shared memory.
+__global__ void __launch_bounds__(32 * kRunWarps, kRunCtas)
+    lines_decompress_kernel(const __grid_constant__ LineRun R, const AxisEntry *__restrict__ ent, const int64_t *__restrict__ t_int,
+                            const int32_t *__restrict__ qb, float *__restrict__ rec, uint32_t *err_word) {
+    extern __shared__ __align__(16) uint32_t run_smem[];
+    const uint32_t warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Axis 2's entries of all targets: {pre | cc << 16, jj | stencil << 16 | bb << 19}.
+    uint2 *tab = reinterpret_cast<uint2 *>(run_smem);
+    float *s = reinterpret_cast<float *>(run_smem + R.tab_words + warp * R.line_words);
+    float *ts = s + R.line_words - R.nb2 * R.rounds;
+    for (uint32_t r = 0; r < R.rounds; r++)
+        for (uint32_t k = threadIdx.x; k < R.r[r].count; k += blockDim.x) {
+            const AxisEntry e = load_entry(ent + R.r[r].ent2 + k);
+            tab[R.r[r].first + k] = make_uint2((uint32_t)e.pre | e.cc << 16, e.jj | e.stencil << 16 | e.bb << 19);
         }
-        store_lines(fg, col, sl, rec);
+    __syncthreads();
+    for (uint32_t line = blockIdx.x * warps + warp; line < R.lines; line += gridDim.x * warps) {
+        const RunLine l = run_line(R, ent, rec, line);
+        auto load_qbs = [&](const LineQBs &L, uint32_t r, uint32_t k, int32_t (&q)[kRunAhead]) {
+            const uint32_t count = R.r[r].count, first = R.r[r].first;
+#pragma unroll
+            for (uint32_t j = 0; j < kRunAhead; j++) {
+                if (k + 32 * j >= count) break;
+                const uint32_t i = k + 32 * j + lane;
+                q[j] = 0;
+                if (i >= count) continue;
+                const uint2 e = tab[first + i];
+                const uint32_t o = L.mul * (e.x & 0xffff) + (L.u * (e.x >> 16) + (e.y & 0xffff)) * L.w + L.x;
+                if (o < L.limit) q[j] = __ldg(L.q + o);
+                else atomicOr(err_word, 4u);
+            }
+        };
+        int32_t q[kRunAhead];
+        LineQBs L = line_qbs(R.r[0], l, qb);
+        load_qbs(L, 0, 0, q);
+        for (uint32_t k = lane; k < R.known; k += 32) s[padded(k * R.step)] = l.g[k * R.step];
+        for (uint32_t k = lane; k < R.nb2 * R.rounds; k += 32) ts[k] = run_t(R, t_int, l.blk + k / R.rounds, k % R.rounds);
+        __syncwarp();
+        for (uint32_t r = 0; r < R.rounds; r++) {
+            const uint32_t hs = R.r[r].hs, count = R.r[r].count, first = R.r[r].first;
+            const double eb2 = R.r[r].eb2;
+            for (uint32_t k = 0; k < count; k += 32 * kRunAhead) {
+                int32_t next[kRunAhead];
+                if (k + 32 * kRunAhead < count) {
+                    load_qbs(L, r, k + 32 * kRunAhead, next);
+                } else if (r + 1 < R.rounds) {
+                    L = line_qbs(R.r[r + 1], l, qb);
+                    load_qbs(L, r + 1, 0, next);
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < kRunAhead; j++) {
+                    if (k + 32 * j >= count) break;
+                    const uint32_t i = k + 32 * j + lane;
+                    if (i >= count) continue;
+                    const uint32_t ii = hs * (2 * i + 1), w = tab[first + i].y, sc = (w >> 16) & 7;
+                    const float m1 = s[padded(ii - hs)];
+                    float pred;
+                    if (sc <= kStencilQuintic) {
+                        const float p1 = s[padded(ii + hs)], m3 = s[padded(ii - 3 * hs)], p3 = s[padded(ii + 3 * hs)];
+                        if (sc == kStencilCubic) {
+                            const double td = (double)ts[(w >> 19) * R.rounds + r];
+                            pred = cubic(m3, m1, p1, p3, __dsub_rn(0.25, td), __dadd_rn(0.25, td));
+                        } else {
+                            const StencilIn v{m1, p1, m3, p3, s[padded(ii - 5 * hs)], s[padded(ii + 5 * hs)]};
+                            pred = predict_loaded(v, kStencilQuintic, 0.0f);
+                        }
+                    } else {
+                        pred = predict_edge(s, ii, hs, sc);
+                    }
+                    s[padded(ii)] = __double2float_rn(__fma_rn(-(double)q[j], eb2, (double)pred));
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < kRunAhead; j++) q[j] = next[j];
+            }
+            __syncwarp();
+        }
+        const uint32_t hs = R.r[R.rounds - 1].hs;
+        for (uint32_t i = lane * hs; i < R.n2; i += 32 * hs) l.g[i] = s[padded(i)];
+        __syncwarp();
+    }
+}
+
+// One block along axis 2: no table, everything follows from a target's index. kLanes lanes per line
+// (16: two lines in a warp, which then share the coarse rounds' steps). A round's interior targets
+// are 1 .. cubics; their shared-memory addresses move by a constant from step to step, because a step
+// of kLanes targets is a multiple of 32 values. The targets at the line's ends (the first, and up to
+// two last) are lanes 0 to 2's, in one step of their own.
+template <uint32_t kLanes>
+__global__ void __launch_bounds__(32 * kRunWarps, kRunCtas)
+    lines_decompress_one_kernel(const __grid_constant__ LineRun R, const AxisEntry *__restrict__ ent,
+                                const int64_t *__restrict__ t_int, const int32_t *__restrict__ qb, float *__restrict__ rec,
+                                uint32_t *err_word) {
+    extern __shared__ __align__(16) uint32_t run_smem[];
+    constexpr uint32_t kPer = 32 / kLanes;
+    const uint32_t groups = blockDim.x / kLanes, group = threadIdx.x / kLanes, lane = threadIdx.x & 31,
+                   sub = threadIdx.x & (kLanes - 1);
+    float *s = reinterpret_cast<float *>(run_smem + group * R.line_words);
+    float *ts = s + R.line_words - R.rounds;
+    const uint32_t step = gridDim.x * groups;
+    for (uint32_t at = blockIdx.x * groups + group; at - group % kPer < R.lines; at += step) {
+        const bool real = at < R.lines;  // a group past the last line works on that one and stores nothing
+        const RunLine l = run_line(R, ent, rec, real ? at : R.lines - 1);
+        auto end_target = [&](uint32_t r) { return sub == 0 ? 0 : R.r[r].cubics + sub; };  // lanes 0 to 2
+        auto load = [&](const LineQBs &L, uint32_t o) {
+            if (o < L.limit) return __ldg(L.q + o);
+            atomicOr(err_word, 4u);
+            return 0;
+        };
+        auto load_ends = [&](LineQBs &L, uint32_t r) {
+            L.x += L.u * R.r[r].count * L.w;
+            const uint32_t i = end_target(r);
+            return sub < 3 && i < R.r[r].count ? load(L, i * L.w + L.x) : 0;
+        };
+        auto load_inner = [&](const LineQBs &L, uint32_t r, uint32_t k, int32_t (&q)[kRunAhead]) {
+            const uint32_t cubics = R.r[r].cubics;
+#pragma unroll
+            for (uint32_t j = 0; j < kRunAhead; j++) {
+                if (k + kLanes * j >= cubics) break;
+                const uint32_t i = k + kLanes * j + sub;
+                q[j] = i < cubics ? load(L, (i + 1) * L.w + L.x) : 0;
+            }
+        };
+        int32_t q[kRunAhead], qe;
+        LineQBs L = line_qbs(R.r[0], l, qb);
+        qe = load_ends(L, 0);
+        load_inner(L, 0, 0, q);
+        for (uint32_t k = sub; k < R.known; k += kLanes) s[padded(k * R.step)] = l.g[k * R.step];
+        for (uint32_t r = sub; r < R.rounds; r += kLanes) ts[r] = run_t(R, t_int, l.blk, r);
+        __syncwarp();
+        for (uint32_t r = 0; r < R.rounds; r++) {
+            const uint32_t hs = R.r[r].hs, cubics = R.r[r].cubics, quintics = R.r[r].quintics;
+            const double eb2 = R.r[r].eb2, td = (double)ts[r], c1 = __dsub_rn(0.25, td), c2 = __dadd_rn(0.25, td);
+            const uint32_t ie = end_target(r);
+            const int32_t q_end = qe;
+            // Inner targets, from 1: addresses of the target and its neighbours.
+            const uint32_t i0 = hs * (2 * sub + 3), move = 2 * hs * kLanes / 32 * 33;
+            const float *a3 = s + padded(i0 - 3 * hs), *a1 = s + padded(i0 - hs), *b1 = s + padded(i0 + hs),
+                        *b3 = s + padded(i0 + 3 * hs);
+            float *c = s + padded(i0);
+            uint32_t k = 0;
+            do {
+                int32_t next[kRunAhead];
+                if (k + kLanes * kRunAhead < cubics) {
+                    load_inner(L, r, k + kLanes * kRunAhead, next);
+                } else if (r + 1 < R.rounds) {
+                    L = line_qbs(R.r[r + 1], l, qb);
+                    qe = load_ends(L, r + 1);
+                    load_inner(L, r + 1, 0, next);
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < kRunAhead; j++) {
+                    if (k + kLanes * j >= cubics) break;
+                    const uint32_t i = k + kLanes * j + sub;
+                    if (i < cubics) {
+                        float pred;
+                        if (i - 1 < quintics) {
+                            const uint32_t ii = hs * (2 * i + 3);
+                            const StencilIn v{*a1, *b1, *a3, *b3, s[padded(ii - 5 * hs)], s[padded(ii + 5 * hs)]};
+                            pred = predict_loaded(v, kStencilQuintic, 0.0f);
+                        } else {
+                            pred = cubic(*a3, *a1, *b1, *b3, c1, c2);
+                        }
+                        *c = __double2float_rn(__fma_rn(-(double)q[j], eb2, (double)pred));
+                    }
+                    a3 += move;
+                    a1 += move;
+                    b1 += move;
+                    b3 += move;
+                    c += move;
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < kRunAhead; j++) q[j] = next[j];
+                k += kLanes * kRunAhead;
+            } while (k < cubics);
+            if (sub < 3 && ie < R.r[r].count) {
+                const uint32_t ii = hs * (2 * ie + 1);
+                const float pred = predict_edge(s, ii, hs, stencil_case(ii, hs, R.n2, false));
+                s[padded(ii)] = __double2float_rn(__fma_rn(-(double)q_end, eb2, (double)pred));
+            }
+            __syncwarp();
+        }
+        // The warp stores its lines one after another, whole sectors at a time.
+        const uint32_t hs = R.r[R.rounds - 1].hs;
+        for (uint32_t m = 0; m < kPer; m++) {
+            float *g = reinterpret_cast<float *>(__shfl_sync(0xffffffffu, (unsigned long long)l.g, m * kLanes));
+            if (!__shfl_sync(0xffffffffu, real, m * kLanes)) continue;
+            const float *line = s + ((int)m - (int)(lane / kLanes)) * (int)R.line_words;
+            for (uint32_t i = lane * hs; i < R.n2; i += 32 * hs) g[i] = line[padded(i)];
+        }
+        __syncwarp();
     }
 }
 
@@ -324,21 +559,111 @@ __global__ void __launch_bounds__(fastsel::kThreads, 6)
 
 uint32_t lines_smem_limit() { return 96 * 1024; }
 
-cudaError_t launch_lines_decompress(const FieldGeom &fg, const RoundGeom *rounds, const AxisEntry *ent, const uint64_t *qoff,
-                                    const int64_t *t_int, const int32_t *qb, float *rec, uint32_t *err, uint32_t set,
-                                    uint32_t line_bytes, cudaStream_t st) {
-    const uint32_t items = column_count(set, (uint32_t)fg.block_num[0], (uint32_t)fg.block_num[1]);
-    if (items == 0) return cudaSuccess;
-    if (fg.block_num[2] > kMaxColumnBlocks) return cudaErrorInvalidValue;
-    const uint32_t smem = (uint32_t)(align16(sizeof(DecShared)) + line_bytes);
-    cudaError_t e = cudaFuncSetAttribute(lines_decompress_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// The launch's CTAs: the most warps on an SM, `per` lines each; of equals the wider CTA (fewer copies
+// of the table), unless that leaves SMs without lines.
+struct RunShape {
+    uint32_t warps, ctas;  // of a CTA, of an SM
+};
+static RunShape run_shape(uint64_t tab_words, uint64_t line_words, uint32_t per, uint64_t lines) {
+    RunShape s{1, 0};
+    for (uint32_t w = kRunWarps; w >= 1; w /= 2) {
+        const uint64_t bytes = 4 * (tab_words + w * per * line_words);
+        if (bytes > kRunSmem) continue;
+        const uint32_t c = (uint32_t)std::min<uint64_t>(kRunWarps * kRunCtas / w, kRunSm / (bytes + 1024));
+        if (c * w > s.ctas * s.warps || (w >= 4 && lines < 148ull * 2 * w * per)) s = {w, c};
+    }
+    return s;
+}
+
+// Where a run goes line by line. A line costs its rounds' steps whatever its length, 1.1 ns in all at
+// five rounds, so short lines are better off round by round, where a step holds several lines
+// (512x512xn: n = 32 140 against 240 us, n = 64 260 against 298; 256x256x512 in nine rounds 510 against
+// 185), unless they are so few that launches are what the rounds cost (24x20x17: 39 against 11 us). With
+// a table, a CTA must also fit as often as its registers allow: with half of the warps the rounds are
+// as fast (64x64x4096 in four rounds: 203 against 238 us; 256x256x512 in three: 362 against 199).
+constexpr uint64_t kRunTargets = 96, kRunFewLines = 4096;
+
+uint32_t lines_run_length(const FieldGeom &fg, const RoundGeom *rounds, uint32_t count) {
+    uint32_t len = 0, used = 0;
+    uint64_t targets = 0, lines = 0;
+    for (; len < count && rounds[len].dir == 2; len++) {
+        if (!rounds[len].targets) continue;
+        used++;
+        targets += rounds[len].tcount[2];
+        lines = rounds[len].tcount[0] * rounds[len].tcount[1];
+    }
+    if (used < 2 || used > kRunRounds || (targets < kRunTargets && lines > kRunFewLines)) return 0;
+    if (fg.origin[0] || fg.origin[1] || fg.origin[2] || fg.n[2] >= 65536) return 0;  // 16-bit entries
+    // 32-bit offsets within a row of blocks' QBs.
+    const uint64_t c0 = std::min(fg.block_shape[0] + 1, fg.n[0]), c1 = std::min(fg.block_shape[1] + 1, fg.n[1]);
+    if (c0 * c1 >= (1ull << 31) / fg.n[2]) return 0;
+    const bool one = fg.block_num[2] == 1;
+    const RunShape s = run_shape(one ? 0 : 2 * targets, fg.n[2] + fg.n[2] / 32 + 1 + fg.block_num[2] * used, 1, lines);
+    return s.ctas * s.warps >= (one ? 1 : kRunWarps * kRunCtas) ? len : 0;
+}
+
+cudaError_t launch_lines_decompress(const FieldGeom &fg, const RoundGeom *rounds, uint32_t len, uint32_t l0, const AxisEntry *ent,
+                                    const uint64_t *qoff, const int64_t *t_int, const int32_t *qb, float *rec, uint32_t *err,
+                                    cudaStream_t st) {
+    LineRun R{};
+    R.n1n2 = fg.n[1] * fg.n[2];
+    R.n2 = (uint32_t)fg.n[2];
+    for (uint32_t l = 0; l < len; l++) {
+        const RoundGeom &rg = rounds[l];
+        if (rg.targets == 0) continue;
+        if (R.rounds == 0) {
+            R.ent0 = rg.ent_off[0];
+            R.ent1 = rg.ent_off[1];
+            R.total1 = rg.total[1];
+            R.lines = (uint32_t)(rg.tcount[0] * rg.tcount[1]);
+            R.T1 = (uint32_t)rg.tcount[1];
+            R.step = (uint32_t)(2 * rg.hs);
+            R.known = (R.n2 + R.step - 1) / R.step;
+        }
+        RunRound &m = R.r[R.rounds++];
+        m.eb2 = (double)rg.eb + (double)rg.eb;
+        m.qoff = qoff[l0 + l + 1];
+        m.qb_total = rg.qb_total;
+        m.ent2 = rg.ent_off[2];
+        m.hs = (uint32_t)rg.hs;
+        m.count = (uint32_t)rg.tcount[2];
+        m.first = R.targets;
+        m.total2 = (uint32_t)rg.total[2];
+        m.order = (uint32_t)rg.order;
+        m.l = l0 + l;
+        // Targets i >= 1 with (2 i + 1) hs + 3 hs < n2, and i >= 2 with (2 i + 1) hs + 5 hs < n2.
+        auto below = [&](uint64_t reach, uint32_t from) {
+            const uint64_t end = reach < R.n2 ? (R.n2 - reach + 2 * rg.hs - 1) / (2 * rg.hs) : 0;
+            return end > from ? (uint32_t)(end - from) : 0u;
+        };
+        m.cubics = below(4 * rg.hs, 1);
+        m.quintics = fg.quintic ? below(6 * rg.hs, 2) : 0;
+        R.targets += m.count;
+    }
+    R.nb1 = (uint32_t)fg.block_num[1];
+    R.nb2 = (uint32_t)fg.block_num[2];
+    R.layers = fg.layer_num;
+    R.tp = (float)fg.t_precision;
+    const bool one = R.nb2 == 1;
+    R.tab_words = one ? 0 : 2 * R.targets;
+    R.line_words = R.n2 + R.n2 / 32 + 1 + R.nb2 * R.rounds;
+    RunShape sh = run_shape(R.tab_words, R.line_words, 1, R.lines);
+    uint32_t per = 1;
+    if (one && R.lines >= 148 * 2 * 16) {
+        // Two lines a warp where that leaves the SMs their warps.
+        const RunShape two = run_shape(R.tab_words, R.line_words, 2, R.lines);
+        if (two.warps * two.ctas == kRunWarps * kRunCtas) {
+            sh = two;
+            per = 2;
+        }
+    }
+    const uint32_t warps = sh.warps, ctas = sh.ctas;
+    const uint32_t smem = 4 * (R.tab_words + warps * per * R.line_words);
+    auto kernel = !one ? lines_decompress_kernel : per == 2 ? lines_decompress_one_kernel<16> : lines_decompress_one_kernel<32>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRunSmem);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lines_decompress_kernel, 256, smem);
-    if (e != cudaSuccess) return e;
-    const uint64_t cap = 148ull * (per_sm > 0 ? per_sm : 1);
-    lines_decompress_kernel<<<(unsigned)(items < cap ? items : cap), 256, smem, st>>>(fg, rounds, ent, qoff, t_int, qb, rec, set,
-                                                                                      items, err);
+    const uint32_t grid = std::min((R.lines + warps * per - 1) / (warps * per), 148 * ctas);
+    kernel<<<grid, 32 * warps, smem, st>>>(R, ent, t_int, qb, rec, err);
     count_launch();
     return cudaGetLastError();
 }

@@ -101,6 +101,13 @@ cudaError_t launch_round_compress(const FieldGeom &fg, const RoundGeom &rg, cons
 cudaError_t launch_round_decompress(const FieldGeom &fg, const RoundGeom &rg, uint32_t l, const AxisEntry *ent,
                                     const int64_t *t_int, const int32_t *qb, float *rec, uint32_t *err, cudaStream_t st);
 
+// Consecutive rounds along axis 2 decompressed line by line in one launch (k_lines.cu). The first: how
+// many of the `count` rounds at `rounds` one launch takes (0: none, the rounds go one by one). The
+// second: `len` rounds at `rounds`, round l0 of the plan first; qoff has the streams' offsets in qb.
+uint32_t lines_run_length(const FieldGeom &fg, const RoundGeom *rounds, uint32_t count);
+cudaError_t launch_lines_decompress(const FieldGeom &fg, const RoundGeom *rounds, uint32_t len, uint32_t l0, const AxisEntry *ent,
+                                    const uint64_t *qoff, const int64_t *t_int, const int32_t *qb, float *rec, uint32_t *err,
+                                    cudaStream_t st);
 // Fused rounds for plans whose every round runs along axis 2 (k_lines.cu). rounds and qoff (the
 // stream offsets, pivots first) are device copies of the plan's round table; line_bytes is the
 // size of one column's lines (at most lines_smem_limit()), and the field has at most 64 blocks
@@ -110,9 +117,6 @@ cudaError_t launch_round_decompress(const FieldGeom &fg, const RoundGeom &rg, ui
 // indices of the same set.
 enum : uint32_t { kColumnsAll = 0, kColumnsInterior = 1, kColumnsEdge = 2 };
 uint32_t lines_smem_limit();
-cudaError_t launch_lines_decompress(const FieldGeom &fg, const RoundGeom *rounds, const AxisEntry *ent, const uint64_t *qoff,
-                                    const int64_t *t_int, const int32_t *qb, float *rec, uint32_t *err, uint32_t set,
-                                    uint32_t line_bytes, cudaStream_t st);
 // A full pass (resume_in == nullptr) or the resumption of the listed (column, round) pairs. Blocks
 // handed to the exact path are listed per round in bail_blocks + round * nblocks (bail_count[round])
 // and their columns in resume_out (resume_count).
