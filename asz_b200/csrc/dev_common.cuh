@@ -130,6 +130,15 @@ struct BatchField {
     uint32_t tpl_log2[64];          // threads per target line (log2), per round
 };
 
+// A batch field's data range (one launch for all fields): as range_kernel's results, which start at
+// INT32_MAX, INT32_MIN and 0.
+struct RangeField {
+    const float *x;
+    uint64_t n;
+    int32_t range[2];
+    unsigned long long nonfinite;
+};
+
 // One round's targets of a probe frame's target block, in the block's loop order, and what the host's
 // reductions need of each.
 struct ProbeSpan {

@@ -218,6 +218,8 @@ struct asz_ctx {
     PinnedBuf plan_host, plan_words;
     DevBuf fam_tab, fam_mem, fam_points;  // predictor-family probes: tables, frames, the targets' points
     PinnedBuf fam_host;
+    DevBuf prep_mem;  // a batch's ranges and slopes
+    PinnedBuf prep_host;
     bool have_last = false;
     // Profiling (asz_profile_*).
     bool prof = false;
@@ -919,6 +921,8 @@ void asz_destroy(asz_ctx *c) {
     c->plan_words.release();
     for (DevBuf *b : {&c->fam_tab, &c->fam_mem, &c->fam_points}) b->release();
     c->fam_host.release();
+    c->prep_mem.release();
+    c->prep_host.release();
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
     asz::host::sweep_release(c->sweep);
@@ -1133,6 +1137,13 @@ int encode_set_done(asz_ctx *ctx) {  // after the synchronisation
     return ASZ_OK;
 }
 
+float range_value(int32_t k) {  // of an ordered-int key
+    const uint32_t b = k >= 0 ? (uint32_t)k : ((uint32_t)k ^ 0x7fffffffu);
+    float f;
+    std::memcpy(&f, &b, 4);
+    return f;
+}
+
 // first_max: a zero maximum takes the sign of the first largest element (std::max_element)
 // instead of the last one (std::minmax_element).
 int compute_range(asz_ctx *ctx, const float *d_in, u64 N, float &mn, float &mx, bool first_max = false) {
@@ -1154,14 +1165,8 @@ int compute_range(asz_ctx *ctx, const float *d_in, u64 N, float &mn, float &mx, 
     CK(cudaMemcpyAsync(&hw->misc, dm, offsetof(MiscLayout, dec_err), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (h.nonfinite) return fail(ctx, ASZ_E_DATA, "input contains a nonfinite value");
-    auto tof = [](int32_t k) {
-        uint32_t b = k >= 0 ? (uint32_t)k : ((uint32_t)k ^ 0x7fffffffu);
-        float f;
-        std::memcpy(&f, &b, 4);
-        return f;
-    };
-    mn = tof(h.range[0]);
-    mx = tof(h.range[1]);
+    mn = range_value(h.range[0]);
+    mx = range_value(h.range[1]);
     if (mn == 0.0f || mx == 0.0f) {
         // minmax_element keeps the first smallest and the last largest element; with zeros of
         // both signs present, that decides the stored sign.
@@ -1207,73 +1212,16 @@ void slope_boxes(const uint64_t dims[3], const asz_params &p, float abs_eb, Samp
     }
 }
 
-// get_default_slope on given boxes over `field` (dims fdims): the whole field, or a compact copy of
-// the boxes' samples whose boxes keep the samples' order.
-int default_slope_on(asz_ctx *ctx, const float *field, const uint64_t fdims[3], SampleBox boxes[3], const asz_params &p,
-                     float abs_eb, float mn, float mx, const std::vector<float> &cand_t, float &slope_out,
-                     float &max_invalid_out, int &reason_out) {
-    FieldGeom fg{};
-    for (int a = 0; a < 3; a++) fg.n[a] = fdims[a];
-    const uint64_t *dims = fdims;
-    const float *d_in = field;
+void slope_evals(const asz_params &p, float abs_eb, const std::vector<float> &cand_t, ProxyEval *evals) {
     const float ebs[2] = {abs_eb * p.default_slope_eb_span, abs_eb / p.default_slope_eb_span};
-    MiscLayout *dm = ctx->misc.as<MiscLayout>();
-    uint32_t cap = 1;
-    for (int d = 0; d < 3; d++) {
-        boxes[d].log2_off = boxes[d].n ? log2_table(ctx, boxes[d].n) : 0;
-        cap = std::max<uint32_t>(cap, boxes[d].n);
-    }
-    const uint32_t ne = (uint32_t)(2 * cand_t.size());
-    if (ne > 64) return fail(ctx, ASZ_E_UNSUPPORTED, "too many t candidates for the default slope");
-    ProxyEval evals[64];
     for (int i = 0; i < 2; i++)
         for (size_t k = 0; k < cand_t.size(); k++) evals[i * cand_t.size() + k] = ProxyEval{cand_t[k], ebs[i]};
-    int rc = upload_log2(ctx);
-    if (rc) return rc;
-    uint32_t bcap, tcap;
-    u64 sstride;
-    scratch_dims(cap, bcap, tcap, sstride);
-    CK(ctx->scratch.reserve(3 * sstride));
-    rc = proxy_upload(ctx, boxes, 3, evals, ne);
-    if (rc) return rc;
-    const float R = mx - mn;
-    // The shared-memory exact kernel when the maps fit, else the same kernel with global scratch;
-    // the serial kernel when a key exceeds int32 (the exact kernels then report error bit 2).
-    bool serial = cap > exact_cap();
-    const MiscLayout *res = nullptr;
-    if (!serial) {
-        {
-            ProfScope ps_slope(ctx, "slope", 0);
-            CK(launch_slope_exact(dm->boxes, dm->evals, ne, d_in, dims[1] * dims[2], dims[2], ctx->log2arena.as<float>(),
-                                  R * R, dm->h1, dm->x, dm->m, &dm->perr, exact_cap(), cap, 3, ctx->stream));
-        }
-        rc = proxy_results(ctx, res);
-        if (rc) return rc;
-        if (res->perr) {
-            serial = true;
-            CK(cudaMemsetAsync(&dm->perr, 0, 4, ctx->stream));
-        }
-    }
-    if (serial) {
-        bool done = false;
-        rc = abmap_exact_global(ctx, ne, d_in, dims[1] * dims[2], dims[2], R * R, cap, 3, "slope_global", done);
-        if (rc) return rc;
-        serial = !done;
-    }
-    if (serial) {
-        ProfScope ps_slope(ctx, "slope_serial", 0);
-        CK(launch_slope_v0(fg, dm->boxes, dm->evals, ne, d_in, ctx->log2arena.as<float>(), R * R, ctx->scratch.as<uint8_t>(),
-                           sstride, cap, bcap, tcap, dm->h1, dm->x, dm->m, &dm->perr, 3, ctx->stream));
-    }
-    if (serial) {
-        rc = proxy_results(ctx, res);
-        if (rc) return rc;
-    } else {
-        res = &((HostWords *)ctx->words.p)->misc;  // read with the last launch's error word
-    }
-    const float *h1 = res->h1, *x = res->x;
-    const uint32_t *m = res->m;
-    if (res->perr) return fail(ctx, ASZ_E_DEVICE, "default-slope kernel reported an internal error");
+}
+
+// The slope from the three boxes' proxies.
+int slope_of(asz_ctx *ctx, const asz_params &p, const std::vector<float> &cand_t, const float *h1, const float *x, const uint32_t *m,
+             float &slope_out, float &max_invalid_out, int &reason_out) {
+    const uint32_t ne = (uint32_t)(2 * cand_t.size());
     float avg_h1[2] = {0, 0}, avg_psnr[2] = {0, 0};
     u64 valid[2] = {0, 0};
     for (int d = 0; d < 3; d++) {
@@ -1322,6 +1270,72 @@ int default_slope_on(asz_ctx *ctx, const float *field, const uint64_t fdims[3], 
         slope_out = psnr_diff / h1_diff;
     }
     return ASZ_OK;
+}
+
+// get_default_slope on given boxes over `field` (dims fdims): the whole field, or a compact copy of
+// the boxes' samples whose boxes keep the samples' order.
+int default_slope_on(asz_ctx *ctx, const float *field, const uint64_t fdims[3], SampleBox boxes[3], const asz_params &p,
+                     float abs_eb, float mn, float mx, const std::vector<float> &cand_t, float &slope_out,
+                     float &max_invalid_out, int &reason_out) {
+    FieldGeom fg{};
+    for (int a = 0; a < 3; a++) fg.n[a] = fdims[a];
+    const uint64_t *dims = fdims;
+    const float *d_in = field;
+    MiscLayout *dm = ctx->misc.as<MiscLayout>();
+    uint32_t cap = 1;
+    for (int d = 0; d < 3; d++) {
+        boxes[d].log2_off = boxes[d].n ? log2_table(ctx, boxes[d].n) : 0;
+        cap = std::max<uint32_t>(cap, boxes[d].n);
+    }
+    const uint32_t ne = (uint32_t)(2 * cand_t.size());
+    if (ne > 64) return fail(ctx, ASZ_E_UNSUPPORTED, "too many t candidates for the default slope");
+    ProxyEval evals[64];
+    slope_evals(p, abs_eb, cand_t, evals);
+    int rc = upload_log2(ctx);
+    if (rc) return rc;
+    uint32_t bcap, tcap;
+    u64 sstride;
+    scratch_dims(cap, bcap, tcap, sstride);
+    CK(ctx->scratch.reserve(3 * sstride));
+    rc = proxy_upload(ctx, boxes, 3, evals, ne);
+    if (rc) return rc;
+    const float R = mx - mn;
+    // The shared-memory exact kernel when the maps fit, else the same kernel with global scratch;
+    // the serial kernel when a key exceeds int32 (the exact kernels then report error bit 2).
+    bool serial = cap > exact_cap();
+    const MiscLayout *res = nullptr;
+    if (!serial) {
+        {
+            ProfScope ps_slope(ctx, "slope", 0);
+            CK(launch_slope_exact(dm->boxes, dm->evals, ne, d_in, dims[1] * dims[2], dims[2], ctx->log2arena.as<float>(),
+                                  R * R, dm->h1, dm->x, dm->m, &dm->perr, exact_cap(), cap, 3, ctx->stream));
+        }
+        rc = proxy_results(ctx, res);
+        if (rc) return rc;
+        if (res->perr) {
+            serial = true;
+            CK(cudaMemsetAsync(&dm->perr, 0, 4, ctx->stream));
+        }
+    }
+    if (serial) {
+        bool done = false;
+        rc = abmap_exact_global(ctx, ne, d_in, dims[1] * dims[2], dims[2], R * R, cap, 3, "slope_global", done);
+        if (rc) return rc;
+        serial = !done;
+    }
+    if (serial) {
+        ProfScope ps_slope(ctx, "slope_serial", 0);
+        CK(launch_slope_v0(fg, dm->boxes, dm->evals, ne, d_in, ctx->log2arena.as<float>(), R * R, ctx->scratch.as<uint8_t>(),
+                           sstride, cap, bcap, tcap, dm->h1, dm->x, dm->m, &dm->perr, 3, ctx->stream));
+    }
+    if (serial) {
+        rc = proxy_results(ctx, res);
+        if (rc) return rc;
+    } else {
+        res = &((HostWords *)ctx->words.p)->misc;  // read with the last launch's error word
+    }
+    if (res->perr) return fail(ctx, ASZ_E_DEVICE, "default-slope kernel reported an internal error");
+    return slope_of(ctx, p, cand_t, res->h1, res->x, res->m, slope_out, max_invalid_out, reason_out);
 }
 
 int default_slope(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const asz_params &p, float abs_eb, float mn,
@@ -2767,18 +2781,21 @@ int encode_fields(asz_ctx *ctx, const std::vector<EncodeArgs> &A, std::vector<as
     CK(ctx->hist.reserve(std::max<u64>(hist_total, 1) * 8));
     CK(cudaMemsetAsync(ctx->hist.p, 0, std::max<u64>(hist_total, 1) * 8, st));
     unsigned long long *d_hist = ctx->hist.as<unsigned long long>();
+    std::vector<HistStream> hs;
+    u64 hist_bytes = 0;
     for (u64 f = 0; f < nf; f++) {
         const EncodeArgs &a = A[f];
-        const u64 L = a.plan->pred.size();
-        std::vector<StreamOut> &so = SO[f];
-        ProfScope ps_hist(ctx, "histogram", (a.G->nblocks * L) * 8 + a.N * 4);
-        if (so[0].count)
-            CK(launch_histogram<int64_t>(a.d_tint, so[0].count, so[0].lo, (u64)(so[0].hi - so[0].lo) + 1, d_hist + so[0].hist_off,
-                                         st));
-        for (u64 s2 = 0; s2 <= L; s2++)
-            if (so[s2 + 1].count && !so[s2 + 1].prebuilt)
-                CK(launch_histogram<int32_t>(a.d_qb + (*a.qb_off)[s2], (*a.qb_len)[s2], so[s2 + 1].lo,
-                                             (u64)(so[s2 + 1].hi - so[s2 + 1].lo) + 1, d_hist + so[s2 + 1].hist_off, st));
+        for (u64 s2 = 0; s2 < SO[f].size(); s2++) {
+            const StreamOut &o = SO[f][s2];
+            if (!o.count || o.prebuilt) continue;
+            const void *sym = s2 == 0 ? (const void *)a.d_tint : (const void *)(a.d_qb + (*a.qb_off)[s2 - 1]);
+            hs.push_back(HistStream{sym, o.count, o.lo, (u64)(o.hi - o.lo) + 1, d_hist + o.hist_off, s2 == 0, 0});
+            hist_bytes += o.count * (s2 == 0 ? 8 : 4);
+        }
+    }
+    if (!hs.empty()) {
+        ProfScope ps_hist(ctx, "histogram", hist_bytes);
+        CK(launch_histogram_set(hs.data(), (uint32_t)hs.size(), st));
     }
     std::optional<HostScope> hs_h(std::in_place, ctx, "host:codes_hist_d2h");
     CK(ctx->enc_host.reserve(std::max<u64>(hist_total, 1) * 8));
@@ -3942,7 +3959,80 @@ struct BatchItem {
     Geometry G;
     std::vector<u64> qb_off, qb_len;
     u64 o_in = 0, o_rec = 0, o_qb = 0, o_tval = 0, o_tint = 0, o_ent = 0, o_prox = 0;
+    bool have_range = false;              // from the launch for all fields
+    const SlopeOut *slope_at = nullptr;  // likewise, in the context's pinned buffer
 };
+
+// Ranges and default slopes of a batch's fields, a launch and a wait each for all fields. What is out of
+// the ordinary is left to the single-field calls, field by field, with their errors: nonfinite values,
+// a constant field, a zero extremum (its sign takes another look), groups that the shared-memory
+// replay does not take.
+int batch_slopes(asz_ctx *ctx, std::vector<BatchItem> &B, const asz_params &p, float rel_eb, const std::vector<float> &cand) {
+    cudaStream_t st = ctx->stream;
+    const uint32_t nf = (uint32_t)B.size(), ne = (uint32_t)(2 * cand.size());
+    if (nf < 2 || nf > 65535 || ne > 64) return ASZ_OK;
+    CK(ctx->prep_host.reserve(nf * (sizeof(SlopeField) + sizeof(SlopeOut))));
+    CK(ctx->prep_mem.reserve(nf * (sizeof(SlopeField) + sizeof(SlopeOut))));
+    u64 most = 0, bytes = 0;
+    {
+        RangeField *h = (RangeField *)ctx->prep_host.p, *d = ctx->prep_mem.as<RangeField>();
+        for (uint32_t f = 0; f < nf; f++) {
+            h[f] = RangeField{B[f].d_in, B[f].N, {INT32_MAX, INT32_MIN}, 0};
+            most = std::max(most, B[f].N);
+            bytes += B[f].N * 4;
+        }
+        CK(cudaMemcpyAsync(d, h, nf * sizeof(RangeField), cudaMemcpyHostToDevice, st));
+        {
+            ProfScope ps(ctx, "range", bytes);
+            CK(launch_range_batch(d, nf, most, st));
+        }
+        CK(cudaMemcpyAsync(h, d, nf * sizeof(RangeField), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (uint32_t f = 0; f < nf; f++) {
+            BatchItem &b = B[f];
+            b.mn = range_value(h[f].range[0]);
+            b.mx = range_value(h[f].range[1]);
+            b.have_range = !h[f].nonfinite && b.mn != 0.0f && b.mx != 0.0f && b.mn != b.mx;
+            if (b.have_range) b.abs_eb = rel_eb * (b.mx - b.mn);
+        }
+    }
+    SlopeField *h = (SlopeField *)ctx->prep_host.p, *d = ctx->prep_mem.as<SlopeField>();
+    std::vector<uint32_t> taken;
+    uint32_t cap = 1;
+    for (uint32_t f = 0; f < nf; f++) {
+        const BatchItem &b = B[f];
+        if (!b.have_range) continue;
+        SlopeField &s = h[taken.size()];
+        std::memset(&s, 0, sizeof(s));
+        slope_boxes(b.dims, p, b.abs_eb, s.boxes);
+        uint32_t n = 1;
+        for (const SampleBox &x : s.boxes) n = std::max(n, x.n);
+        if (n > exact_cap()) continue;
+        cap = std::max(cap, n);
+        for (SampleBox &x : s.boxes) x.log2_off = x.n ? log2_table(ctx, x.n) : 0;
+        slope_evals(p, b.abs_eb, cand, s.evals);
+        s.orig = b.d_in;
+        s.n1n2 = b.dims[1] * b.dims[2];
+        s.n2 = b.dims[2];
+        s.R2 = (b.mx - b.mn) * (b.mx - b.mn);
+        taken.push_back(f);
+    }
+    if (taken.empty()) return ASZ_OK;
+    const int rc = upload_log2(ctx);
+    if (rc) return rc;
+    SlopeOut *ho = (SlopeOut *)(h + nf), *dout = (SlopeOut *)(d + nf);
+    CK(cudaMemcpyAsync(d, h, taken.size() * sizeof(SlopeField), cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(dout, 0, taken.size() * sizeof(SlopeOut), st));
+    {
+        ProfScope ps(ctx, "slope", 0);
+        CK(launch_slope_batch(d, (uint32_t)taken.size(), ne, ctx->log2arena.as<float>(), dout, exact_cap(), cap, st));
+    }
+    CK(cudaMemcpyAsync(ho, dout, taken.size() * sizeof(SlopeOut), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (size_t i = 0; i < taken.size(); i++)
+        if (!ho[i].err) B[taken[i]].slope_at = &ho[i];  // err: a key beyond int32
+    return ASZ_OK;
+}
 
 // Launch shapes that change no result: CTAs per SM of the persistent selection and round
 // kernels, and a shift of the threads per target line (fewer threads per line, more lines per CTA).
@@ -4010,17 +4100,25 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     BR.h2d_s = secs(t_h2d, clk::now());
     auto t_prep = clk::now();
     const std::vector<float> cand = candidate_t(p);
+    if ((rc = batch_slopes(ctx, B, p, rel_eb, cand))) return rc;
     u64 nb_total = 0, ent_total = 0, tint_total = 0, qb_total = 0;
     uint32_t capmax = 1;
     std::vector<uint32_t> cap_round(L, 1);  // largest group of each round over the fields
     for (uint32_t f = 0; f < nf; f++) {
         BatchItem &b = B[f];
         const std::string tag = "field " + std::to_string(f) + ": ";
-        rc = compute_range(ctx, b.d_in, b.N, b.mn, b.mx);
-        if (rc) return fail(ctx, rc, tag + ctx->err);
-        if (b.mn == b.mx) return fail(ctx, ASZ_E_DATA, tag + "max_val==min_val");
-        b.abs_eb = rel_eb * (b.mx - b.mn);
-        rc = default_slope(ctx, b.d_in, b.dims, p, b.abs_eb, b.mn, b.mx, cand, b.slope, b.max_invalid, b.reason);
+        if (!b.have_range) {
+            rc = compute_range(ctx, b.d_in, b.N, b.mn, b.mx);
+            if (rc) return fail(ctx, rc, tag + ctx->err);
+            if (b.mn == b.mx) return fail(ctx, ASZ_E_DATA, tag + "max_val==min_val");
+            b.abs_eb = rel_eb * (b.mx - b.mn);
+        }
+        if (b.slope_at) {
+            const SlopeOut &o = *b.slope_at;
+            rc = slope_of(ctx, p, cand, o.h1, o.x, o.m, b.slope, b.max_invalid, b.reason);
+        } else {
+            rc = default_slope(ctx, b.d_in, b.dims, p, b.abs_eb, b.mn, b.mx, cand, b.slope, b.max_invalid, b.reason);
+        }
         if (rc) return fail(ctx, rc, tag + ctx->err);
         build_geometry(b.dims, plan, p, b.abs_eb, b.slope, quintic, b.G);
         if (!kernel_limits_ok(b.G)) return fail(ctx, ASZ_E_UNSUPPORTED, tag + "field too large for 32-bit line indexing");

@@ -27,8 +27,10 @@ __device__ __forceinline__ int32_t ord_key(float v) {
 }
 
 // out[0] = min key, out[1] = max key (ordered-int encoding), out[2] = count of non-finite values.
-__global__ void range_kernel(const float4 *__restrict__ x4, uint64_t n4, const float *__restrict__ tail, uint64_t ntail,
-                             int32_t *out, unsigned long long *nonfinite) {
+__device__ __forceinline__ void range_of(const float *__restrict__ x, uint64_t n, int32_t *out, unsigned long long *nonfinite) {
+    // 128-bit loads from the first 16-byte boundary on; the values before it and behind the last one.
+    const uint64_t head = min((uint64_t)((16 - (uintptr_t)x % 16) % 16 / 4), n), n4 = (n - head) / 4, ends = n - 4 * n4;
+    const float4 *x4 = reinterpret_cast<const float4 *>(x + head);
     int32_t mn = INT32_MAX, mx = INT32_MIN;
     unsigned long long bad = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -56,8 +58,8 @@ __global__ void range_kernel(const float4 *__restrict__ x4, uint64_t n4, const f
         take(v3);
     }
     for (; i < n4; i += stride) take(__ldg(x4 + i));
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < ntail; i += stride) {
-        float v = tail[i];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < ends; i += stride) {
+        const float v = x[i < head ? i : i + 4 * n4];
         if (!isfinite(v)) bad++;
         else {
             mn = min(mn, ord_key(v));
@@ -74,6 +76,15 @@ __global__ void range_kernel(const float4 *__restrict__ x4, uint64_t n4, const f
         atomicMax(&out[1], mx);
         if (bad) atomicAdd(nonfinite, bad);
     }
+}
+
+__global__ void range_kernel(const float *__restrict__ x, uint64_t n, int32_t *out, unsigned long long *nonfinite) {
+    range_of(x, n, out, nonfinite);
+}
+// The fields of a batch (y): eight of 16 MB 0.17 -> 0.05 ms, and one wait of the host.
+__global__ void range_batch_kernel(RangeField *F) {
+    RangeField &f = F[blockIdx.y];
+    range_of(f.x, f.n, f.range, &f.nonfinite);
 }
 
 // First and last index of a zero (either sign), for the sign of a zero minimum or maximum.
@@ -580,12 +591,16 @@ static unsigned grid_for(uint64_t n, unsigned threads, unsigned cap) {
     return (unsigned)(b < cap ? (b ? b : 1) : cap);
 }
 
+static unsigned range_grid(uint64_t n, unsigned cap) { return grid_for(std::max<uint64_t>(n / 4, 1), 256, cap); }
+
 cudaError_t launch_range(const float *x, uint64_t n, int32_t *out, unsigned long long *nonfinite, cudaStream_t st) {
-    // 128-bit loads when the pointer allows; otherwise (and for the tail) scalar loads.
-    uint64_t n4 = ((uintptr_t)x % 16 == 0) ? n / 4 : 0;
-    uint64_t ntail = n - 4 * n4;
-    range_kernel<<<grid_for(n4 ? n4 : ntail, 256, 148 * 8), 256, 0, st>>>((const float4 *)x, n4, x + 4 * n4, ntail, out,
-                                                                           nonfinite);
+    range_kernel<<<range_grid(n, 148 * 8), 256, 0, st>>>(x, n, out, nonfinite);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_range_batch(RangeField *F, uint32_t nf, uint64_t most, cudaStream_t st) {
+    range_batch_kernel<<<dim3(range_grid(most, std::max(148 * 8 / nf, 1u)), nf), 256, 0, st>>>(F);
     count_launch();
     return cudaGetLastError();
 }

@@ -19,25 +19,25 @@
 namespace asz {
 
 // ---------------------------------------------------------------------------------------------
-// Histogram of symbols in [offset, offset+range). Counts are 64-bit.
+// Histogram of symbols in [offset, offset+range). Counts are 64-bit; of a range up to kHistShared a CTA
+// counts in shared memory first. A thread takes runs of kHistRun consecutive symbols, from run r0 on in
+// steps of dr, and adds equal neighbours together: most symbols of a stream are a few values, often
+// repeated, so this saves most atomics.
+constexpr uint32_t kHistRun = 8, kHistShared = 8192;
 template <class T>
-__global__ void histogram_kernel(const T *__restrict__ s, uint64_t n, int64_t offset, uint64_t range,
-                                 unsigned long long *__restrict__ hist) {
+__device__ __forceinline__ void histogram_of(const T *__restrict__ s, uint64_t n, int64_t offset, uint64_t range,
+                                             unsigned long long *__restrict__ hist, uint64_t r0, uint64_t r1, uint64_t dr) {
     extern __shared__ unsigned int sh[];
-    const bool use_sh = range <= 8192;
+    const bool use_sh = range <= kHistShared;
     if (use_sh) {
         for (uint64_t i = threadIdx.x; i < range; i += blockDim.x) sh[i] = 0;
         __syncthreads();
     }
-    // A thread takes runs of kHistRun consecutive symbols and adds equal neighbours together:
-    // most symbols of a stream are a few values, often repeated, so this saves most atomics.
-    constexpr uint32_t kHistRun = 8;
     auto add = [&](uint64_t v, uint32_t c) {
         if (use_sh) atomicAdd(&sh[v], c);
         else atomicAdd(&hist[v], (unsigned long long)c);
     };
-    const uint64_t nruns = (n + kHistRun - 1) / kHistRun;
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < nruns; r += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t r = r0; r < r1; r += dr) {
         const uint64_t i0 = r * kHistRun, i1 = min(i0 + kHistRun, n);
         uint64_t cur = (uint64_t)((int64_t)s[i0] - offset);
         uint32_t c = 1;
@@ -58,6 +58,29 @@ __global__ void histogram_kernel(const T *__restrict__ s, uint64_t n, int64_t of
         for (uint64_t i = threadIdx.x; i < range; i += blockDim.x)
             if (sh[i]) atomicAdd(&hist[i], (unsigned long long)sh[i]);
     }
+}
+
+template <class T>
+__global__ void histogram_kernel(const T *__restrict__ s, uint64_t n, int64_t offset, uint64_t range,
+                                 unsigned long long *__restrict__ hist) {
+    histogram_of(s, n, offset, range, hist, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, (n + kHistRun - 1) / kHistRun,
+                 (uint64_t)gridDim.x * blockDim.x);
+}
+
+// The streams of a set, a CTA per tile of a stream. A launch per stream was bound by the launches and
+// by CTAs too few to fill the chip: the 80 streams of eight fields (33M values) 0.56 -> 0.10 ms.
+__global__ void histogram_set_kernel(const __grid_constant__ HistSet set) {
+    uint32_t lo = 0, hi = set.n;  // the last stream that starts at or before this tile
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (set.s[mid].tile <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const HistStream &h = set.s[lo];
+    const uint64_t runs = (h.n + kHistRun - 1) / kHistRun, r = (uint64_t)(blockIdx.x - h.tile) * set.tile_runs;
+    const uint64_t r0 = r + threadIdx.x, r1 = min(r + set.tile_runs, runs);
+    if (h.wide) histogram_of((const int64_t *)h.sym, h.n, h.lo, h.range, h.hist, r0, r1, blockDim.x);
+    else histogram_of((const int32_t *)h.sym, h.n, h.lo, h.range, h.hist, r0, r1, blockDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -595,6 +618,34 @@ __global__ void fill_kernel(T *__restrict__ out, uint64_t n, T v) {
 
 // ---------------------------------------------------------------------------------------------
 // Host-callable launchers (declared in launch.h).
+
+cudaError_t launch_histogram_set(const HistStream *streams, uint32_t n, cudaStream_t st) {
+    // Tiles of up to 16384 symbols, smaller where the chip would not be full of them.
+    uint64_t runs = 0;
+    for (uint32_t i = 0; i < n; i++) runs += (streams[i].n + kHistRun - 1) / kHistRun;
+    const uint64_t tile = std::min<uint64_t>(std::max<uint64_t>((runs / (148 * 8) + 255) / 256 * 256, 256), 2048);
+    for (uint32_t at = 0; at < n;) {
+        HistSet set{};
+        set.tile_runs = (uint32_t)tile;
+        uint64_t tiles = 0, range = 0;
+        for (; at < n && set.n < HistSet::kMost; at++) {
+            const uint64_t t = ((streams[at].n + kHistRun - 1) / kHistRun + tile - 1) / tile;
+            if (t == 0) continue;
+            if (tiles + t > INT32_MAX) break;
+            HistStream &h = set.s[set.n++] = streams[at];
+            h.tile = (uint32_t)tiles;
+            tiles += t;
+            if (h.range <= kHistShared) range = std::max(range, h.range);
+        }
+        if (set.n == 0) {
+            if (at < n) return cudaErrorInvalidValue;
+            break;
+        }
+        histogram_set_kernel<<<(unsigned)tiles, 256, range * sizeof(unsigned int), st>>>(set);
+        count_launch();
+    }
+    return cudaGetLastError();
+}
 
 template <class T>
 cudaError_t launch_histogram(const T *s, uint64_t n, int64_t offset, uint64_t range, unsigned long long *hist,

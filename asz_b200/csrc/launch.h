@@ -51,6 +51,8 @@ struct PlanCand {
 };
 
 cudaError_t launch_range(const float *x, uint64_t n, int32_t *out, unsigned long long *nonfinite, cudaStream_t st);
+// The ranges of a batch's fields, of at most `most` values each, in place.
+cudaError_t launch_range_batch(RangeField *F, uint32_t nf, uint64_t most, cudaStream_t st);
 cudaError_t launch_zero_first_last(const float *x, uint64_t n, unsigned long long *first, unsigned long long *last,
                                    cudaStream_t st);
 // Batches (host/batch.cpp): one launch per round for every field of a batch. The fast selection and
@@ -187,6 +189,10 @@ cudaError_t launch_plan_mse(const PlanCand *cands, uint32_t ncands, const float 
 cudaError_t launch_slope_exact(const SampleBox *boxes, const ProxyEval *evals, uint32_t n_evals, const float *orig,
                                uint64_t n1n2, uint64_t n2, const float *log2arena, float R2, float *h1, float *x,
                                uint32_t *m_out, uint32_t *err, uint32_t cap, uint32_t most, uint32_t nboxes, cudaStream_t st);
+// The default slopes of a batch's fields, n_evals evaluations each (out zero before); cap and most as
+// launch_slope_exact, over all fields.
+cudaError_t launch_slope_batch(const SlopeField *fields, uint32_t nf, uint32_t n_evals, const float *log2arena, SlopeOut *out,
+                               uint32_t cap, uint32_t most, cudaStream_t st);
 cudaError_t launch_slope_v0(const FieldGeom &fg, const SampleBox *boxes, const ProxyEval *evals, uint32_t n_evals,
                             const float *orig, const float *log2arena, float R2, uint8_t *scratch, uint64_t scratch_stride,
                             uint32_t cap, uint32_t bcap, uint32_t tcap, float *h1, float *x, uint32_t *m_out, uint32_t *err,
@@ -195,6 +201,21 @@ cudaError_t launch_slope_v0(const FieldGeom &fg, const SampleBox *boxes, const P
 template <class T>
 cudaError_t launch_histogram(const T *s, uint64_t n, int64_t offset, uint64_t range, unsigned long long *hist,
                              cudaStream_t st);
+// The histograms of several streams (zero before) in one launch for every HistSet::kMost of them.
+struct HistStream {
+    const void *sym;
+    uint64_t n;
+    int64_t lo;  // the symbol of hist[0]
+    uint64_t range;
+    unsigned long long *hist;
+    uint32_t wide, tile;  // int64 symbols (else int32); the launcher's: the stream's first tile
+};
+struct HistSet {
+    static constexpr uint32_t kMost = 80;  // 3.8 KB of the launch's parameters
+    HistStream s[kMost];
+    uint32_t n, tile_runs;
+};
+cudaError_t launch_histogram_set(const HistStream *streams, uint32_t n, cudaStream_t st);
 // Tiled encoding of several streams of one symbol type in one launch (k_huff.cu). toff: exclusive
 // prefix of the streams' tile counts (ns + 1 entries, tiles of enc_tile<T>() symbols);
 // tile_state needs ntiles + 1 entries and err one, both zero before the launch, as each stream's out.

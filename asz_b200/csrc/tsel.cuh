@@ -34,6 +34,19 @@ struct ProxyEval {
     float t, abs_eb;
 };
 
+// A field of a batch for the default slope: the three boxes' proxies of all its fields are one launch.
+struct SlopeField {
+    const float *orig;
+    uint64_t n1n2, n2;
+    float R2;
+    SampleBox boxes[3];
+    ProxyEval evals[64];
+};
+struct SlopeOut {
+    float h1[3 * 64], x[3 * 64];  // by box and evaluation
+    uint32_t m[3], err;
+};
+
 // Per-round table of the up to 27 block classes (first/middle/last along each axis).
 struct ClassInfo {
     uint32_t ss;         // sampling_stride (needs glibc cbrt, so computed on the host)
