@@ -3285,14 +3285,45 @@ struct DecodeRun {
     uint32_t nst = 0, max_lut_bits = 1;
     u64 ntiles = 0, nchunks = 0;
 };
-constexpr u64 kChunkBits = 1024;
+
+// The bits until a wrong start falls in step with the codewords are geometrically distributed, their
+// mean about 1.8 b^2 at b bits a symbol (simulated for normal and Laplace symbols, 4 to 11 bits).
+double step_bits(u64 bits, u64 values) {
+    const double b = (double)bits / (double)values;
+    return 1.8 * b * b;
+}
+
+// Words of a stream's chunks: 32, or 8. A chunk is a thread's serial work, so where chunks of 1024 bits do
+// not fill the chip, shorter ones take a third of the time (40x48x64 at 1e-3, 130 KB: 58 + 42 -> 33 +
+// 18 us of synchronising and writing; at 1e-2, 46 KB: 76 + 52 -> 31 + 20; 256^3 at 1e-2, 4.4 MB: 99 + 86
+// -> 75 + 68). They cost more halo (a quarter of the lanes instead of a sixteenth) and more turns where a
+// wrong start runs through most of a chunk (256^3 at 1e-3, 16 MB: 90 + 90 -> 143 + 64; 400^3 at 1e-2, 15 MB:
+// 174 + 294 -> 250 + 234; 20^3 at 1e-5, 12 bits and more a symbol: 61 + 17 -> 100 + 21), so only where the
+// payloads, and the payloads times their step, are small, and
+// a stream's step within a chunk. Codes of about one length (of one, where they are short) hardly ever
+// fall in step: there each run of chunks costs a pass, so the runs stay long.
+void decode_words(std::vector<DecStream> &ds, const std::vector<const HuffParsed *> &codes) {
+    double bits = 0, steps = 0;
+    for (const DecStream &d : ds) {
+        bits += (double)(d.bit_end - d.bit_begin);
+        steps += (double)(d.bit_end - d.bit_begin) * step_bits(d.bit_end - d.bit_begin, d.count);
+    }
+    const bool few = bits <= 48e6 && steps <= 2.5e9;
+    for (size_t i = 0; i < ds.size(); i++) {
+        DecStream &d = ds[i];
+        const bool one_run = d.bit_end - d.bit_begin <= 8 * 32 * decode_run(8);  // no guesses
+        const double step = step_bits(d.bit_end - d.bit_begin, d.count);
+        const bool falls_in = step <= 250 && codes[i]->max_len >= codes[i]->min_len + (step <= 30 ? 1 : 3);
+        d.words = few && (one_run || falls_in) ? 8 : 32;
+    }
+}
 
 // Tables and descriptors to the device, and the first synchronisation pass. The stream bytes are on
 // the device at d_base (256-byte aligned, padded by kDecodePad).
 int decode_begin(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8_t *d_base, MiscLayout *dm, cudaStream_t st,
                  DecodeRun &r) {
-    const u64 C = kChunkBits;
     std::vector<DecStream> ds;
+    std::vector<const HuffParsed *> codes;
     std::vector<uint32_t> tile_stream;
     std::vector<uint32_t> luts, lut2s, childs;
     u64 nchunks = 0;
@@ -3308,9 +3339,6 @@ int decode_begin(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8_t
         DecStream d{};
         d.bit_begin = hp.payload_off * 8;
         d.bit_end = d.bit_begin + hp.payload_bits;
-        d.chunk0 = nchunks;
-        d.nchunks = std::max<u64>(1, (hp.payload_bits + C - 1) / C);
-        d.tile0 = tile_stream.size();
         d.lut_off = luts.size();
         d.lut2_off = lut2s.size();
         d.child_off = childs.size();
@@ -3323,11 +3351,19 @@ int decode_begin(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8_t
         luts.resize((luts.size() + 3) & ~size_t(3));
         lut2s.insert(lut2s.end(), hp.lut2.begin(), hp.lut2.end());
         childs.insert(childs.end(), hp.child.begin(), hp.child.end());
-        const u64 tiles = (d.nchunks + kDecodeTile - 1) / kDecodeTile;
-        tile_stream.insert(tile_stream.end(), tiles, (uint32_t)ds.size());
-        nchunks += d.nchunks;
         r.max_lut_bits = std::max(r.max_lut_bits, hp.lut_bits);
         ds.push_back(d);
+        codes.push_back(&hp);
+    }
+    decode_words(ds, codes);
+    for (size_t i = 0; i < ds.size(); i++) {
+        DecStream &d = ds[i];
+        const u64 C = 32 * d.words;
+        d.chunk0 = nchunks;
+        d.nchunks = std::max<u64>(1, (d.bit_end - d.bit_begin + C - 1) / C);
+        d.tile0 = tile_stream.size();
+        tile_stream.insert(tile_stream.end(), (d.nchunks + decode_tile(d.words) - 1) / decode_tile(d.words), (uint32_t)i);
+        nchunks += d.nchunks;
     }
     CK(cudaMemsetAsync(&dm->dec_err, 0, 8, st));  // and dec_changed
     if (ds.empty()) return ASZ_OK;
@@ -3365,20 +3401,16 @@ int decode_begin(asz_ctx *ctx, const std::vector<DecodeJob> &jobs, const uint8_t
     r.nchunks = nchunks;
     CK(cudaMemsetAsync(r.cnt + nchunks, 0, 8, st));
     ProfScope ps(ctx, "huff_decode_sync", 0);
-    CK(launch_decode_sync(r.base, C, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 1, r.start, r.end, r.cnt, r.moved,
+    CK(launch_decode_sync(r.base, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 1, r.start, r.end, r.cnt, r.moved,
                           &dm->dec_err, st));
     // A second pass where a run's guess is likely to miss somewhere (it costs about 10 us; finding out
-    // at the end costs the whole decoding and reconstruction again). The bits until a wrong start
-    // falls in step are geometrically distributed, their mean about 1.8 b^2 at b bits a symbol
-    // (simulated for normal and Laplace symbols, 4 to 11 bits).
+    // at the end costs the whole decoding and reconstruction again).
     double misses = 0;
-    for (const DecStream &d : ds) {
-        const double b = (double)(d.bit_end - d.bit_begin) / (double)d.count;
-        misses += (double)(d.nchunks / kDecodeRun) * std::exp(-(double)(kDecodeHalo * C) / (1.8 * b * b));
-    }
+    for (const DecStream &d : ds)
+        misses += (double)(d.nchunks / decode_run(d.words)) * std::exp(-(double)(32 * kDecodeHaloWords) / step_bits(d.bit_end - d.bit_begin, d.count));
     if (misses > 0.01) {
         CK(launch_decode_restart(r.ds, r.nst, nchunks, r.end, r.start, r.moved, &dm->dec_changed, st));
-        CK(launch_decode_sync(r.base, C, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 0, r.start, r.end, r.cnt,
+        CK(launch_decode_sync(r.base, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 0, r.start, r.end, r.cnt,
                               r.moved, &dm->dec_err, st));
         CK(cudaMemsetAsync(&dm->dec_changed, 0, 4, st));
     }
@@ -3397,7 +3429,7 @@ int decode_values(asz_ctx *ctx, const DecodeRun &r, MiscLayout *dm, cudaStream_t
     CK(launch_scan_u64(r.cnt, r.off, r.nchunks + 1, ctx->cubtmp.p, tb, st));
     CK(launch_decode_check(r.ds, r.nst, r.ts, r.ntiles, r.off, r.start, r.end, &dm->dec_err, &dm->dec_changed, st));
     ProfScope ps_w(ctx, "huff_decode_write", 0);
-    CK(launch_decode_write(r.base, kChunkBits, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, r.start, r.off, &dm->dec_err,
+    CK(launch_decode_write(r.base, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, r.start, r.off, &dm->dec_err,
                            st));
     return ASZ_OK;
 }
@@ -3412,9 +3444,9 @@ int decode_settle(asz_ctx *ctx, const DecodeRun &r, MiscLayout *dm, cudaStream_t
         CK(cudaStreamSynchronize(st));
         if (!changed) return ASZ_OK;
         // Every pass that moves a start fixes at least one more run, so this ends.
-        if (it > r.ntiles * (kDecodeTile / kDecodeRun) + 2) return fail(ctx, ASZ_E_DATA, "Huffman payload does not synchronise");
+        if (it > r.ntiles * (kDecodeThreads / 32) + 2) return fail(ctx, ASZ_E_DATA, "Huffman payload does not synchronise");
         ProfScope ps(ctx, "huff_decode_sync", 0);
-        CK(launch_decode_sync(r.base, kChunkBits, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 0, r.start, r.end, r.cnt,
+        CK(launch_decode_sync(r.base, r.ds, r.ts, r.ntiles, r.max_lut_bits, r.lut, r.lut2, r.child, 0, r.start, r.end, r.cnt,
                               r.moved, &dm->dec_err, st));
     }
 }

@@ -301,7 +301,7 @@ bool parse_stream(const uint8_t *buf, uint64_t len, uint64_t &pos, HuffParsed &o
         std::vector<LongLeaf> longer;
         std::vector<uint32_t> open{0};
         uint64_t turn = 0, leaves = 0, nodes = 1;
-        uint32_t max_len = 0;
+        uint32_t min_len = 64, max_len = 0;
         bool in_range = true, fits = true;
         while (!open.empty()) {
             unsigned inner;
@@ -331,6 +331,7 @@ bool parse_stream(const uint8_t *buf, uint64_t len, uint64_t &pos, HuffParsed &o
             }
             o.child[2 * (size_t)open.back() + ((turn >> d) & 1)] = 0x80000000u | (uint32_t)sym;
             leaves++;
+            min_len = std::min(min_len, l);
             max_len = std::max(max_len, l);
             in_range = in_range && (sym < std::max<uint64_t>(o.maxval, 1) || o.maxval >= (1ull << 31));
             fits = fits && sym < (1ull << kLutValueBits);
@@ -360,6 +361,8 @@ bool parse_stream(const uint8_t *buf, uint64_t len, uint64_t &pos, HuffParsed &o
             err = "Huffman symbol outside its range";
             return false;
         }
+        o.min_len = min_len;
+        o.max_len = max_len;
         o.lut_bits = std::min(max_len, kLutBits);
         o.lut.resize(1ull << o.lut_bits);  // a shorter table's entries are the first ones
         uint32_t sub = kLut2Bits;

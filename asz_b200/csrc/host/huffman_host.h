@@ -56,6 +56,7 @@ struct HuffParsed {
     std::vector<uint32_t> lut, lut2;
     std::vector<uint32_t> child;   // 2 per node: a node, or a symbol with the top bit set
     uint32_t lut_bits = 0;
+    uint32_t min_len = 0, max_len = 0;  // of a code, in bits
 };
 
 // Parse the tree at buf[pos] and the length word that follows; advances pos past the payload.

@@ -288,11 +288,11 @@ struct DecodeTables {
     uint32_t lut_bits;
 };
 
-// A chunk's words: 32 of its own after a lead of up to 31 bits, and two more that its last codeword
+// A chunk's words: W of its own after a lead of up to 31 bits, and two more that its last codeword
 // may reach. The odd stride keeps a warp's reads, at about the same place of its chunks, on
 // different banks.
-constexpr uint32_t kSlotWords = 35;
-constexpr uint32_t kDecodeSlotBytes = ((kDecodeTile + kDecodeHalo) * kSlotWords * 4 + 15) / 16 * 16;
+ASZ_HD constexpr uint32_t slot_words(uint32_t W) { return W + 3; }
+constexpr uint32_t kDecodeSlotBytes = ((decode_tile(32) + decode_halo(32)) * slot_words(32) * 4 + 15) / 16 * 16;  // the most
 
 // The 32 payload bits from bit `pos` of a slot on.
 __device__ __forceinline__ uint32_t peek(const uint32_t *slot, uint32_t pos) {
@@ -348,12 +348,12 @@ __device__ __forceinline__ void stage_lut(uint4 *lut_sh, const uint32_t *__restr
 
 // The words of kSlots chunks from chunk `first` of the stream on (negative: none there) into their
 // slots. Words outside the payload read as zero.
-template <uint32_t kSlots>
+template <uint32_t W, uint32_t kSlots>
 __device__ __forceinline__ void stage_payload(uint32_t *slots, const uint8_t *__restrict__ base, const DecStream &d, int64_t first) {
     const uint32_t *words = reinterpret_cast<const uint32_t *>(base);
     const int64_t lo = (int64_t)(d.bit_begin >> 5), hi = (int64_t)(d.bit_end >> 5) + 1;  // kDecodePad lies behind
-    const int64_t w0 = lo + first * 32;
-    constexpr uint32_t kWords = kSlots * 32 + 2, kUnroll = 8;
+    const int64_t w0 = lo + first * W;
+    constexpr uint32_t kWords = kSlots * W + 2, kUnroll = 8;
     for (uint32_t i0 = threadIdx.x; i0 < kWords; i0 += kUnroll * kDecodeThreads) {
         uint32_t v[kUnroll];
 #pragma unroll
@@ -363,21 +363,23 @@ __device__ __forceinline__ void stage_payload(uint32_t *slots, const uint8_t *__
         }
 #pragma unroll
         for (uint32_t u = 0; u < kUnroll; u++) {
-            const uint32_t i = i0 + u * kDecodeThreads, slot = i >> 5, j = i & 31;
-            if (slot < kSlots) slots[slot * kSlotWords + j] = v[u];
-            if (j < 2 && slot && slot <= kSlots) slots[(slot - 1) * kSlotWords + 32 + j] = v[u];
+            const uint32_t i = i0 + u * kDecodeThreads, slot = i / W, j = i % W;
+            if (slot < kSlots) slots[slot * slot_words(W) + j] = v[u];
+            if (j < 2 && slot && slot <= kSlots) slots[(slot - 1) * slot_words(W) + W + j] = v[u];
         }
     }
 }
 
 // One chunk's decoding, in bits from its slot's start: where it stopped and how many values it met.
-// marks[j * kDecodeThreads] keeps the first codeword's start from 128 (j + 1) bits after `lead` on, with
+// marks[j * kDecodeThreads] keeps a codeword's start about j + 1 eighths of the chunk after `lead`, with
 // the values before it in the upper half. A chunk that has to start elsewhere is read until it meets
 // one of them (codewords fall in step after a geometrically distributed number of bits, about 30 at 4
 // bits a symbol and 130 at 10; from there on it is decoded already).
-constexpr uint32_t kMarkBits = 128, kMarks = 7;
+constexpr uint32_t kMarks = 7;
 
+template <uint32_t W>
 struct ChunkRun {
+    static constexpr uint32_t kMarkBits = 4 * W;
     uint32_t end = 0, count = 0;
 
     __device__ __forceinline__ void decode(const uint32_t *slot, uint32_t lead, uint32_t pos, uint32_t lim, const DecodeTables &T,
@@ -411,13 +413,70 @@ struct ChunkRun {
 // recording where it stopped (end[k]) and how many values it produced (count[k]). First pass: every
 // chunk starts at its first bit, and then, within its warp, where its predecessor ended, until no
 // start moves. A warp's first chunk has its predecessor in another warp, so a warp's first
-// kDecodeHalo lanes decode the chunks before its own as well: a wrong guess nearly always meets the
-// true codewords within those 2048 bits (a 161x257x349 quintic stream at 1e-4 needed five passes
+// lanes decode the chunks before its own as well: a wrong guess nearly always meets the
+// true codewords within those bits (a 161x257x349 quintic stream at 1e-4 needed five passes
 // over all chunks, with the host waiting for each; now it is this one). What it nearly always is,
 // decode_check_kernel checks; a warp whose first chunk did start elsewhere is settled by the later
 // passes, which start at start[] and decode only from a moved first chunk on (moved[k] != 0).
+template <uint32_t W>
+__device__ __forceinline__ bool sync_tile(const uint8_t *__restrict__ base, const DecStream &d, uint64_t tile, bool fresh,
+                                          const uint32_t *__restrict__ luts, const uint32_t *__restrict__ lut2s,
+                                          const uint32_t *__restrict__ childs, int first_pass, uint64_t *__restrict__ start,
+                                          uint64_t *__restrict__ end, uint64_t *__restrict__ count,
+                                          const uint32_t *__restrict__ moved, uint32_t *slots, uint4 *lut_sh, uint32_t *marks,
+                                          uint32_t *err_word) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t kl0 = (int64_t)((tile - d.tile0) * decode_tile(W)) - (int)decode_halo(W);
+    if (!first_pass) {
+        const uint64_t mine = (uint64_t)(tile - d.tile0) * decode_tile(W) + threadIdx.x;
+        if (!__syncthreads_or(threadIdx.x < decode_tile(W) && mine < d.nchunks && moved[d.chunk0 + mine])) return false;
+    }
+    __syncthreads();  // the tile before is done with the shared memory
+    if (fresh) stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
+    stage_payload<W, decode_tile(W) + decode_halo(W)>(slots, base, d, kl0);
+    for (uint32_t j = 0; j < kMarks; j++) marks[j * kDecodeThreads] = 0;
+    __syncthreads();
+    const DecodeTables T{reinterpret_cast<const uint32_t *>(lut_sh), lut2s + d.lut2_off, childs + d.child_off, d.lut_bits};
+    const int at_slot = warp * (int)decode_run(W) + lane;
+    const int64_t kl = kl0 + at_slot;
+    const uint32_t *slot = slots + at_slot * slot_words(W);
+    const bool own = lane >= (int)decode_halo(W) && kl < (int64_t)d.nchunks;
+    const bool in = first_pass ? kl >= 0 && kl < (int64_t)d.nchunks : own;
+    const bool after = in && lane > (first_pass ? 0 : (int)decode_halo(W)) && kl > 0;  // has a predecessor here
+    const uint64_t k = d.chunk0 + (uint64_t)kl;
+    // Positions relative to the chunk's slot.
+    const uint32_t lead = (uint32_t)(d.bit_begin & 31), span = 32 * W;
+    const uint64_t first = d.bit_begin + (uint64_t)kl * span, origin = first - lead;
+    const uint32_t lim = in ? lead + (uint32_t)min((uint64_t)span, d.bit_end - first) : 0;
+    uint32_t s = lead;
+    ChunkRun<W> run;
+    bool need = in;
+    if (in && !first_pass) {
+        s = (uint32_t)(start[k] - origin);
+        run.end = (uint32_t)(end[k] - origin);
+        run.count = (uint32_t)count[k];
+        need = moved[k] != 0;
+    }
+    // Each turn makes at least one more chunk of the warp final.
+    for (uint32_t turn = 0; turn <= 32; turn++) {
+        if (need) run.decode(slot, lead, s, lim, T, marks, err_word);
+        __syncwarp();
+        const uint32_t before = __shfl_up_sync(0xffffffffu, run.end, 1);
+        const uint32_t at = after ? before - span : s;
+        need = at != s;
+        s = at;
+        if (!__any_sync(0xffffffffu, need)) break;
+    }
+    if (own) {
+        start[k] = origin + s;
+        end[k] = origin + run.end;
+        count[k] = run.count;
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(kDecodeThreads, 4)
-    decode_sync_kernel(const uint8_t *__restrict__ base, uint64_t chunk_bits, const DecStream *__restrict__ streams,
+    decode_sync_kernel(const uint8_t *__restrict__ base, const DecStream *__restrict__ streams,
                        const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const uint32_t *__restrict__ luts,
                        const uint32_t *__restrict__ lut2s, const uint32_t *__restrict__ childs, int first_pass,
                        uint64_t *__restrict__ start, uint64_t *__restrict__ end, uint64_t *__restrict__ count,
@@ -426,59 +485,16 @@ __global__ void __launch_bounds__(kDecodeThreads, 4)
     __shared__ uint32_t marks_sh[kMarks * kDecodeThreads];
     uint32_t *const slots = reinterpret_cast<uint32_t *>(dec_smem);
     uint4 *const lut_sh = dec_smem + kDecodeSlotBytes / 16;
-    uint32_t staged = 0xffffffffu;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *const marks = marks_sh + threadIdx.x;
+    uint32_t staged = 0xffffffffu;
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint32_t si = tile_stream[tile];
         const DecStream &d = streams[si];
-        const int64_t kl0 = (int64_t)((tile - d.tile0) * kDecodeTile) - (int)kDecodeHalo;
-        if (!first_pass) {
-            const uint64_t mine = (uint64_t)(tile - d.tile0) * kDecodeTile + threadIdx.x;
-            if (!__syncthreads_or(threadIdx.x < kDecodeTile && mine < d.nchunks && moved[d.chunk0 + mine])) continue;
-        }
-        __syncthreads();  // the tile before is done with the shared memory
-        if (si != staged) stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
-        stage_payload<kDecodeTile + kDecodeHalo>(slots, base, d, kl0);
-        for (uint32_t j = 0; j < kMarks; j++) marks[j * kDecodeThreads] = 0;
-        __syncthreads();
-        staged = si;
-        const DecodeTables T{reinterpret_cast<const uint32_t *>(lut_sh), lut2s + d.lut2_off, childs + d.child_off, d.lut_bits};
-        const int at_slot = warp * (int)kDecodeRun + lane;
-        const int64_t kl = kl0 + at_slot;
-        const uint32_t *slot = slots + at_slot * kSlotWords;
-        const bool own = lane >= (int)kDecodeHalo && kl < (int64_t)d.nchunks;
-        const bool in = first_pass ? kl >= 0 && kl < (int64_t)d.nchunks : own;
-        const bool after = in && lane > (first_pass ? 0 : (int)kDecodeHalo) && kl > 0;  // has a predecessor here
-        const uint64_t k = d.chunk0 + (uint64_t)kl;
-        // Positions relative to the chunk's slot.
-        const uint32_t lead = (uint32_t)(d.bit_begin & 31), span = (uint32_t)chunk_bits;
-        const uint64_t first = d.bit_begin + (uint64_t)kl * chunk_bits, origin = first - lead;
-        const uint32_t lim = in ? lead + (uint32_t)min((uint64_t)span, d.bit_end - first) : 0;
-        uint32_t s = lead;
-        ChunkRun run;
-        bool need = in;
-        if (in && !first_pass) {
-            s = (uint32_t)(start[k] - origin);
-            run.end = (uint32_t)(end[k] - origin);
-            run.count = (uint32_t)count[k];
-            need = moved[k] != 0;
-        }
-        // Each turn makes at least one more chunk of the warp final.
-        for (uint32_t turn = 0; turn <= 32; turn++) {
-            if (need) run.decode(slot, lead, s, lim, T, marks, err_word);
-            __syncwarp();
-            const uint32_t before = __shfl_up_sync(0xffffffffu, run.end, 1);
-            const uint32_t at = after ? before - span : s;
-            need = at != s;
-            s = at;
-            if (!__any_sync(0xffffffffu, need)) break;
-        }
-        if (own) {
-            start[k] = origin + s;
-            end[k] = origin + run.end;
-            count[k] = run.count;
-        }
+        const bool done = d.words == 8 ? sync_tile<8>(base, d, tile, si != staged, luts, lut2s, childs, first_pass, start, end, count,
+                                                      moved, slots, lut_sh, marks, err_word)
+                                       : sync_tile<32>(base, d, tile, si != staged, luts, lut2s, childs, first_pass, start, end, count,
+                                                       moved, slots, lut_sh, marks, err_word);
+        if (done) staged = si;  // its table is in shared memory
     }
 }
 
@@ -520,11 +536,11 @@ __global__ void decode_check_kernel(const DecStream *__restrict__ streams, uint3
                                     const uint64_t *__restrict__ start, const uint64_t *__restrict__ end, uint32_t *err_word,
                                     uint32_t *changed) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    constexpr uint32_t kRuns = kDecodeTile / kDecodeRun;
+    constexpr uint32_t kRuns = kDecodeThreads / 32;
     if (i < ntiles * kRuns) {
         const uint64_t tile = i / kRuns;
         const DecStream &d = streams[tile_stream[tile]];
-        const uint64_t kl = (tile - d.tile0) * kDecodeTile + i % kRuns * kDecodeRun, k = d.chunk0 + kl;
+        const uint64_t kl = (tile - d.tile0) * decode_tile(d.words) + i % kRuns * decode_run(d.words), k = d.chunk0 + kl;
         if (kl && kl < d.nchunks && start[k] != end[k - 1]) *changed = 1u;
     }
     if (i >= nstreams) return;
@@ -537,8 +553,73 @@ __global__ void decode_check_kernel(const DecStream *__restrict__ streams, uint3
 
 // Pass B over all tiles: write the values (symbol index + offset) of chunk k at its offset in its
 // stream's output (int64 for the t stream, int32 for QB streams).
+template <uint32_t W>
+__device__ __forceinline__ void write_tile(const uint8_t *__restrict__ base, const DecStream &d, uint64_t tile, bool fresh,
+                                           const uint32_t *__restrict__ luts, const uint32_t *__restrict__ lut2s,
+                                           const uint32_t *__restrict__ childs, const uint64_t *__restrict__ start,
+                                           const uint64_t *__restrict__ off, uint32_t *slots, uint4 *lut_sh, uint32_t *err_word) {
+    const uint64_t kl0 = (tile - d.tile0) * decode_tile(W), kl = kl0 + threadIdx.x;
+    __syncthreads();
+    if (fresh) stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
+    stage_payload<W, decode_tile(W)>(slots, base, d, (int64_t)kl0);
+    __syncthreads();
+    if (threadIdx.x >= decode_tile(W) || kl >= d.nchunks) return;
+    const DecodeTables T{reinterpret_cast<const uint32_t *>(lut_sh), lut2s + d.lut2_off, childs + d.child_off, d.lut_bits};
+    const uint32_t *slot = slots + threadIdx.x * slot_words(W);
+    const uint64_t k = d.chunk0 + kl;
+    const uint32_t lead = (uint32_t)(d.bit_begin & 31);
+    const uint64_t first = d.bit_begin + kl * (32 * W);
+    uint32_t pos = (uint32_t)(start[k] - (first - lead));
+    const uint32_t lim = lead + (uint32_t)min((uint64_t)(32 * W), d.bit_end - first);
+    if (pos >= lim) return;
+    const uint64_t o0 = off[k] - off[d.chunk0], count = d.count;
+    if (o0 >= count) {
+        atomicOr(err_word, 16u);
+        return;
+    }
+    const uint32_t room = (uint32_t)min(count - o0, (uint64_t)0xffffffffu);  // values left of the stream
+    uint32_t o = 0;
+    if (d.wide) {
+        int64_t *out = static_cast<int64_t *>(d.out) + o0;
+        const int64_t offset = d.offset;
+        while (pos < lim && o < room) out[o++] = (int64_t)decode_sym(slot, pos, T) + offset;
+    } else {
+        // int32 values go out four at a time as one 16-byte store once the position is aligned:
+        // whole sectors leave the thread instead of one value per store.
+        int32_t *out = static_cast<int32_t *>(d.out) + o0;
+        const uint32_t offset = (uint32_t)(int32_t)d.offset;
+        const uint32_t head = min(room, (uint32_t)(-(intptr_t)((uintptr_t)out >> 2) & 3));  // up to the alignment
+        while (pos < lim && o < head) out[o++] = (int32_t)(decode_sym(slot, pos, T) + offset);
+        while (pos < lim && o + 4 <= room) {
+            int4 v;
+            v.x = (int32_t)(decode_sym(slot, pos, T) + offset);
+            if (pos >= lim) {
+                out[o++] = v.x;
+                break;
+            }
+            v.y = (int32_t)(decode_sym(slot, pos, T) + offset);
+            if (pos >= lim) {
+                out[o] = v.x, out[o + 1] = v.y;
+                o += 2;
+                break;
+            }
+            v.z = (int32_t)(decode_sym(slot, pos, T) + offset);
+            if (pos >= lim) {
+                out[o] = v.x, out[o + 1] = v.y, out[o + 2] = v.z;
+                o += 3;
+                break;
+            }
+            v.w = (int32_t)(decode_sym(slot, pos, T) + offset);
+            *reinterpret_cast<int4 *>(out + o) = v;
+            o += 4;
+        }
+        while (pos < lim && o < room) out[o++] = (int32_t)(decode_sym(slot, pos, T) + offset);
+    }
+    if (pos < lim || pos >= kBadPath) atomicOr(err_word, 16u);
+}
+
 __global__ void __launch_bounds__(kDecodeThreads, 4)
-    decode_write_kernel(const uint8_t *__restrict__ base, uint64_t chunk_bits, const DecStream *__restrict__ streams,
+    decode_write_kernel(const uint8_t *__restrict__ base, const DecStream *__restrict__ streams,
                         const uint32_t *__restrict__ tile_stream, uint64_t ntiles, const uint32_t *__restrict__ luts,
                         const uint32_t *__restrict__ lut2s, const uint32_t *__restrict__ childs,
                         const uint64_t *__restrict__ start, const uint64_t *__restrict__ off, uint32_t *err_word) {
@@ -549,65 +630,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 4)
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint32_t si = tile_stream[tile];
         const DecStream &d = streams[si];
-        const uint64_t kl0 = (tile - d.tile0) * kDecodeTile, kl = kl0 + threadIdx.x;
-        __syncthreads();
-        if (si != staged) stage_lut(lut_sh, luts + d.lut_off, d.lut_bits);
-        stage_payload<kDecodeTile>(slots, base, d, (int64_t)kl0);
-        __syncthreads();
+        if (d.words == 8) write_tile<8>(base, d, tile, si != staged, luts, lut2s, childs, start, off, slots, lut_sh, err_word);
+        else write_tile<32>(base, d, tile, si != staged, luts, lut2s, childs, start, off, slots, lut_sh, err_word);
         staged = si;
-        if (threadIdx.x >= kDecodeTile || kl >= d.nchunks) continue;
-        const DecodeTables T{reinterpret_cast<const uint32_t *>(lut_sh), lut2s + d.lut2_off, childs + d.child_off, d.lut_bits};
-        const uint32_t *slot = slots + threadIdx.x * kSlotWords;
-        const uint64_t k = d.chunk0 + kl;
-        const uint32_t lead = (uint32_t)(d.bit_begin & 31);
-        const uint64_t first = d.bit_begin + kl * chunk_bits;
-        uint32_t pos = (uint32_t)(start[k] - (first - lead));
-        const uint32_t lim = lead + (uint32_t)min(chunk_bits, d.bit_end - first);
-        if (pos >= lim) continue;
-        const uint64_t o0 = off[k] - off[d.chunk0], count = d.count;
-        if (o0 >= count) {
-            atomicOr(err_word, 16u);
-            continue;
-        }
-        const uint32_t room = (uint32_t)min(count - o0, (uint64_t)0xffffffffu);  // values left of the stream
-        uint32_t o = 0;
-        if (d.wide) {
-            int64_t *out = static_cast<int64_t *>(d.out) + o0;
-            const int64_t offset = d.offset;
-            while (pos < lim && o < room) out[o++] = (int64_t)decode_sym(slot, pos, T) + offset;
-        } else {
-            // int32 values go out four at a time as one 16-byte store once the position is aligned:
-            // whole sectors leave the thread instead of one value per store.
-            int32_t *out = static_cast<int32_t *>(d.out) + o0;
-            const uint32_t offset = (uint32_t)(int32_t)d.offset;
-            const uint32_t head = min(room, (uint32_t)(-(intptr_t)((uintptr_t)out >> 2) & 3));  // up to the alignment
-            while (pos < lim && o < head) out[o++] = (int32_t)(decode_sym(slot, pos, T) + offset);
-            while (pos < lim && o + 4 <= room) {
-                int4 v;
-                v.x = (int32_t)(decode_sym(slot, pos, T) + offset);
-                if (pos >= lim) {
-                    out[o++] = v.x;
-                    break;
-                }
-                v.y = (int32_t)(decode_sym(slot, pos, T) + offset);
-                if (pos >= lim) {
-                    out[o] = v.x, out[o + 1] = v.y;
-                    o += 2;
-                    break;
-                }
-                v.z = (int32_t)(decode_sym(slot, pos, T) + offset);
-                if (pos >= lim) {
-                    out[o] = v.x, out[o + 1] = v.y, out[o + 2] = v.z;
-                    o += 3;
-                    break;
-                }
-                v.w = (int32_t)(decode_sym(slot, pos, T) + offset);
-                *reinterpret_cast<int4 *>(out + o) = v;
-                o += 4;
-            }
-            while (pos < lim && o < room) out[o++] = (int32_t)(decode_sym(slot, pos, T) + offset);
-        }
-        if (pos < lim || pos >= kBadPath) atomicOr(err_word, 16u);
     }
 }
 
@@ -767,7 +792,7 @@ static size_t decode_smem(uint32_t max_lut_bits) {
     return kDecodeSlotBytes + std::max<size_t>(((size_t)1 << max_lut_bits) * 4, 16);
 }
 
-cudaError_t launch_decode_sync(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
+cudaError_t launch_decode_sync(const uint8_t *base, const DecStream *streams, const uint32_t *tile_stream,
                                uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
                                const uint32_t *childs,
                                int first_pass, uint64_t *start, uint64_t *end, uint64_t *count, const uint32_t *moved,
@@ -775,7 +800,7 @@ cudaError_t launch_decode_sync(const uint8_t *base, uint64_t chunk_bits, const D
     const size_t sh = decode_smem(max_lut_bits);
     const cudaError_t e = cudaFuncSetAttribute(decode_sync_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (e != cudaSuccess) return e;
-    decode_sync_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, chunk_bits, streams, tile_stream, ntiles, luts, lut2s,
+    decode_sync_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, streams, tile_stream, ntiles, luts, lut2s,
                                                                       childs, first_pass, start, end, count, moved, err);
     count_launch();
     return cudaGetLastError();
@@ -793,21 +818,21 @@ cudaError_t launch_decode_restart(const DecStream *streams, uint32_t nstreams, u
 cudaError_t launch_decode_check(const DecStream *streams, uint32_t nstreams, const uint32_t *tile_stream, uint64_t ntiles,
                                 const uint64_t *off, const uint64_t *start, const uint64_t *end, uint32_t *err,
                                 uint32_t *changed, cudaStream_t st) {
-    const uint64_t n = std::max<uint64_t>(ntiles * (kDecodeTile / kDecodeRun), nstreams);
+    const uint64_t n = std::max<uint64_t>(ntiles * (kDecodeThreads / 32), nstreams);
     decode_check_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(streams, nstreams, tile_stream, ntiles, off, start, end, err,
                                                                       changed);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_decode_write(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
+cudaError_t launch_decode_write(const uint8_t *base, const DecStream *streams, const uint32_t *tile_stream,
                                 uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
                                const uint32_t *childs,
                                 const uint64_t *start, const uint64_t *off, uint32_t *err, cudaStream_t st) {
     const size_t sh = decode_smem(max_lut_bits);
     const cudaError_t e = cudaFuncSetAttribute(decode_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (e != cudaSuccess) return e;
-    decode_write_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, chunk_bits, streams, tile_stream, ntiles, luts, lut2s, childs,
+    decode_write_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, streams, tile_stream, ntiles, luts, lut2s, childs,
                                                                        start, off, err);
     count_launch();
     return cudaGetLastError();

@@ -31,12 +31,15 @@ struct DecStream {
     int64_t offset;                // added to each symbol index
     void *out;                     // int64 values when wide, else int32
     uint32_t lut_bits, wide;
+    uint32_t words;                // of a chunk: 8 or 32
 };
 
-// A decode CTA has a tile of chunks, a run of them a warp, whose first lanes decode the chunks before
-// its run as well.
-constexpr uint32_t kDecodeThreads = 256, kDecodeHalo = 2, kDecodeRun = 32 - kDecodeHalo,
-                   kDecodeTile = kDecodeThreads / 32 * kDecodeRun;
+// A decode CTA has a tile of chunks of W words, a run of them a warp, whose first lanes decode the chunks
+// before its run as well (2048 bits of them, whatever W is).
+constexpr uint32_t kDecodeThreads = 256, kDecodeHaloWords = 64;
+ASZ_HD constexpr uint32_t decode_halo(uint32_t W) { return kDecodeHaloWords / W; }
+ASZ_HD constexpr uint32_t decode_run(uint32_t W) { return 32 - decode_halo(W); }
+ASZ_HD constexpr uint32_t decode_tile(uint32_t W) { return kDecodeThreads / 32 * decode_run(W); }
 
 // One candidate predictor of a plan-search layer (generate_config.tpp:526-604): its sample lattice
 // (start, stride and count per axis; loop nest ax[0] outer .. ax[2] inner), stencil geometry along
@@ -235,7 +238,7 @@ template <class T>
 cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uint64_t *toff, uint64_t ntiles, uint64_t *tile_state,
                                 uint64_t *err, cudaStream_t st);
 cudaError_t launch_scan_u64(const uint64_t *in, uint64_t *out, uint64_t n, void *tmp, size_t &tmp_bytes, cudaStream_t st);
-cudaError_t launch_decode_sync(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
+cudaError_t launch_decode_sync(const uint8_t *base, const DecStream *streams, const uint32_t *tile_stream,
                                uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
                                const uint32_t *childs,
                                int first_pass, uint64_t *start, uint64_t *end, uint64_t *count, const uint32_t *moved,
@@ -245,7 +248,7 @@ cudaError_t launch_decode_restart(const DecStream *streams, uint32_t nstreams, u
 cudaError_t launch_decode_check(const DecStream *streams, uint32_t nstreams, const uint32_t *tile_stream, uint64_t ntiles,
                                 const uint64_t *off, const uint64_t *start, const uint64_t *end, uint32_t *err,
                                 uint32_t *changed, cudaStream_t st);
-cudaError_t launch_decode_write(const uint8_t *base, uint64_t chunk_bits, const DecStream *streams, const uint32_t *tile_stream,
+cudaError_t launch_decode_write(const uint8_t *base, const DecStream *streams, const uint32_t *tile_stream,
                                 uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
                                const uint32_t *childs,
                                 const uint64_t *start, const uint64_t *off, uint32_t *err, cudaStream_t st);
