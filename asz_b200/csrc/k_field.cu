@@ -706,9 +706,10 @@ static cudaError_t launch_round_compress_lines(const FieldGeom &fg, const RoundG
     const unsigned warps = (unsigned)std::max<size_t>(1, std::min<size_t>(8, kStageBudget / per_warp));
     const size_t smem = warps * per_warp + (hist ? kHistWin * sizeof(uint32_t) : 0);
     cudaError_t e;
+    // The limit is the most that any launch uses: it is one for all threads of the process.
     if (smem > 48 * 1024 &&
-        (e = cudaFuncSetAttribute(round_compress_line_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-            cudaSuccess)
+        (e = cudaFuncSetAttribute(round_compress_line_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kStageBudget + kHistWin * sizeof(uint32_t)))) != cudaSuccess)
         return e;
     int occ = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, round_compress_line_kernel, (int)(32 * warps), smem)) !=

@@ -791,14 +791,17 @@ static unsigned decode_grid(uint64_t ntiles) { return (unsigned)(ntiles < 148 * 
 static size_t decode_smem(uint32_t max_lut_bits) {
     return kDecodeSlotBytes + std::max<size_t>(((size_t)1 << max_lut_bits) * 4, 16);
 }
+constexpr uint32_t kDecodeLutBits = 12;  // a table's most; the kernels' limit is one for all threads and streams
 
 cudaError_t launch_decode_sync(const uint8_t *base, const DecStream *streams, const uint32_t *tile_stream,
                                uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
                                const uint32_t *childs,
                                int first_pass, uint64_t *start, uint64_t *end, uint64_t *count, const uint32_t *moved,
                                uint32_t *err, cudaStream_t st) {
+    if (max_lut_bits > kDecodeLutBits) return cudaErrorInvalidValue;
     const size_t sh = decode_smem(max_lut_bits);
-    const cudaError_t e = cudaFuncSetAttribute(decode_sync_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    const cudaError_t e =
+        cudaFuncSetAttribute(decode_sync_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem(kDecodeLutBits));
     if (e != cudaSuccess) return e;
     decode_sync_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, streams, tile_stream, ntiles, luts, lut2s,
                                                                       childs, first_pass, start, end, count, moved, err);
@@ -829,8 +832,10 @@ cudaError_t launch_decode_write(const uint8_t *base, const DecStream *streams, c
                                 uint64_t ntiles, uint32_t max_lut_bits, const uint32_t *luts, const uint32_t *lut2s,
                                const uint32_t *childs,
                                 const uint64_t *start, const uint64_t *off, uint32_t *err, cudaStream_t st) {
+    if (max_lut_bits > kDecodeLutBits) return cudaErrorInvalidValue;
     const size_t sh = decode_smem(max_lut_bits);
-    const cudaError_t e = cudaFuncSetAttribute(decode_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    const cudaError_t e =
+        cudaFuncSetAttribute(decode_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decode_smem(kDecodeLutBits));
     if (e != cudaSuccess) return e;
     decode_write_kernel<<<decode_grid(ntiles), kDecodeThreads, sh, st>>>(base, streams, tile_stream, ntiles, luts, lut2s, childs,
                                                                        start, off, err);

@@ -680,7 +680,8 @@ cudaError_t launch_lines_compress(const FieldGeom &fg, const RoundGeom *rounds, 
     if (items == 0) return cudaSuccess;
     if (fg.block_num[2] > kMaxColumnBlocks) return cudaErrorInvalidValue;
     const uint32_t smem = (uint32_t)(align16(sizeof(CompShared)) + line_bytes);
-    cudaError_t e = cudaFuncSetAttribute(lines_compress_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(lines_compress_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(align16(sizeof(CompShared)) + lines_smem_limit()));
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lines_compress_kernel, fastsel::kThreads, smem);

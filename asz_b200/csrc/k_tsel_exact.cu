@@ -793,14 +793,16 @@ uint32_t slope_batches(uint32_t n_evals) { return (n_evals + kTeams - 1) / kTeam
 namespace {
 
 // Shared memory of a launch whose largest group has `most` samples and whose kernel takes groups of
-// up to `cap`: the side-by-side tables where they fit.
+// up to `cap`: the side-by-side tables where they fit. The kernel's limit is the most that any launch
+// uses: it is one for all threads of the process, and for launches that a graph keeps.
 cudaError_t exact_shared(const void *kernel, uint32_t cap, uint32_t most, Layout &lo) {
     int dev = 0, lim = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    lo = exact_layout(most < cap ? most : cap, (uint32_t)lim - kExactStatic);
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lo.total);
+    const uint32_t limit = (uint32_t)lim - kExactStatic;
+    lo = exact_layout(most < cap ? most : cap, limit);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
 }
 
 }  // namespace
