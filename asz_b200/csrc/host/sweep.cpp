@@ -19,6 +19,8 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <utility>
@@ -40,7 +42,7 @@ namespace {
 using u64 = uint64_t;
 using clk = std::chrono::steady_clock;
 
-// Per stream of a batch: the framed stream, the zstd output and a zstd context, kept across rows and
+// Per stream in work at a time: the framed stream, the zstd output and a zstd context, kept across rows and
 // calls so that their pages are mapped once (first writes to fresh pages cost as much as zstd).
 struct WorkerScratch {
     std::vector<uint8_t> buf, z;
@@ -50,7 +52,7 @@ struct WorkerScratch {
 struct SweepState {
     DevBuf coef, qb, part, sums, mm, hist, first, tab, pay, enc;
     PinnedBuf small, counts, payload;
-    std::vector<WorkerScratch> ws;
+    std::vector<std::unique_ptr<WorkerScratch>> ws;
 };
 
 struct Predictor {
@@ -237,8 +239,8 @@ void sweep_release(void *state) {
     s->small.release();
     s->counts.release();
     s->payload.release();
-    for (WorkerScratch &w : s->ws)
-        if (w.cc) ZSTD_freeCCtx(w.cc);
+    for (auto &w : s->ws)
+        if (w->cc) ZSTD_freeCCtx(w->cc);
     delete s;
 }
 }  // namespace asz::host
@@ -442,10 +444,22 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
             // Frame each stream (save + encode, huffman.hpp) and compress it with zstd level 3.
             std::vector<u64> hb(kc), zb(kc);
             std::vector<char> zok(kc, 1);
-            if (W.ws.size() < kc) W.ws.resize(kc);
+            std::mutex idle_mu;
+            std::vector<WorkerScratch *> idle;
+            for (auto &w : W.ws) idle.push_back(w.get());
             host::ctx_parallel(ctx, kc, [&](u64 k) {
                 const HuffCode &c = code[k];
-                WorkerScratch &sc = W.ws[k];
+                WorkerScratch *mine;
+                {
+                    std::lock_guard<std::mutex> g(idle_mu);
+                    if (idle.empty()) {
+                        W.ws.push_back(std::make_unique<WorkerScratch>());
+                        idle.push_back(W.ws.back().get());
+                    }
+                    mine = idle.back();
+                    idle.pop_back();
+                }
+                WorkerScratch &sc = *mine;
                 const u64 pay = c.maxval == 1 ? 0 : (c.bits + 7) / 8, len = c.save_size() + 8 + pay;
                 if (sc.buf.size() < len) sc.buf.resize(len);
                 write_tree(c, sc.buf.data());
@@ -458,6 +472,8 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
                 zok[k] = !ZSTD_isError(n);
                 hb[k] = len;
                 zb[k] = n;
+                std::lock_guard<std::mutex> g(idle_mu);
+                idle.push_back(mine);
             });
             const double enc_s = std::chrono::duration<double>(clk::now() - t_enc).count();
             for (u64 k = 0; k < kc; k++) {
