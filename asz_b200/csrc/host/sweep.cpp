@@ -4,9 +4,10 @@
 // Per relative error bound, the predictor's coefficients go through in batches sized to the
 // device memory: one launch predicts and quantises every target for every coefficient of the
 // batch (k_sweep.cu); histograms and first positions of the QB symbols follow on the device; the
-// host builds each stream's Huffman code and H1; one tiled launch encodes all streams; the host
-// frames each stream as huffman_encoder_class<int64_t>::save + encode and compresses it with
-// libzstd level 3 on its threads (lossless_encode_and_write_csv, :400-440).
+// host builds each stream's Huffman code and H1; the streams are encoded, copied out and compressed
+// one behind the other: while a stream is encoded the one before it crosses to the host, where
+// libzstd level 3 takes those that are there, framed as huffman_encoder_class<int64_t>::save + encode,
+// on the worker threads (lossless_encode_and_write_csv, :400-440).
 //
 // Host floating point restates the reference's forms under its -Ofast build and is compiled with
 // -ffp-contract=off: the grid constants (a division in a loop becomes a product with the rounded
@@ -42,17 +43,40 @@ namespace {
 using u64 = uint64_t;
 using clk = std::chrono::steady_clock;
 
-// Per stream in work at a time: the framed stream, the zstd output and a zstd context, kept across rows and
-// calls so that their pages are mapped once (first writes to fresh pages cost as much as zstd).
+// Per stream in work at a time: the zstd output and a zstd context, kept across rows and calls so that
+// their pages are mapped once (first writes to fresh pages cost as much as zstd).
 struct WorkerScratch {
-    std::vector<uint8_t> buf, z;
+    std::vector<uint8_t> z;
     ZSTD_CCtx *cc = nullptr;
 };
+
+// Streams of fewer symbols are encoded and copied out together: below, a launch and a copy each cost
+// more than the wait for the others.
+constexpr u64 kGroupSymbols = 1ull << 22;
 
 struct SweepState {
     DevBuf coef, qb, part, sums, mm, hist, first, tab, pay, enc;
     PinnedBuf small, counts, payload;
     std::vector<std::unique_ptr<WorkerScratch>> ws;
+    cudaStream_t copies = nullptr;   // payloads on their way to the host
+    std::vector<cudaEvent_t> events;  // two a group of streams: encoded, and there
+    // Makes the copies' stream and at least n events.
+    cudaError_t reserve_events(size_t n) {
+        cudaError_t e = cudaSuccess;
+        if (!copies) e = cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking);
+        while (e == cudaSuccess && events.size() < n) {
+            cudaEvent_t ev = nullptr;
+            e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+            if (e == cudaSuccess) events.push_back(ev);
+        }
+        return e;
+    }
+};
+
+// Whatever way a call returns, its copies no longer run: the buffers they use are the next call's.
+struct CopiesEnd {
+    cudaStream_t s;
+    ~CopiesEnd() { cudaStreamSynchronize(s); }
 };
 
 struct Predictor {
@@ -241,6 +265,8 @@ void sweep_release(void *state) {
     s->payload.release();
     for (auto &w : s->ws)
         if (w->cc) ZSTD_freeCCtx(w->cc);
+    for (cudaEvent_t e : s->events) cudaEventDestroy(e);
+    if (s->copies) cudaStreamDestroy(s->copies);
     delete s;
 }
 }  // namespace asz::host
@@ -282,6 +308,234 @@ extern "C" int asz_sweep_targets(const uint64_t dims[3], const char *predictor, 
     return visited == g.targets ? ASZ_OK : ASZ_E_DEVICE;
 }
 
+namespace {
+
+// What the batches of one call share.
+struct SweepCall {
+    asz_ctx *ctx;
+    SweepState &W;
+    const SweepGeom &g;
+    const float *d_in;
+    double range, rel_eb, abs_eb, neg_2_eb;
+    const std::vector<std::pair<double, double>> &grid;
+    const Predictor &p;
+    asz_sweep_row *rows;  // of this error bound
+};
+constexpr int kWide = INT_MAX;  // a QB does not fit Q
+
+// Coefficients k0 .. k0 + kc - 1 of one error bound, with QBs of type Q.
+template <class Q>
+int sweep_batch(const SweepCall &S_, u64 k0, u64 kc) {
+    asz_ctx *const ctx = S_.ctx;
+    SweepState &W = S_.W;
+    const u64 S = S_.g.targets;
+    auto bad = [&](int code, const std::string &m) { return host::ctx_fail(ctx, code, m); };
+    cudaStream_t st = host::ctx_stream(ctx);
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    const uint32_t nparts = sweep_predict_grid(S_.g);
+    const size_t mm_at = kc * 3 * sizeof(double), ss_at = mm_at + kc * 2 * sizeof(long long);
+    CK(W.coef.reserve(kc * sizeof(SweepCoef)));
+    CK(W.qb.reserve(kc * S * sizeof(Q)));
+    CK(W.part.reserve(kc * nparts * 3 * sizeof(double)));
+    CK(W.sums.reserve(ss_at + kc * sizeof(SweepStream)));
+    CK(W.small.reserve(kc * (sizeof(SweepCoef) + 3 * sizeof(double) + 2 * sizeof(long long) + sizeof(SweepStream))));
+    SweepCoef *h_coef = (SweepCoef *)W.small.p;
+    double *h_sums = (double *)(h_coef + kc);
+    long long *h_mm = (long long *)(h_sums + 3 * kc);
+    SweepStream *h_ss = (SweepStream *)(h_mm + 2 * kc);
+    double *d_sums = W.sums.as<double>();
+    long long *d_mm = (long long *)(W.sums.as<uint8_t>() + mm_at);
+    SweepStream *d_ss = (SweepStream *)(W.sums.as<uint8_t>() + ss_at);
+    Q *d_qb = W.qb.as<Q>();
+    for (u64 k = 0; k < kc; k++) {
+        h_coef[k] = make_coef(S_.p, S_.grid[k0 + k].first, S_.grid[k0 + k].second);
+        h_mm[2 * k] = LLONG_MAX;
+        h_mm[2 * k + 1] = LLONG_MIN;
+    }
+    CK(cudaMemcpyAsync(W.coef.p, h_coef, kc * sizeof(SweepCoef), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_mm, h_mm, kc * 2 * sizeof(long long), cudaMemcpyHostToDevice, st));
+    CK(launch_sweep_predict<Q>(S_.d_in, S_.g, W.coef.as<SweepCoef>(), (uint32_t)kc, S_.abs_eb, S_.neg_2_eb, d_qb, S,
+                               W.part.as<double>(), d_mm, st));
+    CK(launch_sweep_sums(W.part.as<double>(), nparts, (uint32_t)kc, d_sums, st));
+    CK(cudaMemcpyAsync(h_sums, d_sums, ss_at, cudaMemcpyDeviceToHost, st));  // the sums and the extremes
+    CK(cudaStreamSynchronize(st));
+    if (sizeof(Q) == 4)
+        for (u64 k = 0; k < kc; k++)
+            if (h_mm[2 * k] == LLONG_MIN) return kWide;
+    const auto t_enc = clk::now();
+    // Histograms and first positions of every stream of the batch.
+    std::vector<u64> hoff(kc + 1, 0);
+    for (u64 k = 0; k < kc; k++) {
+        const u64 r = (u64)(h_mm[2 * k + 1] - h_mm[2 * k]) + 1;
+        if (h_mm[2 * k] > h_mm[2 * k + 1] || r > kMaxSymbolRange)
+            return bad(ASZ_E_UNSUPPORTED, "QB symbol range exceeds 2^27 values");
+        h_ss[k] = SweepStream{h_mm[2 * k], r, hoff[k]};
+        hoff[k + 1] = hoff[k] + r;
+    }
+    const u64 htot = hoff[kc];
+    CK(W.hist.reserve(htot * 8));
+    CK(W.first.reserve(htot * 8));
+    CK(W.counts.reserve(htot * 16));
+    CK(cudaMemsetAsync(W.hist.p, 0, htot * 8, st));
+    CK(cudaMemsetAsync(W.first.p, 0xff, htot * 8, st));
+    CK(cudaMemcpyAsync(d_ss, h_ss, kc * sizeof(SweepStream), cudaMemcpyHostToDevice, st));
+    CK(launch_sweep_stats<Q>(d_qb, S, (uint32_t)kc, d_ss, W.hist.as<unsigned long long>(), W.first.as<unsigned long long>(), st));
+    u64 *h_hist = (u64 *)W.counts.p, *h_first = h_hist + htot;
+    CK(cudaMemcpyAsync(h_hist, W.hist.p, htot * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h_first, W.first.p, htot * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    // Codes on the host threads.
+    std::vector<HuffCode> code(kc);
+    std::vector<double> h1(kc);
+    std::vector<std::string> cerr(kc);
+    std::vector<char> ok(kc, 1);
+    host::ctx_parallel(ctx, kc, [&](u64 k) {
+        std::vector<u64> hv(h_hist + hoff[k], h_hist + hoff[k + 1]);
+        ok[k] = build_code(hv, h_mm[2 * k], h_mm[2 * k + 1], S, true, code[k], cerr[k]);
+    });
+    for (u64 k = 0; k < kc; k++)
+        if (!ok[k]) return bad(ASZ_E_UNSUPPORTED, cerr[k]);
+    // Groups of streams that are encoded in one launch and copied out behind it. A stream's frame in
+    // the pinned buffer is its tree and length word (front), then the payload; a stream alone in its
+    // group is copied straight there, others together to where the group begins, and from there by
+    // the worker.
+    struct Group {
+        u64 k0, k1, es0, toff0, state0, tiles;
+        u64 at;  // in the pinned buffer, of groups of several streams
+    };
+    std::vector<Group> groups;
+    std::vector<EncStream> es;
+    std::vector<u64> toff, tab_off(kc, 0), word_off(kc + 1, 0), frame(kc), front(kc), pay(kc), group_of(kc);
+    u64 tab_tot = 0, states = 0, host_end = 0;
+    for (u64 k = 0; k < kc; k++) {
+        tab_off[k] = tab_tot;
+        tab_tot += code[k].table.size();
+        pay[k] = code[k].maxval == 1 ? 0 : (code[k].bits + 7) / 8;
+        word_off[k + 1] = word_off[k] + (pay[k] + 3) / 4;
+        front[k] = code[k].save_size() + 8;
+        frame[k] = (host_end + front[k] + 63) / 64 * 64 - front[k];  // the payload on a line of its own
+        host_end = frame[k] + front[k] + word_off[k + 1] * 4 - word_off[k] * 4;
+    }
+    CK(W.tab.reserve(std::max<u64>(tab_tot, 1) * sizeof(CodeEntry)));
+    CK(W.pay.reserve(std::max<u64>(word_off[kc], 1) * 4));
+    for (u64 k = 0; k < kc;) {
+        Group G{k, k, es.size(), toff.size(), states, 0, host_end};
+        toff.push_back(0);
+        do {
+            group_of[k] = groups.size();
+            if (pay[k]) {
+                es.push_back(EncStream{d_qb + k * S, S, h_mm[2 * k], W.tab.as<CodeEntry>() + tab_off[k],
+                                       W.pay.as<uint32_t>() + word_off[k]});
+                G.tiles += (S + enc_tile<Q>() - 1) / enc_tile<Q>();
+                toff.push_back(G.tiles);
+            }
+            k++;
+        } while (k < kc && (k - G.k0) * S < kGroupSymbols);
+        G.k1 = k;
+        if (G.k1 - G.k0 > 1) host_end += (word_off[G.k1] - word_off[G.k0]) * 4;
+        states += G.tiles + 1;
+        groups.push_back(G);
+    }
+    const u64 tab_at = (host_end + 15) / 16 * 16;
+    CK(W.payload.reserve(tab_at + tab_tot * sizeof(CodeEntry)));
+    CK(W.reserve_events(2 * groups.size()));
+    CodeEntry *h_tab = (CodeEntry *)(W.payload.p + tab_at);
+    for (u64 k = 0; k < kc; k++) std::memcpy(h_tab + tab_off[k], code[k].table.data(), code[k].table.size() * sizeof(CodeEntry));
+    const u64 o_toff = (es.size() * sizeof(EncStream) + 15) / 16 * 16, o_err = o_toff + (toff.size() * 8 + 15) / 16 * 16,
+              o_state = o_err + 16, end = o_state + states * 8;
+    CK(W.enc.reserve(end));
+    uint8_t *eb = W.enc.as<uint8_t>();
+    CopiesEnd copies_end{W.copies};
+    if (!es.empty()) {
+        CK(cudaMemcpyAsync(W.tab.p, h_tab, tab_tot * sizeof(CodeEntry), cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(W.pay.p, 0, word_off[kc] * 4, st));
+        CK(cudaMemcpyAsync(eb, es.data(), es.size() * sizeof(EncStream), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(eb + o_toff, toff.data(), toff.size() * 8, cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(eb + o_err, 0, end - o_err, st));
+    }
+    for (u64 i = 0; i < groups.size(); i++) {
+        const Group &G = groups[i];
+        const u64 es1 = i + 1 < groups.size() ? groups[i + 1].es0 : es.size();
+        if (es1 == G.es0) continue;
+        CK(launch_encode_tiles<Q>((const EncStream *)eb + G.es0, (uint32_t)(es1 - G.es0), (const u64 *)(eb + o_toff) + G.toff0,
+                                  G.tiles, (u64 *)(eb + o_state) + G.state0, (u64 *)(eb + o_err), st));
+        CK(cudaEventRecord(W.events[2 * i], st));
+        CK(cudaStreamWaitEvent(W.copies, W.events[2 * i], 0));
+        uint8_t *to = W.payload.p + (G.k1 - G.k0 > 1 ? G.at : frame[G.k0] + front[G.k0]);
+        CK(cudaMemcpyAsync(to, W.pay.as<uint32_t>() + word_off[G.k0], (word_off[G.k1] - word_off[G.k0]) * 4,
+                           cudaMemcpyDeviceToHost, W.copies));
+        CK(cudaEventRecord(W.events[2 * i + 1], W.copies));
+    }
+    // Frame each stream (save + encode, huffman.hpp) and compress it with zstd level 3.
+    std::vector<u64> zb(kc);
+    std::vector<char> zok(kc, 1), there(kc, 1);
+    std::mutex idle_mu;
+    std::vector<WorkerScratch *> idle;
+    for (auto &w : W.ws) idle.push_back(w.get());
+    host::ctx_parallel(ctx, kc, [&](u64 k) {
+        const HuffCode &c = code[k];
+        WorkerScratch *mine;
+        {
+            std::lock_guard<std::mutex> g(idle_mu);
+            if (idle.empty()) {
+                W.ws.push_back(std::make_unique<WorkerScratch>());
+                idle.push_back(W.ws.back().get());
+            }
+            mine = idle.back();
+            idle.pop_back();
+        }
+        WorkerScratch &sc = *mine;
+        uint8_t *const buf = W.payload.p + frame[k];
+        const u64 len = front[k] + pay[k];
+        write_tree(c, buf);
+        write_len_word(c, buf + front[k] - 8);
+        h1[k] = h1_of(h_hist + hoff[k], h_first + hoff[k], hoff[k + 1] - hoff[k], h_mm[2 * k], S);
+        if (pay[k]) {
+            const Group &G = groups[group_of[k]];
+            there[k] = cudaSetDevice(dev) == cudaSuccess && cudaEventSynchronize(W.events[2 * group_of[k] + 1]) == cudaSuccess;
+            if (G.k1 - G.k0 > 1) std::memcpy(buf + front[k], W.payload.p + G.at + (word_off[k] - word_off[G.k0]) * 4, pay[k]);
+        }
+        if (sc.z.size() < ZSTD_compressBound(len)) sc.z.resize(ZSTD_compressBound(len));
+        if (!sc.cc) sc.cc = ZSTD_createCCtx();
+        const size_t n = sc.cc ? ZSTD_compressCCtx(sc.cc, sc.z.data(), sc.z.size(), buf, len, 3)
+                               : ZSTD_compress(sc.z.data(), sc.z.size(), buf, len, 3);
+        zok[k] = !ZSTD_isError(n);
+        zb[k] = n;
+        std::lock_guard<std::mutex> g(idle_mu);
+        idle.push_back(mine);
+    });
+    if (!es.empty()) {
+        u64 enc_err = 0;
+        CK(cudaMemcpyAsync(&enc_err, eb + o_err, sizeof(u64), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        CK(cudaStreamSynchronize(W.copies));
+        if (enc_err) return bad(ASZ_E_DEVICE, "Huffman encoder: a tile's wait for the tiles before it timed out");
+    }
+    const double enc_s = std::chrono::duration<double>(clk::now() - t_enc).count();
+    for (u64 k = 0; k < kc; k++) {
+        if (!there[k]) return bad(ASZ_E_CUDA, "waiting for a stream's payload failed");
+        if (!zok[k]) return bad(ASZ_E_DATA, "zstd compression failed");
+        asz_sweep_row &r = S_.rows[k0 + k];
+        std::memset(&r, 0, sizeof r);
+        r.rel_eb = S_.rel_eb;
+        r.c0 = S_.grid[k0 + k].first;
+        r.c1 = S_.grid[k0 + k].second;
+        r.samples = S;
+        r.huffman_bytes = front[k] + pay[k];
+        r.zstd_bytes = zb[k];
+        r.mse_sum = h_sums[3 * k];
+        r.rmse_sum = h_sums[3 * k + 1];
+        r.mae_sum = h_sums[3 * k + 2];
+        r.h1 = h1[k];
+        r.encode_seconds = enc_s / (double)kc;
+        finish_row(r, S_.range);
+    }
+    return ASZ_OK;
+}
+
+}  // namespace
+
 extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const uint64_t dims[3], const char *predictor,
                          const char *targets, const char *six_grid, const double *rel_eb, uint64_t n_eb, asz_sweep_row *rows,
                          uint64_t cap, uint64_t *n_rows, float *min_max) {
@@ -309,7 +563,6 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
     *n_rows = n_eb * K;
     if (cap < n_eb * K) return bad(ASZ_E_ARG, "row buffer too small");
     if (S == 0) return bad(ASZ_E_DATA, "no prediction targets");
-    cudaStream_t st = host::ctx_stream(ctx);
     void *&sp = host::ctx_sweep_state(ctx);
     if (!sp) sp = new SweepState();
     SweepState &W = *(SweepState *)sp;
@@ -329,170 +582,35 @@ extern "C" int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const u
     if (!(mx > mn)) return bad(ASZ_E_DATA, "constant input");
     const double range = (double)mx - (double)mn;
 
-    // Coefficients per batch: their QB streams share the device with the field.
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    const u64 budget = std::max<u64>(S * 8, std::min<u64>(free_b / 3, 24ull << 30));
-    const u64 KB = std::max<u64>(1, std::min<u64>(K, budget / (S * 8)));
-    const uint32_t nparts = sweep_predict_grid(g);
-    CK(W.coef.reserve(KB * sizeof(SweepCoef)));
-    CK(W.qb.reserve(KB * S * 8));
-    CK(W.part.reserve(KB * nparts * 3 * sizeof(double)));
-    CK(W.sums.reserve(KB * 3 * sizeof(double) + KB * 2 * sizeof(long long)));
-    CK(W.small.reserve(KB * (sizeof(SweepCoef) + 3 * sizeof(double) + 2 * sizeof(long long))));
-    SweepCoef *h_coef = (SweepCoef *)W.small.p;
-    double *h_sums = (double *)(h_coef + KB);
-    long long *h_mm = (long long *)(h_sums + 3 * KB);
-    double *d_sums = W.sums.as<double>();
-    long long *d_mm = (long long *)(d_sums + 3 * KB);
-    int64_t *d_qb = W.qb.as<int64_t>();
-
+    // Coefficients per batch: their QB streams share the device with the field. The device's free
+    // memory is asked for only where the buffer that is there does not hold them all (the question
+    // takes 0.1 to 0.3 ms).
+    u64 budget = 0;
+    auto most = [&](u64 size, u64 &kb) -> int {
+        kb = K;
+        if (W.qb.cap >= K * S * size) return ASZ_OK;
+        if (!budget) {
+            size_t free_b = 0, total_b = 0;
+            CK(cudaMemGetInfo(&free_b, &total_b));
+            budget = std::max<u64>(S * 8, std::min<u64>(free_b / 3, 24ull << 30));
+        }
+        kb = std::max<u64>(1, std::min<u64>(K, budget / (S * size)));
+        return ASZ_OK;
+    };
+    u64 KB = 0, KB8 = 0;
+    if ((rc = most(4, KB))) return rc;
     for (u64 e = 0; e < n_eb; e++) {
         const double abs_eb = rel_eb[e] * range;  // :195-196
-        const double neg_2_eb = 1 / (2 * abs_eb);
+        const SweepCall call{ctx, W, g, d_in, range, rel_eb[e], abs_eb, 1 / (2 * abs_eb), grid, p, rows + e * K};
         for (u64 k0 = 0; k0 < K; k0 += KB) {
             const u64 kc = std::min<u64>(KB, K - k0);
-            for (u64 k = 0; k < kc; k++) {
-                h_coef[k] = make_coef(p, grid[k0 + k].first, grid[k0 + k].second);
-                h_mm[2 * k] = LLONG_MAX;
-                h_mm[2 * k + 1] = LLONG_MIN;
+            rc = sweep_batch<int32_t>(call, k0, kc);
+            if (rc == kWide) {
+                if (!KB8 && (rc = most(8, KB8))) return rc;
+                rc = ASZ_OK;
+                for (u64 k = k0; k < k0 + kc && !rc; k += KB8) rc = sweep_batch<int64_t>(call, k, std::min<u64>(KB8, k0 + kc - k));
             }
-            CK(cudaMemcpyAsync(W.coef.p, h_coef, kc * sizeof(SweepCoef), cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(d_mm, h_mm, kc * 2 * sizeof(long long), cudaMemcpyHostToDevice, st));
-            CK(launch_sweep_predict(d_in, g, W.coef.as<SweepCoef>(), (uint32_t)kc, abs_eb, neg_2_eb, d_qb, S,
-                                    W.part.as<double>(), d_mm, st));
-            CK(launch_sweep_sums(W.part.as<double>(), nparts, (uint32_t)kc, d_sums, st));
-            CK(cudaMemcpyAsync(h_sums, d_sums, kc * 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(h_mm, d_mm, kc * 2 * sizeof(long long), cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            const auto t_enc = clk::now();
-            // Histograms and first positions of every stream of the batch.
-            std::vector<u64> hoff(kc + 1, 0);
-            for (u64 k = 0; k < kc; k++) {
-                const u64 r = (u64)(h_mm[2 * k + 1] - h_mm[2 * k]) + 1;
-                if (h_mm[2 * k] > h_mm[2 * k + 1] || r > kMaxSymbolRange)
-                    return bad(ASZ_E_UNSUPPORTED, "QB symbol range exceeds 2^27 values");
-                hoff[k + 1] = hoff[k] + r;
-            }
-            const u64 htot = hoff[kc];
-            CK(W.hist.reserve(htot * 8));
-            CK(W.first.reserve(htot * 8));
-            CK(W.counts.reserve(htot * 16));
-            CK(cudaMemsetAsync(W.hist.p, 0, htot * 8, st));
-            CK(cudaMemsetAsync(W.first.p, 0xff, htot * 8, st));
-            for (u64 k = 0; k < kc; k++) {
-                const int64_t *s = d_qb + k * S;
-                CK(launch_sweep_stats(s, S, h_mm[2 * k], hoff[k + 1] - hoff[k], W.hist.as<unsigned long long>() + hoff[k],
-                                      W.first.as<unsigned long long>() + hoff[k], st));
-            }
-            u64 *h_hist = (u64 *)W.counts.p, *h_first = h_hist + htot;
-            CK(cudaMemcpyAsync(h_hist, W.hist.p, htot * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(h_first, W.first.p, htot * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            // Codes and H1 on the host threads.
-            std::vector<HuffCode> code(kc);
-            std::vector<double> h1(kc);
-            std::vector<std::string> cerr(kc);
-            std::vector<char> ok(kc, 1);
-            host::ctx_parallel(ctx, kc, [&](u64 k) {
-                const u64 r = hoff[k + 1] - hoff[k];
-                std::vector<u64> hv(h_hist + hoff[k], h_hist + hoff[k] + r);
-                ok[k] = build_code(hv, h_mm[2 * k], h_mm[2 * k + 1], S, true, code[k], cerr[k]);
-                h1[k] = h1_of(h_hist + hoff[k], h_first + hoff[k], r, h_mm[2 * k], S);
-            });
-            for (u64 k = 0; k < kc; k++)
-                if (!ok[k]) return bad(ASZ_E_UNSUPPORTED, cerr[k]);
-            // Encode every stream that has a payload in one tiled launch.
-            std::vector<EncStream> es;
-            std::vector<u64> toff{0}, tab_off(kc, 0), word_off(kc + 1, 0);
-            u64 tab_tot = 0;
-            for (u64 k = 0; k < kc; k++) {
-                tab_off[k] = tab_tot;
-                tab_tot += code[k].table.size();
-                word_off[k + 1] = word_off[k] + (code[k].maxval == 1 ? 0 : (code[k].bits + 31) / 32);
-            }
-            CK(W.tab.reserve(std::max<u64>(tab_tot, 1) * sizeof(CodeEntry)));
-            CK(W.pay.reserve(std::max<u64>(word_off[kc], 1) * 4));
-            CK(W.payload.reserve(std::max<u64>(word_off[kc], 1) * 4 + tab_tot * sizeof(CodeEntry)));
-            CodeEntry *h_tab = (CodeEntry *)(W.payload.p + word_off[kc] * 4);
-            for (u64 k = 0; k < kc; k++) {
-                std::memcpy(h_tab + tab_off[k], code[k].table.data(), code[k].table.size() * sizeof(CodeEntry));
-                if (code[k].maxval == 1) continue;
-                es.push_back(EncStream{d_qb + k * S, S, h_mm[2 * k], W.tab.as<CodeEntry>() + tab_off[k],
-                                       W.pay.as<uint32_t>() + word_off[k]});
-                toff.push_back(toff.back() + (S + enc_tile<int64_t>() - 1) / enc_tile<int64_t>());
-            }
-            const u64 nt = toff.back();
-            if (nt) {
-                CK(cudaMemcpyAsync(W.tab.p, h_tab, tab_tot * sizeof(CodeEntry), cudaMemcpyHostToDevice, st));
-                CK(cudaMemsetAsync(W.pay.p, 0, word_off[kc] * 4, st));
-                const u64 o_toff = (es.size() * sizeof(EncStream) + 15) / 16 * 16,
-                          o_err = o_toff + (toff.size() * 8 + 15) / 16 * 16, o_state = o_err + 16, end = o_state + (nt + 1) * 8;
-                CK(W.enc.reserve(end));
-                uint8_t *eb = W.enc.as<uint8_t>();
-                CK(cudaMemcpyAsync(eb, es.data(), es.size() * sizeof(EncStream), cudaMemcpyHostToDevice, st));
-                CK(cudaMemcpyAsync(eb + o_toff, toff.data(), toff.size() * 8, cudaMemcpyHostToDevice, st));
-                CK(cudaMemsetAsync(eb + o_err, 0, end - o_err, st));
-                CK(launch_encode_tiles<int64_t>((const EncStream *)eb, (uint32_t)es.size(), (const u64 *)(eb + o_toff), nt,
-                                                (u64 *)(eb + o_state), (u64 *)(eb + o_err), st));
-                u64 enc_err = 0;
-                CK(cudaMemcpyAsync(&enc_err, eb + o_err, sizeof(u64), cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(W.payload.p, W.pay.p, word_off[kc] * 4, cudaMemcpyDeviceToHost, st));
-                CK(cudaStreamSynchronize(st));
-                if (enc_err) return host::ctx_fail(ctx, ASZ_E_DEVICE, "Huffman encoder: a tile's wait for the tiles before it timed out");
-            }
-            // Frame each stream (save + encode, huffman.hpp) and compress it with zstd level 3.
-            std::vector<u64> hb(kc), zb(kc);
-            std::vector<char> zok(kc, 1);
-            std::mutex idle_mu;
-            std::vector<WorkerScratch *> idle;
-            for (auto &w : W.ws) idle.push_back(w.get());
-            host::ctx_parallel(ctx, kc, [&](u64 k) {
-                const HuffCode &c = code[k];
-                WorkerScratch *mine;
-                {
-                    std::lock_guard<std::mutex> g(idle_mu);
-                    if (idle.empty()) {
-                        W.ws.push_back(std::make_unique<WorkerScratch>());
-                        idle.push_back(W.ws.back().get());
-                    }
-                    mine = idle.back();
-                    idle.pop_back();
-                }
-                WorkerScratch &sc = *mine;
-                const u64 pay = c.maxval == 1 ? 0 : (c.bits + 7) / 8, len = c.save_size() + 8 + pay;
-                if (sc.buf.size() < len) sc.buf.resize(len);
-                write_tree(c, sc.buf.data());
-                write_len_word(c, sc.buf.data() + c.save_size());
-                if (pay) std::memcpy(sc.buf.data() + c.save_size() + 8, W.payload.p + word_off[k] * 4, pay);
-                if (sc.z.size() < ZSTD_compressBound(len)) sc.z.resize(ZSTD_compressBound(len));
-                if (!sc.cc) sc.cc = ZSTD_createCCtx();
-                const size_t n = sc.cc ? ZSTD_compressCCtx(sc.cc, sc.z.data(), sc.z.size(), sc.buf.data(), len, 3)
-                                       : ZSTD_compress(sc.z.data(), sc.z.size(), sc.buf.data(), len, 3);
-                zok[k] = !ZSTD_isError(n);
-                hb[k] = len;
-                zb[k] = n;
-                std::lock_guard<std::mutex> g(idle_mu);
-                idle.push_back(mine);
-            });
-            const double enc_s = std::chrono::duration<double>(clk::now() - t_enc).count();
-            for (u64 k = 0; k < kc; k++) {
-                if (!zok[k]) return bad(ASZ_E_DATA, "zstd compression failed");
-                asz_sweep_row &r = rows[e * K + k0 + k];
-                std::memset(&r, 0, sizeof r);
-                r.rel_eb = rel_eb[e];
-                r.c0 = grid[k0 + k].first;
-                r.c1 = grid[k0 + k].second;
-                r.samples = S;
-                r.huffman_bytes = hb[k];
-                r.zstd_bytes = zb[k];
-                r.mse_sum = h_sums[3 * k];
-                r.rmse_sum = h_sums[3 * k + 1];
-                r.mae_sum = h_sums[3 * k + 2];
-                r.h1 = h1[k];
-                r.encode_seconds = enc_s / (double)kc;
-                finish_row(r, range);
-            }
+            if (rc) return rc;
         }
     }
     return ASZ_OK;

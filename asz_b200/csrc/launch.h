@@ -300,12 +300,19 @@ ASZ_HD bool sweep_target(const SweepGeom &g, uint64_t it, uint64_t i[3], uint64_
 struct SweepCoef {
     double c0, c1, w, lo, hi;
 };
+// Q: int32_t or int64_t; QBs that int32_t does not hold leave INT64_MIN, INT64_MAX in mm.
+template <class Q>
 cudaError_t launch_sweep_predict(const float *d, const SweepGeom &g, const SweepCoef *coef, uint32_t ncoef, double abs_eb,
-                                 double neg_2_eb, int64_t *qb, uint64_t qb_stride, double *part, long long *mm,
-                                 cudaStream_t st);
+                                 double neg_2_eb, Q *qb, uint64_t qb_stride, double *part, long long *mm, cudaStream_t st);
 uint32_t sweep_predict_grid(const SweepGeom &g);
 cudaError_t launch_sweep_sums(const double *part, uint32_t nparts, uint32_t ncoef, double *sums, cudaStream_t st);
-cudaError_t launch_sweep_stats(const int64_t *s, uint64_t n, int64_t offset, uint64_t range, unsigned long long *hist,
-                               unsigned long long *first, cudaStream_t st);
+// One QB stream's smallest symbol, its number of bins and the first of them in the tables.
+struct SweepStream {
+    int64_t offset;
+    uint64_t range, at;
+};
+template <class Q>
+cudaError_t launch_sweep_stats(const Q *qb, uint64_t n, uint32_t ns, const SweepStream *streams, unsigned long long *hists,
+                               unsigned long long *firsts, cudaStream_t st);
 
 }  // namespace asz
