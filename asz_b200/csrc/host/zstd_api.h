@@ -1,5 +1,5 @@
 // The libzstd entry points this library calls. The system provides libzstd.so.1 without its
-// development header, so the prototypes of zstd's stable public API are declared here.
+// development header, so the prototypes of zstd's public API are declared here.
 #pragma once
 #include <cstddef>
 
@@ -20,6 +20,11 @@ size_t ZSTD_compressCCtx(ZSTD_CCtx *cctx, void *dst, size_t dstCapacity, const v
 ZSTD_DCtx *ZSTD_createDCtx(void);
 size_t ZSTD_freeDCtx(ZSTD_DCtx *dctx);
 size_t ZSTD_decompressDCtx(ZSTD_DCtx *dctx, void *dst, size_t dstCapacity, const void *src, size_t srcSize);
+// zstd's block functions, for frames whose headers this library reads itself: blocks in order into one
+// buffer, those that libzstd does not decode announced by ZSTD_insertBlock.
+size_t ZSTD_decompressBegin(ZSTD_DCtx *dctx);
+size_t ZSTD_decompressBlock(ZSTD_DCtx *dctx, void *dst, size_t dstCapacity, const void *src, size_t srcSize);
+size_t ZSTD_insertBlock(ZSTD_DCtx *dctx, const void *blockStart, size_t blockSize);
 }
 
 #define ZSTD_CONTENTSIZE_UNKNOWN (0ULL - 1)

@@ -366,11 +366,16 @@ int asz_sweep(asz_ctx *ctx, const float *data, int on_device, const uint64_t dim
  * of every target equals its position in the reference's block-major loops
  * (compress.tpp:53-88). Returns the number of violations (0), or a negative error code. */
 int64_t asz_check_geometry(const uint64_t dims[3], const char *plan, uint64_t block_pivot_ratio, int quintic);
+
 /* The same for a frame whose blocks and pivot lattice start at `origin` (the predictor-family
  * probe's local contexts, predictor_family.tpp:40-60): positions below the origin, and the
  * origin's faces off the pivot lattice, keep their input values and are never written. */
 int64_t asz_check_geometry_frame(const uint64_t dims[3], const uint64_t origin[3], const char *plan,
                                  uint64_t block_pivot_ratio, int quintic);
+
+/* Host-side self-check of the block-wise zstd unpacking: in[0, len) into out[0, raw). 1: unpacked;
+ * 0: not a frame that it takes (ZSTD_decompress decides then); -1: a fault. */
+int64_t asz_check_unframe(const uint8_t *in, uint64_t len, uint8_t *out, uint64_t raw);
 
 /* Host-side run of the device's std::unordered_map order emulation (no GPU involved), for
  * checking it against the real container: keys are (a[i], b[i]) pairs with the reference's
