@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kEncThreads, 4)
         }
         __syncthreads();
         // Words out, shifted to the tile's offset: word i takes the high bits of packed word i - 1.
-        const uint64_t bit0 = s_excl;
+        const uint64_t bit0 = s_excl + E.bit0;
         const uint32_t shift = (uint32_t)(bit0 & 31);
         const uint32_t nw = (shift + total + 31) >> 5;
         uint32_t *out = E.out + (bit0 >> 5);

@@ -232,7 +232,8 @@ struct EncStream {
     uint64_t n;
     int64_t offset;         // the symbol of code table entry 0
     const CodeEntry *tab;
-    uint32_t *out;          // payload words
+    uint32_t *out;          // payload words, zero before
+    uint32_t bit0 = 0;      // of the payload in the first word
 };
 template <class T>
 cudaError_t launch_encode_tiles(const EncStream *streams, uint32_t ns, const uint64_t *toff, uint64_t ntiles, uint64_t *tile_state,
