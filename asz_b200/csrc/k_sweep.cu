@@ -32,8 +32,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // A thread takes kSweepCoefs coefficients at once: a target's index (two 64-bit divisions), its loads
 // and its conversions are the same for all of them. With a coefficient a thread those cost more than
-// the prediction itself (100x500x500, 13 coefficients: 1.30 -> 0.77 ms, bound by double arithmetic and
-// conversions at 16 warps an SM).
+// the prediction itself (100x500x500, 13 coefficients: 1.30 -> 0.77 ms). Then a warp waits for its loads and
+// conversions, at 16 warps an SM: three CTAs an SM, with a few spilled registers, take 0.61 ms.
 constexpr uint32_t kSweepCoefs = 4;
 
 // Running figures of one thread and one coefficient: the three sums and the QB extremes.
@@ -96,7 +96,7 @@ __device__ __forceinline__ void sweep_one(const float *__restrict__ d, const Swe
 // of one line, with neighbouring items on neighbouring lines: a warp then reads neighbouring lines
 // (adjacent along axis 2), and each thread writes its segment's QB run in order.
 template <class Q, bool SIX>
-__global__ void __launch_bounds__(kSweepThreads)
+__global__ void __launch_bounds__(kSweepThreads, 3)
     sweep_predict_kernel(const float *__restrict__ d, SweepGeom g, const SweepCoef *__restrict__ coef, uint32_t ncoef,
                          double abs_eb, double neg_2_eb, Q *__restrict__ qb, uint64_t qb_stride, double *__restrict__ part,
                          long long *__restrict__ mm) {
