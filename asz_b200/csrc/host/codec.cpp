@@ -3508,6 +3508,15 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     uint8_t *const bsp = ctx->raw_in.p;
     std::memset(bsp + raw, 0, kDecodePad);
     CK(ctx->pre.reserve(raw + kDecodePad));
+    // The pieces on their way to the device are there before a call returns, also one that refuses the
+    // stream: the next call uses the same buffers, perhaps on another stream.
+    struct SendEnd {
+        cudaStream_t s;
+        bool sending = true;
+        ~SendEnd() {
+            if (sending) cudaStreamSynchronize(s);
+        }
+    } send_end{st};
     {
         HostScope hs(ctx, "host:zstd");
         if (!ctx->zd) ctx->zd = ZSTD_createDCtx();
@@ -3627,9 +3636,9 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
         if (counts[l + 2] < G.rounds[l].qb_total) return fail(ctx, ASZ_E_DATA, "compressed stream has too few QBs");
     // Device: stream bytes, t codes, QB streams.
     CK(ctx->misc.reserve(sizeof(MiscLayout)));
-    // What is left of the copy to the device; a call that returned before leaves it to the stream.
-    auto t0 = clk::now();
+    auto t0 = clk::now();  // what is left of the copy to the device
     CK(cudaStreamSynchronize(st));
+    send_end.sending = false;
     R.h2d_s += secs(t0, clk::now());
     std::vector<u64> qoff(L + 1);
     u64 qtot = 0;
