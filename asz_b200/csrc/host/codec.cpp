@@ -4448,9 +4448,13 @@ static int compress_batch_impl(asz_ctx *ctx, uint32_t count, const float *const 
     rc = upload_shape(best[2]);
     if (rc) return rc;
     // ---- The round sequence as a CUDA graph (captured once per batch layout; the inputs' addresses are
-    // in the fields' records, which every call uploads).
+    // in the fields' records, which every call uploads). The largest groups, which follow from the
+    // number of samples a group and not from the shapes, size the captured launches, and say whether
+    // the one with global scratch is among them.
     std::vector<uint64_t> graph_key = shape_key;
     graph_key.insert(graph_key.end(), best.begin(), best.end());
+    graph_key.insert(graph_key.end(), cap_round.begin(), cap_round.end());
+    for (u64 v : {(u64)capmax, gstride, (u64)ggrid}) graph_key.push_back(v);
     for (DevBuf *d : {&ctx->b_rec, &ctx->b_qb, &ctx->b_tval, &ctx->b_tint, &ctx->b_ent, &ctx->b_cls, &ctx->b_rounds,
                       &ctx->b_qoff, &ctx->b_range, &ctx->b_range0, &ctx->b_prox, &ctx->b_amb, &ctx->b_cnt, &ctx->b_fields,
                       &ctx->b_goff, &ctx->b_poff, &ctx->b_ioff, &ctx->b_queue, &ctx->b_hand, &ctx->b_spill, &ctx->scratch,

@@ -90,3 +90,30 @@ def test_batch_device_inputs_and_errors(gpu_ctx):
     bad = fs[:2] + [np.zeros((10, 10, 10), np.float32)]
     with pytest.raises(api.AszError, match="field 2: max_val==min_val"):
         gpu_ctx.compress_batch(bad, 1e-3, plan, "cubic", p)
+
+
+def test_batch_sampling_number_changes(gpu_ctx):
+    """Calls of the same shapes and plan on one context with another number of samples a group: what
+    the captured sequence was made for (the largest groups, and whether any exceeds the exact kernel's
+    shared memory) changes with it, so a sequence captured for the small groups is not replayed for the
+    large ones. A batch of other shapes in between has taken the first capture's place."""
+    import asz_b200.api as api
+    from asz_b200 import fields
+    rng = np.random.default_rng(47)
+    fs = []
+    for shape in [(60, 66, 75), (71, 62, 64)]:
+        fs.append(fields.grf_field(shape, 4.0, rng).astype(np.float32) + rng.random(shape).astype(np.float32) * 0.5)
+    plan = ",".join(["cubic0_012", "cubic1_012", "cubic2_012"] * 2)
+    par = {n: api.default_params(block_pivot_ratio=6, h1_block_sampling_num=n) for n in (64, 256, 2048)}
+    want = {n: [gpu_ctx.compress(f, 1e-4, plan, "cubic", p)[0] for f in fs] for n, p in par.items()}
+    assert want[2048] != want[256]
+    with api.Context(0) as ctx:
+        last = None
+        for n in (2048, None, 256, 2048, 2048, 64, 256, 256, 64):
+            if n is None:
+                ctx.compress_batch([fs[0][:40], fs[1][:40]], 1e-4, plan, "cubic", par[256])
+            else:
+                blobs, _, br = ctx.compress_batch(fs, 1e-4, plan, "cubic", par[n])
+                assert [bytes(b) for b in blobs] == want[n], n
+                assert br.graph_reused == (n == last)
+            last = n
