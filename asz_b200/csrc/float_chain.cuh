@@ -81,7 +81,9 @@ __device__ __forceinline__ float warp_chain(const double *x, int n, const Step &
 #pragma unroll
             for (int i = 0; i < kChainPer; i++) {
                 ok[i] = c.ulps(v[i], r[i]);
-                if (lane * kChainPer + i < done) ok[i] = true, r[i] = 0;
+                // What is added already, and places past the last term, which a sum that is not a
+                // number would reject.
+                if (lane * kChainPer + i < done || b + lane * kChainPer + i >= n) ok[i] = true, r[i] = 0;
                 sum += r[i];  // r <= 2^24
             }
             uint32_t incl = sum;  // <= 32 * 2^26
