@@ -8,12 +8,22 @@
 // scan gives the running sums, and the batch is accepted up to the first thread whose terms tie or
 // leave the binade. That thread takes its terms one by one, and the rest of the batch follows in
 // the new binade. A sum crosses each binade once, so there are about log2(sum / first term) such
-// steps.
+// steps. The subnormal floats and the first binade above them have one ulp and count as one binade
+// (m from 0 on), so sums of terms of any size, also none but zeros, are taken this way. An infinite
+// sum and one that is not a number stay what they are.
 //
-// The tie test keeps a margin of 2^-20: a term known to a relative 2^-52, or an addition that is
-// rounded to double before it is rounded to float, moves x / u by less than 2^-27 (x / u < 2^24),
-// so neither can bring it across a half from outside the margin. A term that is negative or not
-// finite fails the test too and is added by itself.
+// Ties are common in the sums of a field of whole numbers or of few significant bits, once the sum's
+// ulp is twice the squares' last place: most terms tie then. Where a batch had one, block_chain
+// gives each thread's sum for an even and for an odd m, and scans the pairs, so that no tie ends a pass;
+// warp_chain, whose batches are short, adds what is left of a batch term by term after kChainTies of
+// them. The plan search of 100x500x500 bytes at 5e-2, with a pass for each thread that had a tie, took
+// 62 ms, now 4.1; of values of 1e-25, with every term rejected while the sum was below 2^-100, 220, now 7.
+//
+// The tie test of warp_chain keeps a margin of 2^-20: a term known to a relative 2^-52, or an addition
+// that is rounded to double before it is rounded to float, moves x / u by less than 2^-27
+// (x / u < 2^24), so neither can bring it across a half from outside the margin. block_chain's terms
+// are squares, exact in double, and its step rounds once: its ties are exact. A term that is negative
+// or not finite fails the test too and is added by itself.
 #pragma once
 #include <cstdint>
 
@@ -23,35 +33,51 @@ namespace asz {
 struct ChainSum {
     float s;
     uint32_t m;
-    int ex;
     double inv_u;
-    bool normal;  // well inside the normal floats
-    __device__ __forceinline__ explicit ChainSum(float v) : s(v), m(0), ex(0), inv_u(0.0), normal(v >= 0x1p-100f && v < 0x1p120f) {
-        if (normal) {
-            ex = (int)(__float_as_uint(v) >> 23) - 126;  // v = f 2^ex, f in [1/2, 1): ulp 2^(ex - 24)
-            m = (__float_as_uint(v) & 0x7fffffu) | 0x800000u;
-            inv_u = __longlong_as_double((long long)(1023 + 24 - ex) << 52);
+    bool regular;  // finite and not negative
+    __device__ __forceinline__ explicit ChainSum(float v) : s(v), m(0), inv_u(0.0), regular(v >= 0.0f && v <= 0x1.fffffep127f) {
+        if (regular) {
+            const uint32_t bits = __float_as_uint(v) & 0x7fffffffu, e = max(bits >> 23, 1u);
+            m = bits - ((e - 1) << 23);  // v = m 2^(e - 150)
+            inv_u = __longlong_as_double((long long)(1023 + 150 - (int)e) << 52);
         }
     }
-    // The sum after `add` more ulps (m + add < 2^24).
-    __device__ __forceinline__ float after(uint32_t add) const {
-        return add == 0 ? s : __uint_as_float(((uint32_t)(ex + 126) << 23) | ((m + add) & 0x7fffffu));
-    }
+    // The sum after `add` more ulps (m + add < 2^24): the floats of a binade are consecutive integers.
+    __device__ __forceinline__ float after(uint32_t add) const { return add == 0 ? s : __uint_as_float(__float_as_uint(s) + add); }
+    // A sum that no term of this kind changes.
+    __device__ __forceinline__ bool absorbs(double x) const { return s != s || (s > 0.0f && !regular && x >= 0.0); }
     // Rounded ulps of one term; false if the term has to be added by itself.
     __device__ __forceinline__ bool ulps(double x, uint32_t &r) const {
         r = 0;
-        if (!normal) return x == 0.0 && s >= 0.0f;
+        if (!regular) return absorbs(x);
         const double t = __dmul_rn(x, inv_u);
         if (!(t >= 0.0 && t < 0x1p24)) return false;
         const double w = rint(t);
         r = (uint32_t)__double2uint_rn(w);
         return fabs(__dsub_rn(t, w)) < 0.5 - 0x1p-20;  // the difference is exact
     }
+    // Adds one exactly known term's ulps to the sums from an even (even) and from an odd m.
+    __device__ __forceinline__ bool ulps2(double x, uint32_t &even, uint32_t &odd) const {
+        if (!regular) return absorbs(x);
+        const double t = __dmul_rn(x, inv_u);
+        if (!(t >= 0.0 && t < 0x1p24)) return false;
+        const double w = rint(t);
+        const uint32_t r = (uint32_t)__double2uint_rn(w);
+        if (fabs(__dsub_rn(t, w)) == 0.5) {  // to the even one of the two sums around it
+            const uint32_t low = r - (w > t);
+            even += low + ((even + low) & 1u);
+            odd += low + ((odd + low + 1u) & 1u);
+        } else {
+            even += r;
+            odd += r;
+        }
+        return true;
+    }
 };
 
 // Terms of warp_chain lie in its batches' order: four consecutive ones a lane, without bank
 // conflicts.
-constexpr int kChainPer = 4, kChainBatch = 32 * kChainPer, kChainHead = 12;
+constexpr int kChainPer = 4, kChainBatch = 32 * kChainPer, kChainHead = 12, kChainTies = 8;
 __device__ __forceinline__ int chain_slot(int k) {
     return (k & ~(kChainBatch - 1)) + (k & (kChainPer - 1)) * 32 + ((k & (kChainBatch - 1)) / kChainPer);
 }
@@ -74,7 +100,7 @@ __device__ __forceinline__ float warp_chain(const double *x, int n, const Step &
 #pragma unroll
         for (int i = 0; i < kChainPer; i++) v[i] = b + lane * kChainPer + i < n ? x[b + i * 32 + lane] : 0.0;
         int done = b == 0 ? head : 0;  // terms of the batch already added
-        while (true) {
+        for (int steps = 0;; steps++) {
             const ChainSum c(s);
             uint32_t r[kChainPer], sum = 0;
             bool ok[kChainPer];
@@ -98,7 +124,7 @@ __device__ __forceinline__ float warp_chain(const double *x, int n, const Step &
 #pragma unroll
             for (int i = 0; i < kChainPer; i++) {
                 if (at != kChainPer) continue;
-                if (!ok[i] || (c.normal && c.m + acc + r[i] >= (1u << 24))) at = i;
+                if (!ok[i] || (c.regular && c.m + acc + r[i] >= (1u << 24))) at = i;
                 else acc += r[i];
             }
             const unsigned bad = __ballot_sync(0xffffffffu, at != kChainPer);
@@ -108,23 +134,59 @@ __device__ __forceinline__ float warp_chain(const double *x, int n, const Step &
             const int k = f * kChainPer + __shfl_sync(0xffffffffu, at, f);
             s = step(s, b + k);  // the same on every lane
             done = k + 1;
-            if (b + done >= n) break;
+            if (steps == kChainTies)
+                for (; done < kChainBatch && b + done < n; done++) s = step(s, b + done);
+            if (done == kChainBatch || b + done >= n) break;
         }
     }
     return s;
 }
 
+// Increments of m over some terms, from an even and from an odd m.
+struct ChainInc {
+    uint32_t even, odd;
+    __device__ __forceinline__ uint32_t from(uint32_t m) const { return m & 1u ? odd : even; }
+    // These terms, then those of b. Sums above 2^24 need not be right, only above 2^24.
+    __device__ __forceinline__ ChainInc then(const ChainInc &b) const {
+        return ChainInc{even + b.from(even), odd + b.from(odd + 1u)};
+    }
+};
+
 // Scratch of block_chain, in shared memory.
 struct ChainShared {
-    uint32_t total[2][32], first[2][32];
+    ChainInc total[2][32];
+    uint32_t first[2][32];
     float s;
 };
 
-// A CTA of 1024 threads: as warp_chain, with a batch of 1024 kPer terms (load(k0, x) fetches the
-// terms from k0 on, zero past the end). Two barriers a batch, three where a thread steps by itself.
+template <bool kTies>
+struct ChainTies {
+    static constexpr bool value = kTies;
+};
+
+// Inclusive scan over the warp; without ties the two increments are one.
+template <bool kTies>
+__device__ __forceinline__ ChainInc chain_scan(ChainInc v) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t e = __shfl_up_sync(0xffffffffu, v.even, o);
+        if (kTies) {
+            const uint32_t d = __shfl_up_sync(0xffffffffu, v.odd, o);
+            if (lane >= o) v = ChainInc{e, d}.then(v);
+        } else if (lane >= o) {
+            v.even += e;
+        }
+    }
+    return v;
+}
+
+// A CTA of 1024 threads: as warp_chain, with a batch of 1024 kPer terms, squares of x (load(k0, x) fetches
+// the values from k0 on, zero past the end; step is exact but for one rounding). Two barriers a pass,
+// three where a thread steps by itself. A batch's first pass stops at a tie, the others take ties as well.
 template <int kPer, class Load, class Step>
 __device__ float block_chain(ChainShared &sh, float s, uint64_t n, const Load &load, const Step &step) {
-    constexpr uint32_t kT = 1024;
+    constexpr uint32_t kT = 1024, kFull = 1u << 24;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     uint32_t parity = 0;
     float next[kPer];
@@ -136,36 +198,37 @@ __device__ float block_chain(ChainShared &sh, float s, uint64_t n, const Load &l
         for (int i = 0; i < kPer; i++) x[i] = next[i];
         load(k0 + (uint64_t)kT * kPer, next);  // in flight over this batch
         uint32_t from = 0;
-        while (true) {
+        auto pass = [&](auto kTies) {  // true: the batch is done
+            constexpr bool kWithTies = decltype(kTies)::value;
             const ChainSum c(s);
-            uint32_t ulps = 0;
+            ChainInc mine{0, 0};
             bool ok = true;
             if (tid >= from) {
 #pragma unroll
                 for (int i = 0; i < kPer; i++) {
-                    uint32_t r;
-                    ok = c.ulps(__dmul_rn((double)x[i], (double)x[i]), r) && ok;
-                    ulps += r;
+                    const double t = __dmul_rn((double)x[i], (double)x[i]);
+                    if (kWithTies) {
+                        ok = c.ulps2(t, mine.even, mine.odd) && ok;
+                    } else {
+                        uint32_t r;
+                        ok = c.ulps(t, r) && ok;
+                        mine.even += r;
+                    }
                 }
             }
-            ulps = min(ulps, 1u << 24);
-            uint32_t incl = ulps;
-#pragma unroll
-            for (uint32_t o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (lane == 31) sh.total[parity][w] = min(incl, 1u << 24);
+            auto cap = [&](ChainInc v) { return ChainInc{min(v.even, kFull), min(v.odd, kFull)}; };
+            const ChainInc incl = chain_scan<kWithTies>(cap(mine));
+            if (lane == 31) sh.total[parity][w] = cap(incl);
             __syncthreads();
-            uint32_t wt = sh.total[parity][lane];  // running totals of the warps (32 of them)
-#pragma unroll
-            for (uint32_t o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, wt, o);
-                if (lane >= o) wt += y;
-            }
-            const uint32_t all = __shfl_sync(0xffffffffu, wt, 31);
-            const uint32_t before = w ? __shfl_sync(0xffffffffu, wt, w - 1) : 0u;
-            ok = ok && (!c.normal || c.m + before + incl < (1u << 24));
+            const ChainInc wt = chain_scan<kWithTies>(sh.total[parity][lane]);  // of the warps (32 of them)
+            // The sum before this thread's warp, before this thread and after it, and after all.
+            const uint32_t run = kWithTies ? wt.from(c.m) : wt.even;
+            const uint32_t all = __shfl_sync(0xffffffffu, run, 31), warps = __shfl_sync(0xffffffffu, run, (int)w - 1);
+            const uint32_t before_warp = w ? warps : 0u;
+            const uint32_t in_warp = kWithTies ? incl.from(c.m + before_warp) : incl.even;
+            const uint32_t lanes = __shfl_up_sync(0xffffffffu, in_warp, 1);
+            const uint32_t before = before_warp + (lane ? lanes : 0u);
+            ok = ok && (!c.regular || c.m + before_warp + in_warp < kFull);
             const unsigned bad = __ballot_sync(0xffffffffu, !ok);
             if (lane == 0) sh.first[parity][w] = bad ? w * 32 + (uint32_t)__ffs(bad) - 1 : kT;
             __syncthreads();
@@ -173,10 +236,10 @@ __device__ float block_chain(ChainShared &sh, float s, uint64_t n, const Load &l
             parity ^= 1;
             if (f == kT) {
                 s = c.after(all);
-                break;
+                return true;
             }
             if (tid == f) {
-                float v = c.after(before + incl - ulps);
+                float v = c.after(before);
 #pragma unroll
                 for (int i = 0; i < kPer; i++)
                     if (k0 + i < n) v = step(v, x[i]);
@@ -185,8 +248,10 @@ __device__ float block_chain(ChainShared &sh, float s, uint64_t n, const Load &l
             __syncthreads();
             s = sh.s;
             from = f + 1;
-            if (from == kT) break;
-        }
+            return from == kT;
+        };
+        if (pass(ChainTies<false>())) continue;
+        while (!pass(ChainTies<true>())) {}
     }
     return s;
 }

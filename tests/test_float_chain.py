@@ -32,7 +32,7 @@ def _terms(kind, n, rng):
         d[n // 2] = np.inf
     elif kind == "ties":  # odd squares, which tie from a sum of 2^24 on
         d = rng.integers(0, 2, n) * 2 + 1.0
-        d[: min(n, 40)] = 1001
+        d[:17] = 1001
     elif kind == "zeros":
         d[:] = 0
     elif kind != "plain":
@@ -56,3 +56,16 @@ def test_warp(chain, kind, n):
     got = chain.warp_weighted(d.ctypes, cnt.ctypes, n, C.byref(last), C.byref(steps))
     assert last.value < n
     assert _same(got, chain.serial_weighted(d.ctypes, cnt.ctypes, n))
+    # The first twelve terms, one for each binade that the rest of the sum crosses, and ties.
+    assert kind == "ties" or steps.value <= 12 + 48
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n", [1, 8, 1023, 8191, 8192, 8193, 20000])
+def test_block(chain, kind, n):
+    d = _terms(kind, n, np.random.default_rng(n))
+    barriers = C.c_int(0)
+    got = chain.block_square(d.ctypes, n, C.byref(barriers))
+    assert _same(got, chain.serial_square(d.ctypes, n))
+    # Three barriers a pass at most: two passes a batch, and one for each binade that the sum crosses.
+    assert barriers.value <= 3 * (2 * (n // 8192 + 1) + 64)
