@@ -218,26 +218,50 @@ __device__ __forceinline__ void team_clear(TeamShared &sh) {
 // A group is 3 to 1600 samples in the plans met in use: a CTA of 256 threads spent its time at the
 // barriers between its passes, ten groups one after another, and on float atomics in shared memory,
 // which are compare-and-swap loops (256^3 field, 12k groups, 38 MB of samples: 100 us forward, 122
-// backward). A warp per group needs no barrier and has 40 groups an SM under way; the histogram is
-// in fixed point, whose atomics are single instructions, with the scale that n samples of weight 1
-// just fit 32 bits in (at least 2^20, finer than a float's ulp once a bin holds 16 samples), so its
-// sums are exact in any order: 29 us forward, 43 backward, the same without the atomics or the double
-// sums, so what is left is the latency of a group's chain of loads; sixteen in flight a lane and five
-// CTAs an SM were the best of 8 and 16 loads, 4 to 8 CTAs (37 and 55 us with eight loads). Above
-// kWarpMost samples a group is a CTA's.
+// backward). A warp per group needs no barrier and has 40 groups an SM under way; the histogram is in
+// whole numbers, whose atomics are single instructions and whose sums are exact in any order: 35 us
+// forward, 51 backward. It is the latency of a group's chain of loads (of 8 and 16 loads in flight a lane and
+// 4 to 8 CTAs an SM, sixteen and five were the best). Above kWarpMost samples a group is a CTA's.
+//
+// The weights are those that a float has, and more. A bin has two words: how many samples begin in it
+// and the sum of their fractions f, of which a sample weighs 1 - f in its bin and f in the next. f is
+// taken in steps of 2^-T: the sum's leading bits are in one word, its last ones below the count in the
+// other, so that 4095 samples leave T = 28, and 2047 and fewer 31. A coordinate of 1/32 and more, or a
+// negative one (rounded when it moves up to its bin), is a whole number of such steps already; what
+// the ones between 0 and 1/32 have below a step is summed beside them. (One word a bin, of steps of 2^-20 in
+// the largest groups, took 31 and 47 us, and where samples weigh a millionth of a bin, the gradient was off by
+// 200 times what a float's rounding explains.)
 constexpr uint32_t kWarpMost = 4095;
 constexpr int kProxyThreads = 256;
 constexpr int kInFlight = 8;  // samples a lane loads ahead (two words each)
 
+// The words of a bin for groups of n samples.
+struct FracWords {
+    int frac, low;  // bits of the fractions' leading part, below the counts too, and of their last part
+    __device__ __forceinline__ explicit FracWords(uint32_t n) {
+        frac = __clz(n);
+        low = min(2 * frac - 32, 31 - frac);
+    }
+    // n < 2^(32 - frac): the counts fit above 2^frac, n last parts (at most 2^low) below it, and n
+    // leading parts (at most 2^frac) a word.
+    __device__ __forceinline__ float one() const { return __uint_as_float((uint32_t)(127 + frac + low) << 23); }
+    __device__ __forceinline__ long long sum(uint32_t count, uint32_t lead) const {  // of the fractions, in steps
+        return ((long long)lead << low) + (count & ((1u << frac) - 1));
+    }
+    __device__ __forceinline__ long long samples(uint32_t count) const { return (long long)(count >> frac) << (frac + low); }
+};
+
 template <bool kGrad>
-__device__ double warp_proxy(uint32_t *hist, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
+__device__ double warp_proxy(uint32_t *counts, uint32_t *leads, const float *__restrict__ A, const float *__restrict__ B, uint32_t n,
                              const Meta &mt, float t, float R2) {
     const int lane = threadIdx.x & 31;
     const float inv2eb = 0.5f / mt.eb;
-    const int frac = __clz(n);  // n < 2^(32 - frac): n 2^frac fits 32 bits
-    const float one = __uint_as_float((uint32_t)(127 + frac) << 23);
-    const uint32_t unit = 1u << frac;
+    const FracWords F(n);
+    const float one = F.one();
+    const uint32_t low_mask = (1u << F.low) - 1;
+    const uint32_t unit = 1u << F.frac;
     double m = 0.0, ra = 0.0, H = 0.0;
+    float below = 0.0f;
     int klo = kBins, khi = -1;
     for (uint32_t s0 = lane; s0 < n; s0 += 32 * kInFlight) {
         float a[kInFlight], b[kInFlight];
@@ -256,8 +280,9 @@ __device__ double warp_proxy(uint32_t *hist, const float *__restrict__ A, const 
             bool cl;
             bin_of(r, inv2eb, f, k0, cl);
             const uint32_t w = __float2uint_rn(f * one);
-            atomicAdd(&hist[k0], unit - w);
-            atomicAdd(&hist[k0 + 1], w);
+            if (k0 == kHalfBins && f < 0x1p-5f) below += f * one - (float)w;
+            atomicAdd(&counts[k0], unit + (w & low_mask));
+            atomicAdd(&leads[k0], w >> F.low);
             klo = min(klo, k0);
             khi = max(khi, k0 + 1);
             m = fma((double)r, (double)r, m);
@@ -266,14 +291,31 @@ __device__ double warp_proxy(uint32_t *hist, const float *__restrict__ A, const 
     }
     klo = __reduce_min_sync(0xffffffffu, klo);
     khi = __reduce_max_sync(0xffffffffu, khi);
+    if (__any_sync(0xffffffffu, below != 0.0f))
+        for (int o = 16; o; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
     __syncwarp();
-    const float inv_n = 1.0f / ((float)n * one);
-    for (int i = klo + lane; i <= khi; i += 32) {
-        const float p = (float)hist[i] * inv_n;
-        const float l2 = log2f(p + kEps);
-        H -= (double)p * (double)l2;
-        // h'(p) takes the bin's place until the gradient's pass
-        hist[i] = kGrad ? __float_as_uint(-(l2 + p / (p + kEps) * kInvLn2)) : 0u;
+    const float inv = 1.0f / ((float)n * one);
+    // From the last bins on, as a bin takes the fractions of the one before.
+    for (int i0 = klo + (khi - klo) / 32 * 32; i0 >= klo; i0 -= 32) {
+        const int i = i0 + lane;
+        float w = 0.0f;
+        if (i <= khi) {
+            const uint32_t c = counts[i];
+            long long v = F.samples(c) - F.sum(c, leads[i]);
+            if (i > klo) v += F.sum(counts[i - 1], leads[i - 1]);
+            w = __ll2float_rn(v);
+            if (i == kHalfBins) w -= below;
+            if (i == kHalfBins + 1) w += below;
+        }
+        __syncwarp();
+        if (i <= khi) {
+            const float p = w * inv;
+            const float l2 = log2f(p + kEps);
+            H -= (double)p * (double)l2;
+            // h'(p) takes the count's place until the gradient's pass
+            counts[i] = kGrad ? __float_as_uint(-(l2 + p / (p + kEps) * kInvLn2)) : 0u;
+            leads[i] = 0u;
+        }
     }
     for (int o = 16; o; o >>= 1) {
         m += __shfl_xor_sync(0xffffffffu, m, o);
@@ -300,12 +342,12 @@ __device__ double warp_proxy(uint32_t *hist, const float *__restrict__ A, const 
             bool cl;
             bin_of(fmaf(a[i], t, b[i]), inv2eb, f, k0, cl);
             if (!cl)
-                gh = fma((double)(__uint_as_float(hist[k0 + 1]) - __uint_as_float(hist[k0])), (double)(a[i] * inv2eb), gh);
+                gh = fma((double)(__uint_as_float(counts[k0 + 1]) - __uint_as_float(counts[k0])), (double)(a[i] * inv2eb), gh);
         }
     }
     for (int o = 16; o; o >>= 1) gh += __shfl_xor_sync(0xffffffffu, gh, o);
     __syncwarp();
-    for (int i = klo + lane; i <= khi; i += 32) hist[i] = 0u;
+    for (int i = klo + lane; i <= khi; i += 32) counts[i] = 0u;
     __syncwarp();
     return gradient(S, gh, n, mt);
 }
@@ -317,18 +359,18 @@ __global__ void __launch_bounds__(kProxyThreads, 5)
                  uint64_t groups, float *__restrict__ out) {
     constexpr uint32_t kWarps = kProxyThreads / 32;
     __shared__ union Both {
-        uint32_t warp[kWarps][kBins];
+        uint32_t warp[kWarps][2][kBins];
         PassShared team;
         __device__ Both() {}
     } sh;
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = lane; i < kBins; i += 32) sh.warp[w][i] = 0u;
+    for (int i = lane; i < 2 * kBins; i += 32) sh.warp[w][0][i] = 0u;
     __syncwarp();
     for (uint64_t g = blockIdx.x * (uint64_t)kWarps + w; g < groups; g += (uint64_t)gridDim.x * kWarps) {
         const uint32_t o = off[g], n = off[g + 1] - o;
         if (n > kWarpMost) continue;
         double v = 0.0;
-        if (n) v = warp_proxy<kGrad>(sh.warp[w], A + o, B + o, n, load_meta(meta, g), t[g], R2);
+        if (n) v = warp_proxy<kGrad>(sh.warp[w][0], sh.warp[w][1], A + o, B + o, n, load_meta(meta, g), t[g], R2);
         if (lane == 0) out[g] = n == 0 ? 0.0f : kGrad ? (float)(v * (double)gJ[g]) : (float)v;
     }
     bool cleared = false;
