@@ -3673,12 +3673,17 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     rc = host_words(ctx, hw);
     if (rc) return rc;
     const volatile uint32_t *words = hw->dec;  // dec_err, dec_changed, err
-    auto t_core = clk::now();
+    struct Marks {  // between the decoding and the reconstruction, and behind it
+        asz_ctx *c;
+        cudaEvent_t decoded = prof_event(c), rebuilt = prof_event(c);
+        ~Marks() {
+            for (cudaEvent_t e : {decoded, rebuilt}) c->event_pool.push_back(e);
+        }
+    } marks{ctx};
     for (int attempt = 0;; attempt++) {
         rc = decode_values(ctx, run, dm, st);
         if (rc) return rc;
-        if (attempt == 0) R.huffman_s = secs(t_h, clk::now());
-        t_core = clk::now();
+        CK(cudaEventRecord(marks.decoded, st));
         HostScope hs_rec(ctx, "host:reconstruct");
         CK(cudaMemsetAsync(&dm->err, 0, 4, st));
         {
@@ -3701,6 +3706,7 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
                                        ctx->qb.as<int32_t>() + qoff[l + 1], d_out, &dm->err, st));
             l++;
         }
+        CK(cudaEventRecord(marks.rebuilt, st));
         CK(cudaMemcpyAsync(hw->dec, &dm->dec_err, 12, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (!words[1]) break;
@@ -3715,7 +3721,10 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     if (decw & 32u) return fail(ctx, ASZ_E_DATA, "Huffman payload contains too few values");
     if (decw & 64u) return fail(ctx, ASZ_E_DATA, "Huffman payload contains too many values");
     if (errw) return fail(ctx, ASZ_E_DEVICE, "reconstruction kernels reported an internal error");
-    R.core_s = secs(t_core, clk::now());
+    float core_ms = 0;
+    CK(cudaEventElapsedTime(&core_ms, marks.decoded, marks.rebuilt));
+    R.core_s = core_ms / 1000.0;
+    R.huffman_s = secs(t_h, clk::now()) - R.core_s;
     if (!out_on_device) {
         auto t1 = clk::now();
         rc = copy_out(ctx, out, d_out, N * sizeof(float), st);

@@ -79,10 +79,14 @@ typedef struct asz_report {
     double default_slope_s;   /* "Get default slope time" */
     double plan_s;            /* "Generate config time" (auto plans) */
     double family_s;          /* "Predictor family selection time" */
-    double core_s;            /* "Core compression time" without zstd (GPU rounds + Huffman) */
-    double huffman_s;         /* "Huffman compression time" / "Huffman decompression time" */
-    double zstd_s;            /* "Zstd compression time" / "Zstd decompression time" */
-    double h2d_s, d2h_s;      /* host<->device copies inside the call */
+    double core_s;            /* "Core compression time" without zstd (GPU rounds + Huffman); of a decompression
+                               * "Prediction reconstruction time": the reconstruction on the device */
+    double huffman_s;         /* "Huffman compression time" / "Huffman decompression time": the streams' headers and
+                               * trees on the host, what is left of the copy to the device, and the decoding there */
+    double zstd_s;            /* "Zstd compression time" / "Zstd decompression time"; a large stream (4 MB unpacked)
+                               * is on its way to the device meanwhile */
+    double h2d_s, d2h_s;      /* host<->device copies inside the call; of a decompression's stream, what is left to
+                               * wait for when it is unpacked and its headers are read */
     double total_s;           /* wall time of the whole call */
     float min_val, max_val, abs_eb, default_slope;
     float max_err, psnr, cr, br;
