@@ -301,19 +301,21 @@ struct HostScope {
 
 struct ProfScope {
     asz_ctx *c;
+    cudaStream_t st;
     cudaEvent_t a = nullptr, b = nullptr;
     size_t slot = 0;
-    ProfScope(asz_ctx *ctx, const char *name, uint64_t bytes) : c(ctx) {
+    ProfScope(asz_ctx *ctx, const char *name, uint64_t bytes) : ProfScope(ctx, name, bytes, ctx->stream) {}
+    ProfScope(asz_ctx *ctx, const char *name, uint64_t bytes, cudaStream_t s) : c(ctx), st(s) {
         if (!c->prof) return;
         slot = prof_slot(c, name);
         c->prof_slots[slot].bytes += bytes;
         a = prof_event(c);
         b = prof_event(c);
-        cudaEventRecord(a, c->stream);
+        cudaEventRecord(a, st);
     }
     ~ProfScope() {
         if (!a) return;
-        cudaEventRecord(b, c->stream);
+        cudaEventRecord(b, st);
         c->pending.push_back({a, b, slot});
     }
 };
@@ -1556,7 +1558,11 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
             total += (own + kPlanAlign - 1) / kPlanAlign * kPlanAlign;
         }
         std::vector<u64> num(nc);
-        for (uint32_t c = 0; c < nc; c++) num[c] = pc[c].cnt[0] * pc[c].cnt[1] * pc[c].cnt[2];
+        u64 samples = 0;
+        for (uint32_t c = 0; c < nc; c++) {
+            num[c] = pc[c].cnt[0] * pc[c].cnt[1] * pc[c].cnt[2];
+            samples += num[c];
+        }
         CK(ctx->plan_qb.reserve(std::max<u64>(total, 1) * 4));
         CK(ctx->plan_e.reserve(std::max<u64>(total, 1) * 4));
         // Upload: the candidates and their ranges' start values. Counted on the device: ranges and
@@ -1577,7 +1583,7 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         const PlanCand *d_pc = (const PlanCand *)aux;
         int32_t *d_qb = ctx->plan_qb.as<int32_t>();
         {
-            ProfScope ps_(ctx, "plan_sample", total * 8);
+            ProfScope ps_(ctx, "plan_sample", samples * 8);
             CK(launch_plan_sample(d_in, dims[1], dims[2], d_pc, nc, most, d_qb, ctx->plan_e.as<float>(), (int32_t *)(aux + at_range),
                                   (unsigned long long *)(aux + at_win), st));
         }
@@ -1589,7 +1595,10 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         }
         CK(cudaEventRecord(ctx->round_ev[0], st));
         CK(cudaStreamWaitEvent(ctx->side, ctx->round_ev[0], 0));
-        CK(launch_plan_mse(d_pc, nc, ctx->plan_e.as<float>(), (float *)(aux + at_mse), ctx->side));
+        {
+            ProfScope ps_(ctx, "plan_mse", samples * 4, ctx->side);
+            CK(launch_plan_mse(d_pc, nc, ctx->plan_e.as<float>(), (float *)(aux + at_mse), ctx->side));
+        }
         CK(cudaMemcpyAsync(haux + at_mse, aux + at_mse, nc * 4, cudaMemcpyDeviceToHost, ctx->side));
         CK(cudaEventRecord(ctx->round_ev[1], ctx->side));
         struct SideDone {  // no return leaves the side stream at work on these buffers
@@ -1660,11 +1669,14 @@ int plan_search(asz_ctx *ctx, const float *d_in, const uint64_t dims[3], const a
         CK(cudaMemsetAsync(ctx->plan_pay.p, 0, std::max<u64>(words, 1) * 4, st));
         {
             EncodeSet set;
+            u64 encoded = 0;
             for (uint32_t c = 0; c < nc; c++)
-                if (num[c] && codes[c].maxval != 1)
+                if (num[c] && codes[c].maxval != 1) {
                     set.add(0, EncStream{d_qb + pc[c].off, num[c], sym_lo[c], ctx->codes.as<CodeEntry>() + code_off[c],
                                          ctx->plan_pay.as<uint32_t>() + word_off[c]});
-            ProfScope ps_(ctx, "plan_encode", total * 4);
+                    encoded += num[c];
+                }
+            ProfScope ps_(ctx, "plan_encode", encoded * 4);
             if ((rc = launch_encode_set(ctx, set, st))) return rc;
         }
         CK(ctx->plan_words.reserve(std::max<u64>(words, 1) * 4));
@@ -1762,6 +1774,32 @@ struct CoreOut {
     std::vector<PreCode> pre;  // index s: QB stream s (0: pivots, 1..L: rounds)
     std::vector<int32_t> range;  // [min, max] per QB stream
 };
+
+// A round's blocks per class (first, middle, last along each axis), for the selection's algorithmic
+// bytes (one read of the 5 operands, 4 neighbours + original, per sample) and the group size of the
+// most populous class, which picks the kernel's CTA width.
+u64 round_sample_bytes(const Geometry &G, u64 l, uint32_t &common_samples) {
+    u64 per_axis[3][3];
+    for (int a = 0; a < 3; a++) {
+        const u64 nb = G.fg.block_num[a];
+        per_axis[a][0] = 1;
+        per_axis[a][1] = nb > 2 ? nb - 2 : 0;
+        per_axis[a][2] = nb >= 2 ? 1 : 0;
+    }
+    u64 bytes = 0, most = 0;
+    common_samples = 0;
+    for (int c = 0; c < 27; c++) {
+        const ClassInfo &ci = G.classes[l][c];
+        if (ci.fallback || !ci.n) continue;
+        const u64 blocks = per_axis[0][c / 9] * per_axis[1][(c / 3) % 3] * per_axis[2][c % 3];
+        bytes += blocks * ci.n * 20;
+        if (blocks > most || (blocks == most && ci.n > common_samples)) {
+            most = blocks;
+            common_samples = ci.n;
+        }
+    }
+    return bytes;
+}
 
 int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
     const float *d_in = a.d_in;
@@ -2105,28 +2143,8 @@ int run_core(asz_ctx *ctx, const CoreArgs &a, CoreOut &o, asz_report &R) {
             uint32_t *d_list = ctx->tlist.as<uint32_t>(), *d_lcount = &dm->rw.list_count[l % 64];
             uint32_t *d_spill = ctx->spill.as<uint32_t>(), *d_scount = &dm->rw.spill_count[l % 64];
             if (tsel_mode == 0) {
-                // Blocks per class (first, middle, last along each axis), for the algorithmic bytes
-                // (one read of the 5 operands, 4 neighbours + original, per sample) and the group
-                // size of the most populous class, which picks the kernel's CTA width.
-                u64 per_axis[3][3];
-                for (int a = 0; a < 3; a++) {
-                    const u64 nb = G.fg.block_num[a];
-                    per_axis[a][0] = 1;
-                    per_axis[a][1] = nb > 2 ? nb - 2 : 0;
-                    per_axis[a][2] = nb >= 2 ? 1 : 0;
-                }
-                u64 sample_bytes = 0, most = 0;
-                uint32_t common_samples = 0;
-                for (int c = 0; c < 27; c++) {
-                    const ClassInfo &ci = G.classes[l][c];
-                    if (ci.fallback || !ci.n) continue;
-                    const u64 blocks = per_axis[0][c / 9] * per_axis[1][(c / 3) % 3] * per_axis[2][c % 3];
-                    sample_bytes += blocks * ci.n * 20;
-                    if (blocks > most || (blocks == most && ci.n > common_samples)) {
-                        most = blocks;
-                        common_samples = ci.n;
-                    }
-                }
+                uint32_t common_samples;
+                const u64 sample_bytes = round_sample_bytes(G, l, common_samples);
                 ProfScope ps(ctx, "tsel_fast", sample_bytes);
                 CK(launch_tsel_fast(G.fg, rg, (uint32_t)l, cls, d_rec, d_in, ctx->log2arena.as<float>(), R2, t_default, d_tval,
                                     d_tint, &dm->rw.fb, d_list, d_lcount, ctx->overrides.as<uint32_t>(), nov, dm->rw.why, st,
@@ -2400,7 +2418,10 @@ int family_by_frames(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std:
             CK(ctx->fam_tab.reserve(L * sizeof(ProbeSpan)));
             CK(ctx->fam_points.reserve(std::max<u64>(points, 1) * sizeof(ProbePoint)));
             CK(cudaMemcpyAsync(ctx->fam_tab.p, spans.data(), L * sizeof(ProbeSpan), cudaMemcpyHostToDevice, st));
-            CK(launch_probe_points(ctx->fam_tab.as<ProbeSpan>(), (uint32_t)L, most, ctx->fam_points.as<ProbePoint>(), st));
+            {
+                ProfScope ps(ctx, "probe_points", points * 2 * sizeof(ProbePoint));
+                CK(launch_probe_points(ctx->fam_tab.as<ProbeSpan>(), (uint32_t)L, most, ctx->fam_points.as<ProbePoint>(), st));
+            }
             CK(cudaMemcpyAsync(held.back().data(), ctx->fam_points.p, points * sizeof(ProbePoint), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
         }
@@ -2571,11 +2592,21 @@ int family_batch(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::arr
     unsigned long long *hand = (unsigned long long *)(dv + d_hand), *spill = (unsigned long long *)(dv + d_spill),
                        *spill2 = (unsigned long long *)(dv + d_spill2);
     const float t_default = 4.0f / 16, *log2 = ctx->log2arena.as<float>();
-    CK(launch_pivot_compress_batch(F, (const u64 *)(dt + t_poff), nf, pivots, st));
+    {
+        ProfScope ps(ctx, "pivot_compress", pivots * 12);
+        CK(launch_pivot_compress_batch(F, (const u64 *)(dt + t_poff), nf, pivots, st));
+    }
     for (u64 l = 0; l < L; l++) {
         uint32_t *q = (uint32_t *)(dv + d_queue) + 5 * l;
+        u64 sample_bytes = 0, round_targets = 0;
+        if (ctx->prof)
+            for (const Geometry &g : G) {
+                uint32_t common;
+                sample_bytes += round_sample_bytes(g, l, common);
+                round_targets += g.rounds[l].targets;
+            }
         {
-            ProfScope ps(ctx, "tsel_fast", 0);
+            ProfScope ps(ctx, "tsel_fast", sample_bytes);
             CK(launch_tsel_fast_batch(F, goff, nf, (uint32_t)l, log2, t_default, q, hand, q + 2,
                                       (uint32_t)std::min<u64>(blocks, 148 * 16), st));
         }
@@ -2583,13 +2614,18 @@ int family_batch(asz_ctx *ctx, const FamilyProbe &pr, const std::vector<std::arr
             ProfScope ps(ctx, "tsel_exact", 0);
             CK(launch_tsel_exact_batch(F, (uint32_t)l, log2, t_default, hand, q + 2, spill, q + 3, exact_cap(), cap_round[l], 148, st));
         }
-        if (ggrid)
+        if (ggrid) {
+            ProfScope ps(ctx, "tsel_exact_global", 0);
             CK(launch_tsel_exact_global_batch(F, (uint32_t)l, log2, t_default, spill, q + 3, spill2, q + 4,
                                               ctx->gscratch.as<uint8_t>(), gstride, capmax, ggrid, st));
-        ProfScope ps(ctx, "round_compress", 0);
+        }
+        ProfScope ps(ctx, "round_compress", round_targets * 12);
         CK(launch_round_compress_batch(F, ioff + l * (nf + 1), nf, (uint32_t)l, q + 1, 148 * 5, true, st));
     }
-    CK(launch_probe_points((const ProbeSpan *)(dt + t_spans), (uint32_t)(nf * L), most, ctx->fam_points.as<ProbePoint>(), st));
+    {
+        ProfScope ps(ctx, "probe_points", points * 2 * sizeof(ProbePoint));
+        CK(launch_probe_points((const ProbeSpan *)(dt + t_spans), (uint32_t)(nf * L), most, ctx->fam_points.as<ProbePoint>(), st));
+    }
     CK(cudaMemcpyAsync(ctx->fam_host.p, ctx->fam_points.p, points * sizeof(ProbePoint), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(ht, dv + d_cnt, mem - d_cnt, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

@@ -40,3 +40,23 @@ def test_decompression_times(gpu_ctx):
     for r in reps:
         assert r.huffman_s > writing + prof["huff_decode_sync"].ms / 1e3
         assert r.zstd_s + r.h2d_s + r.core_s < r.total_s and r.huffman_s + r.core_s < r.total_s
+
+
+def test_profile_has_every_kernel(gpu_ctx):
+    """The plan search and the family probes (their bytes: what a kernel reads and writes at least)."""
+    import asz_b200.api as api
+    from asz_b200 import fields
+    f = fields.grf_field((60, 150, 170), 3.0, np.random.default_rng(4)).astype(np.float32)
+    p = api.default_params(block_pivot_ratio=3)
+    plan = "cubic0_012,cubic1_120,cubic2_021"
+    run = {fam: _profiled(gpu_ctx, lambda: gpu_ctx.compress(f, 1e-3, plan, fam, p)) for fam in ("cubic", "auto")}
+    # The probes' kernels are the rounds' own, with their bytes, and the gather of their targets.
+    for k in ("pivot_compress", "tsel_fast", "round_compress"):
+        assert run["auto"][k].launches > run["cubic"][k].launches, k
+        assert run["auto"][k].bytes > run["cubic"][k].bytes, k
+    assert run["auto"]["probe_points"].launches > 0 and run["auto"]["probe_points"].ms > 0
+    got = _profiled(gpu_ctx, lambda: gpu_ctx.compress(f, 1e-3, None, "cubic", p))
+    layers = got["plan_sample"].launches
+    assert layers > 3 and got["plan_mse"].launches == layers and got["plan_mse"].ms > 0
+    # A QB and an error written of each sample, and the error read again.
+    assert got["plan_sample"].bytes == 2 * got["plan_mse"].bytes
