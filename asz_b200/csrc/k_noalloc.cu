@@ -66,8 +66,13 @@ __device__ Partial block_reduce(float mx, double s, Partial *sh) {
 // a tile is 8192 elements, so that a field of 16.8 M values is 2048 CTAs, more than the chip holds at
 // once. Tiles of 65536 with single 4-byte loads, 256 CTAs of the same field, took 78 us of kernel
 // for its 134 MB; this form takes 28. Larger fields, up to the scratch's limit, take larger tiles
-// (the number of partials is what the scratch bounds). Arrays that are not 16-byte aligned go
-// through 4-byte loads.
+// (the number of partials is what the scratch bounds). An array off a 16-byte boundary is read by 4-byte
+// loads, in the same order: where an array lies changes no bit of the result.
+__device__ __forceinline__ float4 load4(const float *p, bool aligned) {
+    if (aligned) return __ldcs(reinterpret_cast<const float4 *>(p));
+    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
 __device__ __forceinline__ void take(float a, float b, float &mx, double &s) {
     mx = fmaxf(mx, fabsf(__fsub_rn(a, b)));
     const double d = (double)a - (double)b;
@@ -75,8 +80,8 @@ __device__ __forceinline__ void take(float a, float b, float &mx, double &s) {
 }
 
 __global__ void __launch_bounds__(kThreads)
-    stats_noalloc_kernel(const float *__restrict__ x, const float *__restrict__ y, uint64_t n, uint64_t tile, bool aligned,
-                         unsigned char *scratch) {
+    stats_noalloc_kernel(const float *__restrict__ x, const float *__restrict__ y, uint64_t n, uint64_t tile, bool x_aligned,
+                         bool y_aligned, unsigned char *scratch) {
     __shared__ Partial sh[kThreads / 32];
     __shared__ bool last;
     Control *ctl = (Control *)scratch;
@@ -86,21 +91,19 @@ __global__ void __launch_bounds__(kThreads)
     float mx = 0.0f;
     double s = 0.0;
     uint64_t i = begin;
-    if (aligned) {
-        constexpr int kV = 4;
-        for (; i + kV * 4 * kThreads <= end; i += kV * 4 * kThreads) {
-            const float4 *xv = reinterpret_cast<const float4 *>(x + i) + threadIdx.x,
-                         *yv = reinterpret_cast<const float4 *>(y + i) + threadIdx.x;
-            float4 a[kV], b[kV];
+    constexpr int kV = 4;
+    for (; i + kV * 4 * kThreads <= end; i += kV * 4 * kThreads) {
+        const float *xv = x + i + 4 * threadIdx.x, *yv = y + i + 4 * threadIdx.x;
+        float4 a[kV], b[kV];
 #pragma unroll
-            for (int k = 0; k < kV; k++) a[k] = __ldcs(xv + k * kThreads), b[k] = __ldcs(yv + k * kThreads);
+        for (int k = 0; k < kV; k++)
+            a[k] = load4(xv + 4 * k * kThreads, x_aligned), b[k] = load4(yv + 4 * k * kThreads, y_aligned);
 #pragma unroll
-            for (int k = 0; k < kV; k++) {
-                take(a[k].x, b[k].x, mx, s);
-                take(a[k].y, b[k].y, mx, s);
-                take(a[k].z, b[k].z, mx, s);
-                take(a[k].w, b[k].w, mx, s);
-            }
+        for (int k = 0; k < kV; k++) {
+            take(a[k].x, b[k].x, mx, s);
+            take(a[k].y, b[k].y, mx, s);
+            take(a[k].z, b[k].z, mx, s);
+            take(a[k].w, b[k].w, mx, s);
         }
     }
     for (i += threadIdx.x; i < end; i += kThreads) take(x[i], y[i], mx, s);
@@ -175,8 +178,8 @@ extern "C" int asz_error_stats_noalloc(const float *x, const float *y, uint64_t 
     Control h;
     cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(Control), st);
     if (e == cudaSuccess) {
-        stats_noalloc_kernel<<<(unsigned)tiles, kThreads, 0, st>>>(x, y, n, tile, (((uintptr_t)x | (uintptr_t)y) & 15) == 0,
-                                                                   scratch);
+        stats_noalloc_kernel<<<(unsigned)tiles, kThreads, 0, st>>>(x, y, n, tile, ((uintptr_t)x & 15) == 0,
+                                                                   ((uintptr_t)y & 15) == 0, scratch);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, scratch, sizeof(Control), cudaMemcpyDeviceToHost, st);

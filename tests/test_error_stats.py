@@ -24,3 +24,17 @@ def test_lengths_and_alignment(n, off):
     # n additions of non-negative doubles in any order: relative error below n 2^-53 each way.
     ref = 10 * np.log10(9.0 / np.mean(d * d))
     assert abs(p - ref) <= 10 / np.log(10) * (2 * n + 8) * 2.0 ** -53 + 4e-15 * abs(ref)
+
+
+@pytest.mark.parametrize("n", [4096, 70000, 1 << 21])
+def test_same_bits_at_any_alignment(n):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    for _ in range(8):
+        x, y = torch.randn(n, generator=g, device="cuda"), torch.randn(n, generator=g, device="cuda")
+        got = []
+        for off in [(0, 0), (1, 1), (0, 3), (2, 0)]:
+            a, b = (torch.empty(n + 4, device="cuda")[o: o + n].copy_(v) for o, v in zip(off, (x, y)))
+            torch.cuda.synchronize()
+            got.append(api.error_stats_noalloc(a, b, 3.0))
+        assert len(set(got)) == 1, got
