@@ -3543,7 +3543,6 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
     CK(ctx->raw_in.reserve(raw + kDecodePad));
     uint8_t *const bsp = ctx->raw_in.p;
     std::memset(bsp + raw, 0, kDecodePad);
-    CK(ctx->pre.reserve(raw + kDecodePad));
     // The pieces on their way to the device are there before a call returns, also one that refuses the
     // stream: the next call uses the same buffers, perhaps on another stream.
     struct SendEnd {
@@ -3559,9 +3558,12 @@ extern "C" int asz_decompress(asz_ctx *ctx, const uint8_t *in, size_t len, const
         // Large streams go to the device piece by piece while the rest is still being unpacked (512^3 at
         // 1e-3, 109 MB: 11.7 ms and the copy's 2.0, now 2.0 together); small ones are unpacked in less time
         // than the threads need to wake.
+        // The device's memory is taken when the first piece is there, so not for a frame that only claims a
+        // size.
         u64 sent = 0;
         cudaError_t sent_err = cudaSuccess;
         auto send = [&](u64 to) {
+            if ((sent_err = ctx->pre.reserve(raw + kDecodePad)) != cudaSuccess) return false;
             if (to > sent) sent_err = cudaMemcpyAsync(ctx->pre.as<uint8_t>() + sent, bsp + sent, to - sent, cudaMemcpyHostToDevice, st);
             sent = to;
             return sent_err == cudaSuccess;

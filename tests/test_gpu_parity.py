@@ -324,6 +324,22 @@ def _zstd3(raw: bytes) -> bytes:
     return buf.raw[:n]
 
 
+def test_refused_stream_takes_no_device_memory(gpu_ctx):
+    """A frame that claims 512 MiB and holds nothing valid is refused before device memory is taken for it."""
+    import torch
+    import asz_b200.api as api
+    size = 512 << 20
+    frame = b"\x28\xb5\x2f\xfd" + bytes([0xE0]) + size.to_bytes(8, "little")  # one segment, 8 bytes of content size
+    with api.Context(0) as ctx:
+        ctx.compress(np.random.default_rng(1).random((20, 20, 20)).astype(np.float32), 1e-3, "cubic2_012", "cubic")
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for rest in (b"\x05\x00\x00" + bytes(40), b"\x07\x00\x00", bytes([0x2C, 0, 0]) + b"\xff" * 5):
+            with pytest.raises(api.AszError, match="ZSTD_decompress error"):
+                ctx.decompress(frame + rest, (20, 20, 20), 1e-3)
+        assert before - torch.cuda.mem_get_info()[0] < size // 2
+
+
 def test_corrupt_payload_bits(gpu_ctx):
     """Bit flips inside the Huffman payloads (re-wrapped in a valid zstd frame): the decoder either
     reports a corrupt stream or decodes some other valid stream, never faults, and the context
