@@ -247,11 +247,9 @@ class Context:
             raise AszError(rc, self._L.asz_last_error(self._c).decode())
 
     def _take(self, out, n: int) -> bytes:
-        """The bytes of a library output, which is released. A large one is copied on the library's worker
-        threads: its pages are fresh, and one thread maps and fills them at a few GB/s."""
+        """The bytes of a library output, which is released. The library copies them, a large one on its
+        worker threads: its pages are fresh, and one thread maps and fills them at a few GB/s."""
         try:
-            if n <= 32 << 20:
-                return C.string_at(out, n)
             blob = _new_bytes(None, n)
             self._L.asz_copy_output(self._c, _bytes_at(blob), out, n)
             return blob

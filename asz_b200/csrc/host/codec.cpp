@@ -959,9 +959,10 @@ void asz_free(void *p) {
 
 void asz_copy_output(asz_ctx *ctx, void *dst, const void *src, size_t n) {
     if (!ctx || !dst || !src) return;
-    // Up to kOwnMapping one thread is the better one: 13 MB take it 0.7 ms against 0.1, but zstd then
-    // writes the next stream into lines that the other cores share, which cost it 1 ms. 110 MB into
-    // fresh pages: 45 ms by one thread, 4 by all.
+    // The line is where malloc maps a block by itself: from there on its pages are fresh, and one thread maps
+    // and fills 32 MB in 15 ms, 64 MB in 30 and 110 MB in 50, all of them in 1.3, 2.2 and 3.9. Below, the heap's
+    // pages are mapped (24 MB: 3.0 against 0.2 ms, 13 MB: 1.9 against 0.1), but after a copy by all threads zstd
+    // writes the next stream into lines that the other cores share, which cost it 1 ms at 13 MB.
     if (n <= kOwnMapping) {
         std::memcpy(dst, src, n);
         return;

@@ -336,10 +336,11 @@ __device__ __forceinline__ uint32_t decode_sym(const uint32_t *slot, uint32_t &p
 }
 
 // ---------------------------------------------------------------------------------------------
-// Batched decoding of every stream of a .asz in one launch per pass. Chunks of chunk_bits bits
-// are numbered globally (stream after stream); tiles of blockDim.x chunks never cross a stream,
-// so a CTA stages one stream's lookup table for a tile. Bit positions are absolute from the
-// 16-byte aligned stream buffer `base`.
+// Batched decoding of every stream of a .asz in one launch per pass. A stream's chunks have
+// DecStream::words words, 8 or 32, and are numbered globally (stream after stream); a tile of them
+// (decode_tile: 192 or 240) never crosses a stream, so a CTA stages one stream's lookup table for a tile.
+// When synchronising, a warp has the next decode_run chunks (24 or 30) and decodes the decode_halo
+// before them as well. Bit positions are absolute from the 16-byte aligned stream buffer `base`.
 
 __device__ __forceinline__ void stage_lut(uint4 *lut_sh, const uint32_t *__restrict__ lut, uint32_t lut_bits) {
     const uint4 *v = reinterpret_cast<const uint4 *>(lut);
@@ -785,8 +786,9 @@ template cudaError_t launch_encode_tiles<int32_t>(const EncStream *, uint32_t, c
 template cudaError_t launch_encode_tiles<int64_t>(const EncStream *, uint32_t, const uint64_t *, uint64_t, uint64_t *, uint64_t *,
                                                   cudaStream_t);
 
-// Persistent decode grid: up to 4 CTAs of 256 threads per SM, each with a tile's payload and a table
-// of up to 16 KB.
+// Persistent decode grid: 4 CTAs of 256 threads per SM, each with a tile's payload and a table of up to
+// 16 KB. With a table of 12 bits the synchronising kernel, which has its marks beside them, takes 58,464
+// bytes a CTA, and three of them an SM: the last 148 CTAs follow the others.
 static unsigned decode_grid(uint64_t ntiles) { return (unsigned)(ntiles < 148 * 4 ? (ntiles ? ntiles : 1) : 148 * 4); }
 static size_t decode_smem(uint32_t max_lut_bits) {
     return kDecodeSlotBytes + std::max<size_t>(((size_t)1 << max_lut_bits) * 4, 16);

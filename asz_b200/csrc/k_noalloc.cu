@@ -65,7 +65,7 @@ __device__ Partial block_reduce(float mx, double s, Partial *sh) {
 // HBM-bound: 8 bytes an element. A thread has eight 16-byte loads in flight (four of each array) and
 // a tile is 8192 elements, so that a field of 16.8 M values is 2048 CTAs, more than the chip holds at
 // once. Tiles of 65536 with single 4-byte loads, 256 CTAs of the same field, took 78 us of kernel
-// for its 134 MB; this form takes 28. Larger fields, up to the scratch's limit, take larger tiles
+// for its 134 MB; this form takes 31 (out of DRAM). Larger fields, up to the scratch's limit, take larger tiles
 // (the number of partials is what the scratch bounds). An array off a 16-byte boundary is read by 4-byte
 // loads, in the same order: where an array lies changes no bit of the result.
 __device__ __forceinline__ float4 load4(const float *p, bool aligned) {
